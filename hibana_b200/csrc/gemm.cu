@@ -407,7 +407,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
   const int tile_a = blockIdx.x;
   int tile_b = blockIdx.y, split = blockIdx.z;
@@ -466,52 +466,61 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t smem_base = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+  const uint32_t full_base = __shfl_sync(0xffffffffu, smem_u32(full), 0);
   prof_mark(p, 0, t_entry);
   // Let the kernel after this one be scheduled now (it waits for this grid's completion before it reads anything
   // this grid writes): its launch latency and prologue overlap this grid's main loop.
   if (p.early_launch) grid_dep_launch();
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      // side 0 = A operand (+ its scales), side 1 = B operand (+ its scales) of K tile i into stage i % S
-      auto load_side = [&](int i, int side) {
-        const int s = i % S;
-        uint8_t* st = smem + s * C::STAGE_BYTES;
-        const int kt = kt0 + i;
-        const int kx = (KIND == kGemmBf16 || KIND == kGemmW3) ? kt * 64 : kt * 128;
-        if (side == 0) {
-          if constexpr (KIND == kGemmW3) {
-            bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES,
-                      p.w3_tiles + (static_cast<size_t>(a_row0 >> 7) * p.k_tiles + kt) * 4096, 4096, &full[s]);
-            return;
-          }
-          tma_load_2d(st, &tma, &full[s], kx, a_row0);
-          if constexpr (KIND == kGemmNvfp4)
-            bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES,
-                      p.sfa + (static_cast<size_t>(a_row0 >> 7) * p.ka_a + kt * 4) * 512, 2048, &full[s]);
-        } else {
-          tma_load_2d(st + A_TILE_BYTES, &tmb, &full[s], kx, b_row0);
-          if constexpr (KIND == kGemmNvfp4) {
-#pragma unroll
-            for (int rb = 0; rb < C::NRB; ++rb)
-              bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES + C::SFA_BYTES + rb * 2048,
-                        p.sfb + (static_cast<size_t>((b_row0 >> 7) + rb) * p.ka_b + kt * 4) * 512, 2048, &full[s]);
-          }
+    // The whole warp walks the loop (waits included) and one elected lane issues (elect_one). Issued by `lane == 0`
+    // instead, every copy, scale-factor copy and MMA first moved its operands to uniform registers: 50 ns each, 0.9 us
+    // per 256-element K tile, which bounded every NVFP4 shape of the framework.
+    const int ua_row0 = __shfl_sync(0xffffffffu, a_row0, 0), ub_row0 = __shfl_sync(0xffffffffu, b_row0, 0);
+    int issued = 0;
+    // side 0 = A operand (+ its scales), side 1 = B operand (+ its scales) of K tile i into stage i % S
+    auto load_side = [&](int i, int side) {
+      const int s = i % S;
+      const uint32_t st = smem_base + s * C::STAGE_BYTES;
+      const uint32_t bar = full_base + s * 8;
+      const int kt = kt0 + i;
+      const int kx = (KIND == kGemmBf16 || KIND == kGemmW3) ? kt * 64 : kt * 128;
+      if (side == 0) {
+        if constexpr (KIND == kGemmW3) {
+          bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES,
+                    p.w3_tiles + (static_cast<size_t>(ua_row0 >> 7) * p.k_tiles + kt) * 4096, 4096, bar);
+          return;
         }
-      };
-      // First ring of stages (their `empty` barriers are trivially free): the weights go first; they depend on
-      // nothing. Then the waits for whoever produces the activations: the preceding grid (programmatic
-      // dependent launch), the source rank of a gathered row tile, or every sender of an expert-parallel
-      // dispatch. Then the activations.
-      const int wside = p.swap ? 0 : 1;
-      const int pre = min(S, nkt);
+        tma_load_2d(st, &tma, bar, kx, ua_row0);
+        if constexpr (KIND == kGemmNvfp4)
+          bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES,
+                    p.sfa + (static_cast<size_t>(ua_row0 >> 7) * p.ka_a + kt * 4) * 512, 2048, bar);
+      } else {
+        tma_load_2d(st + A_TILE_BYTES, &tmb, bar, kx, ub_row0);
+        if constexpr (KIND == kGemmNvfp4) {
+#pragma unroll
+          for (int rb = 0; rb < C::NRB; ++rb)
+            bulk_load(st + A_TILE_BYTES + C::B_TILE_BYTES + C::SFA_BYTES + rb * 2048,
+                      p.sfb + (static_cast<size_t>((ub_row0 >> 7) + rb) * p.ka_b + kt * 4) * 512, 2048, bar);
+        }
+      }
+    };
+    // First ring of stages (their `empty` barriers are trivially free): the weights go first; they depend on
+    // nothing. Then the waits for whoever produces the activations: the preceding grid (programmatic
+    // dependent launch), the source rank of a gathered row tile, or every sender of an expert-parallel
+    // dispatch. Then the activations.
+    const int wside = p.swap ? 0 : 1;
+    const int pre = min(S, nkt);
+    if (elect_one())
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&full[i], C::TX_BYTES);
         load_side(i, wside);
       }
-      grid_dep_wait();
+    __syncwarp();
+    grid_dep_wait();
+    if (lane == 0) {
       bool ready = true;
       if (p.peer_on && p.flag_offset >= 0) {
         // all-gather -> GEMM: the rows of this A tile were pushed into local memory by rank `src`
@@ -550,54 +559,55 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
         *abort = 1;
         set_status(p.status, kTimeoutGate);
       }
-      // On a failed wait the activation side is still loaded (whatever is there): the stages then complete, the
-      // barriers balance and no copy is left in flight; the status word tells the host the result is void.
-      for (int i = 0; i < pre; ++i) {
-        load_side(i, wside ^ 1);
-        ++issued;
-      }
-      for (int i = pre; i < nkt && !*abort; ++i) {
-        const int s = i % S;
-        const uint32_t ph = (i / S) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1, abort, p.status, kTimeoutEmpty)) break;
+      // What the peers stored has been seen by this lane's acquire; the copies are issued by an elected lane of the
+      // same warp (ordered by the barrier below) through the asynchronous proxy.
+      if (p.peer_on || p.ep_gate_flags != nullptr) asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    __syncwarp();
+    // On a failed wait the activation side is still loaded (whatever is there): the stages then complete, the
+    // barriers balance and no copy is left in flight; the status word tells the host the result is void.
+    if (elect_one())
+      for (int i = 0; i < pre; ++i) load_side(i, wside ^ 1);
+    __syncwarp();
+    issued = pre;
+    for (int i = pre; i < nkt && !__any_sync(0xffffffffu, *abort); ++i) {
+      const int s = i % S;
+      const uint32_t ph = (i / S) & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1, abort, p.status, kTimeoutEmpty))) break;
+      if (elect_one()) {
         mbar_expect_tx(&full[s], C::TX_BYTES);
         load_side(i, 0);
         load_side(i, 1);
-        ++issued;
       }
-      if (*abort) {
-        // Wait (bounded) for the copies still in flight so that none lands after the CTA has gone.
-        volatile int ignore = 0;
-        for (int j = max(issued - S, 0); j < issued; ++j)
-          mbar_wait(&full[j % S], (j / S) & 1, &ignore, nullptr, kTimeoutDrain);
-      }
+      __syncwarp();
+      ++issued;
+    }
+    if (*abort && lane == 0) {
+      // Wait (bounded) for the copies still in flight so that none lands after the CTA has gone.
+      volatile int ignore = 0;
+      for (int j = max(issued - S, 0); j < issued; ++j)
+        mbar_wait(&full[j % S], (j / S) & 1, &ignore, nullptr, kTimeoutDrain);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = KIND == kGemmNvfp4 ? make_idesc_nvf4(BM, BN)
-                                 : KIND == kGemmFp8 ? make_idesc_e4m3(BM, BN) : make_idesc_bf16(BM, BN);
-      const uint32_t sfa_t = tmem_base + BN;
-      const uint32_t sfb_t = sfa_t + 16;
-      bool ok = true;
-      for (int i = 0; i < nkt; ++i) {
-        const int s = i % S;
-        const uint32_t ph = (i / S) & 1;
-        if (!mbar_wait(&full[s], ph, abort, p.status, kTimeoutFull)) {
-          ok = false;
-          break;
-        }
-        if constexpr (KIND == kGemmW3) {
-          if (!mbar_wait(&dq[s], ph, abort, p.status, kTimeoutFull)) {
-            ok = false;
-            break;
-          }
-        }
-        tc_fence_after();
-        uint8_t* st = smem + s * C::STAGE_BYTES;
-        const uint64_t adesc = make_desc_sw128(smem_u32(st));
-        const uint64_t bdesc = make_desc_sw128(smem_u32(st + A_TILE_BYTES));
+    constexpr uint32_t idesc = KIND == kGemmNvfp4 ? make_idesc_nvf4(BM, BN)
+                               : KIND == kGemmFp8 ? make_idesc_e4m3(BM, BN) : make_idesc_bf16(BM, BN);
+    const uint32_t sfa_t = tmem_base + BN;
+    const uint32_t sfb_t = sfa_t + 16;
+    bool ok = true;
+    for (int i = 0; i < nkt; ++i) {
+      const int s = i % S;
+      const uint32_t ph = (i / S) & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort, p.status, kTimeoutFull));
+      if constexpr (KIND == kGemmW3)
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&dq[s], ph, abort, p.status, kTimeoutFull));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t st = smem_base + s * C::STAGE_BYTES;
+      const uint64_t adesc = make_desc_sw128(st);
+      const uint64_t bdesc = make_desc_sw128(st + A_TILE_BYTES);
+      if (elect_one()) {
         if constexpr (KIND == kGemmNvfp4) {
-          const uint32_t sf = smem_u32(st + A_TILE_BYTES + C::B_TILE_BYTES);
+          const uint32_t sf = st + A_TILE_BYTES + C::B_TILE_BYTES;
 #pragma unroll
           for (int kb = 0; kb < 4; ++kb) {
             tmem_cp_32x128b_x4(sfa_t + kb * 4, make_desc_sf(sf + kb * 512));
@@ -620,8 +630,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
             mma_f16(tmem_base, adesc + kb * 2, bdesc + kb * 2, idesc, (i > 0 || kb > 0) ? 1u : 0u);
         }
         tc_commit(&empty[s]);
+        if (i == nkt - 1) tc_commit(accum);
       }
-      if (ok) tc_commit(accum);
+      __syncwarp();
     }
   } else {
     const int q = warp & 3;  // TMEM lane quarter this warp may read
@@ -1031,10 +1042,13 @@ bool get_tmap_2d(const TmapKey& key, CUtensorMap* out_map) {
   const cuuint64_t strides[1] = {key.pitch_bytes};
   const cuuint32_t box[2] = {key.box_cols, key.box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUtensorMapDataType dt = key.dtype == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+  const CUtensorMapDataType dt = key.dtype == 0   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                 : key.dtype == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                                                  : CU_TENSOR_MAP_DATA_TYPE_UINT64;
   const CUresult r = fn(m.get(), dt, 2, const_cast<void*>(key.ptr), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        key.dtype == 2 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
   *out_map = *m;
   g_tmaps.emplace(key, std::move(m));
@@ -1083,6 +1097,20 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   while (splits > 1 && (splits - 1) * ((k_tiles + splits - 1) / splits) >= k_tiles) --splits;
   if (splits > 8) splits = 8;   // portable cluster size
 
+  if (a.epilogue == kEpiSiluMulQuant) {
+    // tokens on the N side, whole 128-row feature tiles, no grouped / peer variants; the staging tile of a split-K
+    // CTA sits behind its fp32 partial, which the smallest ring must still hold
+    if (grouped || a.peer != nullptr || a.tok_scale != nullptr || a.q_out == nullptr || a.q_sf == nullptr ||
+        a.q_gscale == nullptr)
+      return cudaErrorInvalidValue;
+    if (a.swap && (a.ra % BM != 0 || a.q_ka * 64 < a.ra / 2 || a.bn > 128)) return cudaErrorInvalidValue;
+    // tokens on the 128-row side: the staged epilogue (output tiles of 128 or 256 columns, no split-K) writes the
+    // packed bytes as aligned 16-byte chunks of two groups: feature count a multiple of 64
+    if (!a.swap && (a.rb % 64 != 0 || a.q_ka * 64 < a.rb / 2 || a.splits != 1 || (a.bn != 128 && a.bn != 256) ||
+                    a.q_ld % 16 != 0 || (reinterpret_cast<uintptr_t>(a.q_out) & 15) != 0))
+      return cudaErrorInvalidValue;
+  }
+
   // byte-typed maps (packed e2m1 or e4m3): inner extent and pitch in bytes, 128-byte boxes
   const bool bytes = fp4 || fp8;
   TmapKey ka{a.a, static_cast<uint64_t>(a.ra), static_cast<uint64_t>(fp4 ? a.k / 2 : a.k),
@@ -1127,19 +1155,6 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   p.q_ka = a.q_ka; p.q_ld = a.q_ld;
   p.prof = g_gemm_prof;
   p.local_reduce = g_local_reduce;
-  if (a.epilogue == kEpiSiluMulQuant) {
-    // tokens on the N side, whole 128-row feature tiles, no grouped / peer variants; the staging tile of a split-K
-    // CTA sits behind its fp32 partial, which the smallest ring must still hold
-    if (grouped || a.peer != nullptr || a.tok_scale != nullptr || a.q_out == nullptr || a.q_sf == nullptr ||
-        a.q_gscale == nullptr)
-      return cudaErrorInvalidValue;
-    if (a.swap && (a.ra % BM != 0 || a.q_ka * 64 < a.ra / 2 || a.bn > 128)) return cudaErrorInvalidValue;
-    // tokens on the 128-row side: the staged epilogue (output tiles of 128 or 256 columns, no split-K) writes the
-    // packed bytes as aligned 16-byte chunks of two groups: feature count a multiple of 64
-    if (!a.swap && (a.rb % 64 != 0 || a.q_ka * 64 < a.rb / 2 || a.splits != 1 || (a.bn != 128 && a.bn != 256) ||
-                    a.q_ld % 16 != 0 || (reinterpret_cast<uintptr_t>(a.q_out) & 15) != 0))
-      return cudaErrorInvalidValue;
-  }
   p.early_launch = g_pdl >= 2;
   p.w3_tiles = w3 ? static_cast<const uint8_t*>(a.a) : nullptr;
   p.ep_gate_flags = nullptr; p.ep_seq_ptr = nullptr; p.ep_row_ret = nullptr; p.ep_done = nullptr;
