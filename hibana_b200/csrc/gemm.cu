@@ -1111,6 +1111,8 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
 
+  if (gemm_pair_ok(a)) return gemm_pair_launch(a, stream);
+
   // byte-typed maps (packed e2m1 or e4m3): inner extent and pitch in bytes, 128-byte boxes
   const bool bytes = fp4 || fp8;
   TmapKey ka{a.a, static_cast<uint64_t>(a.ra), static_cast<uint64_t>(fp4 ? a.k / 2 : a.k),

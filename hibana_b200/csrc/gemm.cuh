@@ -107,17 +107,23 @@ struct GemmArgs {
 // Returns cudaSuccess or the launch error. Tensor maps are built (and cached) inside.
 cudaError_t gemm_launch(const GemmArgs& args, cudaStream_t stream);
 
+// Prefill-sized NVFP4 calls with the tokens on the 128-row side run on SM pairs (gemm_pair.cu); `gemm_pair_ok` says
+// which calls it covers, gemm_launch routes them there.
+bool gemm_pair_ok(const GemmArgs& args);
+cudaError_t gemm_pair_launch(const GemmArgs& args, cudaStream_t stream);
+
 // Bytes of fp32 workspace and number of counters a launch with these arguments needs.
 size_t gemm_workspace_bytes(const GemmArgs& args);
 int gemm_num_tiles(const GemmArgs& args);
 
-// Tensor-map cache (host). 2-D row-major tensor, box = {box_inner elements, box_rows}, 128-byte swizzle.
+// Tensor-map cache (host). 2-D row-major tensor, box = {box_inner elements, box_rows}, 128-byte swizzle
+// (8-byte words: none).
 struct TmapKey {
   const void* ptr;
   uint64_t rows, cols;   // cols = inner extent in elements
   uint64_t pitch_bytes;
   uint32_t box_rows, box_cols;
-  int dtype;             // 0 = bf16, 1 = u8
+  int dtype;             // 0 = bf16, 1 = u8, 2 = u64 (unswizzled)
   bool operator==(const TmapKey& o) const {
     return ptr == o.ptr && rows == o.rows && cols == o.cols && pitch_bytes == o.pitch_bytes &&
            box_rows == o.box_rows && box_cols == o.box_cols && dtype == o.dtype;

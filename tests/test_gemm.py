@@ -223,3 +223,35 @@ def test_silu_mul_requant_epilogue_matches_two_kernels(m, n, k):
     # a second call reuses the persistent buffers and must give the same bytes (captured graphs replay it)
     again = gemm.linear_nvfp4_silu_quant(xq, wq, alpha, out_scale)
     assert torch.equal(again.q, two.q)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(257, 256, 288), (300, 5120, 512), (511, 264, 256), (513, 336, 1312), (700, 18560, 256),
+                                   (1025, 4096, 1088), (2048, 5120, 704), (4100, 2048, 320)])
+@pytest.mark.parametrize("epi", [gemm.EPI_STORE, gemm.EPI_RESIDUAL, gemm.EPI_SILU_MUL])
+def test_gemm_nvfp4_sm_pairs(m, n, k, epi):
+    """Prefill-sized calls on SM pairs: ragged rows, columns and K tiles, last waves of every unit width. Bound per element:
+    one bf16 rounding of the result (two with a residual) plus an fp32 accumulation of K / 64 block products."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(m + n + k)
+    x = torch.randn(m, k, device=dev, generator=g).bfloat16()
+    wq = nvfp4.quantize_weight(torch.randn(n, k, device=dev, generator=g) * 0.05)
+    gs = torch.tensor(6.0 / (6 * 448), device=dev)
+    xq = nvfp4.quantize(x, gs)
+    alpha = (gs * wq.gscale).reshape(1)
+    res = torch.randn(m, n, device=dev, generator=g).bfloat16() if epi == gemm.EPI_RESIDUAL else None
+    y = gemm.linear_nvfp4(xq, wq, alpha, epilogue=epi, residual=res)
+    torch.cuda.synchronize()
+    assert nv.read_status() == 0
+    a, b = xq.dequantize().double(), wq.dequantize().double()
+    acc = a @ b.t()
+    err = (k // 64 + 1) * 2.0 ** -22 * (a.abs() @ b.abs().t())
+    if epi == gemm.EPI_SILU_MUL:
+        gate, up = acc[:, 0::2], acc[:, 1::2]
+        ref = torch.nn.functional.silu(gate) * up
+        # |silu'| <= 1.1; the exponential and the division of the epilogue are good to 2^-20
+        bound = 2.0 ** -8 * ref.abs() + 1.1 * err[:, 0::2] * up.abs() + err[:, 1::2] * gate.abs() + 2.0 ** -20 * ref.abs()
+    else:
+        ref = acc if res is None else acc + res.double()
+        bound = 2.0 ** -8 * (ref.abs() + (acc.abs() if res is not None else 0)) + err
+    assert bool(((y.double() - ref).abs() <= bound + 1e-30).all())
