@@ -13,6 +13,12 @@
 //     one 16-row tile; the online softmax lives in registers; the 4 warps' partial (m, l, O) merge through shared
 //     memory at the end, and KV splits merge through the LSE kernel of attn.cu.
 //
+// e4m3 pools (F8): the tiles hold the codes, which expand to fp16 in registers on their way into the MMAs (exactly; two
+// codes per conversion). The softmax weights enter O += P V as two fp16 terms, hi + lo, 22 bits together: the
+// error against 64-bit attention is that of fp32 weights. Measured per layer against the CUDA-core kernel of attn.cu:
+// 2 x 30011 keys, 40 / 8 heads of 128: 116 -> 36 us (3.4 TB/s); 16 x 8192, 32 / 2 heads: 180 -> 53 us; 4 x 5003, 24 / 4
+// heads of 256: 102 -> 20 us.
+//
 // The KV range of a split is derived on the device from ctx_len, so one captured launch serves any context.
 // Replaces the FlashInfer decode wrapper the reference plans per step (hibana/engine/graphs.py:55,
 // hibana/engine/executor.py:161-169) and the multi-row verify kernel (hibana/kernels/csrc/verify_attn.cu:469).
@@ -24,7 +30,6 @@
 namespace hb {
 namespace {
 
-constexpr int DEC_WARPS = 2;   // two CTAs share an SM: one streams while the other runs its prologue or merge
 constexpr int DEC_STAGES = 3;
 
 struct DecParams {
@@ -44,6 +49,7 @@ struct DecParams {
   float* part_lse;
   int hq, hkv, splits;
   float scale_log2;
+  float kv_scale;             // dequantisation scale of an e4m3 pool (1 for bf16)
   int causal;
   int use_tma;
   int* status;
@@ -77,6 +83,27 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void mma_f16_sync(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two e4m3 bytes -> two fp16 (exact; byte 0 in the low half).
+__device__ __forceinline__ uint32_t e4m3x2_f16(uint32_t two) {
+  uint32_t r;
+  asm("{\n\t.reg .b16 t;\n\tcvt.u16.u32 t, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, t;\n\t}" : "=r"(r) : "r"(two));
+  return r;
+}
+// Softmax weights of two keys as fp16 pairs hi + lo (22 significant bits together, as good as fp32 weights).
+__device__ __forceinline__ void split_f16(float a, float b, uint32_t* hi, uint32_t* lo) {
+  const __half2 h = __floats2half2_rn(a, b);
+  const __half2 l = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
+  *hi = *reinterpret_cast<const uint32_t*>(&h);
+  *lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
 // Transposes an 8x8 matrix of 16-bit elements held one 32-bit pair per lane (the mma fragment layout).
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
   uint32_t d;
@@ -90,18 +117,24 @@ __device__ __forceinline__ void cp16(uint32_t saddr, const void* g) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait2() { asm volatile("cp.async.wait_group 2;" ::: "memory"); }
 
-template <int D>
+template <int D, bool F8>
 struct DecCfg {
+  // Two CTAs share an SM: one streams while the other runs its prologue or merge. An e4m3 tile is half the bytes of a
+  // bf16 one and twice the arithmetic per byte: twice the warps, the same bytes in flight.
+  static constexpr int WARPS = F8 ? 4 : 2;
+  static constexpr int THREADS = WARPS * 32;
+  static constexpr int ESZ = F8 ? 1 : 2;
   static constexpr int KT = D >= 256 ? 16 : 32;        // keys per warp tile
-  static constexpr int HALVES = D / 64;                 // 128-byte column blocks per row
+  static constexpr int BLOCK_ELEMS = 128 / ESZ;         // elements of a 128-byte column block
+  static constexpr int HALVES = D / BLOCK_ELEMS;        // column blocks per row
   static constexpr int BLOCK_BYTES = KT * 128;          // one column block of a tile
-  static constexpr int TILE_BYTES = KT * D * 2;         // one of K or V
+  static constexpr int TILE_BYTES = KT * D * ESZ;       // one of K or V
   static constexpr int STAGE_BYTES = 2 * TILE_BYTES;
   static constexpr int WARP_BYTES = DEC_STAGES * STAGE_BYTES;
   static constexpr int QROWB = D * 2 + 16;              // padded Q row: conflict-free ldmatrix
   static constexpr int Q_BYTES = 16 * QROWB;
-  static constexpr int BAR_OFF = DEC_WARPS * WARP_BYTES + Q_BYTES;
-  static constexpr int SMEM = BAR_OFF + 256 + 1024;
+  static constexpr int BAR_OFF = WARPS * WARP_BYTES + Q_BYTES;
+  static constexpr int SMEM = BAR_OFF + 256 + 1024;     // +0 barriers and abort flags, +128 row scales, +192 merge flag
   static_assert(16 * D * 4 + 16 * 8 <= WARP_BYTES, "merge scratch must fit a warp's ring");
   static_assert(BLOCK_BYTES % 1024 == 0, "column blocks must keep the swizzle atom alignment");
 };
@@ -112,10 +145,11 @@ __device__ __forceinline__ uint32_t dsw(int row, int c) {
   return static_cast<uint32_t>((c >> 3) * (KT * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
 }
 
-template <int D, bool T8>
-__global__ void __launch_bounds__(DEC_WARPS * 32, 2)
+template <int D, bool T8, bool F8>
+__global__ void __launch_bounds__(DecCfg<D, F8>::THREADS, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const DecParams p) {
-  using C = DecCfg<D>;
+  using C = DecCfg<D, F8>;
+  constexpr int DEC_WARPS = C::WARPS;
   grid_dep_wait();     // may run as a programmatic dependent of the RoPE + KV-write kernel
   grid_dep_launch();
   constexpr int KT = C::KT, ROWB = C::QROWB;
@@ -147,13 +181,35 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   const int k1 = min(ctx, k0 + per);
   const int ntiles = k1 > k0 ? (k1 - k0 + KT - 1) / KT : 0;
 
-  // Q rows (zero padded to 16) into shared memory.
+  // Q rows (zero padded to 16) into shared memory. For an e4m3 pool Q becomes fp16, the type K and V expand to
+  // exactly: every row is scaled by a power of two that takes its largest element to [2^14, 2^15), so all that is more
+  // than 2^-31 of the largest keeps its eight significant bits; the inverse factor joins the softmax scale.
+  float* row_scale = reinterpret_cast<float*>(smem + C::BAR_OFF + 128);
   for (int i = tid; i < 16 * (D / 8); i += DEC_WARPS * 32) {
     const int qi = i / (D / 8), c = i % (D / 8);
     uint4 v = make_uint4(0, 0, 0, 0);
     if (qi < nq) {
       const int rr = qi / g, gg = qi % g;
       v = *reinterpret_cast<const uint4*>(p.q + (static_cast<long long>(row0 + rr) * p.hq + kvh * g + gg) * D + c * 8);
+    }
+    if constexpr (F8) {
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      // bit pattern of the largest magnitude (a whole row sits in D / 8 = 16 or 32 consecutive lanes)
+      uint32_t mx = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mx = max(mx, max(w[e] & 0x7FFFu, (w[e] >> 16) & 0x7FFFu));
+#pragma unroll
+      for (int sh = 1; sh < D / 8; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+      const int e2 = static_cast<int>(mx >> 7) - 127;          // exponent of the largest element
+      const int up = mx == 0 || e2 > 127 ? 0 : min(14 - e2, 126);
+      const float f = __uint_as_float(static_cast<uint32_t>(127 + max(up, -126)) << 23);
+      if (c == 0) row_scale[qi] = __uint_as_float(static_cast<uint32_t>(127 - max(up, -126)) << 23);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __half2 h = __floats2half2_rn(bf16_lo(w[e]) * f, bf16_hi(w[e]) * f);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      v = make_uint4(w[0], w[1], w[2], w[3]);
     }
     *reinterpret_cast<uint4*>(qs + qi * ROWB + c * 16) = v;
   }
@@ -164,7 +220,24 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   // form. Q is then the B operand (n = query row, k = head dim).
   uint32_t qf[T8 ? 1 : KS][4];
   uint32_t qb[T8 ? KS : 1][2];
-  if constexpr (!T8) {
+  if constexpr (F8) {
+    // The contraction index of Q K^T is permuted inside each block of 16 head dims so that a thread's four K bytes
+    // are one 32-bit word: positions 2 t4, 2 t4 + 1 | 2 t4 + 8, 2 t4 + 9 stand for dims 4 t4 .. 4 t4 + 3.
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      const uint2 a = *reinterpret_cast<const uint2*>(qs + g4 * ROWB + (ks * 16 + 4 * t4) * 2);
+      if constexpr (T8) {
+        qb[ks][0] = a.x;
+        qb[ks][1] = a.y;
+      } else {
+        const uint2 b2 = *reinterpret_cast<const uint2*>(qs + (g4 + 8) * ROWB + (ks * 16 + 4 * t4) * 2);
+        qf[ks][0] = a.x;
+        qf[ks][1] = b2.x;
+        qf[ks][2] = a.y;
+        qf[ks][3] = b2.y;
+      }
+    }
+  } else if constexpr (!T8) {
     const uint32_t base = smem_u32(qs) + ((lane & 7) + ((lane >> 3) & 1) * 8) * ROWB + (lane >> 4) * 16;
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) ldsm_x4(qf[ks], base + ks * 32);
@@ -203,7 +276,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       uint8_t* kt = ring + st * C::STAGE_BYTES;
       const uint32_t kdst = smem_u32(kt);
       const uint32_t vdst = kdst + C::TILE_BYTES;
-      constexpr int CPR = D / 8;            // 16-byte chunks per row
+      constexpr int CPR = D * C::ESZ / 16;  // 16-byte chunks per row
       constexpr int RPI = 32 / CPR > 0 ? 32 / CPR : 1;   // rows per warp instruction
       const int slot0 = __shfl_sync(0xffffffffu, my_slot, 0);
       const bool run = p.use_tma && __all_sync(0xffffffffu, lane >= KT || (my_slot >= 0 && my_slot == slot0 + lane));
@@ -215,7 +288,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
         if (lane < 2 * C::HALVES) {
           const int h = lane >> 1, is_v = lane & 1;
           tma_load_2d(kt + is_v * C::TILE_BYTES + h * C::BLOCK_BYTES, is_v ? &tmv : &tmk, &full[st],
-                      kvh * p.tma_xh + h * 64, kvh * p.tma_yh + slot0);
+                      kvh * p.tma_xh + h * C::BLOCK_ELEMS, kvh * p.tma_yh + slot0);
         }
       } else {
         tma_mode &= ~(1u << st);
@@ -227,10 +300,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
             const int slot = __shfl_sync(0xffffffffu, my_slot, key);
             const uint32_t so = dsw<KT>(key, part);
             if (slot >= 0) {
-              const __nv_bfloat16* src = p.k_pool + static_cast<long long>(slot) * p.pool_stride +
-                                         static_cast<long long>(kvh) * p.head_stride + part * 8;
-              cp16(kdst + so, src);
-              cp16(vdst + so, p.v_pool + (src - p.k_pool));
+              const long long off = (static_cast<long long>(slot) * p.pool_stride +
+                                     static_cast<long long>(kvh) * p.head_stride) * C::ESZ + part * 16;
+              cp16(kdst + so, reinterpret_cast<const uint8_t*>(p.k_pool) + off);
+              cp16(vdst + so, reinterpret_cast<const uint8_t*>(p.v_pool) + off);
             } else {
               asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kdst + so), "r"(0) : "memory");
               asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vdst + so), "r"(0) : "memory");
@@ -253,6 +326,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   const int row_lo = T8 ? 2 * t4 : g4, row_hi = T8 ? 2 * t4 + 1 : g4 + 8;
   const int lim_lo = p.causal ? ctx - R + (row_lo / g) + 1 : ctx;
   const int lim_hi = p.causal ? ctx - R + (row_hi / g) + 1 : ctx;
+  const float scale_lo = F8 ? p.scale_log2 * p.kv_scale * row_scale[row_lo] : p.scale_log2;
+  const float scale_hi = F8 ? p.scale_log2 * p.kv_scale * row_scale[row_hi] : p.scale_log2;
 
   const bool prof = p.prof != nullptr && tid == 0;
   const long long t_start = prof ? clock64() : 0;
@@ -289,6 +364,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
         s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        if constexpr (F8) {
+#pragma unroll
+          for (int ks = 0; ks < KS; ks += 4) {
+            uint32_t kb[4];
+            ldsm_x4(kb, kbase + dsw<KT>(j * 8 + (lane & 7), ks + (lane >> 3)));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              mma_f16_sync(s[j], qf[ks + i], e4m3x2_f16(kb[i]), e4m3x2_f16(kb[i] >> 16));
+          }
+        } else
 #pragma unroll
         for (int ks = 0; ks < KS; ks += 2) {
           uint32_t kb[4];
@@ -304,8 +389,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
         for (int e = 0; e < 2; ++e) {
           const int kp = kpos0 + j * 8 + 2 * t4 + e;
           const bool in = kp < k1;
-          s[j][e] = (in && kp < lim_lo) ? s[j][e] * p.scale_log2 : -INFINITY;
-          s[j][2 + e] = (in && kp < lim_hi) ? s[j][2 + e] * p.scale_log2 : -INFINITY;
+          s[j][e] = (in && kp < lim_lo) ? s[j][e] * scale_lo : -INFINITY;
+          s[j][2 + e] = (in && kp < lim_hi) ? s[j][2 + e] * scale_hi : -INFINITY;
           mx_lo = fmaxf(mx_lo, s[j][e]);
           mx_hi = fmaxf(mx_hi, s[j][2 + e]);
         }
@@ -322,6 +407,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       l_lo *= a_lo;
       l_hi *= a_hi;
       uint32_t pf[NB / 2][4];
+      uint32_t pl[F8 ? NB / 2 : 1][4];   // low halves of the fp16 weights
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
         const float p0 = mn_lo == -INFINITY ? 0.f : exp2f(s[j][0] - mn_lo);
@@ -330,8 +416,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
         const float p3 = mn_hi == -INFINITY ? 0.f : exp2f(s[j][3] - mn_hi);
         l_lo += p0 + p1;
         l_hi += p2 + p3;
-        pf[j >> 1][(j & 1) * 2] = pack_bf16(p0, p1);
-        pf[j >> 1][(j & 1) * 2 + 1] = pack_bf16(p2, p3);
+        if constexpr (F8) {
+          split_f16(p0, p1, &pf[j >> 1][(j & 1) * 2], &pl[j >> 1][(j & 1) * 2]);
+          split_f16(p2, p3, &pf[j >> 1][(j & 1) * 2 + 1], &pl[j >> 1][(j & 1) * 2 + 1]);
+        } else {
+          pf[j >> 1][(j & 1) * 2] = pack_bf16(p0, p1);
+          pf[j >> 1][(j & 1) * 2 + 1] = pack_bf16(p2, p3);
+        }
       }
 #pragma unroll
       for (int nb = 0; nb < ONB; ++nb) {
@@ -342,6 +433,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       }
 #pragma unroll
       for (int kk = 0; kk < KT / 16; ++kk) {
+        if constexpr (F8) {
+          // A transposing load hands a thread the bytes of dims 2 g4, 2 g4 + 1 of two keys: accumulator blocks
+          // 2 c and 2 c + 1 are the even and the odd dims of 16-dim block c.
+#pragma unroll
+          for (int c = 0; c < D / 16; c += 2) {
+            uint32_t vw[4];
+            ldsm_x4_t(vw, vbase + dsw<KT>(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, c + (lane >> 4)));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t w0 = __byte_perm(vw[2 * i], 0, 0x3120), w1 = __byte_perm(vw[2 * i + 1], 0, 0x3120);
+              const uint32_t e0 = e4m3x2_f16(w0), e1 = e4m3x2_f16(w1);
+              const uint32_t o0 = e4m3x2_f16(w0 >> 16), o1 = e4m3x2_f16(w1 >> 16);
+              mma_f16_sync(o[2 * (c + i)], pf[kk], e0, e1);
+              mma_f16_sync(o[2 * (c + i) + 1], pf[kk], o0, o1);
+              mma_f16_sync(o[2 * (c + i)], pl[kk], e0, e1);
+              mma_f16_sync(o[2 * (c + i) + 1], pl[kk], o0, o1);
+            }
+          }
+        } else
 #pragma unroll
         for (int nb = 0; nb < ONB; nb += 2) {
           uint32_t vb[4];
@@ -356,6 +466,19 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         st[mt][0] = st[mt][1] = st[mt][2] = st[mt][3] = 0.f;
+        if constexpr (F8) {
+#pragma unroll
+          for (int ks = 0; ks < KS; ks += 2) {
+            uint32_t kw[4];
+            ldsm_x4(kw, kbase + dsw<KT>(mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, ks + (lane >> 4)));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t ka[4] = {e4m3x2_f16(kw[2 * i]), e4m3x2_f16(kw[2 * i + 1]), e4m3x2_f16(kw[2 * i] >> 16),
+                                      e4m3x2_f16(kw[2 * i + 1] >> 16)};
+              mma_f16_sync(st[mt], ka, qb[ks + i][0], qb[ks + i][1]);
+            }
+          }
+        } else
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
           uint32_t ka[4];
@@ -371,8 +494,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
         for (int e = 0; e < 2; ++e) {
           const int kp = kpos0 + mt * 16 + g4 + 8 * e;
           const bool in = kp < k1;
-          st[mt][2 * e] = (in && kp < lim_lo) ? st[mt][2 * e] * p.scale_log2 : -INFINITY;
-          st[mt][2 * e + 1] = (in && kp < lim_hi) ? st[mt][2 * e + 1] * p.scale_log2 : -INFINITY;
+          st[mt][2 * e] = (in && kp < lim_lo) ? st[mt][2 * e] * scale_lo : -INFINITY;
+          st[mt][2 * e + 1] = (in && kp < lim_hi) ? st[mt][2 * e + 1] * scale_hi : -INFINITY;
           mx_lo = fmaxf(mx_lo, st[mt][2 * e]);
           mx_hi = fmaxf(mx_hi, st[mt][2 * e + 1]);
         }
@@ -390,6 +513,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       l_lo *= a_lo;
       l_hi *= a_hi;
       uint32_t pb[MT][2];   // P^T as B operand: (k = key, n = query row)
+      uint32_t pl[F8 ? MT : 1][2];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
@@ -398,7 +522,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
           const float p1 = mn_hi == -INFINITY ? 0.f : exp2f(st[mt][2 * e + 1] - mn_hi);
           l_lo += p0;
           l_hi += p1;
-          pb[mt][e] = movmatrix_trans(pack_bf16(p0, p1));
+          if constexpr (F8) {
+            uint32_t hi, lo;
+            split_f16(p0, p1, &hi, &lo);
+            pb[mt][e] = movmatrix_trans(hi);
+            pl[mt][e] = movmatrix_trans(lo);
+          } else {
+            pb[mt][e] = movmatrix_trans(pack_bf16(p0, p1));
+          }
         }
       }
 #pragma unroll
@@ -410,6 +541,21 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       }
 #pragma unroll
       for (int kk = 0; kk < MT; ++kk) {
+        if constexpr (F8) {
+          // rows g4 and g4 + 8 of accumulator block ob are dims 2 g4 and 2 g4 + 1 of 16-dim block ob
+#pragma unroll
+          for (int ob = 0; ob < OB; ob += 2) {
+            uint32_t vw[4];
+            ldsm_x4_t(vw, vbase + dsw<KT>(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, ob + (lane >> 4)));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t w0 = __byte_perm(vw[2 * i], 0, 0x3120), w1 = __byte_perm(vw[2 * i + 1], 0, 0x3120);
+              const uint32_t va[4] = {e4m3x2_f16(w0), e4m3x2_f16(w0 >> 16), e4m3x2_f16(w1), e4m3x2_f16(w1 >> 16)};
+              mma_f16_sync(o[ob + i], va, pb[kk][0], pb[kk][1]);
+              mma_f16_sync(o[ob + i], va, pl[kk][0], pl[kk][1]);
+            }
+          }
+        } else
 #pragma unroll
         for (int ob = 0; ob < OB; ++ob) {
           uint32_t va[4];   // V^T block (16 head-dim x 16 keys) through transposing loads
@@ -432,6 +578,15 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
     l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
     l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+    if constexpr (F8) {
+#pragma unroll
+      for (int c = 0; c < D / 16; ++c) {
+        *reinterpret_cast<float4*>(mo + g4 * D + c * 16 + 4 * t4) =
+            make_float4(o[2 * c][0], o[2 * c + 1][0], o[2 * c][1], o[2 * c + 1][1]);
+        *reinterpret_cast<float4*>(mo + (g4 + 8) * D + c * 16 + 4 * t4) =
+            make_float4(o[2 * c][2], o[2 * c + 1][2], o[2 * c][3], o[2 * c + 1][3]);
+      }
+    } else
 #pragma unroll
     for (int nb = 0; nb < OB; ++nb) {
       *reinterpret_cast<float2*>(mo + g4 * D + nb * 8 + 2 * t4) = make_float2(o[nb][0], o[nb][1]);
@@ -450,6 +605,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
       l_lo += __shfl_xor_sync(0xffffffffu, l_lo, sh);
       l_hi += __shfl_xor_sync(0xffffffffu, l_hi, sh);
     }
+    if constexpr (F8) {
+#pragma unroll
+      for (int ob = 0; ob < OB; ++ob) {
+        *reinterpret_cast<float2*>(mo + row_lo * D + ob * 16 + 2 * g4) = make_float2(o[ob][0], o[ob][2]);
+        *reinterpret_cast<float2*>(mo + row_hi * D + ob * 16 + 2 * g4) = make_float2(o[ob][1], o[ob][3]);
+      }
+    } else
 #pragma unroll
     for (int ob = 0; ob < OB; ++ob) {
       mo[row_lo * D + ob * 16 + g4] = o[ob][0];
@@ -488,7 +650,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
           lt += sc * wo[16 * D + qi * 2 + 1];
         }
       }
-      const float val = lt > 0.f ? acc / lt : 0.f;
+      float val = lt > 0.f ? acc / lt : 0.f;
+      if constexpr (F8) val *= p.kv_scale;
       const int rr = qi / g, gg = qi % g;
       const long long rh = static_cast<long long>(row0 + rr) * p.hq + kvh * g + gg;
       if (direct) {
@@ -599,21 +762,21 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   }
 }
 
-template <int D, bool T8>
+template <int D, bool T8, bool F8>
 int launch_decode(const DecParams& p0, const void* k_pool, const void* v_pool, long long pool_slots, int batch,
                   cudaStream_t st) {
   DecParams p = p0;
-  using C = DecCfg<D>;
+  using C = DecCfg<D, F8>;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attn_decode_kernel<D, T8>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+    if (cudaFuncSetAttribute(attn_decode_kernel<D, T8, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
         cudaSuccess)
       return 3;
     attr = true;
   }
   static const CUtensorMap dummy = {};
   const CUtensorMap *tk = &dummy, *tv = &dummy;
-  const KvTma t = make_kv_tma(k_pool, v_pool, p.pool_stride, p.head_stride, pool_slots, p.hkv, D, C::KT);
+  const KvTma t = make_kv_tma(k_pool, v_pool, p.pool_stride, p.head_stride, pool_slots, p.hkv, D, C::KT, C::ESZ);
   p.use_tma = t.ok;
   p.tma_xh = t.xh;
   p.tma_yh = t.yh;
@@ -621,7 +784,7 @@ int launch_decode(const DecParams& p0, const void* k_pool, const void* v_pool, l
     tk = &t.k;
     tv = &t.v;
   }
-  launch_dep(attn_decode_kernel<D, T8>, dim3(batch, p.hkv, p.splits), dim3(DEC_WARPS * 32), C::SMEM, st, *tk, *tv, p);
+  launch_dep(attn_decode_kernel<D, T8, F8>, dim3(batch, p.hkv, p.splits), dim3(C::THREADS), C::SMEM, st, *tk, *tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -656,15 +819,19 @@ void hb_attn_decode_fuse(void* split_counter, void* q_out, void* q_sf, const voi
   g_dec_fuse.q_out = q_out; g_dec_fuse.q_sf = q_sf; g_dec_fuse.q_gscale = q_gscale; g_dec_fuse.q_ka = q_ka;
 }
 
-// bf16 KV only; rows_per_seq * (hq / hkv) must be <= 16. Partials go through hb_attn_merge when splits > 1 unless
+// bf16 KV, or e4m3 (`kv_fp8`: x = code * kv_scale; head dim 128 or 256, slot and head strides multiples of 16, 16-byte
+// aligned pools); rows_per_seq * (hq / hkv) must be <= 16. Partials go through hb_attn_merge when splits > 1 unless
 // hb_attn_decode_fuse armed the in-kernel merge.
 int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                    long long head_stride,
                    const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,
                    const void* q_indptr, void* out, void* part_o, void* part_lse, int batch, int max_rows, int hq,
-                   int hkv, int d, int splits, float scale, int causal, long long pool_slots, void* status,
-                   void* stream) {
+                   int hkv, int d, int splits, float scale, int kv_fp8, float kv_scale, int causal, long long pool_slots,
+                   void* status, void* stream) {
   if (batch <= 0) return 0;
+  if (kv_fp8 && (pool_stride % 16 != 0 || head_stride % 16 != 0 ||
+                 ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) != 0))
+    return 1;
   if (hq % hkv != 0 || max_rows * (hq / hkv) > 16) return 1;
   DecParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
@@ -682,6 +849,7 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
   p.part_lse = static_cast<float*>(part_lse);
   p.hq = hq; p.hkv = hkv; p.splits = splits < 1 ? 1 : splits;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.kv_scale = kv_fp8 ? kv_scale : 1.f;
   p.causal = causal;
   p.status = static_cast<int*>(status);
   p.prof = g_dec_prof;
@@ -695,12 +863,19 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
   if (p.splits > 1 && (part_o == nullptr || part_lse == nullptr)) return 1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool t8 = max_rows * (hq / hkv) <= 8;
-  if (d == 64) return t8 ? launch_decode<64, true>(p, k_pool, v_pool, pool_slots, batch, st)
-                         : launch_decode<64, false>(p, k_pool, v_pool, pool_slots, batch, st);
-  if (d == 128) return t8 ? launch_decode<128, true>(p, k_pool, v_pool, pool_slots, batch, st)
-                          : launch_decode<128, false>(p, k_pool, v_pool, pool_slots, batch, st);
-  if (d == 256) return t8 ? launch_decode<256, true>(p, k_pool, v_pool, pool_slots, batch, st)
-                          : launch_decode<256, false>(p, k_pool, v_pool, pool_slots, batch, st);
+  if (kv_fp8) {
+    if (d == 128) return t8 ? launch_decode<128, true, true>(p, k_pool, v_pool, pool_slots, batch, st)
+                            : launch_decode<128, false, true>(p, k_pool, v_pool, pool_slots, batch, st);
+    if (d == 256) return t8 ? launch_decode<256, true, true>(p, k_pool, v_pool, pool_slots, batch, st)
+                            : launch_decode<256, false, true>(p, k_pool, v_pool, pool_slots, batch, st);
+    return 1;
+  }
+  if (d == 64) return t8 ? launch_decode<64, true, false>(p, k_pool, v_pool, pool_slots, batch, st)
+                         : launch_decode<64, false, false>(p, k_pool, v_pool, pool_slots, batch, st);
+  if (d == 128) return t8 ? launch_decode<128, true, false>(p, k_pool, v_pool, pool_slots, batch, st)
+                          : launch_decode<128, false, false>(p, k_pool, v_pool, pool_slots, batch, st);
+  if (d == 256) return t8 ? launch_decode<256, true, false>(p, k_pool, v_pool, pool_slots, batch, st)
+                          : launch_decode<256, false, false>(p, k_pool, v_pool, pool_slots, batch, st);
   return 1;
 }
 

@@ -16,6 +16,16 @@
 //                         sum refer to is only raised (and O rescaled in TMEM) when the new maximum exceeds it by
 //                         more than 2^8, so the rescale is rare and the tensor pipe overlaps the softmax.
 //
+// e4m3 pools (F8) run the same pipeline in fp16, to which every e4m3 code expands exactly: eight producer warps load
+// 16 codes per lane, expand them in registers and store the swizzled tiles (two loads in flight per lane: K of the next
+// tile, V of this one). Q rows become fp16 under a power-of-two row scale (exact down to 2^-31 of the row's
+// largest element), and P is the sum of two fp16 tiles, hi + lo, so that the softmax weights keep 22 bits: O += hi V +
+// lo V. Against the fp32 CUDA-core kernel of attn.cu: 4096 tokens, 32 / 2 heads of 128: 8050 -> 390 us; 1237 + 263 tokens,
+// 24 / 4 heads of 256: 2170 -> 84 us. What bounds it is the chain scores -> softmax -> P -> O of each tile, not the MMAs.
+//
+// Few rows on a long context leave most SMs idle, so the context can be cut into splits (merged by hb_attn_merge): 4 rows
+// on 30000 keys, 24 / 4 heads of 256: 1050 us as one range, 63 us in 37.
+//
 // Causal masking follows the ragged-batch rule of the engine: row token j of a sequence with R new rows and
 // context ctx sees keys [0, ctx - R + j]. All waits are bounded; a timeout raises the status word and every role
 // leaves.
@@ -29,10 +39,15 @@
 namespace hb {
 namespace {
 
-constexpr int PF_THREADS = 256;
+template <bool F8>
+struct PfRoles {                  // warps 0-3 softmax, then the producers, then the MMA issuer
+  static constexpr int PROD_WARPS = F8 ? 8 : 3;
+  static constexpr int ISSUER = 4 + PROD_WARPS;
+  static constexpr int PRODUCERS = PROD_WARPS * 32;
+  static constexpr int THREADS = (ISSUER + 1) * 32;
+};
 constexpr int PF_ROWS = 128;      // packed query rows per CTA
 constexpr int PF_STAGES = 2;
-constexpr int PF_PRODUCERS = 96;  // warps 4, 5, 6
 
 struct PfParams {
   const __nv_bfloat16* q;
@@ -47,23 +62,26 @@ struct PfParams {
   const int* ctx_len;
   const int* q_indptr;
   __nv_bfloat16* out;
-  int hq, hkv;
+  float* part_o;              // splits > 1: [T, Hq, splits, D] partial outputs and their log2 sums [T, Hq, splits]
+  float* part_lse;
+  int hq, hkv, splits;
   int use_tma;                // pools are TMA-addressable: contiguous slot runs travel as bulk tensor copies
   float scale_log2;
+  float kv_scale;             // dequantisation scale of an e4m3 pool
   int causal;
   int* status;
   unsigned long long* prof;   // optional cycle counters (null = off)
 };
 
-template <int D>
+template <int D, bool F8>
 struct PfCfg {
   static constexpr int KT = D > 128 ? 64 : 128;               // keys per tile (head dim 256: 64, to fit shared memory)
   static constexpr int HALVES = D / 64;                      // 64-element (128-byte) column blocks of a row
   static constexpr int Q_BYTES = PF_ROWS * D * 2;
   static constexpr int KV_TILE = KT * D * 2;              // one stage of K or of V
   static constexpr int P_BYTES = PF_ROWS * KT * 2;
-  static constexpr int BAR_OFF = Q_BYTES + 2 * PF_STAGES * KV_TILE + P_BYTES;
-  static constexpr int SMEM = BAR_OFF + 256 + 1024;
+  static constexpr int BAR_OFF = Q_BYTES + 2 * PF_STAGES * KV_TILE + P_BYTES * (F8 ? 2 : 1);
+  static constexpr int SMEM = BAR_OFF + 256 + (F8 ? PF_ROWS * 4 : 0) + 1024;   // F8: one scale per packed query row
   static constexpr int TMEM_COLS = 512;                      // S0 [0, KT) S1 [KT, 2 KT) O [2 KT, 2 KT + D)
   static constexpr float RESCALE_GAP = 8.f;                  // log2 units
 };
@@ -95,11 +113,29 @@ __device__ __forceinline__ uint32_t sw_off(int r, int part, int rows) {
   return static_cast<uint32_t>((part >> 3) * rows * 128 + r * 128 + (((part & 7) ^ (r & 7)) << 4));
 }
 
-template <int D>
-__global__ void __launch_bounds__(PF_THREADS, 1)
+// 16 e4m3 codes -> 16 fp16 in two 16-byte chunks, at 16-byte columns 2 `part` and 2 `part` + 1 of row r of a tile.
+__device__ __forceinline__ void store_f16_row16(uint32_t tile, int r, int part, int rows, const uint4& a) {
+  const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+  uint32_t h[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
+        : "=r"(h[2 * i]), "=r"(h[2 * i + 1])
+        : "r"(w[i]));
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + sw_off(r, 2 * part + c, rows)), "r"(h[4 * c]),
+                 "r"(h[4 * c + 1]), "r"(h[4 * c + 2]), "r"(h[4 * c + 3])
+                 : "memory");
+}
+
+template <int D, bool F8>
+__global__ void __launch_bounds__(PfRoles<F8>::THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
-  using C = PfCfg<D>;
+  using C = PfCfg<D, F8>;
   constexpr int KT = C::KT;
+  constexpr int PF_PRODUCERS = PfRoles<F8>::PRODUCERS, ISSUER = PfRoles<F8>::ISSUER;
   constexpr int CPR = D / 8;   // 16-byte chunks per row
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -116,12 +152,15 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
   uint64_t* pv_ready = p_ready + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_ready + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* row_scale = reinterpret_cast<float*>(smem + C::BAR_OFF + 256);   // F8
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler too
   const int g = p.hq / p.hkv;
   const int tok_per_blk = PF_ROWS / g;
   const int b = blockIdx.z, kvh = blockIdx.y;
-  const int qb = gridDim.x - 1 - blockIdx.x;   // heaviest (latest) query blocks first
+  const int split = static_cast<int>(blockIdx.x) % p.splits;
+  const int qb = (gridDim.x - 1 - blockIdx.x) / p.splits;   // heaviest (latest) query blocks first
   const int row0 = p.q_indptr ? p.q_indptr[b] : b;
   const int R = p.q_indptr ? p.q_indptr[b + 1] - row0 : 1;
   const int tok0 = qb * tok_per_blk;
@@ -129,9 +168,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
   const int ntok = min(tok_per_blk, R - tok0);
   const int nrows = ntok * g;
   const int ctx = p.ctx_len[b];
-  // keys [0, kmax) are visible to at least one row of the block
-  const int kmax = p.causal ? min(ctx, ctx - R + tok0 + ntok) : ctx;
-  const int ntiles = (kmax + KT - 1) / KT;
+  // keys [0, vis) are visible to at least one row of the block
+  const int vis = p.causal ? min(ctx, ctx - R + tok0 + ntok) : ctx;
+  // of which this CTA takes [kbeg, kmax): splits are whole tiles, so that only the last one ends inside a tile
+  const int per = ((ctx + p.splits - 1) / p.splits + KT - 1) / KT * KT;
+  const int kbeg = split * per;
+  const int kmax = min(vis, kbeg + per);
+  const int ntiles = kmax > kbeg ? (kmax - kbeg + KT - 1) / KT : 0;
 
   if (tid == 0) {
     for (int s = 0; s < PF_STAGES; ++s) {
@@ -151,20 +194,93 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
       prefetch_tmap(&tmv);
     }
   }
-  if (warp == 7) {
+  if (warp == ISSUER) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
+  }
+  if constexpr (F8) {
+    // Q as scaled fp16 rows, by every warp (CPR = 16 or 32 consecutive lanes hold a row)
+    for (int c = tid; c < PF_ROWS * CPR; c += PfRoles<F8>::THREADS) {      // both are multiples of 32: warp-uniform
+      const int r = c / CPR, part = c % CPR;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (r < nrows)
+        v = *reinterpret_cast<const uint4*>(
+            p.q + (static_cast<long long>(row0 + tok0 + r / g) * p.hq + kvh * g + r % g) * D + part * 8);
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      uint32_t mx = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mx = max(mx, max(w[e] & 0x7FFFu, (w[e] >> 16) & 0x7FFFu));
+#pragma unroll
+      for (int sh = 1; sh < CPR; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+      const int e2 = static_cast<int>(mx >> 7) - 127;
+      const int up = mx == 0 || e2 > 127 ? 0 : min(14 - e2, 126);      // largest element to [2^14, 2^15)
+      const float f = __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
+      if (part == 0) row_scale[r] = __uint_as_float(static_cast<uint32_t>(127 - up) << 23);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __half2 h = __floats2half2_rn(bf16_lo(w[e]) * f, bf16_hi(w[e]) * f);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(q_s + sw_off(r, part, PF_ROWS)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    fence_proxy_async_smem();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t o_tmem = tmem_base + 2 * KT;
 
-  if (warp >= 4 && warp < 7) {
+  if (warp >= 4 && warp < ISSUER) {
     // ------------------------------------------------------------------ producers
     const int ptid = tid - 128;
     const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? p.seq_rows[b] : b) * p.ld_idx;
+    if constexpr (F8) {
+      constexpr int CH = D / 16;                              // 16-code chunks per row
+      constexpr int PER = KT * CH / PF_PRODUCERS;             // chunks of a tile per thread
+      constexpr int RSTEP = PF_PRODUCERS / CH;
+      static_assert(KT * CH % PF_PRODUCERS == 0 && PF_PRODUCERS % CH == 0, "whole chunks per thread");
+      const int part = ptid % CH, r0 = ptid / CH;
+      int sl_now[PER], sl_next[PER];
+      uint4 kreg[PER], vreg[PER];
+      auto slots = [&](int t, int (&sl)[PER]) {               // -1 beyond the visible keys
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const int key = kbeg + t * KT + r0 + i * RSTEP;
+          sl[i] = t < ntiles && key < kmax ? __ldg(idx_row + key) : -1;
+        }
+      };
+      auto load = [&](const void* pool, const int (&sl)[PER], uint4 (&reg)[PER]) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+          reg[i] = sl[i] < 0 ? make_uint4(0, 0, 0, 0)
+                             : __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(pool) +
+                                                                    static_cast<long long>(sl[i]) * p.pool_stride +
+                                                                    kvh * p.head_stride + part * 16));
+      };
+      auto store = [&](uint8_t* tile, const uint4 (&reg)[PER], uint64_t* bar) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) store_f16_row16(smem_u32(tile), r0 + i * RSTEP, part, KT, reg[i]);
+        fence_proxy_async_smem();
+        mbar_arrive(bar);
+      };
+      slots(0, sl_now);
+      slots(1, sl_next);
+      load(p.k_pool, sl_now, kreg);
+      for (int t = 0; t < ntiles; ++t) {
+        const int s = t % PF_STAGES;
+        const uint32_t ph = ((t / PF_STAGES) - 1) & 1;
+        load(p.v_pool, sl_now, vreg);
+        if (t >= PF_STAGES && !mbar_wait(&kempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
+        store(k_s + s * C::KV_TILE, kreg, &kfull[s]);
+        load(p.k_pool, sl_next, kreg);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) sl_now[i] = sl_next[i];
+        slots(t + 2, sl_next);
+        if (t >= PF_STAGES && !mbar_wait(&vempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
+        store(v_s + s * C::KV_TILE, vreg, &vfull[s]);
+      }
+    } else {
     // Q rows (zero padded); they travel in the first cp.async group, i.e. with K tile 0.
     for (int c = ptid; c < PF_ROWS * CPR; c += PF_PRODUCERS) {
       const int r = c / CPR, part = c % CPR;
@@ -189,7 +305,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 #pragma unroll
       for (int i = 0; i < SB; ++i) {
         const int j = pw + 3 * i;
-        const int key = t * KT + j * 32 + lane;
+        const int key = kbeg + t * KT + j * 32 + lane;
         sl[i] = (j < KT / 32 && t < ntiles && key < kmax) ? __ldg(idx_row + key) : -1;
       }
     };
@@ -286,31 +402,38 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing may land after the CTA has gone
     fence_proxy_async_smem();
     if (live) mbar_arrive(&vfull[(ntiles - 1) % PF_STAGES]);
-  } else if (warp == 7) {
+    }
+  } else if (warp == ISSUER) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(PF_ROWS, KT);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(PF_ROWS, D, 0, 1);
-      const uint32_t q_a = smem_u32(q_s), p_a = smem_u32(p_s);
+    {   // the whole warp walks the loop, one elected lane issues (hb_common.cuh, elect_one)
+      // operand format codes of kind::f16: 0 = fp16, 1 = bf16 (bits 7 and 10)
+      constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
+      constexpr uint32_t idesc_qk = make_idesc_bf16(PF_ROWS, KT) & ~(F8 ? kBf16 : 0u);
+      constexpr uint32_t idesc_pv = make_idesc_bf16(PF_ROWS, D, 0, 1) & ~(F8 ? kBf16 : 0u);
+      const uint32_t q_a = __shfl_sync(0xffffffffu, smem_u32(q_s), 0);
+      const uint32_t k_0 = q_a + C::Q_BYTES, v_0 = k_0 + PF_STAGES * C::KV_TILE, p_a = v_0 + PF_STAGES * C::KV_TILE;
       // S(t) = Q K(t)^T into score buffer t % 2; releases the K stage and publishes the scores when done.
       auto issue_qk = [&](int t) -> bool {
         const int s = t % PF_STAGES;
         {
           PF_T0();
-          if (!mbar_wait(&kfull[s], (t / PF_STAGES) & 1, abort, p.status, kTimeoutFull)) return false;
-          PF_ACC(5, true);
+          if (!warp_wait(&kfull[s], (t / PF_STAGES) & 1, abort, p.status, kTimeoutFull)) return false;
+          PF_ACC(5, lane == 0);
         }
         tc_fence_after();
-        const uint32_t k_a = smem_u32(k_s + s * C::KV_TILE);
+        const uint32_t k_a = k_0 + s * C::KV_TILE;
         const uint32_t s_t = tmem_base + (t & 1) * KT;
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint32_t in_row = (ks & 3) * 32;   // 16 elements = 32 bytes inside the 128-byte swizzled row
-          mma_f16(s_t, make_desc_sw128(q_a + (ks >> 2) * (PF_ROWS * 128) + in_row),
-                  make_desc_sw128(k_a + (ks >> 2) * (KT * 128) + in_row), idesc_qk, ks > 0 ? 1u : 0u);
+          for (int ks = 0; ks < D / 16; ++ks) {
+            const uint32_t in_row = (ks & 3) * 32;   // 16 elements = 32 bytes inside the 128-byte swizzled row
+            mma_f16(s_t, make_desc_sw128(q_a + (ks >> 2) * (PF_ROWS * 128) + in_row),
+                    make_desc_sw128(k_a + (ks >> 2) * (KT * 128) + in_row), idesc_qk, ks > 0 ? 1u : 0u);
+          }
+          tc_commit(&kempty[s]);
+          tc_commit(&s_ready[t & 1]);
         }
-        tc_commit(&kempty[s]);
-        tc_commit(&s_ready[t & 1]);
+        __syncwarp();
         return true;
       };
       bool ok = ntiles > 0 && issue_qk(0);
@@ -319,25 +442,31 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         const int s = t % PF_STAGES;
         {
           PF_T0();
-          if (!mbar_wait(p_ready, t & 1, abort, p.status, kTimeoutAccum)) break;
-          PF_ACC(3, true);
+          if (!warp_wait(p_ready, t & 1, abort, p.status, kTimeoutAccum)) break;
+          PF_ACC(3, lane == 0);
         }
         {
           PF_T0();
-          if (!mbar_wait(&vfull[s], (t / PF_STAGES) & 1, abort, p.status, kTimeoutFull)) break;
-          PF_ACC(4, true);
+          if (!warp_wait(&vfull[s], (t / PF_STAGES) & 1, abort, p.status, kTimeoutFull)) break;
+          PF_ACC(4, lane == 0);
         }
         tc_fence_after();
-        const uint32_t v_a = smem_u32(v_s + s * C::KV_TILE);
+        const uint32_t v_a = v_0 + s * C::KV_TILE;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < KT / 16; ++kk) {
-          const uint64_t adesc = make_desc_sw128(p_a + (kk >> 2) * (PF_ROWS * 128) + (kk & 3) * 32);
-          // 16 keys = two 8-row groups 1024 bytes apart; the D / 64 column blocks are KT * 128 bytes apart
-          const uint64_t bdesc = make_desc_sw128_mn(v_a + kk * 2048, KT * 128, 1024);
-          mma_f16(o_tmem, adesc, bdesc, idesc_pv, (t > 0 || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < KT / 16; ++kk) {
+            const uint64_t adesc = make_desc_sw128(p_a + (kk >> 2) * (PF_ROWS * 128) + (kk & 3) * 32);
+            // 16 keys = two 8-row groups 1024 bytes apart; the D / 64 column blocks are KT * 128 bytes apart
+            const uint64_t bdesc = make_desc_sw128_mn(v_a + kk * 2048, KT * 128, 1024);
+            mma_f16(o_tmem, adesc, bdesc, idesc_pv, (t > 0 || kk > 0) ? 1u : 0u);
+            if constexpr (F8)      // the low parts of the weights
+              mma_f16(o_tmem, make_desc_sw128(p_a + C::P_BYTES + (kk >> 2) * (PF_ROWS * 128) + (kk & 3) * 32), bdesc,
+                      idesc_pv, 1u);
+          }
+          tc_commit(&vempty[s]);
+          tc_commit(pv_ready);
         }
-        tc_commit(&vempty[s]);
-        tc_commit(pv_ready);
+        __syncwarp();
         // score buffer t % 2 was read completely before p_ready(t): refill it two tiles ahead
         if (t + 2 < ntiles) ok = issue_qk(t + 2);
       }
@@ -350,6 +479,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     const int tok = tok0 + r / g;
     // last visible key position (inclusive)
     const int lim = row_ok ? (p.causal ? ctx - R + tok : ctx - 1) : -1;
+    const float scale_log2 = F8 ? p.scale_log2 * p.kv_scale * row_scale[r] : p.scale_log2;
     float m_ref = -INFINITY, l = 0.f;   // O and l are relative to 2^m_ref
     const uint32_t p_row = smem_u32(p_s) + r * 128;
     bool ok = true;
@@ -364,7 +494,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         PF_ACC(0, tid == 0);
       }
       tc_fence_after();
-      const int k0 = t * KT;
+      const int k0 = kbeg + t * KT;
       const uint32_t s_t = tmem_base + (t & 1) * KT + tlane;
       // The two passes over the score row are rolled loops over 32-column chunks: fully unrolled, the softmax body
       // alone is several thousand instructions, and streaming that through the instruction cache every tile cost
@@ -382,7 +512,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         for (int j = 0; j < 32; ++j)
           mx4[j & 3] = fmaxf(mx4[j & 3], j <= rc ? __uint_as_float(v[j]) : -INFINITY);
       }
-      const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
       // P(t) overwrites the buffer O += P(t - 1) V(t - 1) reads, and a rescale touches O: both need that MMA done.
       {
         PF_T0();
@@ -421,12 +551,26 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         tmem_ld_wait();
         const int rc = rel - c0;
         uint32_t w[16];
+        uint32_t wl[F8 ? 16 : 1];
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-          const float p0 = j <= rc ? ex2(fmaf(__uint_as_float(v[j]), p.scale_log2, neg_m)) : 0.f;
-          const float p1 = j + 1 <= rc ? ex2(fmaf(__uint_as_float(v[j + 1]), p.scale_log2, neg_m)) : 0.f;
+          // F8: product and difference rounded one after the other, as the maximum was, so that the largest score gives
+          // exactly 2^0 whatever its size (a fused product of scores near 2^40 would overflow the exponential)
+          const float x0 = F8 ? __fadd_rn(__fmul_rn(__uint_as_float(v[j]), scale_log2), neg_m)
+                              : fmaf(__uint_as_float(v[j]), scale_log2, neg_m);
+          const float x1 = F8 ? __fadd_rn(__fmul_rn(__uint_as_float(v[j + 1]), scale_log2), neg_m)
+                              : fmaf(__uint_as_float(v[j + 1]), scale_log2, neg_m);
+          const float p0 = j <= rc ? ex2(x0) : 0.f;
+          const float p1 = j + 1 <= rc ? ex2(x1) : 0.f;
           sum4[(j >> 1) & 3] += p0 + p1;
-          w[j >> 1] = pack_bf16(p0, p1);
+          if constexpr (F8) {
+            const __half2 hi = __floats2half2_rn(p0, p1);
+            const __half2 lo = __floats2half2_rn(p0 - __low2float(hi), p1 - __high2float(hi));
+            w[j >> 1] = *reinterpret_cast<const uint32_t*>(&hi);
+            wl[j >> 1] = *reinterpret_cast<const uint32_t*>(&lo);
+          } else {
+            w[j >> 1] = pack_bf16(p0, p1);
+          }
         }
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
@@ -435,6 +579,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[4 * ch]), "r"(w[4 * ch + 1]),
                        "r"(w[4 * ch + 2]), "r"(w[4 * ch + 3])
                        : "memory");
+          if constexpr (F8)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + C::P_BYTES), "r"(wl[4 * ch]),
+                         "r"(wl[4 * ch + 1]), "r"(wl[4 * ch + 2]), "r"(wl[4 * ch + 3])
+                         : "memory");
         }
       }
       l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
@@ -454,8 +602,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     if (ok && ntiles > 0) ok = warp_wait(pv_ready, (ntiles - 1) & 1, abort, p.status, kTimeoutAccum);
     if (ok) {
       tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* dst = p.out + (static_cast<long long>(row0 + tok) * p.hq + kvh * g + r % g) * D;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if constexpr (F8) inv *= p.kv_scale;
+      const long long rh = static_cast<long long>(row0 + tok) * p.hq + kvh * g + r % g;
+      __nv_bfloat16* dst = p.out + rh * D;
+      if (p.splits > 1 && row_ok) p.part_lse[rh * p.splits + split] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
 #pragma unroll
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t o[32];
@@ -466,7 +617,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 32; ++j) o[j] = 0;
         }
-        if (row_ok) {
+        if (row_ok && p.splits > 1) {
+          float* part = p.part_o + (rh * p.splits + split) * D + c0;
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(part + j) =
+                make_float4(__uint_as_float(o[j]) * inv, __uint_as_float(o[j + 1]) * inv,
+                            __uint_as_float(o[j + 2]) * inv, __uint_as_float(o[j + 3]) * inv);
+        } else if (row_ok) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8)
             *reinterpret_cast<uint4*>(dst + c0 + j) =
@@ -481,21 +639,21 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 7) tmem_dealloc(tmem_base, C::TMEM_COLS);
+  if (warp == ISSUER) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
-template <int D>
+template <int D, bool F8>
 int launch_prefill(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int qblocks, int batch,
                    cudaStream_t st) {
-  using C = PfCfg<D>;
+  using C = PfCfg<D, F8>;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+    if (cudaFuncSetAttribute(attn_prefill_kernel<D, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
         cudaSuccess)
       return 3;
     attr = true;
   }
-  attn_prefill_kernel<D><<<dim3(qblocks, p.hkv, batch), PF_THREADS, C::SMEM, st>>>(*tk, *tv, p);
+  attn_prefill_kernel<D, F8><<<dim3(qblocks * p.splits, p.hkv, batch), PfRoles<F8>::THREADS, C::SMEM, st>>>(*tk, *tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -515,14 +673,21 @@ extern "C" {
 // [12] softmax score load, [13] softmax math incl. the wait for the previous O update, [14] publish P.
 void hb_attn_prefill_profile(void* buf) { g_pf_prof = static_cast<unsigned long long*>(buf); }
 
-// bf16 KV, head dim 64 or 128, group size hq / hkv <= 128. `max_rows` bounds the new rows of any sequence.
+// bf16 KV with head dim 64, 128 or 256, or e4m3 KV (`kv_fp8`: x = code * kv_scale) with head dim 128 or 256, slot and head
+// strides multiples of 16 and 16-byte aligned pools; group size hq / hkv <= 128. `max_rows` bounds the new rows of any
+// sequence. With splits > 1 the context is cut into that many ranges of whole tiles, a CTA each, whose normalised
+// partial rows and log2 sums go to part_o / part_lse for hb_attn_merge.
 int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                     long long head_stride,
                     const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,
-                    const void* q_indptr, void* out, int batch, int max_rows, int hq, int hkv, int d, float scale,
-                    int causal, long long pool_slots, void* status, void* stream) {
+                    const void* q_indptr, void* out, void* part_o, void* part_lse, int splits, int batch, int max_rows,
+                    int hq, int hkv, int d, float scale,
+                    int kv_fp8, float kv_scale, int causal, long long pool_slots, void* status, void* stream) {
   if (batch <= 0 || max_rows <= 0) return 0;
   if (hq % hkv != 0 || hq / hkv > PF_ROWS) return 1;
+  if (kv_fp8 && (pool_stride % 16 != 0 || head_stride % 16 != 0 ||
+                 ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) != 0))
+    return 1;
   PfParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k_pool = static_cast<const __nv_bfloat16*>(k_pool);
@@ -535,8 +700,13 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
   p.ctx_len = static_cast<const int*>(ctx_len);
   p.q_indptr = static_cast<const int*>(q_indptr);
   p.out = static_cast<__nv_bfloat16*>(out);
+  p.part_o = static_cast<float*>(part_o);
+  p.part_lse = static_cast<float*>(part_lse);
+  p.splits = splits < 1 ? 1 : splits;
+  if (p.splits > 1 && (part_o == nullptr || part_lse == nullptr)) return 1;
   p.hq = hq; p.hkv = hkv;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.kv_scale = kv_scale;
   p.causal = causal;
   p.status = static_cast<int*>(status);
   p.prof = g_pf_prof;
@@ -545,6 +715,12 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   static const CUtensorMap dummy = {};
   const CUtensorMap *tk = &dummy, *tv = &dummy;
+  if (kv_fp8) {      // producers load through registers: no tensor maps
+    p.use_tma = p.tma_xh = p.tma_yh = 0;
+    if (d == 128) return launch_prefill<128, true>(p, tk, tv, qblocks, batch, st);
+    if (d == 256) return launch_prefill<256, true>(p, tk, tv, qblocks, batch, st);
+    return 1;
+  }
   const KvTma t = make_kv_tma(k_pool, v_pool, pool_stride, head_stride, pool_slots, hkv, d, 32);
   p.use_tma = t.ok;
   p.tma_xh = t.xh;
@@ -553,9 +729,9 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
     tk = &t.k;
     tv = &t.v;
   }
-  if (d == 64) return launch_prefill<64>(p, tk, tv, qblocks, batch, st);
-  if (d == 128) return launch_prefill<128>(p, tk, tv, qblocks, batch, st);
-  if (d == 256) return launch_prefill<256>(p, tk, tv, qblocks, batch, st);
+  if (d == 64) return launch_prefill<64, false>(p, tk, tv, qblocks, batch, st);
+  if (d == 128) return launch_prefill<128, false>(p, tk, tv, qblocks, batch, st);
+  if (d == 256) return launch_prefill<256, false>(p, tk, tv, qblocks, batch, st);
   return 1;
 }
 

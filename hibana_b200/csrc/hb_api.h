@@ -125,8 +125,7 @@ int hb_attn_merge(const void* part_o, const void* part_lse, void* out, long long
 int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                     long long head_stride,
                     const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,
-                    const void* q_indptr, void* out, int batch, int max_rows, int hq, int hkv, int d, float scale,
-                    int causal, long long pool_slots, void* status, void* stream);
+                    const void* q_indptr, void* out, void* part_o, void* part_lse, int splits, int batch, int max_rows, int hq, int hkv, int d, float scale, int kv_fp8, float kv_scale, int causal, long long pool_slots, void* status, void* stream);
 int hb_gdn_phase1(const void* q, const void* k, const void* v, const void* g, const void* beta, long long ldq,
                   long long ldv, int n, int k_heads, int v_heads, float scale, int l2norm, void* w, void* qg, void* kd,
                   void* m, void* u, void* g_end, void* stream);
@@ -148,7 +147,7 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
                    long long head_stride,
                    const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,
                    const void* q_indptr, void* out, void* part_o, void* part_lse, int batch, int max_rows, int hq,
-                   int hkv, int d, int splits, float scale, int causal, long long pool_slots, void* status,
+                   int hkv, int d, int splits, float scale, int kv_fp8, float kv_scale, int causal, long long pool_slots, void* status,
                    void* stream);
 
 // ---- sampling and speculative acceptance (sample.cu) -----------------------------------------------------

@@ -2,7 +2,7 @@
 
 `paged_attention` is the single entry: query rows of a ragged batch attend to their sequence's context through
 the block table. Kernels: csrc/attn_prefill.cu (tcgen05 prefill), csrc/attn_decode.cu (tensor-core flash-decoding,
-up to 16 query rows per kv head), csrc/attn.cu (general split-KV + LSE merge; fp8 KV, head dim 256 prefill). The plain-PyTorch reference below is the CPU path
+up to 16 query rows per kv head), csrc/attn.cu (general split-KV + LSE merge: NVFP4 KV, fp8 KV under `stable_numerics`). The plain-PyTorch reference below is the CPU path
 and the GPU tests' oracle. Reference counterparts: hibana/kernels/ops.py:131-161 (ragged prefill),
 hibana/model/attention.py:69-126, hibana/kernels/csrc/verify_attn.cu.
 """
@@ -23,14 +23,14 @@ nv.register("hb_attn_paged", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I,
 nv.register("hb_attn_merge", [P, P, P, L, I, I, P])
 nv.register("hb_attn_fp4_scales", [P, P, L, L], void=True)
 nv.register("hb_attn_merge_quant", [P, P, L, I, I, I, P, P, P, I, P])
-nv.register("hb_attn_decode", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, L, P, P])
+nv.register("hb_attn_decode", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, Fl, I, L, P, P])
 
 nv.register("hb_attn_decode_fuse", [P, P, P, P, I], void=True)
 nv.register("hb_attn_decode_tc", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, L, P, P])
 nv.register("hb_attn_decode_tc_profile", [P], void=True)
 nv.register("hb_attn_prefill_profile", [P], void=True)
 nv.register("hb_attn_decode_profile", [P], void=True)
-nv.register("hb_attn_prefill", [P, P, P, L, L, P, L, P, P, P, P, I, I, I, I, I, Fl, I, L, P, P])
+nv.register("hb_attn_prefill", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, Fl, I, L, P, P])
 
 from ..hardware.b200 import NUM_SMS  # noqa: E402
 
@@ -133,9 +133,10 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     fp4 = getattr(k_pool, "sf", None) is not None
     fp8 = k_pool.dtype != torch.bfloat16
     cfg = cfgmod.current()
-    if not fp8 and max_rows * (hq // hkv) <= 16 and d in (64, 128, 256):
+    f8 = fp8 and not fp4 and _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+    if (not fp8 and d in (64, 128, 256) or f8) and max_rows * (hq // hkv) <= 16:
         st = nv.device_state(q.device)
-        tc = d == 128 and cfg.decode_attn == "tc"
+        tc = d == 128 and cfg.decode_attn == "tc" and not f8
         fuse = cfg.fuse_epilogues and not tc and (cfg.fuse_attn_tail or splits == 1)
         xq = None
         if fuse:
@@ -153,10 +154,11 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         args = (q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1),
                 kv_indices.data_ptr(), kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), nv.ptr(q_indptr),
                 nv.ptr(out), workspace.part_o.data_ptr() if splits > 1 else None,
-                workspace.part_lse.data_ptr() if splits > 1 else None, b, max_rows, hq, hkv, d, splits, scale,
-                int(causal), k_pool.shape[0], st.status.data_ptr())
-        fn = nv.lib().hb_attn_decode_tc if tc else nv.lib().hb_attn_decode
-        nv.check(fn(*args, nv.stream()), "hb_attn_decode")
+                workspace.part_lse.data_ptr() if splits > 1 else None, b, max_rows, hq, hkv, d, splits, scale)
+        tail = (int(causal), k_pool.shape[0], st.status.data_ptr(), nv.stream())
+        code = (nv.lib().hb_attn_decode_tc(*args, *tail) if tc
+                else nv.lib().hb_attn_decode(*args, int(f8), kv_scale, *tail))
+        nv.check(code, "hb_attn_decode")
         if xq is not None:
             return xq
         if splits > 1 and not fuse:
@@ -175,6 +177,16 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     res = _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, seq_rows, scale, kv_scale, causal,
                          splits, workspace, out, cfg, fp8, b, t, hq, hkv, d)
     return res if quant_scale is None else nvfp4.quantize(res.view(t, hq * d), quant_scale)
+
+
+def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg) -> bool:
+    """Whether an e4m3 pool takes the tensor-core kernels: whole 128-byte column blocks per row and rows on 16-byte
+    boundaries (bulk copies). Under `stable_numerics` the general kernel stays: it sums a row's keys in the same order
+    however many rows share the call, the tensor-core kernels have one form for up to 8 and one for up to 16 rows."""
+    return (k_pool.dtype == torch.float8_e4m3fn and d in (128, 256) and not cfg.stable_numerics
+            and k_pool.stride(0) % 16 == 0 and k_pool.stride(1) % 16 == 0 and k_pool.stride(2) == 1
+            and v_pool.stride() == k_pool.stride()
+            and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
 
 
 _QUANT_BUFS: dict = {}
@@ -196,13 +208,17 @@ def _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, s
     if getattr(k_pool, "sf", None) is not None:
         fp8 = 2       # NVFP4 pool: the split-KV kernel dequantises rows as it loads them
         nv.lib().hb_attn_fp4_scales(k_pool.sf.data_ptr(), v_pool.sf.data_ptr(), k_pool.sf.stride(0), k_pool.sf.stride(1))
-    if not fp8 and d in (64, 128, 256) and q_indptr is not None and cfg.prefill_attn == "tc":
+    f8 = fp8 is True and _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+    if (not fp8 and d in (64, 128, 256) or f8) and q_indptr is not None and cfg.prefill_attn == "tc":
         st = nv.device_state(q.device)
+        parts = (workspace.part_o.data_ptr(), workspace.part_lse.data_ptr()) if splits > 1 else (None, None)
         nv.check(nv.lib().hb_attn_prefill(
             q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1), kv_indices.data_ptr(),
-            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), b,
-            max_rows, hq, hkv, d, scale, int(causal), k_pool.shape[0], st.status.data_ptr(), nv.stream()),
-                 "hb_attn_prefill")
+            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts, splits,
+            b, max_rows, hq, hkv, d, scale, int(f8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
+            nv.stream()), "hb_attn_prefill")
+        if splits > 1:
+            nv.check(nv.lib().hb_attn_merge(*parts, out.data_ptr(), t * hq, splits, d, nv.stream()), "hb_attn_merge")
         return out
     nv.check(nv.lib().hb_attn_paged(
         q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1), kv_indices.data_ptr(),

@@ -4,6 +4,7 @@ import math
 import pytest
 import torch
 
+from hibana_b200 import _native as nv
 from hibana_b200.ops import attention, basic, nvfp4, sampling
 
 
@@ -537,3 +538,45 @@ def test_nvfp4_kv_kernels_match_reference(rows):
         _close(got, ref, 2e-2)
     from hibana_b200 import _native as nv
     assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hq,hkv,d", [(40, 8, 128), (24, 4, 256), (32, 2, 128), (32, 2, 256), (3, 3, 128)])
+@pytest.mark.parametrize("rows", ["decode", "verify", "prefill"])
+@pytest.mark.parametrize("contiguous", [False, True])
+def test_fp8_attention_tensor_cores(hq, hkv, d, rows, contiguous):
+    """e4m3 pools on the tensor-core kernels against 64-bit attention of the dequantised cache: contexts at the edges of
+    tiles and blocks, scattered slots and runs, every row count form, splits. The weights keep 22 bits and the sums 24, so
+    the result is off by its rounding to bf16: at most 2^-9 per element, hence of the norm (1.1x for the sums)."""
+    g = hq // hkv
+    if rows == "decode":
+        counts, ctxs = [1] * 7, [1, 15, 16, 33, 64, 300, 1025]
+    elif rows == "verify":
+        counts = [max(1, 16 // g), 1, max(1, 8 // g)]
+        ctxs = [max(1, 16 // g), 130, 700]
+    else:
+        counts, ctxs = [20, 1, 150, 65], [20, 200, 150, 577]
+    q, kp, vp, idx, ctx, indptr, sr = _attn_case(len(counts), counts, ctxs, hq, hkv, d, dtype=torch.float8_e4m3fn,
+                                                 contiguous=contiguous)
+    q[0] *= 2.0 ** 40                       # rows of very different size: each has its own fp16 scale
+    q[-1] *= 2.0 ** -30
+    scale, ks = 0.5 / d ** 0.5, 0.25
+    ref = torch.zeros(q.shape, dtype=torch.float64)
+    for i, c in enumerate(ctxs):
+        r0, r1 = int(indptr[i]), int(indptr[i + 1])
+        sl = idx[sr[i], :c].long()
+        k = kp[sl].double().repeat_interleave(g, 1) * ks
+        v = vp[sl].double().repeat_interleave(g, 1) * ks
+        s = torch.einsum("rhd,chd->rhc", q[r0:r1].double(), k) * scale
+        lim = c - (r1 - r0) + torch.arange(r1 - r0)
+        s = s.masked_fill((torch.arange(c)[None] > lim[:, None])[:, None], float("-inf"))
+        ref[r0:r1] = torch.einsum("rhc,chd->rhd", torch.softmax(s, -1), v)
+    kw = {} if rows == "decode" else dict(q_indptr=indptr.cuda(), max_rows=max(counts))
+    kc, vc = (t.cuda() for t in (kp, vp))
+    if contiguous:
+        kc, vc = (t.transpose(0, 1).contiguous().transpose(0, 1) for t in (kc, vc))
+    for splits in (1, 3):
+        got = attention.paged_attention(q.cuda(), kc, vc, idx.cuda(), ctx.cuda(), seq_rows=sr.cuda(), scale=scale,
+                                        kv_scale=ks, splits=splits, **kw).cpu().double()
+        err = (got - ref).norm() / ref.norm()
+        assert nv.read_status() == 0 and float(err) < 1.1 * 2.0 ** -9, float(err)
