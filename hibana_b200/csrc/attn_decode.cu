@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(DecCfg<D, F8>::THREADS, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const DecParams p) {
   using C = DecCfg<D, F8>;
   constexpr int DEC_WARPS = C::WARPS;
+  grid_dep_launch();   // what follows (merge, output projection) waits for this grid before it reads anything
   grid_dep_wait();     // may run as a programmatic dependent of the RoPE + KV-write kernel
-  grid_dep_launch();
   constexpr int KT = C::KT, ROWB = C::QROWB;
   constexpr int NB = KT / 8;     // score n-blocks per tile
   constexpr int KS = D / 16;     // k-steps of Q K^T

@@ -1000,7 +1000,9 @@ cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorM
           (void)cudaGetLastError();
           n = -1;
         }
-        max_clusters[splits] = n;
+        // The query counts one CTA per SM for a kernel that allocates tensor memory. Two do run where shared memory and
+        // tensor memory hold two (BN <= 64): with 148 slots assumed, K was cut half as often as the chip has room for.
+        max_clusters[splits] = BN <= 64 && n > 0 ? 2 * n : n;
       }
       if (max_clusters[splits] >= tiles) break;
     }

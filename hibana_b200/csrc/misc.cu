@@ -215,8 +215,8 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, long
                                      int kv_fp8, float kv_inv_scale, int q_gate, uint8_t* __restrict__ k_sf,
                                      uint8_t* __restrict__ v_sf, long long sf_pool_stride, long long sf_head_stride,
                                      const float2* __restrict__ table) {
+  grid_dep_launch();   // the attention kernel waits for this grid; its launch overlaps the rest of the projection's
   grid_dep_wait();     // may run as a programmatic dependent of the QKV projection
-  grid_dep_launch();
   const int t = blockIdx.x;
   const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int nw = gridDim.y * (blockDim.x >> 5);
@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(
     __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
     long long pool_stride, long long head_stride, int tokens, int hq, int hkv, int d, int q_gate,
     const float2* __restrict__ table) {
-  grid_dep_wait();
   grid_dep_launch();
+  grid_dep_wait();
   const int lanes_per_head = d >> 3;                       // 8, 16 or 32
   const int heads_per_warp = 32 / lanes_per_head;
   const int lane = threadIdx.x & 31;

@@ -105,16 +105,27 @@ norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
                         const __nv_bfloat16* __restrict__ w, float eps, int gemma, int m, int k, int ka,
                         const float* __restrict__ gscale, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                         __nv_bfloat16* __restrict__ normed) {
-  grid_dep_wait();     // launched as a programmatic dependent: the producer of x must have completed
-  grid_dep_launch();   // a GEMM launched as a programmatic dependent may start prefetching its weights
   __shared__ float red[40];
   const int row = blockIdx.x;
   const int tid = threadIdx.x;
+  // A decode step is a chain of short kernels, and this one is latency: the GEMM behind it may become resident and fetch
+  // weights from now on, and what no kernel of the step writes (norm weights, the scale) is read before the wait for the
+  // producer of x. At one row of 5120 the step got 2.0 us shorter per launch.
+  grid_dep_launch();
+  const int nchunk = k >> 3;
+  uint4 wa[MAXC];
+  float gs_early = 0.f;
+  if (row < m) {
+#pragma unroll
+    for (int i = 0; i < MAXC; ++i)
+      if (tid + i * T < nchunk) wa[i] = __ldg(reinterpret_cast<const uint4*>(w) + tid + i * T);
+    if (q != nullptr) gs_early = __ldg(gscale);
+  }
+  grid_dep_wait();
   if (row >= m) {   // padding rows of the last 128-row scale block: zero scales, nothing else
     for (int g = tid; g < ka * 4; g += T) sf[row_sf_off(row, g, ka)] = 0;
     return;
   }
-  const int nchunk = k >> 3;
   float v[MAXC][8];
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * k);
   uint4* rr = residual ? reinterpret_cast<uint4*>(residual + static_cast<size_t>(row) * k) : nullptr;
@@ -144,7 +155,7 @@ norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
   RowOut out;
   out.n = 1;
   out.q[0] = q; out.sf[0] = sf; out.bf[0] = normed;
-  row_finish<T, MAXC>(v, k, w, eps, gemma, red, out, row, ka, gscale);
+  row_finish<T, MAXC>(v, k, w, eps, gemma, red, out, row, ka, &gs_early, wa);
 }
 
 // Zeroes the scale bytes of the padding rows [m, round_up(m, 128)) (used after the per-row kernel).

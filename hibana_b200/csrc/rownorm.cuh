@@ -58,11 +58,12 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 
 // v[i] holds chunk (tid + i * T) of the row (values already rounded to bf16 precision). Computes the RMS over the
 // row, applies the weight, and writes bf16 and / or NVFP4 to every destination at row `out_row`.
+// `w_regs` (may be null) holds this thread's weight chunks, loaded by the caller ahead of time.
 // `red` is shared scratch of >= 33 floats. weight == null skips the normalisation (plain quantise / copy).
 template <int T, int MAXC>
 __device__ __forceinline__ void row_finish(float (&v)[MAXC][8], int h, const __nv_bfloat16* __restrict__ weight,
                                            float eps, int gemma, float* red, const RowOut& out, long long out_row,
-                                           int ka, const float* __restrict__ gscale) {
+                                           int ka, const float* __restrict__ gscale, const uint4* w_regs = nullptr) {
   const int tid = threadIdx.x;
   const int nchunk = h >> 3;
   float rstd = 1.f;
@@ -96,7 +97,7 @@ __device__ __forceinline__ void row_finish(float (&v)[MAXC][8], int h, const __n
     if (live) {
       if (weight != nullptr) {
         float w[8];
-        unpack8(reinterpret_cast<const uint4*>(weight)[c], w);
+        unpack8(w_regs != nullptr ? w_regs[i] : reinterpret_cast<const uint4*>(weight)[c], w);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
           y[e] = __bfloat162float(__float2bfloat16(v[i][e] * rstd * (gemma ? 1.f + w[e] : w[e])));
