@@ -171,98 +171,144 @@ __device__ __forceinline__ unsigned order_key(float v) {   // order-preserving m
 __device__ __forceinline__ float key_value(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
-__device__ __forceinline__ float block_sum256(float v, float* red) {   // 256 threads, deterministic
+// A row's kernels run 1024 threads: a pass over the vocabulary is a chain of L2 loads per thread, so its length is what counts.
+// The masses that decide a draw keep one fixed order of additions whatever the thread count: SUM_T strided accumulators, a
+// tree over each warp, then the warps one after the other.
+constexpr int LAW_T = 1024, LAW_WARPS = LAW_T / 32, SUM_T = 256;
+__device__ __forceinline__ float sum_in_order(float v, float* red) {   // v counts on the first SUM_T threads; whole CTA
   v = warp_sum(v);
   __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) t += red[w];
+  for (int w = 0; w < SUM_T / 32; ++w) t += red[w];
   return t;
 }
-
-__device__ __forceinline__ int block_sum256i(int v, int* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+__device__ __forceinline__ int block_sum_i(int v, int* red) {
+  v = __reduce_add_sync(0xffffffffu, v);
   __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  int t = 0;
+  return __reduce_add_sync(0xffffffffu, red[threadIdx.x & 31]);
+}
+
+// Largest key x of [lo, hi] with f(x) >= want, where f(x) is the sum of weight(v) over the allowed tokens of key >= x (f(lo) >=
+// want, f falls with x, no token is above hi). Every pass over the row sums the tokens above WAYS - 1 thresholds at once, so
+// 32 bits take 8 passes instead of 32, and what lies above the range is carried along, so later passes only look at
+// the few tokens inside it. Deterministic. Whole CTA; `sums` is shared scratch.
+constexpr int WAYS = 16;
+template <typename V, typename T, typename W>
+__device__ unsigned search_key(const T* __restrict__ lr, int vocab, const int* __restrict__ mask, unsigned lo, unsigned hi,
+                               V want, W weight, V (*sums)[LAW_WARPS]) {
+  V beyond = V(0);           // f(hi + 1)
+  while (lo < hi) {
+    const unsigned span = hi - lo, step = span / WAYS + 1;
+    V acc[WAYS - 1];
 #pragma unroll
-  for (int w = 0; w < 8; ++w) t += red[w];
-  return t;
+    for (int j = 0; j < WAYS - 1; ++j) acc[j] = V(0);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < vocab; i += LAW_T) {
+      const float v = ldf<T>(lr, i);
+      const unsigned k = order_key(v);
+      if (k > lo && k <= hi && v > -INFINITY && mask_ok(mask, i)) {
+        const unsigned above = (k - lo) / step;          // thresholds lo + step, lo + 2 step, ... at or below k
+        const V w = weight(v);
+#pragma unroll
+        for (int j = 0; j < WAYS - 1; ++j) acc[j] += above > static_cast<unsigned>(j) ? w : V(0);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < WAYS - 1; ++j) {
+      V t = acc[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if ((threadIdx.x & 31) == 0) sums[j][threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    unsigned best = 0;       // thresholds that hold
+#pragma unroll 1
+    for (; best < span / step; ++best) {
+      V t = sums[best][threadIdx.x & 31];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      t += beyond;
+      if (!(t >= want)) {
+        hi = lo + (best + 1) * step - 1;
+        beyond = t;
+        break;
+      }
+    }
+    lo += best * step;
+  }
+  return lo;
 }
 
 // The sampling law of one row as engine/rejection.py `distribution` defines it: softmax(logits / temp) over the
 // allowed tokens, cut to the first `k_lim` tokens in (value desc, index asc) order (0 = no cut), then to the
 // smallest prefix of that order whose mass reaches p_lim. Draws one token by inverse CDF in index order from the
 // law with token `exclude` removed (-1: nothing removed; the residual of a point-mass draft in speculative
-// sampling) and reports the probability of token `probe` under the law. 256 threads, whole CTA.
+// sampling) and reports the probability of token `probe` under the law. LAW_T threads, whole CTA. With a nucleus
+// cut, 256 threads and one threshold per pass took 165 us at 18992 tokens and 2040 us at 151936; this takes 87 and 480 us, with
+// the same draws.
 template <typename T>
 __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restrict__ mask, float temp, int k_lim,
                         float p_lim, float u01, int exclude, int probe, long long* out, float* out_prob,
                         float* out_probe) {
-  __shared__ float red[8];
-  __shared__ int redi[8];
-  __shared__ float csum[256];
-  __shared__ int ceq[256];
-  __shared__ int s_pick_thread;
+  constexpr int CHUNKS = 256;              // contiguous pieces of the row for the draw
+  __shared__ float red[LAW_WARPS];
+  __shared__ int redi[LAW_WARPS];
+  __shared__ float csum[CHUNKS];
+  __shared__ int ceq[CHUNKS];
+  __shared__ int s_pick, s_eq_base;
   __shared__ float s_base;
-  __shared__ int s_eq_base;
+  __shared__ float sums_f[WAYS - 1][LAW_WARPS];
+  __shared__ int sums_i[WAYS - 1][LAW_WARPS];
   const int tid = threadIdx.x;
   const float inv_t = 1.f / temp;
   float mx = -INFINITY;
-  for (int i = tid; i < vocab; i += 256)
+  for (int i = tid; i < vocab; i += LAW_T)
     if (mask_ok(mask, i)) mx = fmaxf(mx, ldf<T>(lr, i));
   mx = warp_max(mx);
   __syncthreads();
   if ((tid & 31) == 0) red[tid >> 5] = mx;
   __syncthreads();
-  mx = red[0];
-#pragma unroll
-  for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w]);
+  mx = warp_max(red[tid & 31]);
   // ---- top-k cut: tk_key = value of the k-th token, need_k = how many of the tokens equal to it are inside
   unsigned tk_key = 0;     // finite values have keys above 0x007fffff: 0 keeps everything
   int need_k = 0x7fffffff;
   const bool cut_k = k_lim > 0 && k_lim < vocab;
   if (cut_k) {
-    unsigned lo = 0, hi = order_key(mx);
-    while (lo < hi) {
-      const unsigned mid = lo + ((hi - lo + 1) >> 1);
-      int cnt = 0;
-      for (int i = tid; i < vocab; i += 256)
-        if (mask_ok(mask, i)) {
-          const float v = ldf<T>(lr, i);
-          cnt += v > -INFINITY && order_key(v) >= mid;
-        }
-      cnt = block_sum256i(cnt, redi);
-      if (cnt >= k_lim) lo = mid;
-      else hi = mid - 1;
-    }
-    tk_key = lo;
+    tk_key = search_key<int>(lr, vocab, mask, 0u, order_key(mx), k_lim, [](float) { return 1; }, sums_i);
     int above = 0;
-    for (int i = tid; i < vocab; i += 256)
+    for (int i = tid; i < vocab; i += LAW_T)
       if (mask_ok(mask, i)) {
         const float v = ldf<T>(lr, i);
         above += v > -INFINITY && order_key(v) > tk_key;
       }
-    need_k = k_lim - block_sum256i(above, redi);
+    need_k = k_lim - block_sum_i(above, redi);
   }
   // mass above a key and number of tokens equal to it
   float m_above = 0.f;
   int n_eq = 0;
-  for (int i = tid; i < vocab; i += 256)
-    if (mask_ok(mask, i)) {
-      const float v = ldf<T>(lr, i);
-      if (v > -INFINITY) {
+  auto mass_above = [&](unsigned key) {
+    m_above = 0.f;
+    n_eq = 0;
+    if (tid < SUM_T) {
+#pragma unroll 8
+      for (int i = tid; i < vocab; i += SUM_T) {
+        const float v = ldf<T>(lr, i);
+        const bool live = v > -INFINITY && mask_ok(mask, i);
         const unsigned k = order_key(v);
-        if (k > tk_key) m_above += __expf((v - mx) * inv_t);
-        else n_eq += k == tk_key;
+        m_above += live && k > key ? __expf((v - mx) * inv_t) : 0.f;
+        n_eq += live && k == key;
       }
     }
-  m_above = block_sum256(m_above, red);
-  n_eq = block_sum256i(n_eq, redi);
+    m_above = sum_in_order(m_above, red);
+    n_eq = block_sum_i(n_eq, redi);
+  };
+  mass_above(tk_key);
   unsigned t_key = tk_key;
   int need_eq = min(need_k, n_eq);
   float w_t = cut_k ? __expf((key_value(tk_key) - mx) * inv_t) : 0.f;
@@ -270,34 +316,12 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   // ---- nucleus inside the cut: the smallest prefix, in the same order, whose mass reaches p_lim * kept
   if (p_lim < 1.f) {
     const float want = p_lim * kept;
-    unsigned lo = tk_key, hi = order_key(mx);      // mass(key >= lo) = kept >= want
-    while (lo < hi) {
-      const unsigned mid = lo + ((hi - lo + 1) >> 1);     // mid > tk_key: every token at or above it is inside the cut
-      float mass = 0.f;
-      for (int i = tid; i < vocab; i += 256)
-        if (mask_ok(mask, i)) {
-          const float v = ldf<T>(lr, i);
-          if (v > -INFINITY && order_key(v) >= mid) mass += __expf((v - mx) * inv_t);
-        }
-      mass = block_sum256(mass, red);
-      if (mass >= want) lo = mid;
-      else hi = mid - 1;
-    }
+    // mass(key >= tk_key) = kept >= want, and every token above tk_key is inside the cut
+    const unsigned lo = search_key<float>(lr, vocab, mask, tk_key, order_key(mx), want,
+                                          [&](float v) { return __expf((v - mx) * inv_t); }, sums_f);
     if (lo != tk_key || !cut_k) {
       t_key = lo;
-      float above = 0.f;
-      int eq = 0;
-      for (int i = tid; i < vocab; i += 256)
-        if (mask_ok(mask, i)) {
-          const float v = ldf<T>(lr, i);
-          if (v > -INFINITY) {
-            const unsigned k = order_key(v);
-            if (k > t_key) above += __expf((v - mx) * inv_t);
-            else eq += k == t_key;
-          }
-        }
-      m_above = block_sum256(above, red);
-      n_eq = block_sum256i(eq, redi);
+      mass_above(t_key);
       w_t = __expf((key_value(t_key) - mx) * inv_t);
       need_eq = n_eq;
     }
@@ -321,12 +345,12 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
       if (k > t_key) w = __expf((v - mx) * inv_t);
       else if (k == t_key) {
         int before = 0;
-        for (int i = tid; i < tok; i += 256)
+        for (int i = tid; i < tok; i += LAW_T)
           if (mask_ok(mask, i)) {
             const float o = ldf<T>(lr, i);
             before += o > -INFINITY && order_key(o) == t_key;
           }
-        before = block_sum256i(before, redi);
+        before = block_sum_i(before, redi);
         if (before < need_eq) w = w_t;
       }
     }
@@ -339,34 +363,36 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
     w_ex = 0.f;
   }
   const float kept_draw = kept - w_ex;
-  // ---- draw: contiguous chunk per thread, chunk sums scanned by thread 0, the owning thread walks its chunk
-  const int per = (vocab + 255) / 256;
-  const int lo_i = tid * per, hi_i = min(vocab, lo_i + per);
-  float mine = 0.f;
-  int my_eq = 0;
-  for (int i = lo_i; i < hi_i; ++i)
-    if (mask_ok(mask, i)) {
+  // ---- draw: mass and number of threshold tokens per chunk, the chunk the draw falls into, then the token in it; all sums in
+  // index order
+  const int per = (vocab + CHUNKS - 1) / CHUNKS;
+  if (tid < CHUNKS) {
+    float mine = 0.f;
+    int my_eq = 0;
+    const int hi_i = min(vocab, (tid + 1) * per);
+#pragma unroll 8
+    for (int i = tid * per; i < hi_i; ++i) {
       const float v = ldf<T>(lr, i);
-      if (v > -INFINITY) {
-        const unsigned k = order_key(v);
-        if (k > t_key) mine += __expf((v - mx) * inv_t);
-        else if (k == t_key) ++my_eq;
-      }
+      const bool live = v > -INFINITY && mask_ok(mask, i);
+      const unsigned k = order_key(v);
+      mine += live && k > t_key ? __expf((v - mx) * inv_t) : 0.f;
+      my_eq += live && k == t_key;
     }
-  csum[tid] = mine;
-  ceq[tid] = my_eq;
+    csum[tid] = mine;
+    ceq[tid] = my_eq;
+  }
   __syncthreads();
   const float u = u01 * kept_draw;
-  const int ex_thread = exclude >= 0 ? exclude / per : -1;
+  const int ex_chunk = exclude >= 0 ? exclude / per : -1;
   if (tid == 0) {
     float acc = 0.f;
     int eq_seen = 0, pick = -1, last = 0;
     float base = 0.f;
     int eq_base = 0;
-    for (int t = 0; t < 256; ++t) {
+    for (int t = 0; t < CHUNKS; ++t) {
       const int take = max(0, min(ceq[t], need_eq - eq_seen));
       float w = csum[t] + take * w_t;
-      if (t == ex_thread) w = fmaxf(w - w_ex, 0.f);
+      if (t == ex_chunk) w = fmaxf(w - w_ex, 0.f);
       if (w > 0.f) last = t;
       if (pick < 0 && u < acc + w) {
         pick = t;
@@ -380,43 +406,49 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
       pick = last;
       base = -1.f;
     }
-    s_pick_thread = pick;
+    s_pick = pick;
     s_base = base;
     s_eq_base = eq_base;
   }
   __syncthreads();
-  if (tid == s_pick_thread) {
+  if (tid < 32) {        // one warp loads 32 tokens at a time and adds them up in order
     float acc = s_base;
     int eq_seen = s_eq_base, chosen = -1, last_kept = -1;
     float w_chosen = 0.f, w_last = 0.f;
-    for (int i = lo_i; i < hi_i; ++i) {
-      if (!mask_ok(mask, i)) continue;
-      const float v = ldf<T>(lr, i);
-      if (!(v > -INFINITY)) continue;
+    const int hi_i = min(vocab, (s_pick + 1) * per);
+    for (int i0 = s_pick * per; i0 < hi_i && chosen < 0; i0 += 32) {
+      const int i = i0 + tid;
+      float v = -INFINITY;
+      if (i < hi_i && mask_ok(mask, i)) v = ldf<T>(lr, i);
+      const bool live = v > -INFINITY;
       const unsigned k = order_key(v);
+      const unsigned equal = __ballot_sync(0xffffffffu, live && k == t_key);
       float w = 0.f;
-      if (k > t_key) w = __expf((v - mx) * inv_t);
-      else if (k == t_key) {
-        if (eq_seen < need_eq) w = w_t;
-        ++eq_seen;
-      }
+      if (live && k > t_key) w = __expf((v - mx) * inv_t);
+      else if (live && k == t_key && eq_seen + __popc(equal & ((1u << tid) - 1u)) < need_eq) w = w_t;
       if (i == exclude) w = 0.f;
-      if (w <= 0.f) continue;
-      last_kept = i;
-      w_last = w;
-      if (s_base >= 0.f && u < acc + w) {
-        chosen = i;
-        w_chosen = w;
-        break;
+      eq_seen += __popc(equal);
+      for (unsigned left = __ballot_sync(0xffffffffu, w > 0.f); left != 0u; left &= left - 1u) {
+        const int src = __ffs(left) - 1;
+        const float ws = __shfl_sync(0xffffffffu, w, src);
+        last_kept = i0 + src;
+        w_last = ws;
+        if (s_base >= 0.f && u < acc + ws) {
+          chosen = last_kept;
+          w_chosen = ws;
+          break;
+        }
+        acc += ws;
       }
-      acc += w;
     }
     if (chosen < 0) {
       chosen = last_kept < 0 ? 0 : last_kept;
       w_chosen = w_last;
     }
-    *out = chosen;
-    if (out_prob) *out_prob = w_chosen / kept_draw;
+    if (tid == 0) {
+      *out = chosen;
+      if (out_prob) *out_prob = w_chosen / kept_draw;
+    }
   }
   __syncthreads();
 }
@@ -432,7 +464,7 @@ constexpr int SAMPLE_K = 64;  // candidates kept per row for 1 <= top-k <= 64 (t
 // One CTA per row. Keeps the SAMPLE_K largest logits by repeated threshold passes (vocab is read a few times from
 // L2), then softmax / top-p / inverse-CDF draw on the candidates. temperature <= 0 means greedy.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(LAW_T)
 sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ offsets,
@@ -440,8 +472,8 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
               float* __restrict__ out_prob, int skip_greedy) {
   __shared__ float cv[SAMPLE_K];
   __shared__ int ci[SAMPLE_K];
-  __shared__ float wv[8];
-  __shared__ int wi[8];
+  __shared__ float wv[LAW_WARPS];
+  __shared__ int wi[LAW_WARPS];
   __shared__ float s_prev_v;
   __shared__ int s_prev_i;
   const int row = blockIdx.x;
@@ -494,7 +526,7 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; ++w)
+      for (int w = 1; w < LAW_WARPS; ++w)
         if (wv[w] > best || (wv[w] == best && wi[w] < bi)) {
           best = wv[w];
           bi = wi[w];
@@ -605,7 +637,7 @@ __global__ void lattice_walk_kernel(const long long* __restrict__ cand, const fl
 // fall out of the same rule: their law is the one-hot argmax). Uniforms are counter draws at (seed, 2 * (draws + j)
 // + 1) for the test and + 2 for the draw.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(LAW_T)
 spec_targets_kernel(const T* __restrict__ logits, long long ld, int vocab, int k, const long long* __restrict__ drafts,
                     const float* __restrict__ temperature, const int* __restrict__ top_k,
                     const float* __restrict__ top_p, const unsigned long long* __restrict__ seeds,
@@ -747,8 +779,8 @@ int hb_sample(const void* logits, long long ld, int rows, int vocab, int is_f32,
       static_cast<const float*>(top_p), static_cast<const unsigned long long*>(seeds),                     \
       static_cast<const unsigned long long*>(offsets), static_cast<const int*>(bitmask), mask_words,       \
       static_cast<long long*>(out), static_cast<float*>(out_prob), skip_greedy
-  if (is_f32) sample_kernel<float><<<rows, 256, 0, st>>>(static_cast<const float*>(logits), HB_SAMPLE_ARGS);
-  else sample_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SAMPLE_ARGS);
+  if (is_f32) sample_kernel<float><<<rows, LAW_T, 0, st>>>(static_cast<const float*>(logits), HB_SAMPLE_ARGS);
+  else sample_kernel<__nv_bfloat16><<<rows, LAW_T, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SAMPLE_ARGS);
 #undef HB_SAMPLE_ARGS
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
@@ -778,9 +810,9 @@ int hb_spec_targets(const void* logits, long long ld, int batch, int k, int voca
       static_cast<const unsigned long long*>(seeds), static_cast<const unsigned long long*>(draws),           \
       static_cast<const float*>(soft), static_cast<const int*>(bitmask), mask_words,                          \
       static_cast<const long long*>(greedy_pick), static_cast<long long*>(target), static_cast<float*>(p_draft)
-  if (is_f32) spec_targets_kernel<float><<<rows, 256, 0, st>>>(static_cast<const float*>(logits), HB_SPEC_ARGS);
+  if (is_f32) spec_targets_kernel<float><<<rows, LAW_T, 0, st>>>(static_cast<const float*>(logits), HB_SPEC_ARGS);
   else
-    spec_targets_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SPEC_ARGS);
+    spec_targets_kernel<__nv_bfloat16><<<rows, LAW_T, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SPEC_ARGS);
 #undef HB_SPEC_ARGS
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
