@@ -119,3 +119,38 @@ def test_expert_sharing_kernel_matches_reference():
         got_i, got_w = moe.share_experts(ids.cuda(), w.cuda(), e, keep, budget, scale=1.7)
         assert torch.equal(got_i.cpu(), want_i)
         assert torch.allclose(got_w.cpu(), want_w, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,topk,e,lo,n", [(1, 1, 8, 0, 8), (372, 22, 512, 0, 512), (373, 22, 512, 0, 512),
+                                                (4096, 22, 512, 100, 300), (1025, 8, 60, 0, 60)])
+def test_plan_places_pairs_in_order(tokens, topk, e, lo, n):
+    """Segments, positions and work list of the routing plan (one CTA below 8192 pairs, a cluster of eight from there on)
+    against a plain count: whole numbers, all equal."""
+    from hibana_b200 import _native as nv
+    g = torch.Generator().manual_seed(tokens)
+    ids = torch.rand(tokens, e, generator=g).topk(topk, dim=1).indices.int()
+    rows_cap = ((tokens * topk + 127) // 128) * 128 + min(n, tokens * topk) * 128
+    bn, cap = 256, tokens * topk // 256 + 1 + e
+    out = [torch.empty(m, dtype=torch.int32, device="cuda") for m in (e, e, tokens * topk, rows_cap, 1, cap, 1)]
+    cnt, start, pos, src, total, tiles, n_tiles = out
+    idc = ids.cuda()
+    nv.check(nv.lib().hb_moe_plan(idc.data_ptr(), tokens, topk, e, lo, n, 0, cnt.data_ptr(), start.data_ptr(), pos.data_ptr(),
+                                  src.data_ptr(), rows_cap, total.data_ptr(), bn, tiles.data_ptr(), n_tiles.data_ptr(), cap,
+                                  nv.stream()), "hb_moe_plan")
+    flat = ids.view(-1)
+    held = (flat >= lo) & (flat < lo + n)
+    want_cnt = torch.bincount(flat[held].long(), minlength=e)
+    seg = (want_cnt + 127) // 128 * 128
+    want_start = seg.cumsum(0) - seg
+    assert cnt.cpu().tolist() == want_cnt.tolist() and int(total) == int(seg.sum())
+    assert start.cpu().tolist() == want_start.tolist()
+    want_pos = torch.full_like(flat, -1)
+    want_src = torch.full((rows_cap,), -1, dtype=torch.int32)
+    for x in range(lo, lo + n):
+        at = (flat == x).nonzero()[:, 0]
+        want_pos[at] = (want_start[x] + torch.arange(len(at))).int()
+        want_src[int(want_start[x]):int(want_start[x]) + len(at)] = (at // topk).int()
+    assert torch.equal(pos.cpu(), want_pos) and torch.equal(src.cpu(), want_src)
+    want_tiles = [x * 4096 + c for x in range(e) for c in range(-(-int(want_cnt[x]) // bn))]
+    assert int(n_tiles) == len(want_tiles) and tiles[:len(want_tiles)].cpu().tolist() == want_tiles
