@@ -8,6 +8,7 @@ rows to slot 0) and hibana/engine/upload.py (pinned non-blocking upload).
 """
 from __future__ import annotations
 
+import gc
 from typing import Optional, Sequence
 
 import numpy as np
@@ -146,6 +147,7 @@ class ModelRunner:
         """Captures one decode graph per bucket (after a warm-up run of the same body)."""
         if not self.use_graphs:
             return
+        gc.collect()      # a dead engine's graphs must not be destroyed by the collector while this one captures
         for b in (buckets or self.buckets):
             buf = self.bufs[b]
             self._prepare_bucket(buf)

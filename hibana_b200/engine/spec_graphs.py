@@ -24,6 +24,7 @@ acceptance and grammar masks take the eager round. Reference: hibana/engine/spec
 """
 from __future__ import annotations
 
+import gc
 from typing import Optional, Sequence
 
 import numpy as np
@@ -144,6 +145,7 @@ class VerifyGraphs:
     def capture(self) -> None:
         if self.device.type != "cuda" or not self.runner.use_graphs:
             return
+        gc.collect()      # see ModelRunner.capture
         for b, buf in self.bufs.items():
             self._prepare(buf)
             buf.dev.zero_()
@@ -284,6 +286,7 @@ class DraftGraphs:
     def capture(self) -> None:
         if self.device.type != "cuda" or not self.runner.use_graphs:
             return
+        gc.collect()      # see ModelRunner.capture
         for buf in self.bufs.values():
             buf.dev.zero_()
             s = torch.cuda.Stream()
