@@ -1099,10 +1099,18 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   while (splits > 1 && (splits - 1) * ((k_tiles + splits - 1) / splits) >= k_tiles) --splits;
   if (splits > 8) splits = 8;   // portable cluster size
 
-  if (a.epilogue == kEpiSiluMulQuant) {
-    // tokens on the N side, whole 128-row feature tiles, no grouped / peer variants; the staging tile of a split-K
+  if (grouped && (a.epilogue == kEpiSiluMulQuant || a.epilogue == kEpiRelu2Quant)) {
+    // SM pairs only: whole 64-feature spans, every row's packed bytes on 16-byte boundaries
+    const int feats = a.epilogue == kEpiSiluMulQuant ? a.grp_rows_a / 2 : a.grp_rows_a;
+    if (a.q_out == nullptr || a.q_sf == nullptr || a.q_gscale == nullptr || feats % 64 != 0 || a.q_ka * 64 < feats ||
+        a.q_ld % 16 != 0 || (reinterpret_cast<uintptr_t>(a.q_out) & 15) != 0 || !gemm_pair_ok(a))
+      return cudaErrorInvalidValue;
+  } else if (a.epilogue == kEpiRelu2Quant) {
+    return cudaErrorInvalidValue;
+  } else if (a.epilogue == kEpiSiluMulQuant) {
+    // tokens on the N side, whole 128-row feature tiles, no peer variants; the staging tile of a split-K
     // CTA sits behind its fp32 partial, which the smallest ring must still hold
-    if (grouped || a.peer != nullptr || a.tok_scale != nullptr || a.q_out == nullptr || a.q_sf == nullptr ||
+    if (a.peer != nullptr || a.tok_scale != nullptr || a.q_out == nullptr || a.q_sf == nullptr ||
         a.q_gscale == nullptr)
       return cudaErrorInvalidValue;
     if (a.swap && (a.ra % BM != 0 || a.q_ka * 64 < a.ra / 2 || a.bn > 128)) return cudaErrorInvalidValue;
@@ -1309,6 +1317,29 @@ int hb_gemm_grouped(int kind, const void* a, const void* b, const void* sfa, con
     g.grp_tile_cap = tile_cap;
   }
   g.peer = nullptr;
+  const cudaError_t e = hb::gemm_launch(g, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? 0 : static_cast<int>(e);
+}
+
+// The same with the activation (epilogue 7: SiLU-mul of interleaved gate / up rows, 8: squared ReLU) requantised to NVFP4 in
+// the epilogue: q_out [b_rows, q_ld bytes] and q_sf (q_ka K atoms per row block) are the activation operand of the next
+// grouped call over the same rows. Needs the plan's work list for 256-row chunks (`tiles`).
+int hb_gemm_grouped_quant(const void* a, const void* b, const void* sfa, const void* sfb, int experts, int n_per_expert,
+                          int b_rows, int k, const void* alpha_ptr, int epilogue, const void* start, const void* cnt,
+                          void* status, int ka_a, int ka_b, const void* tiles, const void* n_tiles, int tile_cap,
+                          void* q_out, void* q_sf, const void* q_gscale, int q_ka, long long q_ld, void* stream) {
+  hb::GemmArgs g;
+  g.kind = hb::kGemmNvfp4; g.a = a; g.b = b; g.sfa = sfa; g.sfb = sfb;
+  g.ra = experts * n_per_expert; g.rb = b_rows; g.k = k; g.lda = k; g.ldb = k;
+  g.out = nullptr; g.ldo = 0; g.residual = nullptr; g.alpha = 1.f;
+  g.alpha_ptr = static_cast<const float*>(alpha_ptr); g.epilogue = epilogue; g.swap = 1; g.splits = 1;
+  g.workspace = nullptr; g.counters = nullptr; g.status = static_cast<int*>(status); g.bn = 256;
+  g.sf_k_atoms_a = ka_a; g.sf_k_atoms_b = ka_b;
+  g.grp_start = static_cast<const int*>(start); g.grp_cnt = static_cast<const int*>(cnt);
+  g.grp_rows_a = n_per_expert; g.grp_experts = experts; g.grp_chunks = 1;
+  g.grp_tiles = static_cast<const int*>(tiles); g.grp_ntiles = static_cast<const int*>(n_tiles); g.grp_tile_cap = tile_cap;
+  g.peer = nullptr;
+  g.q_out = q_out; g.q_sf = q_sf; g.q_gscale = static_cast<const float*>(q_gscale); g.q_ka = q_ka; g.q_ld = q_ld;
   const cudaError_t e = hb::gemm_launch(g, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }

@@ -29,6 +29,7 @@ enum GemmEpilogue : int {
                          // rows go to q_out, ue4m3 scales to q_sf (128x4-swizzled blocks) with the static per-tensor
                          // scale *q_gscale of the consuming projection. Weights on the 128-row side only; the next
                          // GEMM reads the result as its activation operand with no kernel in between.
+  kEpiRelu2Quant = 8,    // squared ReLU as in kEpiRelu2, requantised to NVFP4 the same way (grouped calls on SM pairs)
 };
 
 // Peer-memory fusion arguments (all ranks pass the same offsets; pointers are this process's mappings).

@@ -18,6 +18,12 @@
 //
 // The last wave of full tiles is cut into narrower units (128 or 64 columns) when that shortens it: 2048 x 5120 makes
 // 160 tiles for 74 clusters, 12 of which would otherwise keep the whole chip for a third full wave.
+//
+// Grouped (mixture-of-experts) mode: a unit is (chunk of up to 256 rows of an expert's segment, 256 of its weight rows), from
+// the work list that the routing plan left on the device. An expert of a 4096-token chunk has about 176 rows, and its
+// GEMM is 4 to 11 K tiles long: as one CTA per 128 x 128 tile, set-up and epilogue took most of the time (fc1 and
+// fc2 of 512 experts, 1024 x 2688, 544 us each over 4096 and 904 tokens; as units 391 and 235). fc1 requantises its
+// activation for fc2 in the epilogue, for which two warps share each lane quarter (464 us with one).
 #include <algorithm>
 
 #include "gemm.cuh"
@@ -32,16 +38,16 @@ namespace {
 
 constexpr int PAIR_M = 256;                   // rows of a unit (128 per CTA)
 constexpr int PAIR_N = 256;                   // columns of a full unit
-constexpr int THREADS = 192;                  // producer warp, MMA warp, four epilogue warps
+constexpr int EPI_WARPS = 8;                  // two per TMEM lane quarter, half of a unit's columns each
+constexpr int THREADS = 64 + EPI_WARPS * 32;  // producer warp, MMA warp, epilogue warps
 constexpr int STAGES = 5;
 constexpr int A_BYTES = 128 * 128;            // 128 rows x 256 packed e2m1
 constexpr int B_BYTES = 128 * 128;            // this CTA's half of the 256 columns
 constexpr int SFA_BYTES = 2048;               // one 128-row block x 4 K atoms
 constexpr int SFB_BYTES = 4096;               // two 128-column blocks x 4 K atoms (each CTA holds all columns' scales)
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
-constexpr int ROW_PITCH = 144;                // staged output row: 128 bytes + 16 (conflict-free 16-byte accesses)
-constexpr int Q_PITCH = 80;                   // staged requantised row: 64 packed bytes, 8 scale bytes, padding
-constexpr int STAGING_BYTES = 4 * 32 * ROW_PITCH;
+constexpr int ROW_PITCH = 80;                 // staged output row: at most 64 + 8 bytes (conflict-free 16-byte accesses)
+constexpr int STAGING_BYTES = EPI_WARPS * 32 * ROW_PITCH;
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + 256;
 constexpr int ACC1_COL = 208;                 // first column of the second accumulator
 constexpr int SFA_COL = 464;                  // 4 K atoms x 4 columns
@@ -63,28 +69,98 @@ struct PairParams {
   int q_ka;
   long long q_ld;
   int* status;
+  // grouped mode
+  const int* grp_start;     // [E] first row of the expert's segment (a multiple of 128)
+  const int* grp_cnt;       // [E] its rows
+  const int* grp_tiles;     // work list: expert * 4096 + chunk of 256 rows
+  const int* grp_ntiles;
+  int grp_rows_b;           // weight rows per expert (n columns)
+  int n_tiles;              // units per list entry; the last one is sub_width wide if that covers its columns
 };
 
 struct Unit {
-  int m0, n0, width;
-  bool live;     // a narrow unit of a ragged last tile can lie past the last column
+  int m0, n0, width;      // first row, first column, columns
+  int b0;                 // first row of the weight matrix
+  int m_end;              // rows from here on are not stored
+  float alpha;
+  bool live;              // a narrow unit of a ragged last tile can lie past the last column
 };
-__device__ __forceinline__ Unit unit_at(const PairParams& p, int u) {
-  Unit x;
-  int t = u, sub = 0;
-  x.width = PAIR_N;
-  if (u >= p.full_units) {
-    const int per = PAIR_N / p.sub_width;
-    t = p.full_units + (u - p.full_units) / per;
-    sub = (u - p.full_units) % per;
-    x.width = p.sub_width;
+
+// The units of one cluster in order. In grouped mode a unit's place takes two dependent loads: the entry after the next and
+// the segment of the next one are under way while the current unit is worked on.
+template <bool GRP>
+struct UnitWalk {
+  const PairParams& p;
+  int u, stride, units;
+  int code_far = 0;                                   // list entry of unit u + 2 stride
+  int code_next = 0, start_next = 0, cnt_next = 0;    // entry, segment and scale of unit u + stride
+  float alpha_next = 0.f;
+  int code = 0, start = 0, cnt = 0;
+  float alpha = 0.f;
+
+  __device__ __forceinline__ UnitWalk(const PairParams& params, int cluster, int clusters) : p(params), u(cluster), stride(clusters) {
+    if constexpr (GRP) {
+      units = *p.grp_ntiles * p.n_tiles;
+      code_far = entry(u);
+      fetch();
+      code_far = entry(u + stride);
+      step();
+      code_far = entry(u + 2 * stride);
+    } else {
+      units = p.units;
+    }
   }
-  // rows fastest: the row tiles that read the same weights run side by side, so the weights leave HBM once
-  x.m0 = (t % p.m_tiles) * PAIR_M;
-  x.n0 = (t / p.m_tiles) * PAIR_N + sub * x.width;
-  x.live = x.n0 < p.n;
-  return x;
-}
+  __device__ __forceinline__ int entry(int unit) const { return unit < units ? p.grp_tiles[unit / p.n_tiles] : 0; }
+  __device__ __forceinline__ void fetch() {
+    code_next = code_far;
+    start_next = p.grp_start[code_next >> 12];
+    cnt_next = p.grp_cnt[code_next >> 12];
+    alpha_next = p.alpha_ptr != nullptr ? p.alpha_ptr[code_next >> 12] : 1.f;
+  }
+  __device__ __forceinline__ void step() {
+    code = code_next; start = start_next; cnt = cnt_next; alpha = alpha_next;
+    fetch();
+  }
+  __device__ __forceinline__ bool more() const { return u < units; }
+  __device__ __forceinline__ void next() {
+    u += stride;
+    if constexpr (GRP) {
+      step();
+      code_far = entry(u + 2 * stride);
+    }
+  }
+  __device__ __forceinline__ int width() const {
+    if constexpr (GRP) return u % p.n_tiles == p.n_tiles - 1 ? p.sub_width : PAIR_N;
+    return u >= p.full_units ? p.sub_width : PAIR_N;
+  }
+  __device__ __forceinline__ Unit unit() const {
+    Unit x;
+    x.width = width();
+    if constexpr (GRP) {
+      x.m0 = start + (code & 4095) * PAIR_M;
+      x.n0 = (u % p.n_tiles) * PAIR_N;
+      x.b0 = (code >> 12) * p.grp_rows_b + x.n0;
+      x.m_end = start + cnt;
+      x.alpha = p.alpha * alpha;
+      x.live = true;
+    } else {
+      int t = u, sub = 0;
+      if (u >= p.full_units) {
+        const int per = PAIR_N / p.sub_width;
+        t = p.full_units + (u - p.full_units) / per;
+        sub = (u - p.full_units) % per;
+      }
+      // rows fastest: the row tiles that read the same weights run side by side, so the weights leave HBM once
+      x.m0 = (t % p.m_tiles) * PAIR_M;
+      x.n0 = (t / p.m_tiles) * PAIR_N + sub * x.width;
+      x.b0 = x.n0;
+      x.m_end = p.m;
+      x.alpha = 0.f;      // one scale for all units: read once by the epilogue
+      x.live = x.n0 < p.n;
+    }
+    return x;
+  }
+};
 
 // ---- the cta_group::2 forms of the wrappers in hb_common.cuh
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {   // one whole warp of each CTA
@@ -129,116 +205,132 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
 
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 
-// One epilogue warp's 32 rows of a unit. `acc` is the accumulator's address for the warp's lanes, `release` the leader's
-// acc_free barrier. Steps of 64 columns; the first step covers the columns the two accumulators share.
+// One epilogue warp's part of a unit: 32 rows x half of its columns, in steps of 32 columns (one tcgen05.ld), two steps in
+// registers at a time. `acc` is the accumulator's address for the warp's lanes, `release` the leader's acc_free barrier.
+// The columns that the two accumulators share come first: the last ones of the first, the first ones of the second.
 template <int EPI>
-__device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x, int buf, uint32_t acc, int row0,
+__device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x, int buf, int half, uint32_t acc, int row0,
                                               uint8_t* staging, float alpha, float q_inv_gs, uint32_t release, int lane) {
-  const int steps = x.width / 64;
-  uint8_t* my_row = staging + lane * (EPI == kEpiSiluMulQuant ? Q_PITCH : ROW_PITCH);
+  const int steps = x.width / 64, groups = (steps + 1) / 2;
+  const int col0 = half * (x.width / 2);            // first column of this half, within the unit
+  uint8_t* my_row = staging + lane * ROW_PITCH;
+  const int row = row0 + lane;
 #pragma unroll 1
-  for (int j = 0; j < steps; ++j) {
-    const int s = buf == 0 ? steps - 1 - j : j;
+  for (int j = 0; j < groups; ++j) {
+    const int s0 = 2 * (buf == 0 ? groups - 1 - j : j);
     uint32_t r[2][32];
-    tmem_ld_32x32(acc + s * 64, r[0]);
-    tmem_ld_32x32(acc + s * 64 + 32, r[1]);
+    tmem_ld_32x32(acc + col0 + s0 * 32, r[0]);
+    if (s0 + 1 < steps) tmem_ld_32x32(acc + col0 + s0 * 32 + 32, r[1]);
     tmem_ld_wait();
     if (j == 0) {
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(release);
     }
-    if constexpr (EPI == kEpiSiluMulQuant) {
-      // 32 accumulator columns are 16 gate / up pairs: one 16-feature NVFP4 group of the thread's token. Same
-      // arithmetic in the same order as the stand-alone quantiser.
-      uint2 packed[2];
-      uint32_t sf[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < 2; ++h) {
+      const int s = s0 + h;
+      if (s >= steps) break;
+      const int c = x.n0 + col0 + s * 32;           // first column of the step
+      if constexpr (EPI == kEpiSiluMulQuant) {
+        // 32 accumulator columns are 16 gate / up pairs: one 16-feature NVFP4 group of the thread's token. Same
+        // arithmetic in the same order as the stand-alone quantiser.
         float y[16];
 #pragma unroll
         for (int t = 0; t < 16; ++t)
           y[t] = __bfloat162float(__float2bfloat16(silu_fast(__uint_as_float(r[h][2 * t]) * alpha) *
                                                    (__uint_as_float(r[h][2 * t + 1]) * alpha)));
-        sf[h] = quant16(y, q_inv_gs, &packed[h]);
-      }
-      *reinterpret_cast<uint4*>(my_row + s * 16) = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
-      *reinterpret_cast<uint16_t*>(my_row + 64 + s * 2) = static_cast<uint16_t>(sf[0] | (sf[1] << 8));
-    } else if constexpr (EPI == kEpiSiluMul) {
+        my_row[64 + s] = static_cast<uint8_t>(quant16(y, q_inv_gs, reinterpret_cast<uint2*>(my_row + s * 8)));
+      } else if constexpr (EPI == kEpiRelu2Quant) {
+        // two groups: squared ReLU, rounded as a bf16 store would, then the same quantiser
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t w[8];
+        for (int g = 0; g < 2; ++g) {
+          float y[16];
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
-          w[t] = pack_bf16(
-              silu_fast(__uint_as_float(r[h][4 * t]) * alpha) * (__uint_as_float(r[h][4 * t + 1]) * alpha),
-              silu_fast(__uint_as_float(r[h][4 * t + 2]) * alpha) * (__uint_as_float(r[h][4 * t + 3]) * alpha));
-        *reinterpret_cast<uint4*>(my_row + h * 32) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(my_row + h * 32 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-      }
-    } else {
+          for (int t = 0; t < 16; ++t) {
+            const float v = __uint_as_float(r[h][g * 16 + t]) * alpha;
+            y[t] = __bfloat162float(__float2bfloat16(v > 0.f ? v * v : 0.f));
+          }
+          my_row[64 + 2 * s + g] =
+              static_cast<uint8_t>(quant16(y, q_inv_gs, reinterpret_cast<uint2*>(my_row + s * 16 + g * 8)));
+        }
+      } else {
+        // bf16 rows through shared memory: whole 16-byte chunks, consecutive lanes along a row
+        constexpr int CHUNKS = EPI == kEpiSiluMul ? 2 : 4;
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < CHUNKS; ++t) {
           uint32_t w[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            w[i] = pack_bf16(__uint_as_float(r[h][8 * t + 2 * i]) * alpha, __uint_as_float(r[h][8 * t + 2 * i + 1]) * alpha);
-          *reinterpret_cast<uint4*>(my_row + h * 64 + t * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-    }
-    if constexpr (EPI != kEpiSiluMulQuant) {
-      // whole 16-byte chunks, consecutive lanes along a row: 128 (64 with SiLU-mul) contiguous bytes per row
-      constexpr int CHUNKS = EPI == kEpiSiluMul ? 4 : 8;
-      const int col0 = EPI == kEpiSiluMul ? (x.n0 >> 1) + s * 32 : x.n0 + s * 64;
-      const int col_end = EPI == kEpiSiluMul ? p.n >> 1 : p.n;
-      const int ch = lane % CHUNKS;
-      const int gcol = col0 + ch * 8;
-      __syncwarp();
-#pragma unroll
-      for (int r0 = 0; r0 < 32; r0 += 32 / CHUNKS) {
-        const int lr = r0 + lane / CHUNKS;
-        const int grow = row0 + lr;
-        if (grow < p.m && gcol + 8 <= col_end) {
-          uint4 v = *reinterpret_cast<const uint4*>(staging + lr * ROW_PITCH + ch * 16);
-          const long long o = static_cast<long long>(grow) * p.ldo + gcol;
-          if constexpr (EPI == kEpiResidual) {
-            const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + o);
-            v.x = pack_bf16(bf16_lo(v.x) + bf16_lo(rr.x), bf16_hi(v.x) + bf16_hi(rr.x));
-            v.y = pack_bf16(bf16_lo(v.y) + bf16_lo(rr.y), bf16_hi(v.y) + bf16_hi(rr.y));
-            v.z = pack_bf16(bf16_lo(v.z) + bf16_lo(rr.z), bf16_hi(v.z) + bf16_hi(rr.z));
-            v.w = pack_bf16(bf16_lo(v.w) + bf16_lo(rr.w), bf16_hi(v.w) + bf16_hi(rr.w));
+          for (int i = 0; i < 4; ++i) {
+            if constexpr (EPI == kEpiSiluMul) {
+              const int e = 16 * t + 4 * i;
+              w[i] = pack_bf16(silu_fast(__uint_as_float(r[h][e]) * alpha) * (__uint_as_float(r[h][e + 1]) * alpha),
+                               silu_fast(__uint_as_float(r[h][e + 2]) * alpha) * (__uint_as_float(r[h][e + 3]) * alpha));
+            } else {
+              w[i] = pack_bf16(__uint_as_float(r[h][8 * t + 2 * i]) * alpha, __uint_as_float(r[h][8 * t + 2 * i + 1]) * alpha);
+            }
           }
-          *reinterpret_cast<uint4*>(p.out + o) = v;
+          *reinterpret_cast<uint4*>(my_row + t * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        const int col_end = EPI == kEpiSiluMul ? p.n >> 1 : p.n;
+        const int ch = lane % CHUNKS;
+        const int gcol = (EPI == kEpiSiluMul ? c >> 1 : c) + ch * 8;
+        __syncwarp();
+#pragma unroll
+        for (int r0 = 0; r0 < 32; r0 += 32 / CHUNKS) {
+          const int lr = r0 + lane / CHUNKS;
+          const int grow = row0 + lr;
+          if (grow < x.m_end && gcol + 8 <= col_end) {
+            uint4 v = *reinterpret_cast<const uint4*>(staging + lr * ROW_PITCH + ch * 16);
+            const long long o = static_cast<long long>(grow) * p.ldo + gcol;
+            if constexpr (EPI == kEpiResidual) {
+              const uint4 rr = *reinterpret_cast<const uint4*>(p.residual + o);
+              v.x = pack_bf16(bf16_lo(v.x) + bf16_lo(rr.x), bf16_hi(v.x) + bf16_hi(rr.x));
+              v.y = pack_bf16(bf16_lo(v.y) + bf16_lo(rr.y), bf16_hi(v.y) + bf16_hi(rr.y));
+              v.z = pack_bf16(bf16_lo(v.z) + bf16_lo(rr.z), bf16_hi(v.z) + bf16_hi(rr.z));
+              v.w = pack_bf16(bf16_lo(v.w) + bf16_lo(rr.w), bf16_hi(v.w) + bf16_hi(rr.w));
+            }
+            *reinterpret_cast<uint4*>(p.out + o) = v;
+          }
+        }
+        __syncwarp();
       }
-      __syncwarp();
     }
   }
-  if constexpr (EPI == kEpiSiluMulQuant) {
+  if constexpr (EPI == kEpiSiluMulQuant || EPI == kEpiRelu2Quant) {
+    // Packed bytes of the half: consecutive lanes along a row, 8 bytes per group (SiLU-mul: a step is one group, else two).
+    // The feature count is a multiple of 64, so a step's groups are in range together.
+    constexpr int GROUPS = EPI == kEpiSiluMulQuant ? 1 : 2;
+    constexpr int SHIFT = EPI == kEpiSiluMulQuant ? 5 : 4;      // columns per group, log2
+    const int c_half = x.n0 + col0;
+    const int ng = steps * GROUPS;                              // 8, 4, 2 or 1
+    const int g = lane % ng;
     __syncwarp();
-    // packed bytes: width / 4 per row, 16-byte chunks of two groups (the feature count is a multiple of 64)
-    const int rows_per = 32 / steps;
-    const int ch = lane % steps;
-    for (int r0 = 0; r0 < 32; r0 += rows_per) {
-      const int lr = r0 + lane / steps;
+    for (int r0 = 0; r0 < 32; r0 += 32 / ng) {
+      const int lr = r0 + lane / ng;
       const int grow = row0 + lr;
-      if (grow < p.m && x.n0 + ch * 64 + 64 <= p.n)
-        *reinterpret_cast<uint4*>(p.q_out + static_cast<size_t>(grow) * p.q_ld + (x.n0 >> 2) + ch * 16) =
-            *reinterpret_cast<const uint4*>(staging + lr * Q_PITCH + ch * 16);
+      if (grow < x.m_end && c_half + ((g + 1) << SHIFT) <= p.n)
+        *reinterpret_cast<uint2*>(p.q_out + static_cast<size_t>(grow) * p.q_ld + (c_half >> SHIFT) * 8 + g * 8) =
+            *reinterpret_cast<const uint2*>(staging + lr * ROW_PITCH + g * 8);
     }
-    if (row0 + lane < p.m) {
-      for (int g2 = 0; g2 < steps; ++g2)
-        if (x.n0 + g2 * 64 + 64 <= p.n)
-          *reinterpret_cast<uint16_t*>(p.q_sf + row_sf_off(row0 + lane, (x.n0 >> 5) + 2 * g2, p.q_ka)) =
-              *reinterpret_cast<const uint16_t*>(my_row + 64 + 2 * g2);
+    if (row < x.m_end) {
+      const int g0 = c_half >> SHIFT;
+      if (ng >= 4 && c_half + (ng << SHIFT) <= p.n) {           // four groups of a K atom are one aligned word
+        for (int w = 0; w < ng; w += 4)
+          *reinterpret_cast<uint32_t*>(p.q_sf + row_sf_off(row, g0 + w, p.q_ka)) =
+              *reinterpret_cast<const uint32_t*>(my_row + 64 + w);
+      } else {
+        for (int w = 0; w < ng; ++w)
+          if (c_half + ((w + 1) << SHIFT) <= p.n) p.q_sf[row_sf_off(row, g0 + w, p.q_ka)] = my_row[64 + w];
+      }
+      if (half == 1 && x.n0 + x.width >= p.n)      // groups that pad the last K tile of the next GEMM read as zero
+        for (int w = p.n >> SHIFT; w < p.q_ka * 4; ++w) p.q_sf[row_sf_off(row, w, p.q_ka)] = 0;
     }
     __syncwarp();
   }
 }
 
-template <int EPI>
+template <int EPI, bool GRP>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
                  const __grid_constant__ CUtensorMap tb_sub, const __grid_constant__ CUtensorMap tsfa,
@@ -249,7 +341,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
   uint64_t* full = reinterpret_cast<uint64_t*>(staging + STAGING_BYTES);   // the leader's count both CTAs' bytes
   uint64_t* empty = full + STAGES;
   uint64_t* accum = empty + STAGES;     // [2] accumulator complete (both CTAs)
-  uint64_t* acc_free = accum + 2;       // leader: the shared columns of the last unit have been read (8 warps)
+  uint64_t* acc_free = accum + 2;       // leader: the shared columns of the last unit have been read (both CTAs' warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -265,7 +357,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
     }
     mbar_init(&accum[0], 1);
     mbar_init(&accum[1], 1);
-    mbar_init(acc_free, 8);
+    mbar_init(acc_free, 2 * EPI_WARPS);
     *abort = 0;
     fence_mbar_init();
     prefetch_tmap(&ta);
@@ -294,18 +386,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
     auto side_b = [&](const Unit& x, int kt, int s) {
       const uint32_t st = smem_base + s * STAGE_BYTES;
       tma_load_2d_pair(st + A_BYTES, x.width == PAIR_N ? &tb : &tb_sub, full0 + s * 8, kt * 128,
-                       x.n0 + static_cast<int>(rank) * (x.width >> 1));
-      tma_load_2d_pair(st + A_BYTES + B_BYTES + SFA_BYTES, &tsfb, full0 + s * 8, kt * 256, x.n0 >> 7);
+                       x.b0 + static_cast<int>(rank) * (x.width >> 1));
+      tma_load_2d_pair(st + A_BYTES + B_BYTES + SFA_BYTES, &tsfb, full0 + s * 8, kt * 256, x.b0 >> 7);
     };
     auto tx_bytes = [](const Unit& x) {
       return 2u * (A_BYTES + SFA_BYTES + SFB_BYTES + static_cast<uint32_t>(x.width) * 64u);
     };
     // The first ring of stages: weights first (they depend on nothing), then the wait for the kernel that produces
     // the activations, then the activations.
+    // (In grouped mode the unit itself comes from the plan's kernels, so all of it waits.)
     int pre = 0;
-    {
-      const Unit x = unit_at(p, cluster);
-      if (cluster < p.units && x.live) pre = min(STAGES, p.k_tiles);
+    if constexpr (!GRP) {
+      const UnitWalk<false> w(p, cluster, clusters);
+      const Unit x = w.unit();
+      if (w.more() && x.live) pre = min(STAGES, p.k_tiles);
       if (elect_one())
         for (int kt = 0; kt < pre; ++kt) {
           if (rank == 0) mbar_expect_tx(&full[kt], tx_bytes(x));
@@ -316,11 +410,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
       if (elect_one())
         for (int kt = 0; kt < pre; ++kt) side_a(x, kt, kt);
       __syncwarp();
+    } else {
+      grid_dep_wait();
     }
     bool ok = true;
-    for (int u = cluster; u < p.units && ok; u += clusters) {
-      const Unit x = unit_at(p, u);
+    for (UnitWalk<GRP> w(p, cluster, clusters); w.more() && ok; w.next()) {
+      Unit x = w.unit();
       if (!x.live) continue;
+      if constexpr (GRP) {
+        x.m0 = __shfl_sync(0xffffffffu, x.m0, 0);
+        x.b0 = __shfl_sync(0xffffffffu, x.b0, 0);
+      }
       for (int kt = 0; kt < p.k_tiles; ++kt, ++i) {
         if (i < pre) continue;
         const int s = i % STAGES;
@@ -347,13 +447,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
       const uint32_t sfa_t = tmem_base + SFA_COL, sfb_t = tmem_base + SFB_COL;
       int i = 0, it = 0;
       bool ok = true;
-      for (int u = cluster; u < p.units && ok; u += clusters) {
-        const Unit x = unit_at(p, u);
-        if (!x.live) continue;
-        const uint32_t idesc = make_idesc_nvf4(PAIR_M, PAIR_N) -
-                               (static_cast<uint32_t>((PAIR_N - x.width) >> 3) << 17);
+      // (of a grouped unit this warp needs no more than its width, which is not in the work list)
+      int units = p.units;
+      if constexpr (GRP) {
+        grid_dep_wait();
+        units = __shfl_sync(0xffffffffu, *p.grp_ntiles, 0) * p.n_tiles;
+      }
+      for (int u = cluster; u < units && ok; u += clusters) {
+        int width = PAIR_N, n0 = 0;
+        if constexpr (GRP) {
+          if (u % p.n_tiles == p.n_tiles - 1) width = p.sub_width;
+        } else {
+          UnitWalk<false> w(p, u, clusters);
+          const Unit x = w.unit();
+          if (!x.live) continue;
+          width = x.width;
+          n0 = x.n0;
+        }
+        const uint32_t idesc = make_idesc_nvf4(PAIR_M, PAIR_N) - (static_cast<uint32_t>((PAIR_N - width) >> 3) << 17);
         const uint32_t acc = tmem_base + ((it & 1) ? ACC1_COL : 0);
-        const uint32_t sfb_u = sfb_t + ((x.n0 & 64) ? 2 : 0);    // a 64-column unit in the upper half of a block
+        const uint32_t sfb_u = sfb_t + ((n0 & 64) ? 2 : 0);      // a 64-column unit in the upper half of a block
         if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_free, (it - 1) & 1, abort, p.status, kTimeoutAccum));
         if (!ok) break;
         tc_fence_after();
@@ -390,18 +503,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
     const int q = warp & 3;      // TMEM lane quarter this warp may read
     const uint32_t tlane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t release = map_to_cta(smem_u32(acc_free), 0);
-    uint8_t* mine = staging + q * 32 * ROW_PITCH;
+    const int half = (warp - 2) >> 2;
+    uint8_t* mine = staging + (warp - 2) * 32 * ROW_PITCH;
     float alpha = p.alpha;
-    if (p.alpha_ptr != nullptr) alpha *= *p.alpha_ptr;
-    const float q_inv_gs = EPI == kEpiSiluMulQuant ? 1.f / *p.q_gscale : 0.f;
+    if (!GRP && p.alpha_ptr != nullptr) alpha *= *p.alpha_ptr;
+    const float q_inv_gs = EPI == kEpiSiluMulQuant || EPI == kEpiRelu2Quant ? 1.f / *p.q_gscale : 0.f;
     int it = 0;
-    for (int u = cluster; u < p.units; u += clusters) {
-      const Unit x = unit_at(p, u);
+    for (UnitWalk<GRP> w(p, cluster, clusters); w.more(); w.next()) {
+      const Unit x = w.unit();
       if (!x.live) continue;
+      if constexpr (GRP) alpha = x.alpha;
       const int buf = it & 1;
       if (!mbar_wait(&accum[buf], (it >> 1) & 1, abort, p.status, kTimeoutAccum)) break;
       tc_fence_after();
-      epilogue_unit<EPI>(p, x, buf, tlane + (buf ? ACC1_COL : 0), x.m0 + static_cast<int>(rank) * 128 + q * 32, mine,
+      epilogue_unit<EPI>(p, x, buf, half, tlane + (buf ? ACC1_COL : 0), x.m0 + static_cast<int>(rank) * 128 + q * 32, mine,
                          alpha, q_inv_gs, release, lane);
       ++it;
     }
@@ -413,7 +528,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int EPI>
+template <int EPI, bool GRP>
 cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_sub, const CUtensorMap& tsfa,
                    const CUtensorMap& tsfb, const PairParams& p, int clusters, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -428,13 +543,13 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = hb_gemm_get_pdl() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI>, ta, tb, tb_sub, tsfa, tsfb, p);
+  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, GRP>, ta, tb, tb_sub, tsfa, tsfb, p);
 }
 
 // Clusters of two that the device holds at once (0 = the kernels could not be set up).
-template <int EPI>
+template <int EPI, bool GRP>
 int resident_clusters() {
-  if (cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+  if (cudaFuncSetAttribute(gemm_pair_kernel<EPI, GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
     return 0;
   cudaLaunchConfig_t q = {};
   q.gridDim = dim3(2);
@@ -446,7 +561,7 @@ int resident_clusters() {
   q.attrs = at;
   q.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<EPI>, &q) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<EPI, GRP>, &q) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
@@ -456,50 +571,75 @@ int resident_clusters() {
 }  // namespace
 
 bool gemm_pair_ok(const GemmArgs& a) {
-  if (a.kind != kGemmNvfp4 || a.swap || a.peer != nullptr || a.grp_cnt != nullptr || a.tok_scale != nullptr ||
-      a.splits > 1 || a.bn != 256)
+  if (a.kind != kGemmNvfp4 || a.peer != nullptr || a.ep != nullptr || a.tok_scale != nullptr || a.bn != 256) return false;
+  const bool grouped = a.grp_cnt != nullptr;
+  if (grouped) {
+    if (!a.swap || a.grp_tiles == nullptr || a.grp_rows_a % 128 != 0) return false;
+  } else if (a.swap || a.splits > 1) {
     return false;
+  }
   if (a.epilogue == kEpiSiluMulQuant) return true;      // gemm_launch has checked its layout
-  if (a.epilogue != kEpiStore && a.epilogue != kEpiResidual && a.epilogue != kEpiSiluMul) return false;
+  if (a.epilogue == kEpiRelu2Quant) return grouped;
+  if (a.epilogue != kEpiStore && (grouped || (a.epilogue != kEpiResidual && a.epilogue != kEpiSiluMul))) return false;
   // 16-byte output chunks
   const int cols = a.epilogue == kEpiSiluMul ? 16 : 8;
-  return a.rb % cols == 0 && a.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
+  return (grouped ? a.grp_rows_a : a.rb) % cols == 0 && a.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(a.residual) & 15) == 0;
 }
 
 cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
   static const int resident = [] {
-    int n = resident_clusters<kEpiStore>();
-    n = std::min(n, resident_clusters<kEpiResidual>());
-    n = std::min(n, resident_clusters<kEpiSiluMul>());
-    return std::min(n, resident_clusters<kEpiSiluMulQuant>());
+    int n = resident_clusters<kEpiStore, false>();
+    n = std::min(n, resident_clusters<kEpiResidual, false>());
+    n = std::min(n, resident_clusters<kEpiSiluMul, false>());
+    n = std::min(n, resident_clusters<kEpiSiluMulQuant, false>());
+    n = std::min(n, resident_clusters<kEpiStore, true>());
+    n = std::min(n, resident_clusters<kEpiRelu2Quant, true>());
+    return std::min(n, resident_clusters<kEpiSiluMulQuant, true>());
   }();
   if (resident < 1) return cudaErrorInvalidConfiguration;
+  const bool grouped = a.grp_cnt != nullptr;
+  // tokens are the A side here; a grouped call names its weights first
+  const void *act = grouped ? a.b : a.a, *act_sf = grouped ? a.sfb : a.sfa;
+  const void *wgt = grouped ? a.a : a.b, *wgt_sf = grouped ? a.sfa : a.sfb;
+  const int rows = grouped ? a.rb : a.ra, wgt_rows = grouped ? a.ra : a.rb;
+  const int act_ka = grouped ? a.sf_k_atoms_b : a.sf_k_atoms_a, wgt_ka = grouped ? a.sf_k_atoms_a : a.sf_k_atoms_b;
+  const int64_t act_ld = grouped ? a.ldb : a.lda, wgt_ld = grouped ? a.lda : a.ldb;
   PairParams p;
-  p.m = a.ra; p.n = a.rb; p.k_tiles = (a.k + 255) / 256;
-  p.m_tiles = (a.ra + PAIR_M - 1) / PAIR_M;
-  const int n_tiles = (a.rb + PAIR_N - 1) / PAIR_N;
-  const int tiles = p.m_tiles * n_tiles;
-  // Width of the units that the last, partial wave of full tiles is cut into: the one with the shortest estimate. A K tile
-  // of a wave costs the larger of the MMAs (0.28 us at 256 columns) and of the bytes the wave's clusters fetch through L2,
-  // which delivers 12.5 TB/s to all SMs together (measured; a full wave of 256-column units is bound by it): 22 KB plus
-  // 64 bytes per column and CTA. Narrow units spread a few tiles over idle SMs but fetch the A rows again.
-  const int rem = tiles % resident;
-  p.sub_width = PAIR_N;
-  double best = 1e30;
-  for (int w = PAIR_N; w >= 64 && rem != 0; w /= 2) {
-    double t = 0;
-    for (int left = rem * (PAIR_N / w); left > 0; left -= resident) {
-      const int live = std::min(left, resident);
-      t += std::max(0.28 * w / PAIR_N, 2.0 * live * (22528 + 64 * w) / 12.5e6) + 0.01;
+  p.m = rows; p.n = grouped ? a.grp_rows_a : a.rb; p.k_tiles = (a.k + 255) / 256;
+  p.m_tiles = (rows + PAIR_M - 1) / PAIR_M;
+  p.n_tiles = (p.n + PAIR_N - 1) / PAIR_N;
+  int clusters;
+  if (grouped) {
+    const int last = p.n - (p.n_tiles - 1) * PAIR_N;      // a multiple of 128
+    p.sub_width = last <= 128 ? 128 : PAIR_N;
+    p.full_units = p.units = 0;                           // the list's length is on the device
+    clusters = resident;
+  } else {
+    const int tiles = p.m_tiles * p.n_tiles;
+    // Width of the units that the last, partial wave of full tiles is cut into: the one with the shortest estimate. A K
+    // tile of a wave costs the larger of the MMAs (0.28 us at 256 columns) and of the bytes the wave's clusters fetch
+    // through L2, which delivers 12.5 TB/s to all SMs together (measured; a full wave of 256-column units is bound by
+    // it): 22 KB plus 64 bytes per column and CTA. Narrow units spread a few tiles over idle SMs but fetch the A rows
+    // again.
+    const int rem = tiles % resident;
+    p.sub_width = PAIR_N;
+    double best = 1e30;
+    for (int w = PAIR_N; w >= 64 && rem != 0; w /= 2) {
+      double t = 0;
+      for (int left = rem * (PAIR_N / w); left > 0; left -= resident) {
+        const int live = std::min(left, resident);
+        t += std::max(0.28 * w / PAIR_N, 2.0 * live * (22528 + 64 * w) / 12.5e6) + 0.01;
+      }
+      if (t < best * 0.97) {
+        best = t;
+        p.sub_width = w;
+      }
     }
-    if (t < best * 0.97) {
-      best = t;
-      p.sub_width = w;
-    }
+    p.full_units = p.sub_width == PAIR_N ? tiles : tiles - rem;
+    p.units = p.full_units + (tiles - p.full_units) * (PAIR_N / p.sub_width);
+    clusters = std::min(resident, p.units);
   }
-  p.full_units = p.sub_width == PAIR_N ? tiles : tiles - rem;
-  p.units = p.full_units + (tiles - p.full_units) * (PAIR_N / p.sub_width);
   p.out = static_cast<__nv_bfloat16*>(a.out); p.ldo = a.ldo;
   p.residual = static_cast<const __nv_bfloat16*>(a.residual);
   p.alpha = a.alpha; p.alpha_ptr = a.alpha_ptr;
@@ -507,28 +647,33 @@ cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
   p.q_out = static_cast<uint8_t*>(a.q_out); p.q_sf = static_cast<uint8_t*>(a.q_sf); p.q_gscale = a.q_gscale;
   p.q_ka = a.q_ka; p.q_ld = a.q_ld;
   p.status = a.status;
+  p.grp_start = a.grp_start; p.grp_cnt = a.grp_cnt; p.grp_tiles = a.grp_tiles; p.grp_ntiles = a.grp_ntiles;
+  p.grp_rows_b = a.grp_rows_a;
 
   const uint64_t cols = static_cast<uint64_t>(a.k / 2);
   const uint32_t sub_rows = static_cast<uint32_t>(p.sub_width / 2);
-  const TmapKey ka{a.a, static_cast<uint64_t>(a.ra), cols, static_cast<uint64_t>(a.lda / 2), 128, 128, 1};
-  const TmapKey kb{a.b, static_cast<uint64_t>(a.rb), cols, static_cast<uint64_t>(a.ldb / 2), 128, 128, 1};
-  const TmapKey kb_sub{a.b, static_cast<uint64_t>(a.rb), cols, static_cast<uint64_t>(a.ldb / 2), sub_rows, 128, 1};
+  const uint64_t pitch_a = static_cast<uint64_t>(act_ld / 2), pitch_b = static_cast<uint64_t>(wgt_ld / 2);
+  const TmapKey ka{act, static_cast<uint64_t>(rows), cols, pitch_a, 128, 128, 1};
+  const TmapKey kb{wgt, static_cast<uint64_t>(wgt_rows), cols, pitch_b, 128, 128, 1};
+  const TmapKey kb_sub{wgt, static_cast<uint64_t>(wgt_rows), cols, pitch_b, sub_rows, 128, 1};
   // scale factors as rows of 128-row blocks: 64 8-byte words per K atom
-  const uint64_t pa = static_cast<uint64_t>(a.sf_k_atoms_a) * 512, pb = static_cast<uint64_t>(a.sf_k_atoms_b) * 512;
-  const TmapKey ksa{a.sfa, static_cast<uint64_t>((a.ra + 127) / 128), pa / 8, pa, 1, 256, 2};
-  const TmapKey ksb{a.sfb, static_cast<uint64_t>((a.rb + 127) / 128), pb / 8, pb, 2, 256, 2};
+  const uint64_t pa = static_cast<uint64_t>(act_ka) * 512, pb = static_cast<uint64_t>(wgt_ka) * 512;
+  const TmapKey ksa{act_sf, static_cast<uint64_t>((rows + 127) / 128), pa / 8, pa, 1, 256, 2};
+  const TmapKey ksb{wgt_sf, static_cast<uint64_t>((wgt_rows + 127) / 128), pb / 8, pb, 2, 256, 2};
   CUtensorMap ta, tb, tb_sub, tsfa, tsfb;
   if (!get_tmap_2d(ka, &ta) || !get_tmap_2d(kb, &tb) || !get_tmap_2d(kb_sub, &tb_sub) || !get_tmap_2d(ksa, &tsfa) ||
       !get_tmap_2d(ksb, &tsfb))
     return cudaErrorInvalidValue;
-  const int clusters = std::min(resident, p.units);
+#define HB_PAIR(EPI, GRP) launch<EPI, GRP>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream)
   switch (a.epilogue) {
-    case kEpiStore: return launch<kEpiStore>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream);
-    case kEpiResidual: return launch<kEpiResidual>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream);
-    case kEpiSiluMul: return launch<kEpiSiluMul>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream);
-    case kEpiSiluMulQuant: return launch<kEpiSiluMulQuant>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream);
+    case kEpiStore: return grouped ? HB_PAIR(kEpiStore, true) : HB_PAIR(kEpiStore, false);
+    case kEpiResidual: return HB_PAIR(kEpiResidual, false);
+    case kEpiSiluMul: return HB_PAIR(kEpiSiluMul, false);
+    case kEpiSiluMulQuant: return grouped ? HB_PAIR(kEpiSiluMulQuant, true) : HB_PAIR(kEpiSiluMulQuant, false);
+    case kEpiRelu2Quant: return HB_PAIR(kEpiRelu2Quant, true);
     default: return cudaErrorInvalidValue;
   }
+#undef HB_PAIR
 }
 
 }  // namespace hb

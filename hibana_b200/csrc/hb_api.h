@@ -29,6 +29,10 @@ int hb_gemm_grouped(int kind, const void* a, const void* b, const void* sfa, con
                     int n_per_expert, int b_rows, int k, void* out, long long ldo, const void* alpha_ptr,
                     int epilogue, const void* start, const void* cnt, int max_rows_per_expert, void* status, int ka_a,
                     int ka_b, int bn_hint, const void* tiles, const void* n_tiles, int tile_cap, void* stream);
+int hb_gemm_grouped_quant(const void* a, const void* b, const void* sfa, const void* sfb, int experts, int n_per_expert,
+                          int b_rows, int k, const void* alpha_ptr, int epilogue, const void* start, const void* cnt,
+                          void* status, int ka_a, int ka_b, const void* tiles, const void* n_tiles, int tile_cap,
+                          void* q_out, void* q_sf, const void* q_gscale, int q_ka, long long q_ld, void* stream);
 int hb_gemm_peer(int kind, const void* a, const void* b, const void* sfa, const void* sfb, int m, int n, int k,
                  void* out, long long ldo, const void* alpha_ptr, int epilogue, const void* const* peer_bases,
                  int world, int rank, int rows_per_rank, long long stage_offset, long long counter_offset,

@@ -25,6 +25,7 @@ nv.register("hb_moe_plan", [P, I, I, I, I, I, I, P, P, P, P, I, P, I, P, P, I, P
 nv.register("hb_moe_gather", [P, L, P, P, P, I, I, P])
 nv.register("hb_moe_combine", [P, L, P, P, P, L, P, L, I, I, I, P])
 nv.register("hb_gemm_grouped", [I, P, P, P, P, I, I, I, I, P, L, P, I, P, P, I, P, I, I, I, P, P, I, P])
+nv.register("hb_gemm_grouped_quant", [P, P, P, P, I, I, I, I, P, I, P, P, P, I, I, P, P, I, P, P, P, I, L, P])
 nv.register("hb_quant_nvfp4_rows", [P, L, I, I, I, P, P, P, I, P, P, P])
 
 
@@ -283,6 +284,13 @@ def tile_hint(pairs: int, experts: int, max_rows: int, fmt: str) -> int:
     return bn
 
 
+def pair_rows(ew: "ExpertWeights", max_rows: int) -> bool:
+    """Whether the grouped GEMMs run on SM pairs over 256-row chunks (csrc/gemm_pair.cu): NVFP4 experts as soon as a chunk
+    would otherwise be a 128-token tile, in geometries whose activation can be requantised in fc1's epilogue."""
+    return (ew.fmt == "nvfp4" and max_rows > 128 and ew.act in ("swiglu", "relu2") and ew.inter % 64 == 0
+            and ew.n1 % 128 == 0 and ew.fc2_rows % 128 == 0)
+
+
 def experts_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ew: ExpertWeights, *,
                     shared: Optional[torch.Tensor] = None, e_lo: int = 0, e_n: Optional[int] = None,
                     id_base: int = 0) -> torch.Tensor:
@@ -304,6 +312,9 @@ def experts_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, e
     while bn_full < max_rows and bn_full < 256:
         bn_full *= 2
     bn_hint = min(bn_hint, bn_full)            # the tile width the grouped GEMMs will use
+    pairs = pair_rows(ew, max_rows)
+    if pairs:
+        bn_hint = 256
     # compact (expert, chunk) work list: the GEMM grids cover the tiles that have rows, not experts x worst case
     tile_cap = -(-(t * topk) // bn_hint) + min(e_n, t * topk)
     tiles = torch.empty(tile_cap, dtype=torch.int32, device=dev)
@@ -321,7 +332,7 @@ def experts_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, e
     n1, h_out = ew.n1, ew.fc2_rows
     epi1 = gemm.EPI_SILU_MUL if ew.act == "swiglu" else gemm.EPI_RELU2 if ew.act == "relu2" else gemm.EPI_STORE
     mid_cols = ew.inter
-    h1 = torch.empty(rows_cap, mid_cols if ew.act == "swiglu" else n1, dtype=torch.bfloat16, device=dev)
+    h1 = None if pairs else torch.empty(rows_cap, mid_cols if ew.act == "swiglu" else n1, dtype=torch.bfloat16, device=dev)
     y = torch.empty(rows_cap, h_out, dtype=torch.bfloat16, device=dev)
     if ew.fmt in ("bf16", "w3"):
         kind = 0 if ew.fmt == "bf16" else 3      # 3: dequant-fused 3-bit experts (csrc/gemm.cu kind w3, grouped)
@@ -348,20 +359,28 @@ def experts_forward(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, e
             nv.check(lib.hb_quant_nvfp4_rows(x.data_ptr(), x.stride(0), rows_cap, h, sf1.shape[1],
                                              ew.fc1_in_scale.data_ptr(), q1.data_ptr(), sf1.data_ptr(), 0,
                                              src.data_ptr(), total.data_ptr(), nv.stream()), "hb_quant_nvfp4_rows")
-        nv.check(lib.hb_gemm_grouped(1, ew.fc1.q.data_ptr(), q1.data_ptr(), ew.fc1.sf.data_ptr(), sf1.data_ptr(), e,
-                                     n1, rows_cap, h, h1.data_ptr(), h1.stride(0), ew.fc1_alpha.data_ptr(), epi1,
-                                     start.data_ptr(), cnt.data_ptr(), max_rows, st.data_ptr(), ew.fc1.ka,
-                                     sf1.shape[1], bn_hint, *tl, nv.stream()), "hb_gemm_grouped")
-        mid = h1                                # the activation (SwiGLU or squared ReLU) ran in the GEMM epilogue
         q2, sf2 = nvfp4._alloc(rows_cap, ew.inter, dev)
-        if by_pair:
-            nv.check(lib.hb_quant_nvfp4_pairs(mid.data_ptr(), mid.stride(0), pos.data_ptr(), t * topk, 0, ew.inter,
-                                              sf2.shape[1], ew.fc2_in_scale.data_ptr(), q2.data_ptr(),
-                                              sf2.data_ptr(), nv.stream()), "hb_quant_nvfp4_pairs")
+        if pairs:
+            epi = gemm.EPI_SILU_MUL_QUANT if ew.act == "swiglu" else gemm.EPI_RELU2_QUANT
+            nv.check(lib.hb_gemm_grouped_quant(ew.fc1.q.data_ptr(), q1.data_ptr(), ew.fc1.sf.data_ptr(), sf1.data_ptr(), e, n1,
+                                               rows_cap, h, ew.fc1_alpha.data_ptr(), epi, start.data_ptr(), cnt.data_ptr(),
+                                               st.data_ptr(), ew.fc1.ka, sf1.shape[1], *tl, q2.data_ptr(), sf2.data_ptr(),
+                                               ew.fc2_in_scale.data_ptr(), sf2.shape[1], ew.inter // 2, nv.stream()),
+                     "hb_gemm_grouped_quant")
         else:
-            nv.check(lib.hb_quant_nvfp4_rows(mid.data_ptr(), mid.stride(0), rows_cap, ew.inter, sf2.shape[1],
-                                             ew.fc2_in_scale.data_ptr(), q2.data_ptr(), sf2.data_ptr(), 0, None,
-                                             total.data_ptr(), nv.stream()), "hb_quant_nvfp4_rows")
+            nv.check(lib.hb_gemm_grouped(1, ew.fc1.q.data_ptr(), q1.data_ptr(), ew.fc1.sf.data_ptr(), sf1.data_ptr(), e,
+                                         n1, rows_cap, h, h1.data_ptr(), h1.stride(0), ew.fc1_alpha.data_ptr(), epi1,
+                                         start.data_ptr(), cnt.data_ptr(), max_rows, st.data_ptr(), ew.fc1.ka,
+                                         sf1.shape[1], bn_hint, *tl, nv.stream()), "hb_gemm_grouped")
+            mid = h1                                # the activation (SwiGLU or squared ReLU) ran in the GEMM epilogue
+            if by_pair:
+                nv.check(lib.hb_quant_nvfp4_pairs(mid.data_ptr(), mid.stride(0), pos.data_ptr(), t * topk, 0, ew.inter,
+                                                  sf2.shape[1], ew.fc2_in_scale.data_ptr(), q2.data_ptr(),
+                                                  sf2.data_ptr(), nv.stream()), "hb_quant_nvfp4_pairs")
+            else:
+                nv.check(lib.hb_quant_nvfp4_rows(mid.data_ptr(), mid.stride(0), rows_cap, ew.inter, sf2.shape[1],
+                                                 ew.fc2_in_scale.data_ptr(), q2.data_ptr(), sf2.data_ptr(), 0, None,
+                                                 total.data_ptr(), nv.stream()), "hb_quant_nvfp4_rows")
         nv.check(lib.hb_gemm_grouped(1, ew.fc2.q.data_ptr(), q2.data_ptr(), ew.fc2.sf.data_ptr(), sf2.data_ptr(), e,
                                      h_out, rows_cap, ew.inter, y.data_ptr(), y.stride(0), ew.fc2_alpha.data_ptr(),
                                      gemm.EPI_STORE, start.data_ptr(), cnt.data_ptr(), max_rows, st.data_ptr(),

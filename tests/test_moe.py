@@ -122,6 +122,32 @@ def test_expert_sharing_kernel_matches_reference():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("t,e,k,h,inter,act", [(129, 5, 2, 256, 384, "relu2"), (300, 40, 6, 512, 640, "relu2"),
+                                               (700, 3, 2, 256, 2688, "relu2"), (300, 16, 4, 128, 192, "swiglu"),
+                                               (1500, 64, 8, 1024, 704, "swiglu")])
+def test_experts_forward_on_sm_pairs(t, e, k, h, inter, act, monkeypatch):
+    """Chunks of 256 rows on SM pairs with the activation requantised in fc1's epilogue give the bytes of the one-CTA tiles
+    followed by the quantiser: the same sums in the same order (empty, partial and several chunks per expert, a last
+    weight tile of 128 rows, plans by one CTA and by a cluster)."""
+    from hibana_b200 import _native as nv
+    ew = _weights(e, h, inter, act, "nvfp4", "cpu", seed=3).to("cuda")
+    g = torch.Generator().manual_seed(t)
+    x = torch.randn(t, h, generator=g).bfloat16().cuda()
+    logits = torch.randn(t, e, generator=g)
+    logits[:, 0] += 3.0                       # a crowded expert
+    logits[:, 1] -= 30.0                      # and an empty one
+    ids, w = moe.route(logits, k)
+    ids, w = ids.cuda(), w.cuda()
+    assert moe.pair_rows(ew, t)
+    got = moe.experts_forward(x, ids, w, ew)
+    half = moe.experts_forward(x, ids, w, ew, e_lo=1, e_n=e - 2)
+    monkeypatch.setattr(moe, "pair_rows", lambda *a: False)
+    assert torch.equal(got, moe.experts_forward(x, ids, w, ew))
+    assert torch.equal(half, moe.experts_forward(x, ids, w, ew, e_lo=1, e_n=e - 2))
+    assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tokens,topk,e,lo,n", [(1, 1, 8, 0, 8), (372, 22, 512, 0, 512), (373, 22, 512, 0, 512),
                                                 (4096, 22, 512, 100, 300), (1025, 8, 60, 0, 60)])
 def test_plan_places_pairs_in_order(tokens, topk, e, lo, n):
