@@ -131,7 +131,9 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device. Every launch asks for it: the raw lookup takes 0.2 us, building
+    a `torch.cuda.Stream` object first took 15, a fifth of the time an eager prefill spends launching."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 CALLS = 0      # native entry points called

@@ -82,12 +82,27 @@ class KvPool:
         if self._shuffled and n >= 32:
             self._free.sort(reverse=True)          # a prefill-sized request gets ascending runs again
             self._shuffled = False
-        out = [self._free.pop() for _ in range(n)]
-        for s in out:
-            self._owned[s] = 1
+        if n == 0:
+            return []
+        out = self._free[:-n - 1:-1]               # what n pops would return
+        del self._free[-n:]
+        if out == list(range(out[0], out[0] + n)):
+            self._owned[out[0]:out[0] + n] = b"\x01" * n
+        else:
+            for s in out:
+                self._owned[s] = 1
         return out
 
     def free(self, ids: Iterable[int]) -> None:
+        ids = list(ids)
+        n = len(ids)
+        # a run of slots, as prompts are handed out: checked and marked as a whole
+        if n >= 32 and 0 < ids[0] <= self.slots + 1 - n and ids == list(range(ids[0], ids[0] + n)) \
+                and self._owned.count(1, ids[0], ids[0] + n) == n:
+            self._owned[ids[0]:ids[0] + n] = bytes(n)
+            self._free.extend(ids)
+            self._shuffled = True
+            return
         for s in ids:
             if s <= 0 or s > self.slots or not self._owned[s]:
                 raise ValueError(f"double free or foreign slot {s}")

@@ -130,13 +130,251 @@ __device__ __forceinline__ void store_f16_row16(uint32_t tile, int r, int part, 
                  : "memory");
 }
 
+// What one CTA works on: a block of query tokens of a sequence, one kv head, one range of its keys.
+struct PfBlock {
+  int g, b, kvh, split, row0, R, tok0, nrows, ctx, kbeg, kmax, ntiles;
+  __device__ __forceinline__ PfBlock(const PfParams& p, int KT) {
+    g = p.hq / p.hkv;
+    const int tok_per_blk = PF_ROWS / g;
+    b = blockIdx.z;
+    kvh = blockIdx.y;
+    split = static_cast<int>(blockIdx.x) % p.splits;
+    const int qb = (gridDim.x - 1 - blockIdx.x) / p.splits;   // heaviest (latest) query blocks first
+    row0 = p.q_indptr ? p.q_indptr[b] : b;
+    R = p.q_indptr ? p.q_indptr[b + 1] - row0 : 1;
+    tok0 = qb * tok_per_blk;
+    const int ntok = min(tok_per_blk, R - tok0);
+    nrows = ntok * g;                                         // none: past the sequence's rows
+    ctx = p.ctx_len[b];
+    // keys [0, vis) are visible to at least one row of the block, of which this CTA takes [kbeg, kmax): splits are whole
+    // tiles, so that only the last one ends inside a tile
+    const int vis = p.causal ? min(ctx, ctx - R + tok0 + ntok) : ctx;
+    const int per = ((ctx + p.splits - 1) / p.splits + KT - 1) / KT * KT;
+    kbeg = split * per;
+    kmax = min(vis, kbeg + per);
+    ntiles = kmax > kbeg ? (kmax - kbeg + KT - 1) / KT : 0;
+  }
+};
+
+// F8: the block's Q rows as fp16 under a power-of-two row scale, by `threads` threads (a multiple of 32).
+template <int D>
+__device__ __forceinline__ void pf_fill_q16(const PfParams& p, const PfBlock& x, uint8_t* q_s, float* row_scale, int tid,
+                                            int threads) {
+  constexpr int CPR = D / 8;
+  const int g = x.g, nrows = x.nrows, row0 = x.row0, tok0 = x.tok0, kvh = x.kvh;
+  // CPR = 16 or 32 consecutive lanes hold a row
+  for (int c = tid; c < PF_ROWS * CPR; c += threads) {      // both are multiples of 32: warp-uniform
+    const int r = c / CPR, part = c % CPR;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (r < nrows)
+      v = *reinterpret_cast<const uint4*>(
+          p.q + (static_cast<long long>(row0 + tok0 + r / g) * p.hq + kvh * g + r % g) * D + part * 8);
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t mx = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) mx = max(mx, max(w[e] & 0x7FFFu, (w[e] >> 16) & 0x7FFFu));
+#pragma unroll
+    for (int sh = 1; sh < CPR; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+    const int e2 = static_cast<int>(mx >> 7) - 127;
+    const int up = mx == 0 || e2 > 127 ? 0 : min(14 - e2, 126);      // largest element to [2^14, 2^15)
+    const float f = __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
+    if (part == 0) row_scale[r] = __uint_as_float(static_cast<uint32_t>(127 - up) << 23);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __half2 h = __floats2half2_rn(bf16_lo(w[e]) * f, bf16_hi(w[e]) * f);
+      w[e] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(q_s + sw_off(r, part, PF_ROWS)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// The producer warps: K and V tiles of the block's keys into their rings (and, for bf16 pools, the Q rows).
+template <int D, bool F8, int PF_PRODUCERS, int NS>
+__device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, const CUtensorMap& tmk, const CUtensorMap& tmv,
+                                           uint8_t* q_s, uint8_t* k_s, uint8_t* v_s, uint64_t* kfull, uint64_t* vfull,
+                                           uint64_t* kempty, uint64_t* vempty, volatile int* abort, int ptid, int lane) {
+  using C = PfCfg<D, F8>;
+  constexpr int KT = C::KT;
+  constexpr int CPR = D / 8;   // 16-byte chunks per row
+  const int g = x.g, b = x.b, kvh = x.kvh, row0 = x.row0, tok0 = x.tok0, nrows = x.nrows, kbeg = x.kbeg, kmax = x.kmax,
+            ntiles = x.ntiles;
+  const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? p.seq_rows[b] : b) * p.ld_idx;
+  if constexpr (F8) {
+    constexpr int CH = D / 16;                              // 16-code chunks per row
+    constexpr int PER = KT * CH / PF_PRODUCERS;             // chunks of a tile per thread
+    constexpr int RSTEP = PF_PRODUCERS / CH;
+    static_assert(KT * CH % PF_PRODUCERS == 0 && PF_PRODUCERS % CH == 0, "whole chunks per thread");
+    const int part = ptid % CH, r0 = ptid / CH;
+    int sl_now[PER], sl_next[PER];
+    uint4 kreg[PER], vreg[PER];
+    auto slots = [&](int t, int (&sl)[PER]) {               // -1 beyond the visible keys
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int key = kbeg + t * KT + r0 + i * RSTEP;
+        sl[i] = t < ntiles && key < kmax ? __ldg(idx_row + key) : -1;
+      }
+    };
+    auto load = [&](const void* pool, const int (&sl)[PER], uint4 (&reg)[PER]) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        reg[i] = sl[i] < 0 ? make_uint4(0, 0, 0, 0)
+                           : __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(pool) +
+                                                                  static_cast<long long>(sl[i]) * p.pool_stride +
+                                                                  kvh * p.head_stride + part * 16));
+    };
+    auto store = [&](uint8_t* tile, const uint4 (&reg)[PER], uint64_t* bar) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) store_f16_row16(smem_u32(tile), r0 + i * RSTEP, part, KT, reg[i]);
+      fence_proxy_async_smem();
+      mbar_arrive(bar);
+    };
+    slots(0, sl_now);
+    slots(1, sl_next);
+    load(p.k_pool, sl_now, kreg);
+    for (int t = 0; t < ntiles; ++t) {
+      const int s = t % NS;
+      const uint32_t ph = ((t / NS) - 1) & 1;
+      load(p.v_pool, sl_now, vreg);
+      if (t >= NS && !mbar_wait(&kempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
+      store(k_s + s * C::KV_TILE, kreg, &kfull[s]);
+      load(p.k_pool, sl_next, kreg);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) sl_now[i] = sl_next[i];
+      slots(t + 2, sl_next);
+      if (t >= NS && !mbar_wait(&vempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
+      store(v_s + s * C::KV_TILE, vreg, &vfull[s]);
+    }
+  } else {
+  // Q rows (zero padded); they travel in the first cp.async group, i.e. with K tile 0.
+  for (int c = ptid; c < PF_ROWS * CPR; c += PF_PRODUCERS) {
+    const int r = c / CPR, part = c % CPR;
+    const uint32_t dst = smem_u32(q_s) + sw_off(r, part, PF_ROWS);
+    if (r < nrows) {
+      const int tok = tok0 + r / g, gg = r % g;
+      cp16(dst, p.q + (static_cast<long long>(row0 + tok) * p.hq + kvh * g + gg) * D + part * 8);
+    } else {
+      st_zero16(dst);
+    }
+  }
+  // A tile is moved as four 32-key sub-blocks, one producer warp each (warp j % 3). Lane l fetches the slot id
+  // of key l of the sub-block. Slots of a sequence are handed out in ascending runs, so most sub-blocks sit in
+  // 32 consecutive pool rows: then one lane issues a bulk tensor copy per 128-byte column block (box = 32 rows
+  // x 64 elements, 128-byte swizzle, row pitch = one pool slot) that completes on the tile's barrier by
+  // transaction bytes. Otherwise (fragmented pool, tail of the context) the warp gathers the rows with 16-byte
+  // cp.async: the LSU path keeps only ~16 KB in flight per SM, an order of magnitude less than the TMA unit.
+  const int pw = ptid >> 5;
+  constexpr int SB = (KT / 32 + 2) / 3;   // sub-blocks per warp and tile
+  // Slot ids of this warp's sub-blocks of tile t (one per lane); -1 beyond the visible keys.
+  auto fetch_slots = [&](int t, int (&sl)[SB]) {
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      const int j = pw + 3 * i;
+      const int key = kbeg + t * KT + j * 32 + lane;
+      sl[i] = (j < KT / 32 && t < ntiles && key < kmax) ? __ldg(idx_row + key) : -1;
+    }
+  };
+  auto copy_tile = [&](int t, const int (&sl)[SB], const __nv_bfloat16* pool, const CUtensorMap* tm, uint8_t* ring,
+                       uint64_t* bar) {
+    uint8_t* tile = ring + (t % NS) * C::KV_TILE;
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      const int j = pw + 3 * i;
+      if (j >= KT / 32) break;
+      const int slot = sl[i];
+      const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
+      const bool run = p.use_tma && __all_sync(0xffffffffu, slot >= 0 && slot == slot0 + lane);
+      if (run) {
+        if (elect_one()) {
+          mbar_add_tx(bar, 32 * D * 2);   // bytes only: the lane's arrival comes with the other producers'
+#pragma unroll
+          for (int h = 0; h < C::HALVES; ++h)
+            tma_load_2d(tile + h * (KT * 128) + j * (32 * 128), tm, bar, kvh * p.tma_xh + h * 64,
+                        kvh * p.tma_yh + slot0);
+        }
+      } else {
+        // lane -> (row = i * (32 / CPR) + lane / CPR, 16-byte column = lane % CPR)
+        constexpr int RPI = 32 / CPR;
+        const int part = lane % CPR;
+        const uint32_t dst0 = smem_u32(tile) + (part >> 3) * (KT * 128);
+#pragma unroll
+        for (int ii = 0; ii < 32 / RPI; ++ii) {
+          const int rr = ii * RPI + lane / CPR;
+          const int s1 = __shfl_sync(0xffffffffu, slot, rr);
+          const int r = j * 32 + rr;
+          const uint32_t dst = dst0 + r * 128 + (((part & 7) ^ (r & 7)) << 4);
+          if (s1 >= 0)
+            cp16(dst, pool + static_cast<long long>(s1) * p.pool_stride + kvh * p.head_stride + part * 8);
+          else st_zero16(dst);
+        }
+      }
+    }
+  };
+  // cp.async groups in order: K0, [K1, V0], [K2, V1], ...  After iteration t commits V(t), "at most two groups
+  // pending" means K(t) and V(t - 1) have landed: fence them for the tensor-core proxy and signal.
+  bool live = ntiles > 0;
+  int sl_v[SB], sl_k[SB], sl_pre[SB];   // slots of tile t (V copy), t + 1 (K copy), t + 2 (in flight)
+  fetch_slots(0, sl_v);
+  fetch_slots(1, sl_k);
+  if (live) copy_tile(0, sl_v, p.k_pool, &tmk, k_s, &kfull[0]);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int t = 0; live && t < ntiles; ++t) {
+    fetch_slots(t + 2, sl_pre);   // latency hides behind the stage waits below
+    if (t + 1 < ntiles) {
+      {
+        PF_T0();
+        if (t + 1 >= NS && !mbar_wait(&kempty[(t + 1) % NS], (((t + 1) / NS) - 1) & 1, abort,
+                                             p.status, kTimeoutEmpty)) {
+          live = false;
+          break;
+        }
+        PF_ACC(6, ptid == 0);
+      }
+      {
+        PF_T0();
+        copy_tile(t + 1, sl_k, p.k_pool, &tmk, k_s, &kfull[(t + 1) % NS]);
+        PF_ACC(8, ptid == 0);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    {
+      PF_T0();
+      if (t >= NS &&
+          !mbar_wait(&vempty[t % NS], ((t / NS) - 1) & 1, abort, p.status, kTimeoutEmpty)) {
+        live = false;
+        break;
+      }
+      PF_ACC(7, ptid == 0);
+    }
+    {
+      PF_T0();
+      copy_tile(t, sl_v, p.v_pool, &tmv, v_s, &vfull[t % NS]);
+      PF_ACC(8, ptid == 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    PF_T0();
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    PF_ACC(9, ptid == 0);
+    fence_proxy_async_smem();
+    mbar_arrive(&kfull[t % NS]);
+    if (t >= 1) mbar_arrive(&vfull[(t - 1) % NS]);
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      sl_v[i] = sl_k[i];
+      sl_k[i] = sl_pre[i];
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing may land after the CTA has gone
+  fence_proxy_async_smem();
+  if (live) mbar_arrive(&vfull[(ntiles - 1) % NS]);
+  }
+}
+
 template <int D, bool F8>
 __global__ void __launch_bounds__(PfRoles<F8>::THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
   using C = PfCfg<D, F8>;
   constexpr int KT = C::KT;
   constexpr int PF_PRODUCERS = PfRoles<F8>::PRODUCERS, ISSUER = PfRoles<F8>::ISSUER;
-  constexpr int CPR = D / 8;   // 16-byte chunks per row
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = smem;
@@ -156,25 +394,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler too
-  const int g = p.hq / p.hkv;
-  const int tok_per_blk = PF_ROWS / g;
-  const int b = blockIdx.z, kvh = blockIdx.y;
-  const int split = static_cast<int>(blockIdx.x) % p.splits;
-  const int qb = (gridDim.x - 1 - blockIdx.x) / p.splits;   // heaviest (latest) query blocks first
-  const int row0 = p.q_indptr ? p.q_indptr[b] : b;
-  const int R = p.q_indptr ? p.q_indptr[b + 1] - row0 : 1;
-  const int tok0 = qb * tok_per_blk;
-  if (tok0 >= R) return;   // uniform: before any barrier or TMEM allocation
-  const int ntok = min(tok_per_blk, R - tok0);
-  const int nrows = ntok * g;
-  const int ctx = p.ctx_len[b];
-  // keys [0, vis) are visible to at least one row of the block
-  const int vis = p.causal ? min(ctx, ctx - R + tok0 + ntok) : ctx;
-  // of which this CTA takes [kbeg, kmax): splits are whole tiles, so that only the last one ends inside a tile
-  const int per = ((ctx + p.splits - 1) / p.splits + KT - 1) / KT * KT;
-  const int kbeg = split * per;
-  const int kmax = min(vis, kbeg + per);
-  const int ntiles = kmax > kbeg ? (kmax - kbeg + KT - 1) / KT : 0;
+  const PfBlock x(p, KT);
+  if (x.nrows <= 0) return;   // uniform: before any barrier or TMEM allocation
+  const int g = x.g, kvh = x.kvh, row0 = x.row0, R = x.R, tok0 = x.tok0, nrows = x.nrows, ctx = x.ctx, split = x.split,
+            kbeg = x.kbeg, ntiles = x.ntiles;
 
   if (tid == 0) {
     for (int s = 0; s < PF_STAGES; ++s) {
@@ -199,30 +422,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     tmem_relinquish();
   }
   if constexpr (F8) {
-    // Q as scaled fp16 rows, by every warp (CPR = 16 or 32 consecutive lanes hold a row)
-    for (int c = tid; c < PF_ROWS * CPR; c += PfRoles<F8>::THREADS) {      // both are multiples of 32: warp-uniform
-      const int r = c / CPR, part = c % CPR;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < nrows)
-        v = *reinterpret_cast<const uint4*>(
-            p.q + (static_cast<long long>(row0 + tok0 + r / g) * p.hq + kvh * g + r % g) * D + part * 8);
-      uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      uint32_t mx = 0;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) mx = max(mx, max(w[e] & 0x7FFFu, (w[e] >> 16) & 0x7FFFu));
-#pragma unroll
-      for (int sh = 1; sh < CPR; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
-      const int e2 = static_cast<int>(mx >> 7) - 127;
-      const int up = mx == 0 || e2 > 127 ? 0 : min(14 - e2, 126);      // largest element to [2^14, 2^15)
-      const float f = __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
-      if (part == 0) row_scale[r] = __uint_as_float(static_cast<uint32_t>(127 - up) << 23);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __half2 h = __floats2half2_rn(bf16_lo(w[e]) * f, bf16_hi(w[e]) * f);
-        w[e] = *reinterpret_cast<const uint32_t*>(&h);
-      }
-      *reinterpret_cast<uint4*>(q_s + sw_off(r, part, PF_ROWS)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    pf_fill_q16<D>(p, x, q_s, row_scale, tid, PfRoles<F8>::THREADS);
     fence_proxy_async_smem();
   }
   tc_fence_before();
@@ -233,176 +433,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 
   if (warp >= 4 && warp < ISSUER) {
     // ------------------------------------------------------------------ producers
-    const int ptid = tid - 128;
-    const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? p.seq_rows[b] : b) * p.ld_idx;
-    if constexpr (F8) {
-      constexpr int CH = D / 16;                              // 16-code chunks per row
-      constexpr int PER = KT * CH / PF_PRODUCERS;             // chunks of a tile per thread
-      constexpr int RSTEP = PF_PRODUCERS / CH;
-      static_assert(KT * CH % PF_PRODUCERS == 0 && PF_PRODUCERS % CH == 0, "whole chunks per thread");
-      const int part = ptid % CH, r0 = ptid / CH;
-      int sl_now[PER], sl_next[PER];
-      uint4 kreg[PER], vreg[PER];
-      auto slots = [&](int t, int (&sl)[PER]) {               // -1 beyond the visible keys
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int key = kbeg + t * KT + r0 + i * RSTEP;
-          sl[i] = t < ntiles && key < kmax ? __ldg(idx_row + key) : -1;
-        }
-      };
-      auto load = [&](const void* pool, const int (&sl)[PER], uint4 (&reg)[PER]) {
-#pragma unroll
-        for (int i = 0; i < PER; ++i)
-          reg[i] = sl[i] < 0 ? make_uint4(0, 0, 0, 0)
-                             : __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(pool) +
-                                                                    static_cast<long long>(sl[i]) * p.pool_stride +
-                                                                    kvh * p.head_stride + part * 16));
-      };
-      auto store = [&](uint8_t* tile, const uint4 (&reg)[PER], uint64_t* bar) {
-#pragma unroll
-        for (int i = 0; i < PER; ++i) store_f16_row16(smem_u32(tile), r0 + i * RSTEP, part, KT, reg[i]);
-        fence_proxy_async_smem();
-        mbar_arrive(bar);
-      };
-      slots(0, sl_now);
-      slots(1, sl_next);
-      load(p.k_pool, sl_now, kreg);
-      for (int t = 0; t < ntiles; ++t) {
-        const int s = t % PF_STAGES;
-        const uint32_t ph = ((t / PF_STAGES) - 1) & 1;
-        load(p.v_pool, sl_now, vreg);
-        if (t >= PF_STAGES && !mbar_wait(&kempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
-        store(k_s + s * C::KV_TILE, kreg, &kfull[s]);
-        load(p.k_pool, sl_next, kreg);
-#pragma unroll
-        for (int i = 0; i < PER; ++i) sl_now[i] = sl_next[i];
-        slots(t + 2, sl_next);
-        if (t >= PF_STAGES && !mbar_wait(&vempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
-        store(v_s + s * C::KV_TILE, vreg, &vfull[s]);
-      }
-    } else {
-    // Q rows (zero padded); they travel in the first cp.async group, i.e. with K tile 0.
-    for (int c = ptid; c < PF_ROWS * CPR; c += PF_PRODUCERS) {
-      const int r = c / CPR, part = c % CPR;
-      const uint32_t dst = smem_u32(q_s) + sw_off(r, part, PF_ROWS);
-      if (r < nrows) {
-        const int tok = tok0 + r / g, gg = r % g;
-        cp16(dst, p.q + (static_cast<long long>(row0 + tok) * p.hq + kvh * g + gg) * D + part * 8);
-      } else {
-        st_zero16(dst);
-      }
-    }
-    // A tile is moved as four 32-key sub-blocks, one producer warp each (warp j % 3). Lane l fetches the slot id
-    // of key l of the sub-block. Slots of a sequence are handed out in ascending runs, so most sub-blocks sit in
-    // 32 consecutive pool rows: then one lane issues a bulk tensor copy per 128-byte column block (box = 32 rows
-    // x 64 elements, 128-byte swizzle, row pitch = one pool slot) that completes on the tile's barrier by
-    // transaction bytes. Otherwise (fragmented pool, tail of the context) the warp gathers the rows with 16-byte
-    // cp.async: the LSU path keeps only ~16 KB in flight per SM, an order of magnitude less than the TMA unit.
-    const int pw = warp - 4;
-    constexpr int SB = (KT / 32 + 2) / 3;   // sub-blocks per warp and tile
-    // Slot ids of this warp's sub-blocks of tile t (one per lane); -1 beyond the visible keys.
-    auto fetch_slots = [&](int t, int (&sl)[SB]) {
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-        const int j = pw + 3 * i;
-        const int key = kbeg + t * KT + j * 32 + lane;
-        sl[i] = (j < KT / 32 && t < ntiles && key < kmax) ? __ldg(idx_row + key) : -1;
-      }
-    };
-    auto copy_tile = [&](int t, const int (&sl)[SB], const __nv_bfloat16* pool, const CUtensorMap* tm, uint8_t* ring,
-                         uint64_t* bar) {
-      uint8_t* tile = ring + (t % PF_STAGES) * C::KV_TILE;
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-        const int j = pw + 3 * i;
-        if (j >= KT / 32) break;
-        const int slot = sl[i];
-        const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
-        const bool run = p.use_tma && __all_sync(0xffffffffu, slot >= 0 && slot == slot0 + lane);
-        if (run) {
-          if (lane == 0) {
-            mbar_add_tx(bar, 32 * D * 2);   // bytes only: this lane's arrival comes with the other producers'
-#pragma unroll
-            for (int h = 0; h < C::HALVES; ++h)
-              tma_load_2d(tile + h * (KT * 128) + j * (32 * 128), tm, bar, kvh * p.tma_xh + h * 64,
-                          kvh * p.tma_yh + slot0);
-          }
-        } else {
-          // lane -> (row = i * (32 / CPR) + lane / CPR, 16-byte column = lane % CPR)
-          constexpr int RPI = 32 / CPR;
-          const int part = lane % CPR;
-          const uint32_t dst0 = smem_u32(tile) + (part >> 3) * (KT * 128);
-#pragma unroll
-          for (int ii = 0; ii < 32 / RPI; ++ii) {
-            const int rr = ii * RPI + lane / CPR;
-            const int s1 = __shfl_sync(0xffffffffu, slot, rr);
-            const int r = j * 32 + rr;
-            const uint32_t dst = dst0 + r * 128 + (((part & 7) ^ (r & 7)) << 4);
-            if (s1 >= 0)
-              cp16(dst, pool + static_cast<long long>(s1) * p.pool_stride + kvh * p.head_stride + part * 8);
-            else st_zero16(dst);
-          }
-        }
-      }
-    };
-    // cp.async groups in order: K0, [K1, V0], [K2, V1], ...  After iteration t commits V(t), "at most two groups
-    // pending" means K(t) and V(t - 1) have landed: fence them for the tensor-core proxy and signal.
-    bool live = ntiles > 0;
-    int sl_v[SB], sl_k[SB], sl_pre[SB];   // slots of tile t (V copy), t + 1 (K copy), t + 2 (in flight)
-    fetch_slots(0, sl_v);
-    fetch_slots(1, sl_k);
-    if (live) copy_tile(0, sl_v, p.k_pool, &tmk, k_s, &kfull[0]);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int t = 0; live && t < ntiles; ++t) {
-      fetch_slots(t + 2, sl_pre);   // latency hides behind the stage waits below
-      if (t + 1 < ntiles) {
-        {
-          PF_T0();
-          if (t + 1 >= PF_STAGES && !mbar_wait(&kempty[(t + 1) % PF_STAGES], (((t + 1) / PF_STAGES) - 1) & 1, abort,
-                                               p.status, kTimeoutEmpty)) {
-            live = false;
-            break;
-          }
-          PF_ACC(6, ptid == 0);
-        }
-        {
-          PF_T0();
-          copy_tile(t + 1, sl_k, p.k_pool, &tmk, k_s, &kfull[(t + 1) % PF_STAGES]);
-          PF_ACC(8, ptid == 0);
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      {
-        PF_T0();
-        if (t >= PF_STAGES &&
-            !mbar_wait(&vempty[t % PF_STAGES], ((t / PF_STAGES) - 1) & 1, abort, p.status, kTimeoutEmpty)) {
-          live = false;
-          break;
-        }
-        PF_ACC(7, ptid == 0);
-      }
-      {
-        PF_T0();
-        copy_tile(t, sl_v, p.v_pool, &tmv, v_s, &vfull[t % PF_STAGES]);
-        PF_ACC(8, ptid == 0);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      PF_T0();
-      asm volatile("cp.async.wait_group 2;" ::: "memory");
-      PF_ACC(9, ptid == 0);
-      fence_proxy_async_smem();
-      mbar_arrive(&kfull[t % PF_STAGES]);
-      if (t >= 1) mbar_arrive(&vfull[(t - 1) % PF_STAGES]);
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-        sl_v[i] = sl_k[i];
-        sl_k[i] = sl_pre[i];
-      }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing may land after the CTA has gone
-    fence_proxy_async_smem();
-    if (live) mbar_arrive(&vfull[(ntiles - 1) % PF_STAGES]);
-    }
+    pf_produce<D, F8, PF_PRODUCERS, PF_STAGES>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty, abort, tid - 128, lane);
   } else if (warp == ISSUER) {
     // ------------------------------------------------------------------ MMA issuer
     {   // the whole warp walks the loop, one elected lane issues (hb_common.cuh, elect_one)
@@ -642,6 +673,366 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
   if (warp == ISSUER) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
+// Head dims up to 128: two softmax warpgroups. One warpgroup's softmax is the longest link of the chain scores -> softmax ->
+// P -> O, and with one warp per scheduler its latencies show (3500 of 4480 cycles per 128-key tile). Here the even and the
+// odd tiles are two independent streams, each with its own softmax warpgroup, issuer lane, score buffer, accumulator and
+// running maximum, on the same Q and the same K / V rings; the streams meet once, at the end. P replaces
+// the scores it came from in TMEM and enters O += P V as the A operand from there (F8: 16 columns of hi, 16 of lo per
+// 32 keys), so it never passes through shared memory.
+constexpr int PP_STAGES = 3;      // K and V rings, shared by both streams
+template <bool F8>
+struct PpRoles {                  // warps 0-3 and 4-7 softmax, then the producers, then one issuer per stream
+  static constexpr int PROD_WARPS = F8 ? 8 : 3;
+  static constexpr int ISSUER = 8 + PROD_WARPS;
+  static constexpr int PRODUCERS = PROD_WARPS * 32;
+  static constexpr int THREADS = (ISSUER + 2) * 32;
+};
+template <int D, bool F8>
+struct PpCfg {
+  static constexpr int KT = 128;
+  static constexpr int BAR_OFF = PfCfg<D, F8>::Q_BYTES + 2 * PP_STAGES * PfCfg<D, F8>::KV_TILE;
+  static constexpr int SCALE_OFF = BAR_OFF + 256;                  // F8: one scale per packed query row
+  static constexpr int SMEM = SCALE_OFF + (F8 ? PF_ROWS * 4 : 0) + 1024;
+  static_assert(PfCfg<D, F8>::KT == KT && 2 * KT + 2 * D <= 512, "a score buffer and an accumulator per stream");
+};
+
+// Two fp32 operations per instruction (same rounding as the scalar forms).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// The weights of one row's `keys` scores at s_t (32 columns at a time): replaces the scores by P and returns their sum. `rel` is the
+// last visible column; WHOLE rows see all of them.
+template <bool F8, bool WHOLE>
+__device__ __forceinline__ float pp_weights(uint32_t s_t, int keys, int rel, float scale_log2, float neg_m) {
+  const uint64_t scale2 = pack2(scale_log2, scale_log2), neg2 = pack2(neg_m, neg_m);
+  uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll 1
+  for (int c0 = 0; c0 < keys; c0 += 32) {
+    uint32_t v[32];
+    tmem_ld_32x32(s_t + c0, v);
+    tmem_ld_wait();
+    const int rc = rel - c0;
+    uint32_t w[16];
+    uint32_t wl[F8 ? 16 : 1];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      // F8: product and difference rounded one after the other, as the maximum was, so that the largest score gives
+      // exactly 2^0 whatever its size (a fused product of scores near 2^40 would overflow the exponential; the paired
+      // mul and add came out fused)
+      float p0, p1;
+      if constexpr (F8) {
+        p0 = __fadd_rn(__fmul_rn(__uint_as_float(v[j]), scale_log2), neg_m);
+        p1 = __fadd_rn(__fmul_rn(__uint_as_float(v[j + 1]), scale_log2), neg_m);
+      } else {
+        unpack2(fma2(pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), scale2, neg2), p0, p1);
+      }
+      p0 = WHOLE || j <= rc ? ex2(p0) : 0.f;
+      p1 = WHOLE || j + 1 <= rc ? ex2(p1) : 0.f;
+      sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], pack2(p0, p1));
+      if constexpr (F8) {
+        const __half2 hi = __floats2half2_rn(p0, p1);
+        const __half2 lo = __floats2half2_rn(p0 - __low2float(hi), p1 - __high2float(hi));
+        w[j >> 1] = *reinterpret_cast<const uint32_t*>(&hi);
+        wl[j >> 1] = *reinterpret_cast<const uint32_t*>(&lo);
+      } else {
+        w[j >> 1] = pack_bf16(p0, p1);
+      }
+    }
+    tmem_st_32x16(s_t + c0, w);                        // over the scores just read
+    if constexpr (F8) tmem_st_32x16(s_t + c0 + 16, wl);
+  }
+  float a, b;
+  unpack2(add2(sum2[0], sum2[1]), a, b);
+  return a + b;
+}
+
+template <int D, bool F8>
+__global__ void __launch_bounds__(PpRoles<F8>::THREADS, 1)
+attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
+  using C = PfCfg<D, F8>;
+  constexpr int KT = C::KT;
+  constexpr int ISSUER = PpRoles<F8>::ISSUER;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* q_s = smem;
+  uint8_t* k_s = smem + C::Q_BYTES;
+  uint8_t* v_s = k_s + PP_STAGES * C::KV_TILE;
+  uint64_t* kfull = reinterpret_cast<uint64_t*>(smem + PpCfg<D, F8>::BAR_OFF);
+  uint64_t* vfull = kfull + PP_STAGES;
+  uint64_t* kempty = vfull + PP_STAGES;
+  uint64_t* vempty = kempty + PP_STAGES;
+  uint64_t* s_ready = vempty + PP_STAGES;      // from here on one per stream
+  uint64_t* p_ready = s_ready + 2;
+  uint64_t* pv_done = p_ready + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float2* ml = reinterpret_cast<float2*>(q_s);     // at the end, over Q: running maximum and sum of both streams' rows
+  float* row_scale = reinterpret_cast<float*>(smem + PpCfg<D, F8>::SCALE_OFF);
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler too
+  const PfBlock x(p, KT);
+  if (x.nrows <= 0) return;   // uniform: before any barrier or TMEM allocation
+  const int ntiles = x.ntiles;
+
+  if (tid == 0) {
+    for (int s = 0; s < PP_STAGES; ++s) {
+      mbar_init(&kfull[s], PpRoles<F8>::PRODUCERS);
+      mbar_init(&vfull[s], PpRoles<F8>::PRODUCERS);
+      mbar_init(&kempty[s], 1);
+      mbar_init(&vempty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_ready[s], 1);
+      mbar_init(&p_ready[s], PF_ROWS);
+      mbar_init(&pv_done[s], 1);
+    }
+    *abort = 0;
+    fence_mbar_init();
+    if (p.use_tma) {
+      prefetch_tmap(&tmk);
+      prefetch_tmap(&tmv);
+    }
+  }
+  if (warp == ISSUER) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if constexpr (F8) {
+    pf_fill_q16<D>(p, x, q_s, row_scale, tid, PpRoles<F8>::THREADS);
+    fence_proxy_async_smem();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  if (warp >= 8 && warp < ISSUER) {
+    pf_produce<D, F8, PpRoles<F8>::PRODUCERS, PP_STAGES>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty, abort, tid - 256,
+                                              lane);
+  } else if (warp >= ISSUER) {
+    // ------------------------------------------------------------------ MMA issuer of one stream
+    constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);      // operand format codes of kind::f16: 0 = fp16, 1 = bf16
+    constexpr uint32_t idesc_qk = make_idesc_bf16(PF_ROWS, KT) & ~(F8 ? kBf16 : 0u);
+    constexpr uint32_t idesc_pv = make_idesc_bf16(PF_ROWS, D, 0, 1) & ~(F8 ? kBf16 : 0u);
+    const int st = warp - ISSUER;
+    const uint32_t q_a = __shfl_sync(0xffffffffu, smem_u32(q_s), 0);
+    const uint32_t s_t = tmem_base + st * KT, o_t = tmem_base + 2 * KT + st * D;
+    for (int t = st, i = 0; t < ntiles; t += 2, ++i) {
+      const int s = t % PP_STAGES;
+      const uint32_t ring = (t / PP_STAGES) & 1;
+      const uint32_t k_a = q_a + C::Q_BYTES + s * C::KV_TILE, v_a = k_a + PP_STAGES * C::KV_TILE;
+      // the score buffer holds P(t - 2) until that tile's O += P V is done
+      if (i > 0 && !warp_wait(&pv_done[st], (i - 1) & 1, abort, p.status, kTimeoutAccum)) break;
+      {
+        PF_T0();
+        if (!warp_wait(&kfull[s], ring, abort, p.status, kTimeoutFull)) break;
+        PF_ACC(5, lane == 0 && st == 0);
+      }
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const uint32_t in_row = (ks & 3) * 32;   // 16 elements = 32 bytes inside the 128-byte swizzled row
+          mma_f16(s_t, make_desc_sw128(q_a + (ks >> 2) * (PF_ROWS * 128) + in_row),
+                  make_desc_sw128(k_a + (ks >> 2) * (KT * 128) + in_row), idesc_qk, ks > 0 ? 1u : 0u);
+        }
+        tc_commit(&kempty[s]);
+        tc_commit(&s_ready[st]);
+      }
+      __syncwarp();
+      {
+        PF_T0();
+        if (!warp_wait(&p_ready[st], i & 1, abort, p.status, kTimeoutAccum)) break;
+        PF_ACC(3, lane == 0 && st == 0);
+      }
+      {
+        PF_T0();
+        if (!warp_wait(&vfull[s], ring, abort, p.status, kTimeoutFull)) break;
+        PF_ACC(4, lane == 0 && st == 0);
+      }
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < KT / 16; ++kk) {
+          // 16 keys = two 8-row groups 1024 bytes apart; the D / 64 column blocks are KT * 128 bytes apart
+          const uint64_t bdesc = make_desc_sw128_mn(v_a + kk * 2048, KT * 128, 1024);
+          const uint32_t a_t = s_t + (kk >> 1) * 32 + (kk & 1) * 8;      // 8 columns of packed pairs
+          mma_f16_ts(o_t, a_t, bdesc, idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
+          if constexpr (F8) mma_f16_ts(o_t, a_t + 16, bdesc, idesc_pv, 1u);   // the low parts of the weights
+        }
+        tc_commit(&vempty[s]);
+        tc_commit(&pv_done[st]);
+      }
+      __syncwarp();
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax of one stream, half of the output columns
+    const int st = warp >> 2;
+    const int r = tid & (PF_ROWS - 1);                   // packed query row = TMEM lane
+    const uint32_t tlane = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t s_t = tmem_base + st * KT + tlane, o_t = tmem_base + 2 * KT + st * D + tlane;
+    const bool row_ok = r < x.nrows;
+    const int tok = x.tok0 + r / x.g;
+    // last visible key position (inclusive)
+    const int lim = row_ok ? (p.causal ? x.ctx - x.R + tok : x.ctx - 1) : -1;
+    const float scale_log2 = F8 ? p.scale_log2 * p.kv_scale * row_scale[r] : p.scale_log2;
+    float m_ref = -INFINITY, l = 0.f;   // O and l of this stream are relative to 2^m_ref
+    bool ok = true;
+    const long long t_begin = p.prof ? clock64() : 0;
+    for (int t = st, i = 0; t < ntiles; t += 2, ++i) {
+      {
+        PF_T0();
+        ok = warp_wait(&s_ready[st], i & 1, abort, p.status, kTimeoutAccum);
+        PF_ACC(0, tid == 0);
+      }
+      if (!ok) break;
+      tc_fence_after();
+      // `rel` = last visible column of this tile for this row; a warp whose rows see the whole tile skips the masking.
+      const int rel = lim - (x.kbeg + t * KT);
+      const bool whole = __all_sync(0xffffffffu, rel >= KT - 1);
+      const long long t_math = p.prof ? clock64() : 0;
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 1
+      for (int c0 = 0; c0 < KT; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32(s_t + c0, v);
+        tmem_ld_wait();
+        if (whole) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(v[j]));
+        } else {
+          const int rc = rel - c0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], j <= rc ? __uint_as_float(v[j]) : -INFINITY);
+        }
+      }
+      const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+      if (i == 0) {
+        m_ref = m_tile;
+      } else if (__any_sync(0xffffffffu, m_tile > m_ref + C::RESCALE_GAP)) {
+        // Raise the reference (all lanes of the warp: tcgen05.ld / st are warp-wide) and rescale O and l. The scores
+        // were issued after this stream's last O += P V had completed.
+        const float m_new = fmaxf(m_ref, m_tile);
+        const float alpha = m_new == -INFINITY ? 1.f : ex2(m_ref - m_new);
+        m_ref = m_new;
+        l *= alpha;
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += 32) {
+          uint32_t o[32];
+          tmem_ld_32x32(o_t + c0, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+          tmem_st_32x32(o_t + c0, o);
+        }
+      }
+      const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
+      const float sum = whole ? pp_weights<F8, true>(s_t, KT, rel, scale_log2, neg_m)
+                              : pp_weights<F8, false>(s_t, KT, rel, scale_log2, neg_m);
+      l += sum;
+      tmem_st_wait();
+      if (p.prof && tid == 0) atomicAdd(p.prof + 13, (unsigned long long)(clock64() - t_math));
+      tc_fence_before();
+      mbar_arrive(&p_ready[st]);
+    }
+    if (p.prof && tid == 0) {
+      atomicAdd(p.prof + 10, (unsigned long long)(clock64() - t_begin));
+      atomicAdd(p.prof + 11, (unsigned long long)((ntiles + 1) / 2));
+    }
+    // This stream's last O += P V (the other's barrier has phases this thread did not follow), then both streams': from
+    // here on no MMA is left, Q included. A stream without tiles (one-tile blocks) has no O.
+    const int n0 = (ntiles + 1) / 2, n1 = ntiles / 2, mine = st == 0 ? n0 : n1;
+    if (ok && mine > 0) ok = warp_wait(&pv_done[st], (mine - 1) & 1, abort, p.status, kTimeoutAccum);
+    __syncwarp();
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    ml[st * PF_ROWS + r] = make_float2(m_ref, l);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (ok) {
+      tc_fence_after();
+      // (without tiles nobody has waited for the copy of Q, which then lands where `ml` is)
+      const float2 none = make_float2(-INFINITY, 0.f);
+      const float2 a = ntiles > 0 ? ml[r] : none, b = ntiles > 0 ? ml[PF_ROWS + r] : none;
+      const float m = fmaxf(a.x, b.x);
+      float wa = a.x == -INFINITY ? 0.f : ex2(a.x - m), wb = b.x == -INFINITY ? 0.f : ex2(b.x - m);
+      const float total = a.y * wa + b.y * wb;
+      float inv = total > 0.f ? 1.f / total : 0.f;
+      if constexpr (F8) inv *= p.kv_scale;
+      wa *= inv;
+      wb *= inv;
+      const long long rh = static_cast<long long>(x.row0 + tok) * p.hq + x.kvh * x.g + r % x.g;
+      __nv_bfloat16* dst = p.out + rh * D;
+      if (p.splits > 1 && row_ok && st == 0)
+        p.part_lse[rh * p.splits + x.split] = total > 0.f ? m + log2f(total) : -INFINITY;
+      const uint32_t o0 = tmem_base + 2 * KT + tlane, o1 = o0 + D;
+#pragma unroll
+      for (int c0 = st * (D / 2); c0 < (st + 1) * (D / 2); c0 += 32) {
+        uint32_t u[32];
+        float o[32];
+        if (n0 > 0) {
+          tmem_ld_32x32(o0 + c0, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = __uint_as_float(u[j]) * wa;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = 0.f;
+        }
+        if (n1 > 0) {
+          tmem_ld_32x32(o1 + c0, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = fmaf(__uint_as_float(u[j]), wb, o[j]);
+        }
+        if (row_ok && p.splits > 1) {
+          float* part = p.part_o + (rh * p.splits + x.split) * D + c0;
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(part + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+        } else if (row_ok) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8)
+            *reinterpret_cast<uint4*>(dst + c0 + j) = make_uint4(pack_bf16(o[j], o[j + 1]), pack_bf16(o[j + 2], o[j + 3]),
+                                                                 pack_bf16(o[j + 4], o[j + 5]), pack_bf16(o[j + 6], o[j + 7]));
+        }
+      }
+      tc_fence_before();
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == ISSUER) tmem_dealloc(tmem_base, 512);
+}
+
+template <int D, bool F8>
+int launch_prefill_pp(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int qblocks, int batch,
+                      cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(attn_prefill_pp_kernel<D, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             PpCfg<D, F8>::SMEM) != cudaSuccess)
+      return 3;
+    attr = true;
+  }
+  attn_prefill_pp_kernel<D, F8><<<dim3(qblocks * p.splits, p.hkv, batch), PpRoles<F8>::THREADS, PpCfg<D, F8>::SMEM, st>>>(
+      *tk, *tv, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
 template <int D, bool F8>
 int launch_prefill(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int qblocks, int batch,
                    cudaStream_t st) {
@@ -717,7 +1108,7 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
   const CUtensorMap *tk = &dummy, *tv = &dummy;
   if (kv_fp8) {      // producers load through registers: no tensor maps
     p.use_tma = p.tma_xh = p.tma_yh = 0;
-    if (d == 128) return launch_prefill<128, true>(p, tk, tv, qblocks, batch, st);
+    if (d == 128) return launch_prefill_pp<128, true>(p, tk, tv, qblocks, batch, st);
     if (d == 256) return launch_prefill<256, true>(p, tk, tv, qblocks, batch, st);
     return 1;
   }
@@ -729,8 +1120,8 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
     tk = &t.k;
     tv = &t.v;
   }
-  if (d == 64) return launch_prefill<64, false>(p, tk, tv, qblocks, batch, st);
-  if (d == 128) return launch_prefill<128, false>(p, tk, tv, qblocks, batch, st);
+  if (d == 64) return launch_prefill_pp<64, false>(p, tk, tv, qblocks, batch, st);
+  if (d == 128) return launch_prefill_pp<128, false>(p, tk, tv, qblocks, batch, st);
   if (d == 256) return launch_prefill<256, false>(p, tk, tv, qblocks, batch, st);
   return 1;
 }

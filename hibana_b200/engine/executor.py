@@ -96,7 +96,7 @@ class Executor:
         if req.total_len + req.params.max_tokens > self.max_ctx:
             raise ValueError(f"prompt + max_tokens exceeds the context limit {self.max_ctx}")
         has_media = bool(getattr(req.media, "images", None))
-        if any(i >= self.target.vocab or (i < 0 and not has_media) for i in req.prompt_ids):
+        if max(req.prompt_ids) >= self.target.vocab or (min(req.prompt_ids) < 0 and not has_media):
             raise ValueError("token id out of range")
 
     def can_admit(self, req: Request, promised: int = 0) -> bool:

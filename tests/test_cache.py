@@ -170,3 +170,25 @@ def test_cache_trace_pins_cache_paths_to_the_cold_run(tmp_path):
     assert rep["pairs"]["cached_vs_cold"]["max_rel_diff"] < 2e-2
     assert rep["pairs"]["restored_vs_cached"]["equal"]            # restore is a byte copy of what the cache held
     assert (tmp_path / "trace.json").exists() and (tmp_path / "trace.pt").exists()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 200])
+def test_kv_pool_runs_of_slots_cpu(n):
+    """Runs of slots are marked as a whole: same slots, same checks as one by one."""
+    from hibana_b200.cache.kv_pool import KvPool
+    pool = KvPool(1, 300, 1, 32)
+    a, b = pool.alloc(n), pool.alloc(5)
+    assert a == list(range(1, n + 1)) and b == list(range(n + 1, n + 6)) and pool.alloc(0) == []
+    pool.free(a)
+    pool.check()
+    with pytest.raises(ValueError):
+        pool.free(a)                               # a second time
+    pool.check()
+    with pytest.raises(ValueError):
+        pool.free(list(range(250, 250 + n)) if n > 51 else [301])      # foreign slots
+    c = pool.alloc(n)
+    assert sorted(c) == a
+    pool.free(iter(c[::-1]))
+    pool.free(b)
+    pool.check()
+    assert pool.free_count == 300
