@@ -111,6 +111,7 @@ int hb_rope_kv_write(const void* qkv, long long ld_qkv, const void* positions, c
                      const void* inv_freq, const void* q_norm_w, const void* k_norm_w, float eps, int gemma_norm,
                      void* q_out, void* k_pool, void* v_pool, long long pool_stride, long long head_stride, int tokens,
                      int hq, int hkv, int d, int rot, int kv_fp8, float kv_inv_scale, int q_gate, void* stream);
+int hb_head_skip(void* y, const void* x, long long ldx, const void* d, long long rows, int inner, int head_dim, void* stream);
 int hb_act_mul(const void* x, const void* gate, void* out, long long rows, int inter, long long ldx, int mode,
                void* stream);
 int hb_embedding(const void* ids, const void* table, void* out, int tokens, int h, long long vocab, void* stream);

@@ -24,6 +24,7 @@ from . import gdn_chunk
 CHUNK = gdn_chunk.CHUNK
 
 P, I, L = nv.P, nv.I, nv.L
+nv.register("hb_head_skip", [P, P, L, P, L, I, I, P])
 nv.register("hb_ssd_phase1", [P, P, P, P, P, P, L, L, L, I, I, I, I, P, P, P, P, P, P])
 
 
@@ -108,5 +109,10 @@ def mamba2_chunked(x, bmat, cmat, dt, a_log, dt_bias, dskip, state, slot_in, slo
             if sout is not None:
                 state[sout[b]] = s.to(state.dtype)
     if dskip is not None:
+        if (native and dskip.dtype == torch.float32 and dskip.is_contiguous() and head_dim % 8 == 0 and x.stride(0) % 8 == 0
+                and x.stride(1) == 1 and x.data_ptr() % 16 == 0):
+            nv.check(nv.lib().hb_head_skip(y.data_ptr(), x.data_ptr(), x.stride(0), dskip.data_ptr(), y.shape[0],
+                                           heads * head_dim, head_dim, nv.stream()), "hb_head_skip")
+            return y
         y = (y.float() + dskip.float().repeat_interleave(head_dim)[None, :] * x.float()).to(x.dtype)
     return y

@@ -580,3 +580,56 @@ def test_fp8_attention_tensor_cores(hq, hkv, d, rows, contiguous):
                                         kv_scale=ks, splits=splits, **kw).cpu().double()
         err = (got - ref).norm() / ref.norm()
         assert nv.read_status() == 0 and float(err) < 1.1 * 2.0 ** -9, float(err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gs,groups", [(8, 5), (24, 3), (64, 4), (72, 2), (120, 3), (136, 2), (256, 2), (264, 2), (512, 1),
+                                       (520, 3), (1024, 2), (1032, 2)])
+@pytest.mark.parametrize("norm_first", [False, True])
+def test_gated_rmsnorm_group_sizes(gs, groups, norm_first):
+    """Every lanes-per-group and chunks-per-lane form against 64 bits: one bf16 rounding, and 2^-14 for the exponential."""
+    g = torch.Generator().manual_seed(gs)
+    h = gs * groups
+    x, z = (torch.randn(11, h + 8, generator=g).bfloat16()[:, :h] for _ in range(2))
+    w = (torch.randn(h, generator=g) * 0.1 + 1).bfloat16()
+    got = basic.gated_rmsnorm(x.cuda(), z.cuda(), w.cuda(), 1e-5, gs, norm_first=norm_first).cpu().double()
+    xd, gate = x.double(), torch.nn.functional.silu(z.double())
+    v = (xd if norm_first else xd * gate).view(11, groups, gs)
+    ref = (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5)).view(11, h) * w.double() * (gate if norm_first else 1)
+    assert bool(((got - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * ref.abs() + 1e-30).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,heads,p", [(1, 1, 8), (37, 6, 64), (130, 128, 64), (5, 3, 128)])
+def test_head_skip_equals_the_elementwise_passes(rows, heads, p):
+    g = torch.Generator().manual_seed(rows)
+    y = torch.randn(rows, heads * p, generator=g).bfloat16().cuda()
+    x = torch.randn(rows, heads * p + 16, generator=g).bfloat16().cuda()[:, :heads * p]
+    d = torch.randn(heads, generator=g).cuda()
+    want = (y.float() + d.repeat_interleave(p)[None, :] * x.float()).to(torch.bfloat16)
+    from hibana_b200.ops import ssd_chunk  # noqa: F401  (declares the entry)
+    nv.check(nv.lib().hb_head_skip(y.data_ptr(), x.data_ptr(), x.stride(0), d.data_ptr(), rows, heads * p, p, nv.stream()),
+             "hb_head_skip")
+    assert torch.equal(y, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("inter", [1, 8, 12, 520])
+@pytest.mark.parametrize("mode", [basic.ACT_SILU_SPLIT, basic.ACT_SILU_PAIRS, basic.ACT_RELU2, basic.ACT_SIGMOID_GATE])
+def test_act_mul_widths(inter, mode):
+    """16-byte and scalar forms against 64 bits: one bf16 rounding, and 2^-14 for the exponential."""
+    g = torch.Generator().manual_seed(inter)
+    cols = 2 * inter if mode in (basic.ACT_SILU_SPLIT, basic.ACT_SILU_PAIRS) else inter
+    x = torch.randn(9, cols, generator=g).bfloat16()
+    gate = torch.randn(9, cols, generator=g).bfloat16() if mode == basic.ACT_SIGMOID_GATE else None
+    got = basic.act_mul(x.cuda(), mode, gate.cuda() if gate is not None else None).cpu().double()
+    xd = x.double()
+    if mode == basic.ACT_SILU_SPLIT:
+        ref = torch.nn.functional.silu(xd[:, :inter]) * xd[:, inter:]
+    elif mode == basic.ACT_SILU_PAIRS:
+        ref = torch.nn.functional.silu(xd[:, 0::2]) * xd[:, 1::2]
+    elif mode == basic.ACT_RELU2:
+        ref = torch.relu(xd) ** 2
+    else:
+        ref = xd * torch.sigmoid(gate.double())
+    assert bool(((got - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * ref.abs() + 1e-30).all())
