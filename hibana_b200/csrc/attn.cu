@@ -355,8 +355,8 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
   extern __shared__ float weight[];     // [splits]
   const long long rh = blockIdx.x;
   const float* lse = part_lse + rh * splits;
-  // The kernel is a chain of L2 round trips: all log sums in one, then eight partials in flight per thread (one after
-  // the other, 18 splits cost 8.2 us; this form).
+  // The kernel is a chain of L2 round trips: all log sums in one, then eight partials in flight per thread: nine
+  // splits merge in 5.2 us, 37 in 8.4 us (dispatch included).
   for (int s = threadIdx.x; s < splits; s += blockDim.x) weight[s] = lse[s];
   __syncthreads();
   float m = -INFINITY;

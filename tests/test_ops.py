@@ -633,3 +633,13 @@ def test_act_mul_widths(inter, mode):
     else:
         ref = xd * torch.sigmoid(gate.double())
     assert bool(((got - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * ref.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("batch,hkv,ctx", [(1, 8, 64), (1, 8, 500), (4, 4, 5056), (3, 2, 2304), (64, 8, 131072)])
+def test_splits_fill_one_wave_before_they_get_short(batch, hkv, ctx):
+    s = attention.choose_splits(batch, hkv, ctx, slots=148)
+    assert s >= 1 and (s == 1 or ctx // s >= attention.MIN_SPLIT_KEYS)
+    if batch * hkv * s > 148 and s > 1:
+        assert ctx // s >= 256
+    elif ctx >= 148 // (batch * hkv) * attention.MIN_SPLIT_KEYS:      # keys enough for the whole wave: nearly all of it
+        assert batch * hkv * s >= 0.9 * 148
