@@ -676,3 +676,326 @@ int hb_ssd_phase1(const void* x, const void* b, const void* c, const void* dt, c
 }
 
 }  // extern "C"
+
+// ---------------------------------------------------------------------------------------------------------------
+// Chunked Mamba-2 (SSD) scan of one sequence in one kernel: the chunk-local factors and the state pass of
+// gdn_chunk_kernel without its W term. With dt_t = softplus(dt + bias), a_t = -exp(a_log) dt_t and gamma its running sum:
+//   V' = dt * X     M[t,i] = e^(gamma_t - gamma_i) <C_t, B_i> (i <= t)     Qg = e^gamma C     Kd = e^(gamma_C - gamma) B
+//   O  = Qg S^T + M V'                                                      S^T <- e^gamma_C S^T + Kd^T V'
+// One CTA per (head, 64 columns of the head), 16 warps, one barrier per chunk. Warps 0..7 (two groups of four, 32 value
+// columns each, the fp32 state in their accumulators) consume the factors of chunk c - 1. Of chunk c, warps 8..11 prepare
+// Qg, Kd and V' and warps 12..15 M, both from the raw B and C rows that were copied during the chunk before.
+//
+// Why one kernel: as two, the factors of all chunks went through memory (Qg, Kd, M and an fp32 dt * X are 53 KB per chunk
+// and head, 470 MB for 4096 tokens and 128 heads, against 84 MB of inputs and outputs), and the second had two CTAs
+// per head, 256 on 148 SMs. 128 heads of 64, scan without the skip term: 4096 tokens 476 -> 243 us, 904 tokens
+// 127 -> 64. Now bound by a chunk's chains of latencies (3.6 us) and about 3400 cycles of shared-memory traffic in it. The
+// two-kernel form's chain is 2 us a chunk, so it stays the faster one for long sequences of few heads (16 heads,
+// 4096 tokens: 162 us against 225); ops/ssd_chunk.py has the rule.
+namespace hb {
+namespace {
+
+struct SsdParams {
+  const __nv_bfloat16* x;    // [n, heads * P]   (pitch ldx)
+  const __nv_bfloat16* b;    // [n, groups * 128] (pitch ldb)
+  const __nv_bfloat16* c;
+  const __nv_bfloat16* dt;   // [n, heads]        (pitch lddt)
+  const float* a_log;        // [heads]
+  const float* dt_bias;      // [heads] or null
+  long long ldx, ldb, lddt;
+  const float* s_in;         // [heads, P, 128] or null (zero state)
+  float* s_out;              // same layout, may be null
+  __nv_bfloat16* o;          // o[row * ldo + h * P + v]
+  long long ldo;
+  int n, nc, heads, groups, p;
+  int wide;                  // rows of b and c can be copied in 16-byte pieces
+};
+
+constexpr int SSD_VN = GC * P_V;                      // one group's V' tile, bf16 [64, 32]
+constexpr int SSD_Q = 0, SSD_KD = GC * P_K, SSD_M = 2 * GC * P_K, SSD_V = SSD_M + GC * P_M;
+constexpr int SSD_STAGE = SSD_V + 2 * SSD_VN;         // factors of one chunk
+constexpr int SSD_RAW = 2 * SSD_STAGE;                // C, then B, of two chunks
+constexpr int SSD_ST = SSD_RAW + 4 * GC * P_K;        // two bf16 copies of S^T (by chunk parity), two groups each
+constexpr int SSD_ST_GROUP = GK * P_V;
+constexpr int SSD_GAM = SSD_ST + 4 * SSD_ST_GROUP;    // gamma, one copy per warp that needs it
+constexpr int SSD_SMEM = SSD_GAM + 4 * GC * 4 + 16;   // + gamma_C of the two stages
+static_assert(SSD_SMEM <= 227 * 1024, "shared memory");
+
+__global__ void __launch_bounds__(512, 1) ssd_chunk_kernel(const SsdParams p) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  const uint32_t sb = smem_u32(sm);
+  float* g_end = reinterpret_cast<float*>(sm + SSD_GAM + 4 * GC * 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.x, v_cta = blockIdx.y * 64;
+  const int qr = lane >> 2, qc = (lane & 3) * 2;   // accumulator row / first column of this lane inside a tile
+
+  if (warp >= 8) {
+    const int w = warp & 3;
+    const bool factors = warp < 12;                // else: M and the copies of raw rows
+    const int grp = h / (p.heads / p.groups);
+    const float a = -__expf(p.a_log[h]);
+    const float bias = p.dt_bias ? p.dt_bias[h] : 0.f;
+    float* gam = reinterpret_cast<float*>(sm + SSD_GAM) + w * GC;
+    const int xcol = v_cta + lane * 2;
+    uint32_t rx[16];
+    // raw bits: a conversion here would wait for the load
+    unsigned short q0 = 0, q1 = 0;
+    const unsigned short* dt_bits = reinterpret_cast<const unsigned short*>(p.dt);
+    auto fetch = [&](int c) {                      // rows past the end: zero
+      const int t0 = c * GC;
+      const int ta = t0 + lane, tb = t0 + 32 + lane;
+      if (ta < p.n) q0 = __ldg(dt_bits + ta * p.lddt + h);
+      if (tb < p.n) q1 = __ldg(dt_bits + tb * p.lddt + h);
+      if (factors) {
+        const __nv_bfloat16* gx = p.x + (t0 + w) * p.ldx + h * p.p + xcol;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int t = t0 + w + 4 * i;
+          rx[i] = 0;
+          if (t < p.n && xcol < p.p) rx[i] = __ldg(reinterpret_cast<const uint32_t*>(gx + i * 4 * p.ldx));
+        }
+        return;
+      }
+      const uint32_t raw = sb + SSD_RAW + (c & 1) * 2 * GC * P_K;
+      // a warp copies rows w, w + 4, ... (8-byte pieces) or pairs of rows (16-byte pieces)
+      const int sub = p.wide ? lane >> 4 : 0, off = p.wide ? (lane & 15) * 16 : lane * 8;
+      const int step = p.wide ? 8 : 4;
+      int r = p.wide ? 2 * w + sub : w;
+      const uint8_t* gc = reinterpret_cast<const uint8_t*>(p.c + grp * GK) + off;
+      const uint8_t* gb = reinterpret_cast<const uint8_t*>(p.b + grp * GK) + off;
+      long long src = (t0 + r) * p.ldb * 2;
+      for (; r < GC; r += step, src += step * p.ldb * 2) {
+        const bool in = t0 + r < p.n;
+        const long long at = in ? src : 0;
+        const uint32_t d = raw + r * P_K + off;
+        if (p.wide) {
+          const int have = in ? 16 : 0;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gc + at), "r"(have) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + GC * P_K), "l"(gb + at), "r"(have) : "memory");
+        } else {
+          const int have = in ? 8 : 0;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gc + at), "r"(have) : "memory");
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + GC * P_K), "l"(gb + at), "r"(have) : "memory");
+        }
+      }
+    };
+    fetch(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    for (int c = 0; c <= p.nc; ++c) {
+      if (c < p.nc) {
+        const int st = (c & 1) * SSD_STAGE, raw = SSD_RAW + (c & 1) * 2 * GC * P_K;
+        const int t0 = c * GC;
+        const float z0 = __uint_as_float(static_cast<uint32_t>(q0) << 16) + bias;
+        const float z1 = __uint_as_float(static_cast<uint32_t>(q1) << 16) + bias;
+        float d0 = 0.f, d1 = 0.f;
+        if (t0 + lane < p.n) d0 = z0 > 20.f ? z0 : log1pf(__expf(z0));
+        if (t0 + 32 + lane < p.n) d1 = z1 > 20.f ? z1 : log1pf(__expf(z1));
+        if (factors) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float d = __shfl_sync(0xffffffffu, i < 8 ? d0 : d1, (w + 4 * i) & 31);
+            *reinterpret_cast<uint32_t*>(sm + st + SSD_V + (lane >> 4) * SSD_VN + (w + 4 * i) * P_V + (lane & 15) * 4) =
+                pack_bf16(bf16_lo(rx[i]) * d, bf16_hi(rx[i]) * d);
+          }
+        }
+        if (c + 1 < p.nc) fetch(c + 1);            // has the rest of this chunk to arrive
+        float g0 = d0 * a, g1 = d1 * a;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float x0 = __shfl_up_sync(0xffffffffu, g0, o), x1 = __shfl_up_sync(0xffffffffu, g1, o);
+          if (lane >= o) {
+            g0 += x0;
+            g1 += x1;
+          }
+        }
+        g1 += __shfl_sync(0xffffffffu, g0, 31);
+        if (factors) {
+          const float g_last = __shfl_sync(0xffffffffu, g1, 31);
+          if (w == 0 && lane == 0) g_end[c & 1] = g_last;
+          const float e0 = __expf(g0), e1 = __expf(g1), f0 = __expf(g_last - g0), f1 = __expf(g_last - g1);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int r = w + 4 * i;
+            const float eg = __shfl_sync(0xffffffffu, i < 8 ? e0 : e1, r & 31);
+            const float ed = __shfl_sync(0xffffffffu, i < 8 ? f0 : f1, r & 31);
+            const int off = r * P_K + lane * 8;
+            const uint2 cc = *reinterpret_cast<const uint2*>(sm + raw + off);
+            const uint2 bb = *reinterpret_cast<const uint2*>(sm + raw + GC * P_K + off);
+            *reinterpret_cast<uint2*>(sm + st + SSD_KD + off) =
+                make_uint2(pack_bf16(bf16_lo(bb.x) * ed, bf16_hi(bb.x) * ed), pack_bf16(bf16_lo(bb.y) * ed, bf16_hi(bb.y) * ed));
+            *reinterpret_cast<uint2*>(sm + st + SSD_Q + off) =
+                make_uint2(pack_bf16(bf16_lo(cc.x) * eg, bf16_hi(cc.x) * eg), pack_bf16(bf16_lo(cc.y) * eg, bf16_hi(cc.y) * eg));
+          }
+        } else {
+          gam[lane] = g0;
+          gam[32 + lane] = g1;
+          __syncwarp();
+          // C B^T for 16 rows, masked and decayed; 16-column tiles above the diagonal stay zero
+          float acc[8][4] = {};
+          const uint32_t a_off = (16 * w + (lane & 15)) * P_K + (lane >> 4) * 16;
+          const int mi = lane >> 3;
+#pragma unroll
+          for (int ks = 0; ks < GK / 16; ++ks) {
+            uint32_t fc[4];
+            ldsm_x4(fc, sb + raw + a_off + ks * 32);
+#pragma unroll
+            for (int jp = 0; jp < 4; ++jp) {
+              if (jp > w) continue;
+              uint32_t fb[4];
+              ldsm_x4(fb, sb + raw + GC * P_K + (16 * jp + (mi >> 1) * 8 + (lane & 7)) * P_K + ks * 32 + (mi & 1) * 16);
+              mma16816(acc[2 * jp], fc, fb[0], fb[1]);
+              mma16816(acc[2 * jp + 1], fc, fb[2], fb[3]);
+            }
+          }
+          const float gt0 = gam[16 * w + qr], gt1 = gam[16 * w + qr + 8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int i = 8 * j + qc;
+            const float2 gi = *reinterpret_cast<const float2*>(gam + i);
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const int t = 16 * w + qr + (e >> 1) * 8;
+              const float gt = e == 0 ? gt0 : gt1;
+              const float v0 = i <= t ? acc[j][e] * __expf(gt - gi.x) : 0.f;
+              const float v1 = i + 1 <= t ? acc[j][e + 1] * __expf(gt - gi.y) : 0.f;
+              *reinterpret_cast<uint32_t*>(sm + st + SSD_M + t * P_M + i * 2) = pack_bf16(v0, v1);
+            }
+          }
+          asm volatile("cp.async.wait_all;" ::: "memory");     // the next chunk's raw rows, before the barrier publishes them
+        }
+      }
+      asm volatile("bar.sync 0, 512;" ::: "memory");           // chunk c is ready, chunk c - 1 consumed
+    }
+    return;
+  }
+
+  const int half = warp >> 2, wr = warp & 3;
+  const int v0 = v_cta + half * VS;
+  const bool live = v0 < p.p;                                  // a head of 32 or 96 columns leaves a group idle
+  const uint32_t st_tile = sb + SSD_ST + half * SSD_ST_GROUP;
+  // fp32 master copy of S^T: warp wr owns key rows 32 wr .. 32 wr + 31 (two 16-row tiles), all 32 value columns
+  float acc_s[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int kr = 32 * wr + 16 * i + qr + (e >> 1) * 8, vc = 8 * j + qc + (e & 1);
+        acc_s[i][j][e] = p.s_in != nullptr && live
+                             ? p.s_in[(static_cast<long long>(h) * p.p + v0 + vc) * GK + kr] : 0.f;
+      }
+  auto publish_state = [&](int parity) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const int kr = 32 * wr + 16 * i + qr + (e >> 1) * 8, vc = 8 * j + qc;
+          *reinterpret_cast<uint32_t*>(sm + SSD_ST + (2 * parity + half) * SSD_ST_GROUP + kr * P_V + vc * 2) =
+              pack_bf16(acc_s[i][j][e], acc_s[i][j][e + 1]);
+        }
+  };
+  publish_state(0);
+  asm volatile("bar.sync 0, 512;" ::: "memory");
+  for (int c = 0; c < p.nc; ++c) {
+    if (live) {
+      const uint32_t st = sb + (c & 1) * SSD_STAGE;
+      const uint32_t vn = st + SSD_V + half * SSD_VN;
+      const uint32_t s_t = st_tile + (c & 1) * 2 * SSD_ST_GROUP;
+      // Qg S^T and M V': rows 16 wr .. 16 wr + 15 of the chunk
+      float a2[4][4] = {};
+      const uint32_t a_off = (16 * wr + (lane & 15)) * P_K + (lane >> 4) * 16;
+#pragma unroll
+      for (int ks = 0; ks < GK / 16; ++ks) {
+        uint32_t fq[4], b[4][2];
+        ldsm_x4(fq, st + SSD_Q + a_off + ks * 32);
+        load_b32(b, s_t, ks * 16, lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma16816(a2[j], fq, b[j][0], b[j][1]);
+      }
+      const float gamma = __expf(g_end[c & 1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc_s[i][j][e] *= gamma;
+      const uint32_t m_off = (16 * wr + (lane & 15)) * P_M + (lane >> 4) * 16;
+      const int mi = lane >> 3;
+#pragma unroll
+      for (int ks = 0; ks < GC / 16; ++ks) {
+        uint32_t fm[4], b[4][2];
+        ldsm_x4(fm, st + SSD_M + m_off + ks * 32);
+        load_b32(b, vn, ks * 16, lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma16816(a2[j], fm, b[j][0], b[j][1]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          // A = Kd^T: element (key row, token) sits at Kd[token][key row]; blocks as in gdn_chunk_kernel
+          const int row = ks * 16 + (mi >> 1) * 8 + (lane & 7), col = 32 * wr + 16 * i + (mi & 1) * 8;
+          uint32_t fa[4];
+          ldsm_x4_t(fa, st + SSD_KD + row * P_K + col * 2);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) mma16816(acc_s[i][j], fa, b[j][0], b[j][1]);
+        }
+      }
+      publish_state((c + 1) & 1);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const int tok = c * GC + 16 * wr + qr + (e >> 1) * 8, vc = 8 * j + qc;
+          if (tok < p.n)
+            *reinterpret_cast<uint32_t*>(p.o + tok * p.ldo + h * p.p + v0 + vc) = pack_bf16(a2[j][e], a2[j][e + 1]);
+        }
+    }
+    asm volatile("bar.sync 0, 512;" ::: "memory");
+  }
+  if (p.s_out != nullptr && live) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int kr = 32 * wr + 16 * i + qr + (e >> 1) * 8, vc = 8 * j + qc + (e & 1);
+          p.s_out[(static_cast<long long>(h) * p.p + v0 + vc) * GK + kr] = acc_s[i][j][e];
+        }
+  }
+}
+
+}  // namespace
+}  // namespace hb
+
+extern "C" {
+
+// The n rows of one sequence; state dim 128, head dim `p` (a multiple of 32). s_in / s_out fp32 [heads, p, 128] (s_in null =
+// zero state, s_out null = do not store); o bf16 rows of pitch ldo.
+int hb_ssd_chunk(const void* x, const void* b, const void* c, const void* dt, const void* a_log, const void* dt_bias,
+                 long long ldx, long long ldb, long long lddt, int n, int heads, int groups, int p, const void* s_in,
+                 void* s_out, void* o, long long ldo, void* stream) {
+  using namespace hb;
+  if (n <= 0) return 0;
+  if (groups <= 0 || heads % groups != 0 || p < VS || p % VS != 0 || (ldx & 1) || (ldb & 3)) return 1;
+  SsdParams q;
+  q.x = static_cast<const __nv_bfloat16*>(x); q.b = static_cast<const __nv_bfloat16*>(b);
+  q.c = static_cast<const __nv_bfloat16*>(c); q.dt = static_cast<const __nv_bfloat16*>(dt);
+  q.a_log = static_cast<const float*>(a_log); q.dt_bias = static_cast<const float*>(dt_bias);
+  q.ldx = ldx; q.ldb = ldb; q.lddt = lddt;
+  q.s_in = static_cast<const float*>(s_in); q.s_out = static_cast<float*>(s_out);
+  q.o = static_cast<__nv_bfloat16*>(o); q.ldo = ldo;
+  q.n = n; q.nc = (n + GC - 1) / GC; q.heads = heads; q.groups = groups; q.p = p;
+  q.wide = ldb % 8 == 0 && ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(ssd_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SSD_SMEM) != cudaSuccess) return 3;
+    attr = true;
+  }
+  ssd_chunk_kernel<<<dim3(heads, (p + 63) / 64), 512, SSD_SMEM, static_cast<cudaStream_t>(stream)>>>(q);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+}  // extern "C"

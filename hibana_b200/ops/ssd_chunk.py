@@ -5,9 +5,11 @@ exp(gamma_t - gamma_i) for i <= t:
 
     Y   = (L * (C B^T)) (dt * X)  +  (e^gamma * C) h0^T          h_C = e^gamma_C h0 + (e^(gamma_C - gamma) * B)^T (dt * X)
 
-which is the chunk recurrence of the gated delta rule without its W term, so phase 2 is the same state-pass
-kernel (csrc/gdn_chunk.cu, value dim = head dim, key dim = state dim 128) and phase 1 one kernel per (chunk, head)
-(`ssd_phase1_kernel`; a handful of batched PyTorch products on the CPU path). The skip term D * x is added at the end. Only the fp32 state format takes this
+which is the chunk recurrence of the gated delta rule without its W term. On the GPU one kernel does all of it
+(`ssd_chunk_kernel` in csrc/gdn_chunk.cu), or, for long sequences of few heads, one kernel per (chunk, head) forms the
+factors (`ssd_phase1_kernel`) and the delta rule's state-pass kernel (value dim = head dim, key dim = state dim 128)
+follows. Operands that neither takes (a wide dt, odd pitches), `ssd_phase1 = torch` and the CPU path form the
+factors with a handful of batched PyTorch products. The skip term D * x is added at the end. Only the fp32 state format takes this
 path; quantised states keep the token-serial kernel. Reference: hibana/kernels/mamba2.py (chunked SSD prefill).
 """
 from __future__ import annotations
@@ -26,6 +28,7 @@ CHUNK = gdn_chunk.CHUNK
 P, I, L = nv.P, nv.I, nv.L
 nv.register("hb_head_skip", [P, P, L, P, L, I, I, P])
 nv.register("hb_ssd_phase1", [P, P, P, P, P, P, L, L, L, I, I, I, I, P, P, P, P, P, P])
+nv.register("hb_ssd_chunk", [P, P, P, P, P, P, L, L, L, I, I, I, I, P, P, P, L, P])
 
 
 def prepare(x, bmat, cmat, dt, a_log, dt_bias, *, heads: int, groups: int, head_dim: int, d_state: int) -> dict:
@@ -76,6 +79,14 @@ def prepare_native(x, bmat, cmat, dt, a_log, dt_bias, *, heads: int, groups: int
     return out
 
 
+def one_kernel(n: int, heads: int, head_dim: int) -> bool:
+    """Whether n rows take `ssd_chunk_kernel`. Its chunk takes 3.6 us against 2 us for the state pass alone, which is made up
+    for by not writing the factors, by one wave of CTAs instead of two, and in short sequences by one launch less. 64-column
+    heads, one kernel / two: 128 heads x 4096 rows 243 / 476 us, 64 x 2048 123 / 131, 8 (of 128) x 777 51 / 67, but
+    16 x 4096 225 / 162."""
+    return heads * head_dim >= 4096 or n <= 1024
+
+
 def mamba2_chunked(x, bmat, cmat, dt, a_log, dt_bias, dskip, state, slot_in, slot_out, *, heads: int, groups: int,
                    head_dim: int, d_state: int, ranges: Sequence[tuple[int, int]],
                    has_init: Optional[Sequence[int]] = None) -> torch.Tensor:
@@ -91,20 +102,28 @@ def mamba2_chunked(x, bmat, cmat, dt, a_log, dt_bias, dskip, state, slot_in, slo
         fused = (native and cfgmod.current().ssd_phase1 == "cuda" and dt.dtype == torch.bfloat16
                  and bmat.stride(0) == cmat.stride(0) and bmat.stride(0) % 4 == 0 and x.stride(0) % 2 == 0
                  and a_log.dtype == torch.float32 and (dt_bias is None or dt_bias.dtype == torch.float32))
+        init = has_init is None or bool(has_init[b])
+        n = r1 - r0
+        if fused and one_kernel(n, heads, head_dim):
+            nv.check(nv.lib().hb_ssd_chunk(x[r0:r1].data_ptr(), bmat[r0:r1].data_ptr(), cmat[r0:r1].data_ptr(),
+                                           dt[r0:r1].data_ptr(), a_log.data_ptr(), nv.ptr(dt_bias), x.stride(0),
+                                           bmat.stride(0), dt.stride(0), n, heads, groups, head_dim,
+                                           nv.ptr(state[sin[b]] if init else None),
+                                           nv.ptr(state[sout[b]] if sout is not None else None), y[r0:r1].data_ptr(),
+                                           y.stride(0), nv.stream()), "hb_ssd_chunk")
+            continue
         if fused:
             ph = prepare_native(x[r0:r1], bmat[r0:r1], cmat[r0:r1], dt[r0:r1], a_log, dt_bias, heads=heads,
                                 groups=groups, head_dim=head_dim)
         else:
             ph = prepare(x[r0:r1], bmat[r0:r1], cmat[r0:r1], dt[r0:r1], a_log, dt_bias, heads=heads, groups=groups,
                          head_dim=head_dim, d_state=d_state)
-        init = has_init is None or bool(has_init[b])
         if native:
             gdn_chunk._native_pass(ph, state[sin[b]] if init else None, state[sout[b]] if sout is not None else None,
                                    y[r0:r1], heads, d_state, head_dim)
         else:
             s0 = state[sin[b]] if init else torch.zeros_like(state[sin[b]])
             oc, s = gdn_chunk.state_pass_ref(ph, s0)
-            n = r1 - r0
             y[r0:r1] = oc.permute(1, 2, 0, 3).reshape(ph["nc"] * CHUNK, heads * head_dim)[:n].to(y.dtype)
             if sout is not None:
                 state[sout[b]] = s.to(state.dtype)

@@ -130,3 +130,32 @@ def test_phase1_kernel_matches_batched_reference(n):
         a, b = got[name].float(), ref[name].float()
         err = (a - b).abs().max().item()
         assert err <= tol * max(1.0, b.abs().max().item()), (name, err, b.abs().max().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,heads,p", [([1], 4, 64), ([63, 64, 65], 4, 32), ([200, 1, 129], 2, 96), ([513], 8, 64),
+                                          ([320, 17], 2, 128), ([1100], 2, 64)])
+def test_ssd_chunk_kernel_against_the_recurrence(rows, heads, p):
+    """Every factor (Qg, Kd, M, V', the state copy) is rounded to bf16 once and the output once: at most five factors of
+    1 + 2^-9 on a term, so the error stays below 2^-6 of the sum of the terms' magnitudes (2^-7 for the state: two)."""
+    from hibana_b200.ops import ssd_chunk
+    groups, n = 2, 128
+    x, bm, cm, dt, a_log, dtb, _, state, indptr, sin, sout = _mamba_case(rows, heads, groups, p, n, seed=11)
+    has_init = torch.tensor([1, 0, 1][:len(rows)], dtype=torch.int32)
+    kw = dict(heads=heads, groups=groups, head_dim=p, d_state=n)
+
+    def scan(x, b, c, st):
+        y = recurrent.mamba2_scan(x, b, c, dt.double(), a_log.double(), dtb.double(), None, st, sin, sout, q_indptr=indptr,
+                                  has_init=has_init, **kw)
+        return y.double(), st
+    ref, st_ref = scan(x.float(), bm.float(), cm.float(), state.clone())
+    mag, st_mag = scan(x.float().abs(), bm.float().abs(), cm.float().abs(), state.abs())
+    wide = torch.cat([x, bm, cm, torch.zeros(x.shape[0], 4).bfloat16()], 1).cuda()      # one pitch, as the convolution leaves them
+    xs, bs, cs = wide[:, :heads * p], wide[:, heads * p:heads * p + groups * n], wide[:, heads * p + groups * n:-4]
+    st = state.cuda()
+    got = ssd_chunk.mamba2_chunked(xs, bs, cs, dt.cuda(), a_log.cuda(), dtb.cuda(), None, st, sin, sout,
+                                   ranges=recurrent._ranges(indptr, len(rows)), has_init=has_init.tolist(), **kw)
+    assert bool(((got.cpu().double() - ref).abs() <= 2.0 ** -6 * mag + 1e-6).all())
+    end = slice(len(rows), None)
+    assert bool(((st.cpu()[end] - st_ref[end]).abs() <= 2.0 ** -7 * st_mag[end] + 1e-6).all())
+    assert torch.equal(st.cpu()[:len(rows)], state[:len(rows)])
