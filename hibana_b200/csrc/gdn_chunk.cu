@@ -5,8 +5,11 @@
 //     V' = U - W S^T                      [64, V]
 //     O  = Qg S^T + M V'                  [64, V]      (M = masked, decayed Q K^T)
 //     S^T <- gamma S^T + Kd^T V'          [K, V]
-// One CTA per (head, 32 columns of V): the columns of the state are independent, so 4 CTAs share a head. The
-// three products run on mma.sync m16n8k16 (bf16 operands, fp32 accumulate; the tiles are 64 x 32 x 128 and the
+// The columns of the state are independent: a group of four warps owns 32 columns of V. A CTA is one group, or two that
+// share W, Qg, Kd and M where one-group CTAs would not fit the chip at once (one is resident per SM): 48 heads of 128
+// columns are 192 CTAs of one group, two waves on 148 SMs, or 96 of two (4096 tokens 282 -> 188 us, 1237 tokens
+// 93 -> 63). Alone on its SM a CTA of one group is the faster one (12 heads, 1500 tokens: 56 us).
+// The three products run on mma.sync m16n8k16 (bf16 operands, fp32 accumulate; the tiles are 64 x 32 x 128 and the
 // chain is serial in the chunk, so the win over a token-serial scan is the 64-fold shorter chain, not tensor
 // throughput). The fp32 master copy of the state lives in accumulator registers for the whole sequence; a bf16
 // copy in shared memory feeds the products. Chunk inputs are double-buffered with cp.async.
@@ -19,20 +22,28 @@ namespace {
 
 constexpr int GC = 64;            // tokens per chunk
 constexpr int GK = 128;           // key dim
-constexpr int VS = 32;            // value columns per CTA
+constexpr int VS = 32;            // value columns of a group of four warps
 constexpr int P_K = GK * 2 + 16;  // row pitch (bytes) of the [64, 128] bf16 tiles
 constexpr int P_M = GC * 2 + 16;  // [64, 64] bf16
-constexpr int P_U = VS * 4 + 16;  // [64, 32] fp32
 constexpr int P_V = VS * 2 + 16;  // [*, 32] bf16 (V' and S^T)
 constexpr int OFF_W = 0;
 constexpr int OFF_Q = OFF_W + GC * P_K;
 constexpr int OFF_KD = OFF_Q + GC * P_K;
 constexpr int OFF_M = OFF_KD + GC * P_K;
 constexpr int OFF_U = OFF_M + GC * P_M;
-constexpr int STAGE = OFF_U + GC * P_U;
-constexpr int OFF_VN = 2 * STAGE;
-constexpr int OFF_ST = OFF_VN + GC * P_V;
-constexpr int G_SMEM = OFF_ST + GK * P_V;
+constexpr int GDN_VN = GC * P_V;              // one group's V' tile
+constexpr int GDN_ST = GK * P_V;              // one group's copy of S^T
+
+// Shared memory of a CTA of G groups: two stages, V' and S^T of every group.
+template <int G>
+struct ChunkSmem {
+  static constexpr int P_U = G * VS * 4 + 16;  // [64, 32 G] fp32
+  static constexpr int STAGE = OFF_U + GC * P_U;
+  static constexpr int OFF_VN = 2 * STAGE;
+  static constexpr int OFF_ST = OFF_VN + G * GDN_VN;
+  static constexpr int BYTES = OFF_ST + G * GDN_ST;
+};
+static_assert(ChunkSmem<2>::BYTES <= 227 * 1024, "shared memory");
 
 struct ChunkParams {
   const __nv_bfloat16* w;     // [H, NC, 64, 128]; null: no W term (V' = U, the Mamba-2 / SSD recurrence)
@@ -81,11 +92,13 @@ __device__ __forceinline__ void load_b32(uint32_t (&b)[4][2], uint32_t tile, int
   b[2][0] = r[0]; b[2][1] = r[1]; b[3][0] = r[2]; b[3][1] = r[3];
 }
 
-__global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
+template <int G>
+__global__ void __launch_bounds__(128 * G) gdn_chunk_kernel(const ChunkParams p) {
   extern __shared__ __align__(16) uint8_t g_smem[];
   const uint32_t sb = smem_u32(g_smem);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.x, v0 = blockIdx.y * VS;
+  using L = ChunkSmem<G>;
+  const int tid = threadIdx.x, group = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31;
+  const int h = blockIdx.x, v_cta = blockIdx.y * VS * G, v0 = v_cta + group * VS;
   const int qr = lane >> 2, qc = (lane & 3) * 2;   // accumulator row / first column of this lane inside a tile
   const int GV = p.vdim;
 
@@ -95,24 +108,28 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
     const uint8_t* gq = reinterpret_cast<const uint8_t*>(p.qg + tile * GC * GK);
     const uint8_t* gk = reinterpret_cast<const uint8_t*>(p.kd + tile * GC * GK);
     const uint8_t* gm = reinterpret_cast<const uint8_t*>(p.m + tile * GC * GC);
-    const uint8_t* gu = reinterpret_cast<const uint8_t*>(p.u + tile * GC * GV + v0);
+    const uint8_t* gu = reinterpret_cast<const uint8_t*>(p.u + tile * GC * GV + v_cta);
     const bool has_w = p.w != nullptr;
-    const uint32_t st = sb + stage * STAGE;
-    for (int i = tid; i < GC * 16; i += 128) {
+    const uint32_t st = sb + stage * L::STAGE;
+    for (int i = tid; i < GC * 16; i += 128 * G) {
       const int r = i >> 4, ch = (i & 15) * 16;
       if (has_w) cp16g(st + OFF_W + r * P_K + ch, gw + r * (GK * 2) + ch);
       cp16g(st + OFF_Q + r * P_K + ch, gq + r * (GK * 2) + ch);
       cp16g(st + OFF_KD + r * P_K + ch, gk + r * (GK * 2) + ch);
     }
-    for (int i = tid; i < GC * 8; i += 128) {
+    for (int i = tid; i < GC * 8; i += 128 * G) {
       const int r = i >> 3, ch = (i & 7) * 16;
       cp16g(st + OFF_M + r * P_M + ch, gm + r * (GC * 2) + ch);
-      cp16g(st + OFF_U + r * P_U + ch, gu + r * (GV * 4) + ch);
+    }
+    for (int i = tid; i < GC * 8 * G; i += 128 * G) {
+      const int r = i / (8 * G), ch = (i % (8 * G)) * 16;
+      cp16g(st + OFF_U + r * L::P_U + ch, gu + r * (GV * 4) + ch);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  // fp32 master copy of S^T: warp w owns key rows 32w .. 32w + 31 (two 16-row tiles), all 32 value columns
+  const int off_vn = L::OFF_VN + group * GDN_VN, off_st = L::OFF_ST + group * GDN_ST;
+  // fp32 master copy of S^T: warp w of a group owns key rows 32w .. 32w + 31 (two 16-row tiles), all 32 value columns
   float acc_s[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -132,7 +149,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
 #pragma unroll
         for (int e = 0; e < 4; e += 2) {
           const int kr = 32 * warp + 16 * i + qr + (e >> 1) * 8, vc = 8 * j + qc;
-          *reinterpret_cast<uint32_t*>(g_smem + OFF_ST + kr * P_V + vc * 2) =
+          *reinterpret_cast<uint32_t*>(g_smem + off_st + kr * P_V + vc * 2) =
               pack_bf16(acc_s[i][j][e], acc_s[i][j][e + 1]);
         }
   };
@@ -149,7 +166,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    const uint32_t st = sb + stage * STAGE;
+    const uint32_t st = sb + stage * L::STAGE;
     // ---- W S^T and Qg S^T (same B fragments): rows 16 warp .. 16 warp + 15 of the chunk
     float a1[4][4] = {}, a2[4][4] = {};
     const uint32_t a_off = (16 * warp + (lane & 15)) * P_K + (lane >> 4) * 16;
@@ -157,7 +174,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
     for (int ks = 0; ks < GK / 16; ++ks) {
       uint32_t fw[4], fq[4], b[4][2];
       ldsm_x4(fq, st + OFF_Q + a_off + ks * 32);
-      load_b32(b, sb + OFF_ST, ks * 16, lane);
+      load_b32(b, sb + off_st, ks * 16, lane);
       if (p.w != nullptr) {
         ldsm_x4(fw, st + OFF_W + a_off + ks * 32);
 #pragma unroll
@@ -172,8 +189,8 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
 #pragma unroll
       for (int e = 0; e < 4; e += 2) {
         const int r = 16 * warp + qr + (e >> 1) * 8, vc = 8 * j + qc;
-        const float2 u = *reinterpret_cast<const float2*>(g_smem + stage * STAGE + OFF_U + r * P_U + vc * 4);
-        *reinterpret_cast<uint32_t*>(g_smem + OFF_VN + r * P_V + vc * 2) = pack_bf16(u.x - a1[j][e], u.y - a1[j][e + 1]);
+        const float2 u = *reinterpret_cast<const float2*>(g_smem + stage * L::STAGE + OFF_U + r * L::P_U + (group * VS + vc) * 4);
+        *reinterpret_cast<uint32_t*>(g_smem + off_vn + r * P_V + vc * 2) = pack_bf16(u.x - a1[j][e], u.y - a1[j][e + 1]);
       }
     __syncthreads();
     // ---- O += M V'
@@ -182,7 +199,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
     for (int ks = 0; ks < GC / 16; ++ks) {
       uint32_t fm[4], b[4][2];
       ldsm_x4(fm, st + OFF_M + m_off + ks * 32);
-      load_b32(b, sb + OFF_VN, ks * 16, lane);
+      load_b32(b, sb + off_vn, ks * 16, lane);
 #pragma unroll
       for (int j = 0; j < 4; ++j) mma16816(a2[j], fm, b[j][0], b[j][1]);
     }
@@ -205,7 +222,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const ChunkParams p) {
 #pragma unroll
     for (int ks = 0; ks < GC / 16; ++ks) {
       uint32_t b[4][2];
-      load_b32(b, sb + OFF_VN, ks * 16, lane);
+      load_b32(b, sb + off_vn, ks * 16, lane);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         // A = Kd^T: element (key row, token) sits at Kd[token][key row]; the four 8x8 blocks of the fragment are
@@ -256,11 +273,19 @@ int hb_gdn_chunk_pass(const void* w, const void* qg, const void* kd, const void*
   p.o = static_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.nc = nc; p.n = n; p.vdim = vdim;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(gdn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(gdn_chunk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChunkSmem<1>::BYTES) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(gdn_chunk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChunkSmem<2>::BYTES) !=
+            cudaSuccess)
       return 3;
     attr = true;
   }
-  gdn_chunk_kernel<<<dim3(heads, vdim / VS), 128, G_SMEM, static_cast<cudaStream_t>(stream)>>>(p);
+  // One group per CTA while all CTAs are resident at once (a CTA of one group is a little faster by itself).
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (vdim % (2 * VS) == 0 && heads * (vdim / VS) > 148)
+    gdn_chunk_kernel<2><<<dim3(heads, vdim / (2 * VS)), 256, ChunkSmem<2>::BYTES, st>>>(p);
+  else
+    gdn_chunk_kernel<1><<<dim3(heads, vdim / VS), 128, ChunkSmem<1>::BYTES, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

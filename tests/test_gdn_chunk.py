@@ -159,3 +159,23 @@ def test_ssd_chunk_kernel_against_the_recurrence(rows, heads, p):
     end = slice(len(rows), None)
     assert bool(((st.cpu()[end] - st_ref[end]).abs() <= 2.0 ** -7 * st_mag[end] + 1e-6).all())
     assert torch.equal(st.cpu()[:len(rows)], state[:len(rows)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 64, 130])
+def test_state_pass_groups_per_cta(rows):
+    """38 heads of 128 columns are more one-group CTAs than SMs, so a CTA is two groups; 19 heads are not. Same sums."""
+    g = torch.Generator().manual_seed(rows)
+    vh = 38
+    q, k = (torch.randn(rows, vh * 128, generator=g).bfloat16().cuda() for _ in range(2))
+    v = torch.randn(rows, vh * 128, generator=g).bfloat16().cuda()
+    gl, beta = -torch.rand(rows, vh, generator=g).cuda(), torch.rand(rows, vh, generator=g).cuda()
+    s_in = (torch.randn(vh, 128, 128, generator=g) * 0.1).cuda()
+    ph = gdn_chunk.prepare_native(q, k, v, gl, beta, k_heads=vh, v_heads=vh, scale=128 ** -0.5, l2norm=True)
+    out, s_out = torch.zeros(rows, vh * 128, dtype=torch.bfloat16, device="cuda"), torch.zeros_like(s_in)
+    gdn_chunk._native_pass(ph, s_in, s_out, out, vh, 128, 128)
+    for h0 in (0, 19):
+        part = {n: t[h0:h0 + 19] if torch.is_tensor(t) else t for n, t in ph.items()}
+        o, s = torch.zeros(rows, 19 * 128, dtype=torch.bfloat16, device="cuda"), torch.zeros_like(s_in[:19])
+        gdn_chunk._native_pass(part, s_in[h0:h0 + 19], s, o, 19, 128, 128)
+        assert torch.equal(o, out[:, h0 * 128:(h0 + 19) * 128]) and torch.equal(s, s_out[h0:h0 + 19])
