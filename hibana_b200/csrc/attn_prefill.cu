@@ -189,8 +189,9 @@ __device__ __forceinline__ void pf_fill_q16(const PfParams& p, const PfBlock& x,
   }
 }
 
-// The producer warps: K and V tiles of the block's keys into their rings (and, for bf16 pools, the Q rows).
-template <int D, bool F8, int PF_PRODUCERS, int NS>
+// The producer warps: K and V tiles of the block's keys into their rings of NS stages (and, for bf16 pools, the Q rows). Tile t
+// is announced on full barrier t % NF.
+template <int D, bool F8, int PF_PRODUCERS, int NS, int NF>
 __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, const CUtensorMap& tmk, const CUtensorMap& tmv,
                                            uint8_t* q_s, uint8_t* k_s, uint8_t* v_s, uint64_t* kfull, uint64_t* vfull,
                                            uint64_t* kempty, uint64_t* vempty, volatile int* abort, int ptid, int lane) {
@@ -237,13 +238,13 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
       const uint32_t ph = ((t / NS) - 1) & 1;
       load(p.v_pool, sl_now, vreg);
       if (t >= NS && !mbar_wait(&kempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
-      store(k_s + s * C::KV_TILE, kreg, &kfull[s]);
+      store(k_s + s * C::KV_TILE, kreg, &kfull[t % NF]);
       load(p.k_pool, sl_next, kreg);
 #pragma unroll
       for (int i = 0; i < PER; ++i) sl_now[i] = sl_next[i];
       slots(t + 2, sl_next);
       if (t >= NS && !mbar_wait(&vempty[s], ph, abort, p.status, kTimeoutEmpty)) break;
-      store(v_s + s * C::KV_TILE, vreg, &vfull[s]);
+      store(v_s + s * C::KV_TILE, vreg, &vfull[t % NF]);
     }
   } else {
   // Q rows (zero padded); they travel in the first cp.async group, i.e. with K tile 0.
@@ -332,7 +333,7 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
       }
       {
         PF_T0();
-        copy_tile(t + 1, sl_k, p.k_pool, &tmk, k_s, &kfull[(t + 1) % NS]);
+        copy_tile(t + 1, sl_k, p.k_pool, &tmk, k_s, &kfull[(t + 1) % NF]);
         PF_ACC(8, ptid == 0);
       }
     }
@@ -348,7 +349,7 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
     }
     {
       PF_T0();
-      copy_tile(t, sl_v, p.v_pool, &tmv, v_s, &vfull[t % NS]);
+      copy_tile(t, sl_v, p.v_pool, &tmv, v_s, &vfull[t % NF]);
       PF_ACC(8, ptid == 0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -356,8 +357,8 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
     asm volatile("cp.async.wait_group 2;" ::: "memory");
     PF_ACC(9, ptid == 0);
     fence_proxy_async_smem();
-    mbar_arrive(&kfull[t % NS]);
-    if (t >= 1) mbar_arrive(&vfull[(t - 1) % NS]);
+    mbar_arrive(&kfull[t % NF]);
+    if (t >= 1) mbar_arrive(&vfull[(t - 1) % NF]);
 #pragma unroll
     for (int i = 0; i < SB; ++i) {
       sl_v[i] = sl_k[i];
@@ -366,7 +367,7 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing may land after the CTA has gone
   fence_proxy_async_smem();
-  if (live) mbar_arrive(&vfull[(ntiles - 1) % NS]);
+  if (live) mbar_arrive(&vfull[(ntiles - 1) % NF]);
   }
 }
 
@@ -434,7 +435,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 
   if (warp >= 4 && warp < ISSUER) {
     // ------------------------------------------------------------------ producers
-    pf_produce<D, F8, PF_PRODUCERS, PF_STAGES>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty, abort, tid - 128, lane);
+    pf_produce<D, F8, PF_PRODUCERS, PF_STAGES, PF_STAGES>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty, abort,
+                                                          tid - 128, lane);
   } else if (warp == ISSUER) {
     // ------------------------------------------------------------------ MMA issuer
     {   // the whole warp walks the loop, one elected lane issues (hb_common.cuh, elect_one)
@@ -685,6 +687,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 // softmax; the rest is the chain of barriers around the two MMAs and K tiles that arrive late (copies of 32 rows; with
 // warps of their own for K and V they came no earlier, and the layer took 125 us).
 constexpr int PP_STAGES = 3;      // K and V rings, shared by both streams
+// Full barriers of a ring. A wait on a phase parity cannot tell phase n from phase n + 2, so whoever waits on a barrier has to
+// wait for every one of its phases. With one barrier per stage a stream would see only every second phase: tile t could
+// pass its wait while the other stream's tile t - 3, whose bulk copies may land later than those of tile t - 2, is still on
+// its way into that stage. Two barriers per stage make each of them one stream's own (t % 6 is even or odd as t is). The
+// empty barriers need no such care: their only waiters, the producers, wait for all phases.
+constexpr int PP_FULL = 2 * PP_STAGES;
+struct PpPlace {
+  int stage, full, parity;        // ring stage, full barrier, and the parity of that barrier's phase
+};
+__host__ __device__ constexpr PpPlace pp_place(int t) { return {t % PP_STAGES, t % PP_FULL, (t / PP_FULL) & 1}; }
 template <bool F8>
 struct PpRoles {                  // warps 0-3 and 4-7 softmax, then the producers, then one issuer per stream
   static constexpr int PROD_WARPS = F8 ? 8 : 3;
@@ -697,6 +709,7 @@ struct PpCfg {
   static constexpr int KT = 128;
   static constexpr int BAR_OFF = PfCfg<D, F8>::Q_BYTES + 2 * PP_STAGES * PfCfg<D, F8>::KV_TILE;
   static constexpr int SCALE_OFF = BAR_OFF + 256;                  // F8: one scale per packed query row
+  static_assert((2 * PP_FULL + 2 * PP_STAGES + 6) * 8 + 8 <= 256, "barriers, TMEM address and abort flag");
   static constexpr int SMEM = SCALE_OFF + (F8 ? PF_ROWS * 4 : 0) + 1024;
   static_assert(PfCfg<D, F8>::KT == KT && 2 * KT + 2 * D <= 512, "a score buffer and an accumulator per stream");
 };
@@ -777,8 +790,8 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
   uint8_t* k_s = smem + C::Q_BYTES;
   uint8_t* v_s = k_s + PP_STAGES * C::KV_TILE;
   uint64_t* kfull = reinterpret_cast<uint64_t*>(smem + PpCfg<D, F8>::BAR_OFF);
-  uint64_t* vfull = kfull + PP_STAGES;
-  uint64_t* kempty = vfull + PP_STAGES;
+  uint64_t* vfull = kfull + PP_FULL;
+  uint64_t* kempty = vfull + PP_FULL;
   uint64_t* vempty = kempty + PP_STAGES;
   uint64_t* s_ready = vempty + PP_STAGES;      // from here on one per stream
   uint64_t* p_ready = s_ready + 2;
@@ -795,9 +808,11 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
   const int ntiles = x.ntiles;
 
   if (tid == 0) {
-    for (int s = 0; s < PP_STAGES; ++s) {
+    for (int s = 0; s < PP_FULL; ++s) {
       mbar_init(&kfull[s], PpRoles<F8>::PRODUCERS);
       mbar_init(&vfull[s], PpRoles<F8>::PRODUCERS);
+    }
+    for (int s = 0; s < PP_STAGES; ++s) {
       mbar_init(&kempty[s], 1);
       mbar_init(&vempty[s], 1);
     }
@@ -827,8 +842,8 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp >= 8 && warp < ISSUER) {
-    pf_produce<D, F8, PpRoles<F8>::PRODUCERS, PP_STAGES>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty, abort, tid - 256,
-                                              lane);
+    pf_produce<D, F8, PpRoles<F8>::PRODUCERS, PP_STAGES, PP_FULL>(p, x, tmk, tmv, q_s, k_s, v_s, kfull, vfull, kempty, vempty,
+                                                                  abort, tid - 256, lane);
   } else if (warp >= ISSUER) {
     // ------------------------------------------------------------------ MMA issuer of one stream
     constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);      // operand format codes of kind::f16: 0 = fp16, 1 = bf16
@@ -838,14 +853,14 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
     const uint32_t q_a = __shfl_sync(0xffffffffu, smem_u32(q_s), 0);
     const uint32_t s_t = tmem_base + st * KT, o_t = tmem_base + 2 * KT + st * D;
     for (int t = st, i = 0; t < ntiles; t += 2, ++i) {
-      const int s = t % PP_STAGES;
-      const uint32_t ring = (t / PP_STAGES) & 1;
+      const PpPlace at = pp_place(t);
+      const int s = at.stage;
       const uint32_t k_a = q_a + C::Q_BYTES + s * C::KV_TILE, v_a = k_a + PP_STAGES * C::KV_TILE;
       // the score buffer holds P(t - 2) until that tile's O += P V is done
       if (i > 0 && !warp_wait(&pv_done[st], (i - 1) & 1, abort, p.status, kTimeoutAccum)) break;
       {
         PF_T0();
-        if (!warp_wait(&kfull[s], ring, abort, p.status, kTimeoutFull)) break;
+        if (!warp_wait(&kfull[at.full], at.parity, abort, p.status, kTimeoutFull)) break;
         PF_ACC(5, lane == 0 && st == 0);
       }
       tc_fence_after();
@@ -867,7 +882,7 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
       }
       {
         PF_T0();
-        if (!warp_wait(&vfull[s], ring, abort, p.status, kTimeoutFull)) break;
+        if (!warp_wait(&vfull[at.full], at.parity, abort, p.status, kTimeoutFull)) break;
         PF_ACC(4, lane == 0 && st == 0);
       }
       tc_fence_after();
@@ -1068,6 +1083,14 @@ extern "C" {
 // [8] producer issues copies, [9] producer waits for landed copies, [10] softmax loop total, [11] tiles,
 // [12] softmax score load, [13] softmax math incl. the wait for the previous O update, [14] publish P.
 void hb_attn_prefill_profile(void* buf) { g_pf_prof = static_cast<unsigned long long*>(buf); }
+
+// Ring stage, full barrier and barrier parity of tile `t` in the two-stream kernel: place[0..2].
+void hb_attn_prefill_place(int t, int* place) {
+  const PpPlace at = pp_place(t);
+  place[0] = at.stage;
+  place[1] = at.full;
+  place[2] = at.parity;
+}
 
 // bf16 KV with head dim 64, 128 or 256, or e4m3 KV (`kv_fp8`: x = code * kv_scale) with head dim 128 or 256, slot and head
 // strides multiples of 16 and 16-byte aligned pools; group size hq / hkv <= 128. `max_rows` bounds the new rows of any

@@ -127,6 +127,7 @@ int hb_attn_merge(const void* part_o, const void* part_lse, void* out, long long
                   void* stream);
 // Tensor-core flash-decoding (attn_decode.cu): bf16 KV, rows_per_sequence * (hq / hkv) <= 16.
 // Prefill / chunked-prefill attention on tcgen05 (bf16 KV, head dim 64 or 128); any number of new rows per sequence.
+void hb_attn_prefill_place(int t, int* place);
 int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                     long long head_stride,
                     const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,

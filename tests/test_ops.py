@@ -643,3 +643,45 @@ def test_splits_fill_one_wave_before_they_get_short(batch, hkv, ctx):
         assert ctx // s >= 256
     elif ctx >= 148 // (batch * hkv) * attention.MIN_SPLIT_KEYS:      # keys enough for the whole wave: nearly all of it
         assert batch * hkv * s >= 0.9 * 148
+
+
+@pytest.mark.parametrize("ntiles", [1, 2, 3, 7, 40])
+def test_prefill_waits_cover_their_tile_cpu(ntiles):
+    """The two-stream prefill kernel's full barriers, replayed on the host: copies may land in any order, and still no stream
+    may pass its wait for a tile that has not landed."""
+    import ctypes
+    import random
+
+    from hibana_b200 import build_native
+    lib = ctypes.CDLL(str(build_native.build()))
+
+    def place(t):
+        out = (ctypes.c_int * 3)()
+        lib.hb_attn_prefill_place(t, out)
+        return tuple(out)
+
+    for seed in range(200):
+        rng = random.Random(seed)
+        phases = {}                              # completed phases per barrier
+        landed, used, flying = set(), set(), []
+        issued, nxt = 0, [0, 1]                  # nxt: the tile each stream waits for
+        for _ in range(100 * ntiles):
+            what = rng.choice(["issue", "land", 0, 1])
+            if what == "issue" and issued < ntiles:
+                # a stage is free once the tile before it there has been used (nobody else writes the stage)
+                before = [t for t in range(issued) if place(t)[0] == place(issued)[0]]
+                if all(t in used for t in before):
+                    flying.append(issued)
+                    issued += 1
+            elif what == "land" and flying:
+                t = flying.pop(rng.randrange(len(flying)))
+                landed.add(t)
+                phases[place(t)[1]] = phases.get(place(t)[1], 0) + 1
+            elif what in (0, 1) and nxt[what] < ntiles:
+                t = nxt[what]
+                _, bar, parity = place(t)
+                if phases.get(bar, 0) & 1 != parity:         # what a parity wait returns
+                    assert t in landed, (seed, t)
+                    used.add(t)
+                    nxt[what] = t + 2
+        assert min(nxt) >= ntiles, nxt
