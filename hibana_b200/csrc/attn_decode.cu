@@ -14,8 +14,8 @@
 //     memory at the end, and KV splits merge through the LSE kernel of attn.cu.
 //
 // e4m3 pools (F8): the tiles hold the codes, which expand to fp16 in registers on their way into the MMAs (exactly; two
-// codes per conversion). The softmax weights enter O += P V as two fp16 terms, hi + lo, 22 bits together: the
-// error against 64-bit attention is that of fp32 weights. Measured per layer against the CUDA-core kernel of attn.cu:
+// codes per conversion). The softmax weights enter O += P V times 2^15 as two fp16 terms, hi + lo: weights down to 2^-18 of
+// the largest keep 22 bits, smaller ones are exact to 2^-40 of it (split_f16). Measured per layer against the CUDA-core kernel of attn.cu:
 // 2 x 30011 keys, 40 / 8 heads of 128: 116 -> 36 us (3.4 TB/s); 16 x 8192, 32 / 2 heads: 180 -> 53 us; 4 x 5003, 24 / 4
 // heads of 256: 102 -> 20 us.
 //
@@ -96,8 +96,13 @@ __device__ __forceinline__ uint32_t e4m3x2_f16(uint32_t two) {
   asm("{\n\t.reg .b16 t;\n\tcvt.u16.u32 t, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, t;\n\t}" : "=r"(r) : "r"(two));
   return r;
 }
-// Softmax weights of two keys as fp16 pairs hi + lo (22 significant bits together, as good as fp32 weights).
+// Softmax weights of two keys (at most 1) times 2^15 as fp16 pairs hi + lo. Without the factor, weights below 2^-14 would
+// fall on the fp16 subnormal grid and those below 2^-25 vanish, although the row sum counts them: with one dominant key of
+// small V over 30011 keys at 2^-24 the output was 2.5e-2 off, with it 2.5e-7 (fp32 weights: 1e-9; the output is bf16).
+constexpr float kWeightScale = 32768.f, kWeightUnscale = 1.f / 32768.f;
 __device__ __forceinline__ void split_f16(float a, float b, uint32_t* hi, uint32_t* lo) {
+  a *= kWeightScale;
+  b *= kWeightScale;
   const __half2 h = __floats2half2_rn(a, b);
   const __half2 l = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
   *hi = *reinterpret_cast<const uint32_t*>(&h);
@@ -651,7 +656,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
         }
       }
       float val = lt > 0.f ? acc / lt : 0.f;
-      if constexpr (F8) val *= p.kv_scale;
+      if constexpr (F8) val *= p.kv_scale * kWeightUnscale;
       const int rr = qi / g, gg = qi % g;
       const long long rh = static_cast<long long>(row0 + rr) * p.hq + kvh * g + gg;
       if (direct) {

@@ -20,9 +20,11 @@
 // e4m3 pools (F8) run the same pipeline in fp16, to which every e4m3 code expands exactly: eight producer warps load
 // 16 codes per lane, expand them in registers and store the swizzled tiles (two loads in flight per lane: K of the next
 // tile, V of this one). Q rows become fp16 under a power-of-two row scale (exact down to 2^-31 of the row's
-// largest element), and P is the sum of two fp16 tiles, hi + lo, so that the softmax weights keep 22 bits: O += hi V +
-// lo V. Against the fp32 CUDA-core kernel of attn.cu: 4096 tokens, 32 / 2 heads of 128: 8050 -> 390 us; 1237 + 263 tokens,
-// 24 / 4 heads of 256: 2170 -> 87 us. What bounds it is the chain scores -> softmax -> P -> O of each tile, not the MMAs.
+// largest element), and P is the sum of two fp16 tiles, hi + lo: O += hi V + lo V. So that small weights do not fall on the
+// fp16 subnormal grid, O and the row sum refer to a value below the running maximum (pf_reference): weights down to 2^-14
+// of the largest keep 22 bits, smaller ones are exact to 2^-36 of it. Against the fp32 CUDA-core kernel of attn.cu: 4096
+// tokens, 32 / 2 heads of 128: 8050 -> 390 us; 1237 + 263 tokens, 24 / 4 heads of 256: 2170 -> 87 us. What bounds it is
+// the chain scores -> softmax -> P -> O of each tile, not the MMAs.
 //
 // Few rows on a long context leave most SMs idle, so the context can be cut into splits (merged by hb_attn_merge): 4 rows
 // on 30000 keys, 24 / 4 heads of 256: 1050 us as one range, 63 us in 37.
@@ -84,7 +86,7 @@ struct PfCfg {
   static constexpr int BAR_OFF = Q_BYTES + 2 * PF_STAGES * KV_TILE + P_BYTES * (F8 ? 2 : 1);
   static constexpr int SMEM = BAR_OFF + 256 + (F8 ? PF_ROWS * 4 : 0) + 1024;   // F8: one scale per packed query row
   static constexpr int TMEM_COLS = 512;                      // S0 [0, KT) S1 [KT, 2 KT) O [2 KT, 2 KT + D)
-  static constexpr float RESCALE_GAP = 8.f;                  // log2 units
+  static constexpr float RESCALE_GAP = F8 ? 4.f : 8.f;       // log2 units; F8: weights stay below 2^(11 + 4), in fp16 range
 };
 
 __device__ __forceinline__ void cp16(uint32_t saddr, const void* g) {
@@ -94,6 +96,16 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// What a row's weights refer to (log2 units) when `mx` is its largest raw score. F8: 2^11 below the maximum. Without that, the
+// weights below 2^-14 of the maximum would be fp16 subnormals and those below 2^-25 vanish, although the row sum counts
+// them: with one dominant key of small V over 30011 keys at 2^-24 the output was 2.5e-2 off, now 4e-6 (the output is bf16). As
+// part of the reference it costs nothing per weight; as a factor on every weight it cost 3 %. Maxima of 2^20 and more stay
+// as they are: there a difference is rounded to steps that could take a weight out of the fp16 range.
+template <bool F8>
+__device__ __forceinline__ float pf_reference(float mx, float scale_log2) {
+  const float m = __fmul_rn(mx, scale_log2);
+  return F8 && fabsf(m) < 1048576.f ? m - 11.f : m;
 }
 // Cycle accounting of one representative thread per role (softmax thread 0, producer 0, the issuer), summed over
 // CTAs into p.prof: where each role's time goes. Costs one predictable branch per site when off.
@@ -546,7 +558,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         for (int j = 0; j < 32; ++j)
           mx4[j & 3] = fmaxf(mx4[j & 3], j <= rc ? __uint_as_float(v[j]) : -INFINITY);
       }
-      const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+      const float m_tile = pf_reference<F8>(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), scale_log2);
       // P(t) overwrites the buffer O += P(t - 1) V(t - 1) reads, and a rescale touches O: both need that MMA done.
       {
         PF_T0();
@@ -589,7 +601,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           // F8: product and difference rounded one after the other, as the maximum was, so that the largest score gives
-          // exactly 2^0 whatever its size (a fused product of scores near 2^40 would overflow the exponential)
+          // the same power of two whatever its size (a fused product of scores near 2^40 would overflow the exponential)
           const float x0 = F8 ? __fadd_rn(__fmul_rn(__uint_as_float(v[j]), scale_log2), neg_m)
                               : fmaf(__uint_as_float(v[j]), scale_log2, neg_m);
           const float x1 = F8 ? __fadd_rn(__fmul_rn(__uint_as_float(v[j + 1]), scale_log2), neg_m)
@@ -749,7 +761,7 @@ __device__ __forceinline__ float pp_weights(uint32_t s_t, int keys, int rel, flo
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
       // F8: product and difference rounded one after the other, as the maximum was, so that the largest score gives
-      // exactly 2^0 whatever its size (a fused product of scores near 2^40 would overflow the exponential; the paired
+      // the same power of two whatever its size (a fused product of scores near 2^40 would overflow the exponential; the paired
       // mul and add came out fused)
       float p0, p1;
       if constexpr (F8) {
@@ -941,7 +953,7 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
           for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], j <= rc ? __uint_as_float(v[j]) : -INFINITY);
         }
       }
-      const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+      const float m_tile = pf_reference<F8>(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), scale_log2);
       if (i == 0) {
         m_ref = m_tile;
       } else if (__any_sync(0xffffffffu, m_tile > m_ref + C::RESCALE_GAP)) {

@@ -685,3 +685,32 @@ def test_prefill_waits_cover_their_tile_cpu(ntiles):
                     used.add(t)
                     nxt[what] = t + 2
         assert min(nxt) >= ntiles, nxt
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hq,hkv,d,rows", [(40, 8, 128, 1), (40, 8, 128, 3), (40, 8, 128, 20), (24, 4, 256, 1),
+                                           (24, 4, 256, 2), (24, 4, 256, 50)])
+@pytest.mark.parametrize("dominant", [11.0, 16.0, 18.0])
+def test_fp8_kv_attention_keeps_small_weights(hq, hkv, d, rows, dominant):
+    """One key of V = 0 that outweighs each of 3000 others by e^11 to e^18 (2^16 to 2^26): the output is the sum of weights
+    that are tiny against the largest. Bound: one rounding to bf16 (2^-9 of the value, 2^-8 allowed) and 1e-4 of a row's
+    root mean square for the weights (exact to 2^-38 of the largest: at 2^-26 that is 2^-12 each, averaged over 3000)."""
+    gen = torch.Generator().manual_seed(5)
+    ctx_n = 3001
+    k = torch.randn(ctx_n + 1, hkv, d, generator=gen)
+    v = torch.randn(ctx_n + 1, hkv, d, generator=gen) + 0.5
+    k[1], v[1] = dominant, 0.0
+    k, v = k.to(torch.float8_e4m3fn), v.to(torch.float8_e4m3fn)
+    q = torch.ones(rows, hq, d, dtype=torch.bfloat16)
+    idx = torch.arange(1, ctx_n + 1, dtype=torch.int32)[None]
+    ctx, indptr = torch.tensor([ctx_n], dtype=torch.int32), torch.tensor([0, rows], dtype=torch.int32)
+    s = torch.einsum("chd->hc", k[1:].double()) / d                       # every query is ones
+    mask = torch.arange(ctx_n)[None, :] > (ctx_n - rows + torch.arange(rows))[:, None]
+    p = torch.softmax(s[None].expand(rows, -1, -1).masked_fill(mask[:, None, :], float("-inf")), -1)
+    ref = torch.einsum("rhc,chd->rhd", p, v[1:].double()).repeat_interleave(hq // hkv, 1)
+    for splits in (1, 5):
+        got = attention.paged_attention(q.cuda(), k.cuda(), v.cuda(), idx.cuda(), ctx.cuda(), q_indptr=indptr.cuda(),
+                                        max_rows=rows, scale=1.0 / d, splits=splits).double().cpu()
+        bound = 2.0 ** -8 * ref.abs() + 1e-4 * ref.pow(2).mean(-1, keepdim=True).sqrt()
+        assert bool(((got - ref).abs() <= bound).all()), ((got - ref).abs() / bound).max().item()
+    assert nv.read_status() == 0
