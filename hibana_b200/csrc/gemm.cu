@@ -32,6 +32,7 @@
 #include <mutex>
 #include <unordered_map>
 #include <memory>
+#include <cstdlib>
 #include <cstring>
 
 #include "hb_common.cuh"
@@ -1000,11 +1001,14 @@ cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorM
           (void)cudaGetLastError();
           n = -1;
         }
-        // The query counts one CTA per SM for a kernel that allocates tensor memory. Two do run where shared memory and
-        // tensor memory hold two (BN <= 64): with 148 slots assumed, K was cut half as often as the chip has room for.
-        max_clusters[splits] = BN <= 64 && n > 0 ? 2 * n : n;
+        max_clusters[splits] = n;
       }
-      if (max_clusters[splits] >= tiles) break;
+      // The query counts one CTA per SM for a kernel that allocates tensor memory. Two do run where shared memory and
+      // tensor memory hold two (BN <= 64): with 148 slots assumed, K was cut half as often as the chip has room for. A
+      // negative split count asks for the wider tiles' limit at every width: the same cuts, so the same order of sums,
+      // whatever the number of tokens.
+      const int room = max_clusters[splits];
+      if ((BN <= 64 && a.splits > 0 ? 2 * room : room) >= tiles) break;
     }
     p.splits = splits;
     grid.z = splits;
@@ -1068,10 +1072,10 @@ static void out_dims(const GemmArgs& a, int* rows, int* cols) {
 }
 
 size_t gemm_workspace_bytes(const GemmArgs& a) {
-  if (a.splits <= 1) return 0;
+  if (std::abs(a.splits) <= 1) return 0;
   int r, c;
   out_dims(a, &r, &c);
-  return static_cast<size_t>(a.splits) * r * c * sizeof(float);
+  return static_cast<size_t>(std::abs(a.splits)) * r * c * sizeof(float);
 }
 
 int gemm_num_tiles(const GemmArgs& a) { return ((a.ra + BM - 1) / BM) * ((a.rb + a.bn - 1) / a.bn); }
@@ -1093,7 +1097,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   if (fp4 && a.bn < 128 && tiles_b != 1 && !grouped) return cudaErrorInvalidValue;
   if (fp4 && grouped && a.bn < 128 && a.grp_chunks != 1) return cudaErrorInvalidValue;
   if (fp4 && (a.sf_k_atoms_a < k_tiles * 4 || a.sf_k_atoms_b < k_tiles * 4)) return cudaErrorInvalidValue;
-  int splits = a.splits < 1 || grouped ? 1 : a.splits;
+  int splits = a.splits == 0 || grouped ? 1 : std::abs(a.splits);      // negative: see launch_t
   if (splits > k_tiles) splits = k_tiles;
   // Every split must own at least one K tile.
   while (splits > 1 && (splits - 1) * ((k_tiles + splits - 1) / splits) >= k_tiles) --splits;

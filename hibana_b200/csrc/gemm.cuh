@@ -76,7 +76,7 @@ struct GemmArgs {
   const float* alpha_ptr;  // optional device scalar multiplied into alpha (dynamic activation scale)
   int epilogue;
   int swap;
-  int splits;           // split-K factor (>= 1)
+  int splits;           // split-K factor, lowered to what is co-resident; negative: lowered alike at every tile width
   float* workspace;     // splits > 1: fp32 [splits][out rows][out cols]
   int* counters;        // splits > 1: one int per output tile, zero before the first launch, self-resetting
   int* status;          // device status word (may be null)

@@ -47,7 +47,8 @@ def set_pdl(on) -> None:
 
 
 def _plan(m: int, n: int, k_tiles: int, max_ws_bytes: int) -> tuple[bool, int, int]:
-    """(swap, bn, splits) for an [m tokens] x [n features] problem."""
+    """(swap, bn, splits) for an [m tokens] x [n features] problem. Negative splits: the launch may lower their number to
+    fit the chip, but by the same amount at every tile width."""
     if m <= 256:
         bn = next(b for b in (16, 32, 64, 128, 256) if b >= m)
         tiles = (n + 127) // 128
@@ -62,6 +63,8 @@ def _plan(m: int, n: int, k_tiles: int, max_ws_bytes: int) -> tuple[bool, int, i
             # Fill the resident CTA slots without spilling into a second, mostly empty wave; every split keeps at
             # least two K tiles.
             splits = max(1, min(slots // tiles, k_tiles // 2, cfgmod.current().max_splits))
+        if cfgmod.current().stable_numerics and splits > 1:
+            splits = -splits
         return True, bn, splits
     return False, (256 if n >= 256 else 128), 1
 

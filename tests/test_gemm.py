@@ -255,3 +255,42 @@ def test_gemm_nvfp4_sm_pairs(m, n, k, epi):
         ref = acc if res is None else acc + res.double()
         bound = 2.0 ** -8 * (ref.abs() + (acc.abs() if res is not None else 0)) + err
     assert bool(((y.double() - ref).abs() <= bound + 1e-30).all())
+
+
+@pytest.mark.parametrize("n,k_tiles", [(5120, 80), (256, 20), (34816, 20)])
+def test_stable_plan_does_not_depend_on_rows_cpu(n, k_tiles):
+    from hibana_b200 import config as cfgmod
+    with cfgmod.using(stable_numerics=True):
+        plans = {gemm._plan(m, n, k_tiles, 0)[2] for m in (1, 16, 64, 65, 128, 129, 256)}
+    assert len(plans) == 1
+    s = plans.pop()
+    assert s == 1 or s < -1       # negative: the launch lowers the number alike at every tile width
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k", [(5120, 5120), (1024, 17408), (7168, 5120)])
+@pytest.mark.parametrize("fmt", ["bf16", "nvfp4", "fp8"])
+def test_stable_numerics_rows_keep_their_bits_at_any_batch(n, k, fmt):
+    """Under `stable_numerics` a row of a projection has the same bits however many rows share the call, on either side of
+    the 64-token tile (two CTAs per SM) and of the 128-token one."""
+    from hibana_b200 import config as cfgmod
+    from hibana_b200.ops import fp8
+    torch.manual_seed(4)
+    x = torch.randn(256, k, device="cuda").bfloat16()
+    w = torch.randn(n, k, device="cuda") * 0.02
+    if fmt == "bf16":
+        wb = w.bfloat16()
+        run = lambda rows: gemm.linear_bf16(rows, wb, epilogue=gemm.EPI_STORE_F32)
+    elif fmt == "nvfp4":
+        wq, gs = nvfp4.quantize_weight(w), torch.tensor(6.0 / (6 * 448), device="cuda")
+        alpha = (gs * wq.gscale).reshape(1)
+        run = lambda rows: gemm.linear_nvfp4(nvfp4.quantize(rows, gs), wq, alpha, epilogue=gemm.EPI_STORE_F32)
+    else:
+        w8, scale = fp8.Fp8Weight.quantize(w), torch.tensor([6.0 / 448], device="cuda")
+        run = lambda rows: fp8.linear_fp8(fp8.quantize_static(rows, scale), w8, x_scale=scale, epilogue=gemm.EPI_STORE_F32)
+    with cfgmod.using(stable_numerics=True):
+        want = run(x[:1]).clone()
+        for m in (2, 16, 64, 65, 80, 128, 130, 256):
+            assert torch.equal(run(x[:m])[:1], want), m
+            assert m < 80 or torch.equal(run(x[:m])[:64], run(x[:64])), m
+    assert nv.read_status() == 0
