@@ -15,7 +15,6 @@ import numpy as np
 import torch
 
 from .. import _native as nv
-from .. import config as cfgmod
 from ..ops import attention, sampling
 from .context import DECODE, PREFILL, VERIFY, ForwardContext
 
@@ -337,14 +336,15 @@ class ModelRunner:
         last = torch.from_numpy(indptr[1:].astype(np.int64) - 1).to(dev) if want == "last" else None
         t = self.model.target
         max_rows = max(counts)
-        splits = 1
-        if cfgmod.current().stable_numerics:
-            pass
-        elif t.attn_layers and b * t.kv_heads * max(1, max_rows // max(1, 32 // max(1, t.q_heads // max(t.kv_heads, 1)))) < 148:
-            splits = attention.choose_splits(b, t.kv_heads, int(ctx_len.max()))
+        splits, workspace = 1, None
+        if t.attn_layers:
+            splits = attention.forward_splits(self.kv.k[0], self.kv.v[0], b, t.q_heads, t.kv_heads, t.head_dim, max_rows,
+                                              int(ctx_len.max()))
+            if splits > 1 and dev.type == "cuda":      # one for all layers
+                workspace = attention.AttnWorkspace(total, t.q_heads, t.head_dim, splits, dev)
         ctx = ForwardContext(mode, positions=pos_d, slots=slots_d, kv_indices=self.block_table, ctx_len=ctx_d,
                              q_indptr=indptr_d, seq_rows=seq_rows_d, max_rows=max_rows, batch=b, sample_rows=last,
-                             attn_splits=splits, comm=self.comm, seq_starts_host=list(counts),
+                             attn_splits=splits, attn_workspace=workspace, comm=self.comm, seq_starts_host=list(counts),
                              state_slots=up(np.asarray(state_slots, dtype=np.int32), torch.int32)
                              if state_slots is not None else seq_rows_d,
                              has_initial_state=up(np.asarray(has_initial_state, dtype=np.int32), torch.int32)

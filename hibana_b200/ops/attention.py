@@ -64,6 +64,39 @@ def choose_splits(batch: int, hkv: int, max_ctx: int, row_chunks: int = 1, slots
     return best
 
 
+# A split prefill writes fp32 partial rows and runs a merge: worth it when every CTA gets rid of this many of its key tiles
+# (32 CTAs of 8 tiles: 22.3 us whole, 22.4 in four ranges; of 16 tiles 34.2 and 24.7; 40 / 8 heads of 128).
+MIN_TILES_SAVED = 6
+
+
+def prefill_splits(batch: int, hq: int, hkv: int, d: int, max_rows: int, max_ctx: int) -> int:
+    """Context ranges of a tensor-core prefill (csrc/attn_prefill.cu): whole key tiles, two at least, and no more CTAs than
+    one wave, of which an SM holds one. A second wave of ranges only adds partial rows to write and merge: 100 rows over
+    30000 keys, 40 / 8 heads, 32 CTAs of whole contexts take 353 us, in 4 ranges 112, in 37 ranges 192; 100 rows over 500
+    keys 16 us whole, 35 in 7 ranges."""
+    if cfgmod.current().stable_numerics:
+        return 1
+    tiles = -(-max_ctx // (128 if d <= 128 else 64))
+    blocks = batch * hkv * -(-max_rows // max(1, 128 // (hq // hkv)))
+    room = min(NUM_SMS // max(1, blocks), 64)
+    if room < 2:
+        return 1
+    per = max(2, -(-tiles // room))
+    return -(-tiles // per) if tiles - per >= MIN_TILES_SAVED else 1
+
+
+def forward_splits(k_pool: torch.Tensor, v_pool: torch.Tensor, batch: int, hq: int, hkv: int, d: int, max_rows: int,
+                   max_ctx: int) -> int:
+    """KV splits of a ragged forward with up to `max_rows` new rows per sequence, for the kernel that will run it."""
+    g = max(1, hq // max(hkv, 1))
+    cfg = cfgmod.current()
+    if max_rows * g > 16 and _prefill_tensor_cores(k_pool, v_pool, d, cfg):
+        return prefill_splits(batch, hq, hkv, d, max_rows, max_ctx)
+    if batch * hkv * max(1, max_rows // max(1, 32 // g)) >= NUM_SMS:
+        return 1
+    return choose_splits(batch, hkv, max_ctx)
+
+
 class AttnWorkspace:
     """Split-KV partial buffers, allocated once (stable addresses for CUDA graphs)."""
 
@@ -135,7 +168,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
             res = out
         return res if quant_scale is None else nvfp4.quantize(res.reshape(t, hq * d), quant_scale)
     b = ctx_len.shape[0]
-    if splits > 1 and (workspace is None or workspace.rows < t or workspace.splits != splits):
+    if splits > 1 and (workspace is None or workspace.rows < t or workspace.part_o.shape[1:] != (hq, splits, d)):
         workspace = AttnWorkspace(t, hq, d, splits, q.device)
     fp4 = getattr(k_pool, "sf", None) is not None
     fp8 = k_pool.dtype != torch.bfloat16
@@ -196,6 +229,13 @@ def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg) -
             and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
 
 
+def _prefill_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg) -> bool:
+    """Whether more than 16 query rows per kv head run in csrc/attn_prefill.cu."""
+    if getattr(k_pool, "sf", None) is not None or cfg.prefill_attn != "tc":
+        return False
+    return d in (64, 128, 256) if k_pool.dtype == torch.bfloat16 else _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+
+
 _QUANT_BUFS: dict = {}
 
 
@@ -215,14 +255,13 @@ def _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, s
     if getattr(k_pool, "sf", None) is not None:
         fp8 = 2       # NVFP4 pool: the split-KV kernel dequantises rows as it loads them
         nv.lib().hb_attn_fp4_scales(k_pool.sf.data_ptr(), v_pool.sf.data_ptr(), k_pool.sf.stride(0), k_pool.sf.stride(1))
-    f8 = fp8 is True and _fp8_tensor_cores(k_pool, v_pool, d, cfg)
-    if (not fp8 and d in (64, 128, 256) or f8) and q_indptr is not None and cfg.prefill_attn == "tc":
+    if q_indptr is not None and _prefill_tensor_cores(k_pool, v_pool, d, cfg):
         st = nv.device_state(q.device)
         parts = (workspace.part_o.data_ptr(), workspace.part_lse.data_ptr()) if splits > 1 else (None, None)
         nv.check(nv.lib().hb_attn_prefill(
             q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1), kv_indices.data_ptr(),
             kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts, splits,
-            b, max_rows, hq, hkv, d, scale, int(f8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
+            b, max_rows, hq, hkv, d, scale, int(fp8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
             nv.stream()), "hb_attn_prefill")
         if splits > 1:
             nv.check(nv.lib().hb_attn_merge(*parts, out.data_ptr(), t * hq, splits, d, nv.stream()), "hb_attn_merge")

@@ -645,6 +645,33 @@ def test_splits_fill_one_wave_before_they_get_short(batch, hkv, ctx):
         assert batch * hkv * s >= 0.9 * 148
 
 
+@pytest.mark.parametrize("batch,hq,hkv,d,rows,ctx", [
+    (1, 40, 8, 128, 29, 200), (1, 40, 8, 128, 100, 500), (1, 40, 8, 128, 100, 2000), (1, 40, 8, 128, 100, 30000),
+    (1, 24, 4, 256, 20, 30000), (3, 32, 2, 128, 20, 5000), (1, 4, 2, 64, 300, 30000), (2, 24, 4, 256, 500, 8000),
+    (1, 40, 8, 128, 2048, 30000), (1, 16, 16, 128, 17, 700)])
+def test_prefill_ranges_fill_one_wave_at_most_cpu(batch, hq, hkv, d, rows, ctx):
+    from hibana_b200 import config as cfgmod
+    from hibana_b200.ops.attention import MIN_TILES_SAVED, NUM_SMS
+    pool = torch.empty(8, hkv, d, dtype=torch.bfloat16)
+    s = attention.forward_splits(pool, pool, batch, hq, hkv, d, rows, ctx)
+    tile = 128 if d <= 128 else 64
+    tiles, blocks = -(-ctx // tile), batch * hkv * -(-rows // (128 // (hq // hkv)))
+    per = -(-(-(-ctx // s)) // tile)                        # key tiles of a range, as the kernel cuts them
+    assert s == 1 or (blocks * s <= NUM_SMS and per >= 2 and tiles - per >= MIN_TILES_SAVED)
+    assert (s - 1) * per < tiles <= s * per                 # no range without keys
+    assert s > 1 or blocks * 2 > NUM_SMS or tiles < 2 + MIN_TILES_SAVED
+    with cfgmod.using(stable_numerics=True):
+        assert attention.forward_splits(pool, pool, batch, hq, hkv, d, rows, ctx) == 1
+
+
+def test_forward_splits_of_other_kernels_cpu():
+    """Up to 16 query rows per kv head, or pools that the tensor-core prefill does not take: the decode rule, one wave at most."""
+    bf, f8 = torch.empty(8, 8, 128, dtype=torch.bfloat16), torch.empty(8, 8, 64, dtype=torch.float8_e4m3fn)
+    assert attention.forward_splits(bf, bf, 1, 40, 8, 128, 3, 5000) == attention.choose_splits(1, 8, 5000) > 1
+    assert attention.forward_splits(f8, f8, 1, 16, 8, 64, 30, 5000) == attention.choose_splits(1, 8, 5000)
+    assert attention.forward_splits(f8, f8, 1, 16, 8, 64, 2000, 5000) == 1
+
+
 @pytest.mark.parametrize("ntiles", [1, 2, 3, 7, 40])
 def test_prefill_waits_cover_their_tile_cpu(ntiles):
     """The two-stream prefill kernel's full barriers, replayed on the host: copies may land in any order, and still no stream
