@@ -36,16 +36,22 @@ from ..hardware.b200 import NUM_SMS  # noqa: E402
 
 
 # One pass of a bf16 decode CTA (two warps, a 32-key tile each). A pass is a chain of latencies, about 1.6 us: one sequence of
-# 500 keys on 8 kv heads takes 16.4 us as one split and 10 us, merge included, in seven (738 -> 728 us per step).
+# 500 keys on 8 kv heads takes 15.1 us as one split and 11.3 us, merge included, in seven.
 MIN_SPLIT_KEYS = 64
+# The merge is a launch of about 4 us: as much as this many keys of a CTA. One sequence on 8 kv heads, whole / in ranges of 64:
+# 128 keys 8.4 / 10.2 us, 256 keys 10.4 / 10.2, 320 keys 11.2 / 10.2; 8 sequences, whole / in two: 256 keys 10.4 / 11.4,
+# 448 keys 13.3 / 13.4, 512 keys 14.2 / 13.3.
+MIN_KEYS_SAVED = 224
 DECODE_CTAS_PER_SM = 2      # csrc/attn_decode.cu: 64-thread CTAs with ~100 KB of rings, two share an SM
 
 
 def choose_splits(batch: int, hkv: int, max_ctx: int, row_chunks: int = 1, slots: int = 0) -> int:
     """KV splits that fill whole waves of the resident CTA slots (the decode kernel streams from every resident
     CTA at once, so a last wave that is a third full costs a whole wave). Within the first wave a split may be as short as
-    MIN_SPLIT_KEYS keys: idle SMs take it. Beyond it one has at least 256 keys, because shorter ones only leave more to
-    merge (4 sequences of 5000 keys on 4 heads: 9 splits take 19.8 us and 5.2 us of merge, 37 take 26.4 and 8.4)."""
+    MIN_SPLIT_KEYS keys, where that takes MIN_KEYS_SAVED keys off every CTA: idle SMs take it. Beyond it one has at least
+    256 keys, because shorter ones only leave more to merge (4 sequences of 5000 keys on 4 heads: 9 splits take 19.8 us and
+    5.2 us of merge, 37 take 26.4 and 8.4). `max_ctx` is the limit that a captured launch is planned for, which the
+    sequences may stay far below: an engine with a limit of 32k runs one of 500 keys in 37 splits, 16 of them with keys."""
     if cfgmod.current().stable_numerics:
         # row-count invariant: one pass over the keys in fixed tiles from position 0, so a token's attention sums
         # in the same order whether it is the only new row of its sequence or one of several verified rows
@@ -61,7 +67,7 @@ def choose_splits(batch: int, hkv: int, max_ctx: int, row_chunks: int = 1, slots
         eff = n / (-(-n // slots) * slots)
         if eff > best_eff + 0.02:     # prefer fewer splits unless the wave efficiency clearly improves
             best, best_eff = s, eff
-    return best
+    return best if max_ctx - -(-max_ctx // best) >= MIN_KEYS_SAVED else 1
 
 
 # A split prefill writes fp32 partial rows and runs a merge: worth it when every CTA gets rid of this many of its key tiles

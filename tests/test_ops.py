@@ -635,6 +635,14 @@ def test_act_mul_widths(inter, mode):
     assert bool(((got - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * ref.abs() + 1e-30).all())
 
 
+@pytest.mark.parametrize("batch", [1, 2, 8, 16])
+def test_no_splits_where_a_merge_costs_more_cpu(batch):
+    """Up to 256 keys a merge takes longer than the keys it saves, with two splits up to 447."""
+    assert all(attention.choose_splits(batch, 8, c, slots=148) == 1 for c in (64, 128, 200, 256))
+    assert attention.choose_splits(8, 8, 447, slots=148) == 1 and attention.choose_splits(8, 8, 448, slots=148) == 2
+    assert attention.choose_splits(1, 8, 320, slots=148) == 5 and attention.choose_splits(1, 8, 500, slots=148) == 7
+
+
 @pytest.mark.parametrize("batch,hkv,ctx", [(1, 8, 64), (1, 8, 500), (4, 4, 5056), (3, 2, 2304), (64, 8, 131072)])
 def test_splits_fill_one_wave_before_they_get_short(batch, hkv, ctx):
     s = attention.choose_splits(batch, hkv, ctx, slots=148)
