@@ -8,7 +8,6 @@ rows to slot 0) and hibana/engine/upload.py (pinned non-blocking upload).
 """
 from __future__ import annotations
 
-import gc
 from typing import Optional, Sequence
 
 import numpy as np
@@ -16,6 +15,7 @@ import torch
 
 from .. import _native as nv
 from ..ops import attention, sampling
+from ..utils import capture
 from .context import DECODE, PREFILL, VERIFY, ForwardContext
 
 # Rows of the packed int32 step buffer.
@@ -146,7 +146,6 @@ class ModelRunner:
         """Captures one decode graph per bucket (after a warm-up run of the same body)."""
         if not self.use_graphs:
             return
-        gc.collect()      # a dead engine's graphs must not be destroyed by the collector while this one captures
         for b in (buckets or self.buckets):
             buf = self.bufs[b]
             self._prepare_bucket(buf)
@@ -160,7 +159,7 @@ class ModelRunner:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             before = nv.LAUNCHES
-            with torch.cuda.graph(g):
+            with capture.graph(g):
                 self._decode_body(buf)
             self.graph_launches[b] = nv.LAUNCHES - before
             buf.graph = g
@@ -171,7 +170,7 @@ class ModelRunner:
                 torch.cuda.synchronize()
                 g2 = torch.cuda.CUDAGraph()
                 before = nv.LAUNCHES
-                with torch.cuda.graph(g2):
+                with capture.graph(g2):
                     self._decode_body(buf, greedy=True)
                 self.graph_launches[b] = nv.LAUNCHES - before     # the common step: report this one
                 buf.graph_greedy = g2

@@ -24,7 +24,6 @@ acceptance and grammar masks take the eager round. Reference: hibana/engine/spec
 """
 from __future__ import annotations
 
-import gc
 from typing import Optional, Sequence
 
 import numpy as np
@@ -32,6 +31,7 @@ import torch
 
 from .. import _native as nv
 from ..ops import attention, sampling
+from ..utils import capture
 from .context import VERIFY, ForwardContext
 from .request import MAX_STOPS
 
@@ -145,7 +145,6 @@ class VerifyGraphs:
     def capture(self) -> None:
         if self.device.type != "cuda" or not self.runner.use_graphs:
             return
-        gc.collect()      # see ModelRunner.capture
         for b, buf in self.bufs.items():
             self._prepare(buf)
             buf.dev.zero_()
@@ -160,7 +159,7 @@ class VerifyGraphs:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             before = nv.LAUNCHES
-            with torch.cuda.graph(g):
+            with capture.graph(g):
                 self._body(buf)
             self.launches[b] = nv.LAUNCHES - before
             buf.graph = g
@@ -286,7 +285,6 @@ class DraftGraphs:
     def capture(self) -> None:
         if self.device.type != "cuda" or not self.runner.use_graphs:
             return
-        gc.collect()      # see ModelRunner.capture
         for buf in self.bufs.values():
             buf.dev.zero_()
             s = torch.cuda.Stream()
@@ -297,7 +295,7 @@ class DraftGraphs:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             before = nv.LAUNCHES
-            with torch.cuda.graph(g):
+            with capture.graph(g):
                 self._body(buf)
             self.launches[buf.bucket] = nv.LAUNCHES - before
             buf.graph = g

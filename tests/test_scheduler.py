@@ -209,3 +209,66 @@ def test_nvtx_ranges_and_ssd_trace_are_switchable(tmp_path):
         llm.executor.ssd.trace("ssd_restore", start=0, end=256, good=256, failed=False)
     line = json.loads((tmp_path / "ssd" / "ssd_trace.jsonl").read_text().splitlines()[-1])
     assert line["event"] == "ssd_restore" and line["good"] == 256
+
+
+def test_collector_is_off_while_any_capture_runs():
+    """The collector is off inside, on again behind the last of several threads, also after an exception, and stays off where
+    it was off before."""
+    import gc
+    import threading
+
+    from hibana_b200.utils.capture import no_collection
+    assert gc.isenabled()
+    inside, leave = threading.Event(), threading.Event()
+
+    def other():
+        with no_collection():
+            inside.set()
+            leave.wait(10)
+
+    th = threading.Thread(target=other)
+    with pytest.raises(RuntimeError):
+        with no_collection():
+            th.start()
+            inside.wait(10)
+            assert not gc.isenabled()
+            raise RuntimeError
+    assert not gc.isenabled()              # the other thread is still inside
+    leave.set()
+    th.join()
+    assert gc.isenabled()
+    gc.disable()
+    try:
+        with no_collection():
+            pass
+        assert not gc.isenabled()
+    finally:
+        gc.enable()
+
+
+@pytest.mark.gpu
+def test_dead_engines_graphs_are_not_destroyed_inside_a_capture():
+    """An engine whose graphs sit in a reference cycle is dropped, then another one captures while the collector would run at
+    almost every allocation."""
+    import gc
+
+    from hibana_b200.engine.executor import Executor
+    from hibana_b200.engine.request import SamplingParams
+    from hibana_b200.models.dense import DenseModel
+    from hibana_b200.target import dense_tiny
+    model = DenseModel(dense_tiny(), "cuda:0", seed=0)
+    sp = SamplingParams(max_tokens=3, ignore_eos=True)
+    want = None
+    old = gc.get_threshold()
+    for _ in range(3):
+        ex = Executor(model, max_batch=2, max_ctx=64)
+        gc.set_threshold(1)
+        try:
+            ex.runner.capture([1, 2])
+        finally:
+            gc.set_threshold(*old)
+        out = [r.output_ids for r in ex.generate_batch([[1, 2, 3], [4, 5]], sp)]
+        assert want is None or out == want
+        want = out
+        ex.cycle = ex
+        del ex
