@@ -82,7 +82,7 @@ class KvPool:
         if self._shuffled and n >= 32:
             self._free.sort(reverse=True)          # a prefill-sized request gets ascending runs again
             self._shuffled = False
-        if n == 0:
+        if n <= 0:
             return []
         out = self._free[:-n - 1:-1]               # what n pops would return
         del self._free[-n:]

@@ -179,6 +179,7 @@ def test_kv_pool_runs_of_slots_cpu(n):
     pool = KvPool(1, 300, 1, 32)
     a, b = pool.alloc(n), pool.alloc(5)
     assert a == list(range(1, n + 1)) and b == list(range(n + 1, n + 6)) and pool.alloc(0) == []
+    assert pool.alloc(-2) == [] and pool.free_count == 300 - n - 5     # nothing asked for, nothing handed out
     pool.free(a)
     pool.check()
     with pytest.raises(ValueError):
