@@ -179,7 +179,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     fp4 = getattr(k_pool, "sf", None) is not None
     fp8 = k_pool.dtype != torch.bfloat16
     cfg = cfgmod.current()
-    f8 = fp8 and not fp4 and _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+    f8 = fp8 and not fp4 and _fp8_tensor_cores(k_pool, v_pool, d, cfg, q, out)
     if (not fp8 and d in (64, 128, 256) or f8) and max_rows * (hq // hkv) <= 16:
         st = nv.device_state(q.device)
         tc = d == 128 and cfg.decode_attn == "tc" and not f8
@@ -225,21 +225,25 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     return res if quant_scale is None else nvfp4.quantize(res.view(t, hq * d), quant_scale)
 
 
-def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg) -> bool:
+def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg, q: Optional[torch.Tensor] = None,
+                      out: Optional[torch.Tensor] = None) -> bool:
     """Whether an e4m3 pool takes the tensor-core kernels: whole 128-byte column blocks per row and rows on 16-byte
-    boundaries (bulk copies). Under `stable_numerics` the general kernel stays: it sums a row's keys in the same order
+    boundaries (bulk copies), query and output rows on 16-byte boundaries (16-byte accesses; the general kernel reads and
+    writes them element by element). Under `stable_numerics` the general kernel stays: it sums a row's keys in the same order
     however many rows share the call, the tensor-core kernels have one form for up to 8 and one for up to 16 rows."""
     return (k_pool.dtype == torch.float8_e4m3fn and d in (128, 256) and not cfg.stable_numerics
             and k_pool.stride(0) % 16 == 0 and k_pool.stride(1) % 16 == 0 and k_pool.stride(2) == 1
             and v_pool.stride() == k_pool.stride()
-            and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
+            and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0
+            and all(x is None or x.data_ptr() % 16 == 0 for x in (q, out)))
 
 
-def _prefill_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg) -> bool:
+def _prefill_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg, q: Optional[torch.Tensor] = None,
+                          out: Optional[torch.Tensor] = None) -> bool:
     """Whether more than 16 query rows per kv head run in csrc/attn_prefill.cu."""
     if getattr(k_pool, "sf", None) is not None or cfg.prefill_attn != "tc":
         return False
-    return d in (64, 128, 256) if k_pool.dtype == torch.bfloat16 else _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+    return d in (64, 128, 256) if k_pool.dtype == torch.bfloat16 else _fp8_tensor_cores(k_pool, v_pool, d, cfg, q, out)
 
 
 _QUANT_BUFS: dict = {}
@@ -261,7 +265,7 @@ def _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, s
     if getattr(k_pool, "sf", None) is not None:
         fp8 = 2       # NVFP4 pool: the split-KV kernel dequantises rows as it loads them
         nv.lib().hb_attn_fp4_scales(k_pool.sf.data_ptr(), v_pool.sf.data_ptr(), k_pool.sf.stride(0), k_pool.sf.stride(1))
-    if q_indptr is not None and _prefill_tensor_cores(k_pool, v_pool, d, cfg):
+    if q_indptr is not None and _prefill_tensor_cores(k_pool, v_pool, d, cfg, q, out):
         st = nv.device_state(q.device)
         parts = (workspace.part_o.data_ptr(), workspace.part_lse.data_ptr()) if splits > 1 else (None, None)
         nv.check(nv.lib().hb_attn_prefill(

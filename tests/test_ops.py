@@ -749,3 +749,36 @@ def test_fp8_kv_attention_keeps_small_weights(hq, hkv, d, rows, dominant):
         bound = 2.0 ** -8 * ref.abs() + 1e-4 * ref.pow(2).mean(-1, keepdim=True).sqrt()
         assert bool(((got - ref).abs() <= bound).all()), ((got - ref).abs() / bound).max().item()
     assert nv.read_status() == 0
+
+
+def _odd_rows(rows, hq, d):
+    """[rows, hq, d] bf16 that starts on a 2-byte boundary."""
+    x = torch.zeros(rows * hq * d + 1, dtype=torch.bfloat16)[1:].view(rows, hq, d)
+    return x.copy_(torch.randn(rows, hq, d, generator=torch.Generator().manual_seed(3)))
+
+
+def test_fp8_kv_rows_off_16_byte_boundaries_take_the_general_kernel_cpu():
+    from hibana_b200 import config as cfgmod
+    pool = torch.zeros(8, 2, 128, dtype=torch.float8_e4m3fn)
+    even, odd = torch.zeros(4, 4, 128, dtype=torch.bfloat16), _odd_rows(4, 4, 128)
+    assert even.data_ptr() % 16 == 0 and odd.data_ptr() % 16 == 2
+    for takes in (attention._fp8_tensor_cores, attention._prefill_tensor_cores):
+        args = (pool, pool, 128, cfgmod.current())
+        assert takes(*args, even, even) and takes(*args, even, None)
+        assert not takes(*args, odd, even) and not takes(*args, even, odd)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 40])
+def test_fp8_kv_attention_of_rows_off_16_byte_boundaries(rows):
+    hq, hkv, d, n = 8, 2, 128, 300
+    gen = torch.Generator().manual_seed(2)
+    k, v = (torch.randn(n + 1, hkv, d, generator=gen).to(torch.float8_e4m3fn) for _ in range(2))
+    q = _odd_rows(rows, hq, d)
+    idx = torch.arange(1, n + 1, dtype=torch.int32)[None]
+    ctx, indptr = torch.tensor([n], dtype=torch.int32), torch.tensor([0, rows], dtype=torch.int32)
+    ref = attention.paged_attention(q, k, v, idx, ctx, q_indptr=indptr, max_rows=rows)
+    base = torch.zeros(rows * hq * d + 1, dtype=torch.bfloat16, device="cuda")
+    odd = base[1:].view(rows, hq, d).copy_(q)
+    got = attention.paged_attention(odd, k.cuda(), v.cuda(), idx.cuda(), ctx.cuda(), q_indptr=indptr.cuda(), max_rows=rows)
+    _close(got, ref, 2e-2)
