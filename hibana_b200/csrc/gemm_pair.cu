@@ -514,7 +514,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
       if (!x.live) continue;
       if constexpr (GRP) alpha = x.alpha;
       const int buf = it & 1;
-      if (!mbar_wait(&accum[buf], (it >> 1) & 1, abort, p.status, kTimeoutAccum)) break;
+      // one verdict per warp: lanes that give up on a wait must not leave the others alone in a warp-wide TMEM load
+      if (!__all_sync(0xffffffffu, mbar_wait(&accum[buf], (it >> 1) & 1, abort, p.status, kTimeoutAccum))) break;
       tc_fence_after();
       epilogue_unit<EPI>(p, x, buf, half, tlane + (buf ? ACC1_COL : 0), x.m0 + static_cast<int>(rank) * 128 + q * 32, mine,
                          alpha, q_inv_gs, release, lane);
