@@ -98,9 +98,16 @@ def forward_splits(k_pool: torch.Tensor, v_pool: torch.Tensor, batch: int, hq: i
     cfg = cfgmod.current()
     if max_rows * g > 16 and _prefill_tensor_cores(k_pool, v_pool, d, cfg):
         return prefill_splits(batch, hq, hkv, d, max_rows, max_ctx)
-    if batch * hkv * max(1, max_rows // max(1, 32 // g)) >= NUM_SMS:
+    ctas = batch * hkv * max(1, max_rows // max(1, 32 // g))       # the general kernel takes up to 32 query rows per CTA
+    if ctas >= NUM_SMS:
         return 1
-    return choose_splits(batch, hkv, max_ctx)
+    splits = choose_splits(batch, hkv, max_ctx)
+    if max_rows * g > 16:
+        # Ranges of less than 256 keys only while about four CTAs per SM run. NVFP4 pools, 40 / 8 and 24 / 4 heads of 128 and
+        # 256: 100 rows over 2000 keys, 7 ranges 363 and 466 us, 18 and 31 ranges 413 and 582; 29 rows over 500 keys, one
+        # range 178 and 251 us, 7 ranges 71 and 87.
+        splits = min(splits, max(max_ctx // 256, 4 * NUM_SMS // ctas, 1))
+    return splits
 
 
 class AttnWorkspace:

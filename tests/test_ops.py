@@ -678,6 +678,9 @@ def test_forward_splits_of_other_kernels_cpu():
     assert attention.forward_splits(bf, bf, 1, 40, 8, 128, 3, 5000) == attention.choose_splits(1, 8, 5000) > 1
     assert attention.forward_splits(f8, f8, 1, 16, 8, 64, 30, 5000) == attention.choose_splits(1, 8, 5000)
     assert attention.forward_splits(f8, f8, 1, 16, 8, 64, 2000, 5000) == 1
+    # many CTAs already: no range of less than 256 keys; few: short ones fill the chip
+    assert attention.forward_splits(f8, f8, 1, 40, 8, 64, 100, 2000) == 7 < attention.choose_splits(1, 8, 2000)
+    assert attention.forward_splits(f8, f8, 1, 40, 8, 64, 29, 500) == attention.choose_splits(1, 8, 500) == 7
 
 
 @pytest.mark.parametrize("ntiles", [1, 2, 3, 7, 40])
