@@ -99,7 +99,7 @@ __global__ void quant_nvfp4_pairs_kernel(const __nv_bfloat16* __restrict__ x, lo
 
 // (residual add +) RMSNorm -> NVFP4 (and / or bf16). One CTA per row on the register-resident row core.
 // Writes the updated residual (bf16) when `residual` is given. gemma != 0 uses weight (1 + w).
-template <int T, int MAXC>
+template <int T, int MAXC, bool EARLY>
 __global__ void __launch_bounds__(T)
 norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                         const __nv_bfloat16* __restrict__ w, float eps, int gemma, int m, int k, int ka,
@@ -110,12 +110,12 @@ norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
   const int tid = threadIdx.x;
   // A decode step is a chain of short kernels, and this one is latency: the GEMM behind it may become resident and fetch
   // weights from now on, and what no kernel of the step writes (norm weights, the scale) is read before the wait for the
-  // producer of x. At one row of 5120 the step got 2.0 us shorter per launch.
+  // producer of x (EARLY). At one row of 5120 the step got 2.0 us shorter per launch.
   grid_dep_launch();
   const int nchunk = k >> 3;
-  uint4 wa[MAXC];
+  uint4 wa[EARLY ? MAXC : 1];
   float gs_early = 0.f;
-  if (row < m) {
+  if (EARLY && row < m) {
 #pragma unroll
     for (int i = 0; i < MAXC; ++i)
       if (tid + i * T < nchunk) wa[i] = __ldg(reinterpret_cast<const uint4*>(w) + tid + i * T);
@@ -155,7 +155,7 @@ norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
   RowOut out;
   out.n = 1;
   out.q[0] = q; out.sf[0] = sf; out.bf[0] = normed;
-  row_finish<T, MAXC>(v, k, w, eps, gemma, red, out, row, ka, &gs_early, wa);
+  row_finish<T, MAXC>(v, k, w, eps, gemma, red, out, row, ka, EARLY ? &gs_early : gscale, EARLY ? wa : nullptr);
 }
 
 // Zeroes the scale bytes of the padding rows [m, round_up(m, 128)) (used after the per-row kernel).
@@ -259,8 +259,13 @@ int hb_norm_quant_nvfp4(const void* x, void* residual, const void* w, float eps,
   constexpr int T = 256;
   const int rows_pad = q != nullptr ? ((m + 127) / 128) * 128 : m;
   const int nchunk = k / 8;
+  // Weights held from the start take registers, which with 2 or 4 chunks per thread cost a resident CTA: late / early, 2048
+  // rows of 2688 10.2 / 11.0 us, of 8192 21.1 / 23.3, 512 rows of 8192 7.8 / 8.9; few rows gain (200 of 8192 5.7 / 5.3, 400
+  // of 2688 4.0 / 3.8), and 1 or 3 chunks at any number (2048 rows of 1024 6.7 / 6.3, 640 of 5120 8.6 / 7.3).
 #define HB_NQ(MAXC)                                                                                              \
-  launch_dep(norm_quant_nvfp4_kernel<T, MAXC>, dim3(rows_pad), dim3(T), 0, st,                                   \
+  launch_dep(MAXC % 2 == 1 || m <= (MAXC == 2 ? 448 : 256) ? norm_quant_nvfp4_kernel<T, MAXC, true>              \
+                                                           : norm_quant_nvfp4_kernel<T, MAXC, false>,            \
+      dim3(rows_pad), dim3(T), 0, st,                                                                            \
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(residual),                               \
       static_cast<const __nv_bfloat16*>(w), eps, gemma, m, k, ka, static_cast<const float*>(gscale),             \
       static_cast<uint8_t*>(q), static_cast<uint8_t*>(sf), static_cast<__nv_bfloat16*>(normed))

@@ -294,3 +294,21 @@ def test_stable_numerics_rows_keep_their_bits_at_any_batch(n, k, fmt):
             assert torch.equal(run(x[:m])[:1], want), m
             assert m < 80 or torch.equal(run(x[:m])[:64], run(x[:64])), m
     assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,few", [(2688, 448), (2064, 448), (8192, 256), (6160, 256), (5120, 448), (1024, 448)])
+def test_norm_quant_rows_do_not_depend_on_how_many_there_are(k, few):
+    """Few rows hold the norm weights from the start, many read them late (2 and 4 chunks per thread): the same bytes."""
+    torch.manual_seed(6)
+    x, res = (torch.randn(few + 1, k, device="cuda").bfloat16() for _ in range(2))
+    w, gs = torch.randn(k, device="cuda").bfloat16(), torch.tensor(0.01, device="cuda")
+    out = []
+    for m in (few, few + 1):
+        r = res[:m].clone()
+        q, y = nvfp4.rmsnorm_quantize(x[:m], w, 1e-6, gs, residual=r, want_normed=True)
+        out.append((q.q[:few], nvfp4.unswizzle_sf(q.sf, m, k // 16)[:few], y[:few], r[:few]))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    ref = (x.float() + res.float()).bfloat16().float()[:few]
+    ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + 1e-6) * w.float()
+    assert bool(((out[0][2].float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
