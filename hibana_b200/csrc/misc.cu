@@ -657,7 +657,9 @@ int hb_act_mul(const void* x, const void* gate, void* out, long long rows, int i
   const long long n = rows * inter;
   if (n <= 0) return 0;
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(gate);
-  if (inter % 8 == 0 && ldx % 8 == 0 && (ptrs & 15) == 0) {
+  // A thread of the vector form computes eight exponentials and divisions one after the other, which few elements do not hide:
+  // scalar / vector, 1 x 5376 1.7 / 2.1 us, 32 x 5376 2.0 / 2.2, 192 x 1024 2.2 / 2.2, 64 x 5376 2.7 / 2.3. Squared ReLU has neither.
+  if (inter % 8 == 0 && ldx % 8 == 0 && (ptrs & 15) == 0 && (mode == 2 || n >= 192 * 1024)) {
     act_mul_vec_kernel<<<static_cast<unsigned>((n / 8 + 255) / 256), 256, 0, ST(stream)>>>(BF(x), BF(gate), BFM(out), rows,
                                                                                            inter, ldx, mode);
     return OK();

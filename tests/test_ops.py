@@ -785,3 +785,16 @@ def test_fp8_kv_attention_of_rows_off_16_byte_boundaries(rows):
     odd = base[1:].view(rows, hq, d).copy_(q)
     got = attention.paged_attention(odd, k.cuda(), v.cuda(), idx.cuda(), ctx.cuda(), q_indptr=indptr.cuda(), max_rows=rows)
     _close(got, ref, 2e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,inter", [(191, 1024), (192, 1024), (400, 520), (25000, 8)])
+@pytest.mark.parametrize("mode", [basic.ACT_SILU_SPLIT, basic.ACT_SILU_PAIRS, basic.ACT_RELU2, basic.ACT_SIGMOID_GATE])
+def test_act_mul_forms_agree(rows, inter, mode):
+    """Rows on 16-byte boundaries (vector form from 192K elements on) and rows off them (scalar form): the same bits."""
+    cols = 2 * inter if mode in (basic.ACT_SILU_SPLIT, basic.ACT_SILU_PAIRS) else inter
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows)).bfloat16().cuda()
+    gate = x.flip(0).contiguous() if mode == basic.ACT_SIGMOID_GATE else None
+    odd = torch.zeros(rows * cols + 4, dtype=torch.bfloat16, device="cuda")[4:].view(rows, cols).copy_(x)
+    assert x.data_ptr() % 16 == 0 and odd.data_ptr() % 16 == 8
+    assert torch.equal(basic.act_mul(x, mode, gate), basic.act_mul(odd, mode, gate))
