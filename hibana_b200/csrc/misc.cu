@@ -79,6 +79,8 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
 // 16-byte chunks per lane; one read of x and z, 16-byte stores. The kernel is bound by issue (an exponential and an IEEE
 // division per element), so no lane idles and no chunk is computed that is not there: 1237 rows of 48 groups of 128 took
 // 66 us with a warp per group and four predicated chunks, 19 us so; 4096 rows of 8 groups of 1024, 115 -> 99.
+// Lanes beyond the end of a group that does not fill them (16, 96 or 640 channels) divide ones, not zeros: a zero dividend sends
+// its warp through the division's slow path (one row of 6 groups of 640: 8.9 us with zeros and four chunks, 4.1 so).
 template <int NC, int L>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
@@ -99,7 +101,8 @@ gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int ci = lane + c * L;
-    xa[c] = za[c] = wa[c] = make_uint4(0, 0, 0, 0);
+    xa[c] = wa[c] = make_uint4(0, 0, 0, 0);
+    za[c] = make_uint4(0x3f803f80, 0x3f803f80, 0x3f803f80, 0x3f803f80);
     if (ci < nchunk) {
       xa[c] = xr[ci];
       if (zr) za[c] = zr[ci];
@@ -474,6 +477,7 @@ static int gated_rmsnorm_reg(const void* x, const void* z, const void* w, void* 
   else if (lanes == 16) HB_GN(1, 16);
   else if (nchunk <= 32) HB_GN(1, 32);
   else if (nchunk <= 64) HB_GN(2, 32);
+  else if (nchunk <= 96) HB_GN(3, 32);
   else HB_GN(4, 32);
 #undef HB_GN
   return OK();

@@ -754,6 +754,22 @@ def test_fp8_kv_attention_keeps_small_weights(hq, hkv, d, rows, dominant):
     assert nv.read_status() == 0
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("gs,groups", [(8, 5), (16, 3), (48, 7), (96, 4), (640, 6), (768, 3), (776, 2), (1000, 1)])
+@pytest.mark.parametrize("norm_first", [False, True])
+def test_gated_rmsnorm_groups_that_leave_lanes_idle(gs, groups, norm_first):
+    """Group sizes whose 16-byte chunks do not fill the lanes: against 64 bits within two bf16 roundings."""
+    g = torch.Generator().manual_seed(gs)
+    x, z = (torch.randn(37, gs * groups, generator=g).bfloat16() for _ in range(2))
+    w = torch.randn(gs * groups, generator=g).bfloat16()
+    got = basic.gated_rmsnorm(x.cuda(), z.cuda(), w.cuda(), 1e-5, gs, norm_first=norm_first).cpu().double()
+    xd, gate = x.double(), torch.nn.functional.silu(z.double())
+    v = (xd if norm_first else xd * gate).view(37, groups, gs)
+    ref = (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5)).view(37, -1) * w.double()
+    ref = ref * gate if norm_first else ref
+    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+
+
 def _odd_rows(rows, hq, d):
     """[rows, hq, d] bf16 that starts on a 2-byte boundary."""
     x = torch.zeros(rows * hq * d + 1, dtype=torch.bfloat16)[1:].view(rows, hq, d)
