@@ -966,6 +966,7 @@ template <int KIND, int BN>
 cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorMap* ta, const CUtensorMap* tb,
                      cudaStream_t stream) {
   using C = Cfg<KIND, BN>;
+  constexpr int K_ELEMS = KIND == kGemmNvfp4 ? 256 : KIND == kGemmFp8 ? 128 : 64;      // of a K tile
   static bool attr_done = false;
   static int max_clusters[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};   // co-resident clusters per cluster size (0 = unknown)
   if (!attr_done) {
@@ -1007,8 +1008,12 @@ cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorM
       // tensor memory hold two (BN <= 64): with 148 slots assumed, K was cut half as often as the chip has room for. A
       // negative split count asks for the wider tiles' limit at every width: the same cuts, so the same order of sums,
       // whatever the number of tokens.
+      // For 64-token tiles the second CTA of an SM pays from 512 elements of K per split on: 64 rows, bf16, 4096 x 1024 in 8
+      // splits of 128 9.2 us, 4 of 256 7.9; 4096 x 2048 in 8 of 256 10.4, 4 of 512 9.2; 5120 x 3072 in 6 of 512 11.1, 3 of 1024 11.9;
+      // 7168 x 5120 with and without the second CTA 15.5 and 23.1.
       const int room = max_clusters[splits];
-      if ((BN <= 64 && a.splits > 0 ? 2 * room : room) >= tiles) break;
+      const bool two = BN < 64 || (BN == 64 && (p.k_tiles + splits - 1) / splits * K_ELEMS >= 512);
+      if ((two && a.splits > 0 ? 2 * room : room) >= tiles) break;
     }
     p.splits = splits;
     grid.z = splits;
