@@ -750,7 +750,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
                 *reinterpret_cast<const uint4*>(tile + lr * PITCH + ch * 16);
         }
         // scale bytes: each lane writes its own row's BN / 32 groups (four groups of a K atom are one 32-bit word
-        // of the swizzled block; the feature count is a multiple of 64, so groups come in valid pairs)
+        // of the swizzled block; the gate and up columns are a multiple of 64, so groups come in valid pairs)
         const int grow = tile_a * BM + q * 32 + lane;
         if (grow < row_lim) {
 #pragma unroll
@@ -1124,7 +1124,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
     if (a.swap && (a.ra % BM != 0 || a.q_ka * 64 < a.ra / 2 || a.bn > 128)) return cudaErrorInvalidValue;
     // tokens on the 128-row side: the staged epilogue (output tiles of 128 or 256 columns, no split-K) writes the
-    // packed bytes as aligned 16-byte chunks of two groups: feature count a multiple of 64
+    // packed bytes as aligned 16-byte chunks of two groups: 32 features, 64 gate and up columns
     if (!a.swap && (a.rb % 64 != 0 || a.q_ka * 64 < a.rb / 2 || a.splits != 1 || (a.bn != 128 && a.bn != 256) ||
                     a.q_ld % 16 != 0 || (reinterpret_cast<uintptr_t>(a.q_out) & 15) != 0))
       return cudaErrorInvalidValue;

@@ -299,7 +299,8 @@ __device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x
   }
   if constexpr (EPI == kEpiSiluMulQuant || EPI == kEpiRelu2Quant) {
     // Packed bytes of the half: consecutive lanes along a row, 8 bytes per group (SiLU-mul: a step is one group, else two).
-    // The feature count is a multiple of 64, so a step's groups are in range together.
+    // Whole steps are in range or none: ungrouped SiLU-mul calls have a multiple of 64 gate and up columns (32 features, so the
+    // last K atom of the next GEMM may hold two groups and two zeroed ones), grouped calls a multiple of 64 features.
     constexpr int GROUPS = EPI == kEpiSiluMulQuant ? 1 : 2;
     constexpr int SHIFT = EPI == kEpiSiluMulQuant ? 5 : 4;      // columns per group, log2
     const int c_half = x.n0 + col0;

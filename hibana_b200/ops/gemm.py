@@ -157,7 +157,7 @@ _REQUANT_BUFS: dict = {}
 def requant_ok(m: int, n: int) -> bool:
     """Shapes the fused SiLU-mul + requant epilogue covers: decode-sized calls with the weights on the 128-row side
     and whole feature tiles, and prefill-sized calls (tokens on the 128-row side, `_plan` picks that above 256 rows)
-    whose feature count is a multiple of 64 (aligned 16-byte chunks of packed values)."""
+    whose feature count n / 2 is a multiple of 32 (aligned 16-byte chunks of packed values)."""
     return (m <= 128 and n % 128 == 0) or (m > 256 and n % 64 == 0)
 
 

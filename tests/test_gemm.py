@@ -312,3 +312,22 @@ def test_norm_quant_rows_do_not_depend_on_how_many_there_are(k, few):
     ref = (x.float() + res.float()).bfloat16().float()[:few]
     ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + 1e-6) * w.float()
     assert bool(((out[0][2].float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(257, 64, 256), (257, 320, 288), (513, 320, 512), (513, 2112, 256), (300, 2112, 1024),
+                                   (600, 10304, 256), (2048, 5120, 256)])
+def test_requant_epilogue_on_sm_pairs_ragged(m, n, k):
+    """SiLU-mul + requantisation with ragged rows, odd multiples of 32 features and a last wave of narrow units: every packed
+    byte and every scale byte of the rows, padding groups included, as SiLU-mul followed by the quantiser leaves them."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    wq = nvfp4.quantize_weight(torch.randn(n, k, device="cuda", generator=g) * 0.05)
+    gs, out_scale = torch.tensor(6.0 / (6 * 448), device="cuda"), torch.tensor(0.002, device="cuda")
+    xq = nvfp4.quantize(torch.randn(m, k, device="cuda", generator=g).bfloat16(), gs)
+    alpha = (gs * wq.gscale).reshape(1)
+    two = nvfp4.quantize(gemm.linear_nvfp4(xq, wq, alpha, epilogue=gemm.EPI_SILU_MUL), out_scale)
+    one = gemm.linear_nvfp4_silu_quant(xq, wq, alpha, out_scale)
+    assert torch.equal(one.q, two.q) and one.sf.shape == two.sf.shape
+    groups = 4 * one.sf.shape[1]
+    assert torch.equal(nvfp4.unswizzle_sf(one.sf, m, groups), nvfp4.unswizzle_sf(two.sf, m, groups))
+    assert nv.read_status() == 0
