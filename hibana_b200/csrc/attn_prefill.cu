@@ -22,9 +22,9 @@
 // tile, V of this one). Q rows become fp16 under a power-of-two row scale (exact down to 2^-31 of the row's
 // largest element), and P is the sum of two fp16 tiles, hi + lo: O += hi V + lo V. So that small weights do not fall on the
 // fp16 subnormal grid, O and the row sum refer to a value below the running maximum (pf_reference): weights down to 2^-14
-// of the largest keep 22 bits, smaller ones are exact to 2^-36 of it. Against the fp32 CUDA-core kernel of attn.cu: 4096
-// tokens, 32 / 2 heads of 128: 8050 -> 390 us; 1237 + 263 tokens, 24 / 4 heads of 256: 2170 -> 87 us. What bounds it is
-// the chain scores -> softmax -> P -> O of each tile, not the MMAs.
+// of the largest keep 22 bits, smaller ones are exact to 2^-36 of it. Against the fp32 CUDA-core kernel of attn.cu: 1237 +
+// 263 tokens, 24 / 4 heads of 256: 2170 -> 87 us. What bounds it is the chain scores -> softmax -> P -> O of each tile, not
+// the MMAs.
 //
 // Few rows on a long context leave most SMs idle, so the context can be cut into splits (merged by hb_attn_merge): 4 rows
 // on 30000 keys, 24 / 4 heads of 256: 1050 us as one range, 63 us in 37.
@@ -695,7 +695,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 // the scores it came from in TMEM and enters O += P V as the A operand from there (F8: 16 columns of hi, 16 of lo per
 // 32 keys), so it never passes through shared memory.
 // One layer, 40 / 8 heads of 128, bf16: 2048 tokens 138 -> 113 us, 4096 in five prompts 239 -> 204, 2048 new tokens over 30000
-// keys 2780 -> 1700; e4m3, 4096 tokens, 32 / 2 heads: 390 -> 280. Per tile of a stream 6400 cycles are left, 2400 of them
+// keys 2780 -> 1700; e4m3, 4096 tokens, 32 / 2 heads: 390 -> 282 (8050 on the CUDA cores). Per tile of a stream 6400 cycles are left, 2400 of them
 // softmax; the rest is the chain of barriers around the two MMAs and K tiles that arrive late (copies of 32 rows; with
 // warps of their own for K and V they came no earlier, and the layer took 125 us).
 constexpr int PP_STAGES = 3;      // K and V rings, shared by both streams

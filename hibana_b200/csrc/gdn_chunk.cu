@@ -282,7 +282,7 @@ int hb_gdn_chunk_pass(const void* w, const void* qg, const void* kd, const void*
   }
   // One group per CTA while all CTAs are resident at once (a CTA of one group is a little faster by itself).
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (vdim % (2 * VS) == 0 && heads * (vdim / VS) > 148)
+  if (vdim % (2 * VS) == 0 && heads * (vdim / VS) > kNumSms)
     gdn_chunk_kernel<2><<<dim3(heads, vdim / (2 * VS)), 256, ChunkSmem<2>::BYTES, st>>>(p);
   else
     gdn_chunk_kernel<1><<<dim3(heads, vdim / VS), 128, ChunkSmem<1>::BYTES, st>>>(p);

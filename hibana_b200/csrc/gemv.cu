@@ -384,7 +384,7 @@ int hb_nvfp4_gemv(const void* wq, const void* wsf, const void* wscale, int n, in
   const int ntiles = n / 16, nchunks = k / kChunk;
   int per_sm = static_cast<int>((220 * 1024) / (smem + 1024));
   per_sm = per_sm > 4 ? 4 : per_sm < 1 ? 1 : per_sm;
-  const int slots = 148 * per_sm;
+  const int slots = kNumSms * per_sm;
   int ksplit = 1;
   for (int cand = 4; cand >= 1; cand >>= 1) {
     const int c = (ntiles * cand + kGemvWarps - 1) / kGemvWarps;

@@ -13,6 +13,8 @@
 
 namespace hb {
 
+constexpr int kNumSms = 148;      // two dies of 74 (hardware/b200.py NUM_SMS)
+
 // Status codes written to the status word (first writer wins; 0 = OK).
 enum Status : int {
   kOk = 0,
@@ -238,9 +240,16 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
 }
 
 // Launch as a programmatic dependent of the kernel before it in the stream (when the library-wide switch is on,
-// see hb_gemm_set_pdl): the grid may be scheduled while its predecessor drains, which hides launch latency. The
-// kernel MUST call grid_dep_wait() before it touches anything its predecessor wrote (and should call
-// grid_dep_launch() right after, so that its own successor can do the same).
+// see hb_gemm_set_pdl): the grid may be scheduled while its predecessor drains, which hides launch latency. The rules:
+//   * every kernel calls grid_dep_wait() before it reads anything that ANY kernel of the step wrote, and before it writes
+//     anything. Kernels may call grid_dep_launch() ahead of their own wait (norm + quantise, RoPE + KV write, decode
+//     attention, merge do), so when a dependent starts, kernels further back than its predecessor may still run;
+//   * before the wait only weights, norm weights and static scales may be read;
+//   * one exception: the one-CTA grouped GEMM (gemm.cu) reads the routing plan before its wait, to leave early. That is safe
+//     because the kernel in front of it (the activation quantiser, the row gather) triggers only after its own wait, which
+//     the plan kernel's end precedes, or is another grouped GEMM behind such a kernel. One that is put in between must do
+//     the same.
+// At level 1 only GEMMs are launched as dependents, so an early trigger matters where a GEMM follows.
 extern "C" int hb_gemm_get_pdl(void);
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

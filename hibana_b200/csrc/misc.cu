@@ -226,7 +226,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, long
                                      int kv_fp8, float kv_inv_scale, int q_gate, uint8_t* __restrict__ k_sf,
                                      uint8_t* __restrict__ v_sf, long long sf_pool_stride, long long sf_head_stride,
                                      const float2* __restrict__ table) {
-  grid_dep_launch();   // the attention kernel waits for this grid; its launch overlaps the rest of the projection's
+  grid_dep_launch();   // at level 2 the attention kernel is a dependent and its launch overlaps the rest of the projection
   grid_dep_wait();     // may run as a programmatic dependent of the QKV projection
   const int t = blockIdx.x;
   const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;

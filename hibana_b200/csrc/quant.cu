@@ -23,7 +23,7 @@ __global__ void quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long lon
                                    uint8_t* __restrict__ sf, int mode, const int* __restrict__ src_rows,
                                    const int* __restrict__ total_rows) {
   grid_dep_wait();     // launched as a programmatic dependent: the producer of x must have completed
-  grid_dep_launch();   // a GEMM launched as a programmatic dependent may start prefetching its weights
+  grid_dep_launch();   // a GEMM may start prefetching its weights; behind the wait, as a grouped one reads the plan (launch_dep)
   const int groups_pad = ka * 4;
   const int rows_pad = ((m + 127) >> 7) << 7;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -77,7 +77,7 @@ __global__ void quant_nvfp4_pairs_kernel(const __nv_bfloat16* __restrict__ x, lo
                                          const float* __restrict__ gscale, uint8_t* __restrict__ q,
                                          uint8_t* __restrict__ sf) {
   grid_dep_wait();
-  grid_dep_launch();
+  grid_dep_launch();   // behind the wait: the grouped GEMM that follows reads the routing plan at once (see launch_dep)
   const int groups_pad = ka * 4;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<long long>(pairs) * groups_pad) return;
