@@ -732,7 +732,7 @@ def test_prefill_waits_cover_their_tile_cpu(ntiles):
 def test_fp8_kv_attention_keeps_small_weights(hq, hkv, d, rows, dominant):
     """One key of V = 0 that outweighs each of 3000 others by e^11 to e^18 (2^16 to 2^26): the output is the sum of weights
     that are tiny against the largest. Bound: one rounding to bf16 (2^-9 of the value, 2^-8 allowed) and 1e-4 of a row's
-    root mean square for the weights (exact to 2^-38 of the largest: at 2^-26 that is 2^-12 each, averaged over 3000)."""
+    root mean square for the weights (exact to 2^-36 of the largest: at 2^-26 that is 2^-10 each, averaged over 3000)."""
     gen = torch.Generator().manual_seed(5)
     ctx_n = 3001
     k = torch.randn(ctx_n + 1, hkv, d, generator=gen)
