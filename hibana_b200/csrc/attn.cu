@@ -112,6 +112,8 @@ struct AttRow {
 
 template <int D, int MAXQ, int FMT>
 __global__ void __launch_bounds__(ATT_THREADS) attn_splitkv_kernel(const AttnParams p) {
+  grid_dep_wait();
+  grid_dep_launch();
   using RL = AttRow<D, FMT>;
   constexpr bool FP8 = FMT == 1, FP4 = FMT == 2, SCALED = FMT != 0;
   constexpr int ESZ = RL::ESZ;
@@ -418,7 +420,7 @@ int launch_attn(const AttnParams& p, int batch, int row_chunks, cudaStream_t st)
     attr = true;
   }
   const dim3 grid(batch, p.hkv * row_chunks, p.splits);
-  attn_splitkv_kernel<D, MAXQ, FP8><<<grid, ATT_THREADS, smem, st>>>(p);
+  launch_dep(attn_splitkv_kernel<D, MAXQ, FP8>, grid, dim3(ATT_THREADS), smem, st, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -500,8 +502,8 @@ int hb_attn_paged(const void* q, const void* k_pool, const void* v_pool, long lo
   }
   if (rc != 0) return rc;
   if (p.splits > 1) {
-    attn_merge_kernel<<<static_cast<unsigned>(static_cast<long long>(total_rows) * hq), 128, p.splits * sizeof(float), st>>>(
-        p.part_o, p.part_lse, p.out, p.splits, d, hq, nullptr, nullptr, nullptr, 0);
+    launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(static_cast<long long>(total_rows) * hq)), dim3(128), p.splits * sizeof(float), st,
+               p.part_o, p.part_lse, p.out, p.splits, d, hq, nullptr, nullptr, nullptr, 0);
     if (cudaGetLastError() != cudaSuccess) return 2;
   }
   return 0;
@@ -511,8 +513,8 @@ int hb_attn_merge(const void* part_o, const void* part_lse, void* out, long long
                   void* stream) {
   if (rows_heads <= 0) return 0;
   launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows_heads)), dim3(128), splits * sizeof(float), static_cast<cudaStream_t>(stream),
-      static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(out), splits,
-      d, 1, static_cast<uint8_t*>(nullptr), static_cast<uint8_t*>(nullptr), static_cast<const float*>(nullptr), 0);
+             static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(out), splits,
+             d, 1, static_cast<uint8_t*>(nullptr), static_cast<uint8_t*>(nullptr), static_cast<const float*>(nullptr), 0);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -523,9 +525,9 @@ int hb_attn_merge_quant(const void* part_o, const void* part_lse, long long rows
   if (rows <= 0) return 0;
   if (d > 256 || d % 16 != 0 || q_out == nullptr || q_sf == nullptr || q_gscale == nullptr) return 1;
   launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows * hq)), dim3(128), splits * sizeof(float), static_cast<cudaStream_t>(stream),
-      static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(nullptr),
-      splits, d, hq, static_cast<uint8_t*>(q_out), static_cast<uint8_t*>(q_sf), static_cast<const float*>(q_gscale),
-      q_ka);
+             static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(nullptr),
+             splits, d, hq, static_cast<uint8_t*>(q_out), static_cast<uint8_t*>(q_sf), static_cast<const float*>(q_gscale),
+             q_ka);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -386,6 +386,8 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
 template <int D, bool F8>
 __global__ void __launch_bounds__(PfRoles<F8>::THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
+  grid_dep_launch();
+  grid_dep_wait();
   using C = PfCfg<D, F8>;
   constexpr int KT = C::KT;
   constexpr int PF_PRODUCERS = PfRoles<F8>::PRODUCERS, ISSUER = PfRoles<F8>::ISSUER;
@@ -793,6 +795,8 @@ __device__ __forceinline__ float pp_weights(uint32_t s_t, int keys, int rel, flo
 template <int D, bool F8>
 __global__ void __launch_bounds__(PpRoles<F8>::THREADS, 1)
 attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
+  grid_dep_launch();
+  grid_dep_wait();
   using C = PfCfg<D, F8>;
   constexpr int KT = C::KT;
   constexpr int ISSUER = PpRoles<F8>::ISSUER;
@@ -1060,8 +1064,8 @@ int launch_prefill_pp(const PfParams& p, const CUtensorMap* tk, const CUtensorMa
       return 3;
     attr = true;
   }
-  attn_prefill_pp_kernel<D, F8><<<dim3(qblocks * p.splits, p.hkv, batch), PpRoles<F8>::THREADS, PpCfg<D, F8>::SMEM, st>>>(
-      *tk, *tv, p);
+  launch_dep(attn_prefill_pp_kernel<D, F8>, dim3(qblocks * p.splits, p.hkv, batch), dim3(PpRoles<F8>::THREADS), PpCfg<D, F8>::SMEM, st,
+             *tk, *tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -1076,7 +1080,7 @@ int launch_prefill(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* 
       return 3;
     attr = true;
   }
-  attn_prefill_kernel<D, F8><<<dim3(qblocks * p.splits, p.hkv, batch), PfRoles<F8>::THREADS, C::SMEM, st>>>(*tk, *tv, p);
+  launch_dep(attn_prefill_kernel<D, F8>, dim3(qblocks * p.splits, p.hkv, batch), dim3(PfRoles<F8>::THREADS), C::SMEM, st, *tk, *tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -94,6 +94,8 @@ __device__ __forceinline__ void load_b32(uint32_t (&b)[4][2], uint32_t tile, int
 
 template <int G>
 __global__ void __launch_bounds__(128 * G) gdn_chunk_kernel(const ChunkParams p) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ __align__(16) uint8_t g_smem[];
   const uint32_t sb = smem_u32(g_smem);
   using L = ChunkSmem<G>;
@@ -283,9 +285,9 @@ int hb_gdn_chunk_pass(const void* w, const void* qg, const void* kd, const void*
   // One group per CTA while all CTAs are resident at once (a CTA of one group is a little faster by itself).
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (vdim % (2 * VS) == 0 && heads * (vdim / VS) > kNumSms)
-    gdn_chunk_kernel<2><<<dim3(heads, vdim / (2 * VS)), 256, ChunkSmem<2>::BYTES, st>>>(p);
+    launch_dep(gdn_chunk_kernel<2>, dim3(heads, vdim / (2 * VS)), dim3(256), ChunkSmem<2>::BYTES, st, p);
   else
-    gdn_chunk_kernel<1><<<dim3(heads, vdim / VS), 128, ChunkSmem<1>::BYTES, st>>>(p);
+    launch_dep(gdn_chunk_kernel<1>, dim3(heads, vdim / VS), dim3(128), ChunkSmem<1>::BYTES, st, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -332,6 +334,8 @@ struct Phase1Params {
 };
 
 __global__ void __launch_bounds__(128, 2) gdn_phase1_kernel(const Phase1Params p) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ __align__(16) uint8_t sm[];
   const uint32_t sb = smem_u32(sm);
   float* a_s = reinterpret_cast<float*>(sm + P1_A);
@@ -539,7 +543,7 @@ int hb_gdn_phase1(const void* q, const void* k, const void* v, const void* g, co
       return 3;
     attr = true;
   }
-  gdn_phase1_kernel<<<dim3(p.nc, v_heads), 128, P1_SMEM, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_dep(gdn_phase1_kernel, dim3(p.nc, v_heads), dim3(128), P1_SMEM, static_cast<cudaStream_t>(stream), p);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -568,6 +572,8 @@ struct SsdP1Params {
 };
 
 __global__ void __launch_bounds__(128, 2) ssd_phase1_kernel(const SsdP1Params p) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ __align__(16) uint8_t sm[];
   const uint32_t sb = smem_u32(sm);
   constexpr int S_C = 0, S_B = GC * P1_PK, S_G = 2 * GC * P1_PK;
@@ -696,7 +702,7 @@ int hb_ssd_phase1(const void* x, const void* b, const void* c, const void* dt, c
     if (cudaFuncSetAttribute(ssd_phase1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 3;
     attr = true;
   }
-  ssd_phase1_kernel<<<dim3(q.nc, heads), 128, smem, static_cast<cudaStream_t>(stream)>>>(q);
+  launch_dep(ssd_phase1_kernel, dim3(q.nc, heads), dim3(128), smem, static_cast<cudaStream_t>(stream), q);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -747,6 +753,8 @@ constexpr int SSD_SMEM = SSD_GAM + 4 * GC * 4 + 16;   // + gamma_C of the two st
 static_assert(SSD_SMEM <= 227 * 1024, "shared memory");
 
 __global__ void __launch_bounds__(512, 1) ssd_chunk_kernel(const SsdParams p) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ __align__(16) uint8_t sm[];
   const uint32_t sb = smem_u32(sm);
   float* g_end = reinterpret_cast<float*>(sm + SSD_GAM + 4 * GC * 4);
@@ -1019,7 +1027,7 @@ int hb_ssd_chunk(const void* x, const void* b, const void* c, const void* dt, co
     if (cudaFuncSetAttribute(ssd_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SSD_SMEM) != cudaSuccess) return 3;
     attr = true;
   }
-  ssd_chunk_kernel<<<dim3(heads, (p + 63) / 64), 512, SSD_SMEM, static_cast<cudaStream_t>(stream)>>>(q);
+  launch_dep(ssd_chunk_kernel, dim3(heads, (p + 63) / 64), dim3(512), SSD_SMEM, static_cast<cudaStream_t>(stream), q);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -920,7 +920,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
     }
     prof_mark(p, 5, t_entry);
     __syncwarp();
-    if (p.splits > 1) cluster_sync_all();   // nobody leaves while a peer may still read its partial
+    if (p.splits > 1) cluster_sync_exit();   // nobody leaves while a peer may still read its partial
     prof_mark(p, 6, t_entry);
   }
   prof_mark(p, 7, t_entry);

@@ -175,6 +175,12 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {   // every thread of every CTA of the cluster
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same meeting without ordering of memory: for CTAs that only must not leave while a peer still reads their shared memory
+// (whose values the peer has used by then). The release above first waits for the thread's global stores to be acknowledged,
+// which nobody in the cluster reads: 1.3 us at the end of a split-K projection.
+__device__ __forceinline__ void cluster_sync_exit() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_t cta) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta));
@@ -241,15 +247,17 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
 
 // Launch as a programmatic dependent of the kernel before it in the stream (when the library-wide switch is on,
 // see hb_gemm_set_pdl): the grid may be scheduled while its predecessor drains, which hides launch latency. The rules:
-//   * every kernel calls grid_dep_wait() before it reads anything that ANY kernel of the step wrote, and before it writes
-//     anything. Kernels may call grid_dep_launch() ahead of their own wait (norm + quantise, RoPE + KV write, decode
-//     attention, merge do), so when a dependent starts, kernels further back than its predecessor may still run;
+//   * every kernel calls grid_dep_wait() in every CTA, before it reads anything that ANY kernel of the step wrote, and before it
+//     writes anything (a grid none of whose CTAs waits could end before its predecessor, and its dependent's wait with it).
+//     Kernels may call grid_dep_launch() ahead of their own wait (norms, RoPE + KV write, attention, merges, plain GEMMs do), so
+//     when a dependent starts, kernels further back than its predecessor may still run;
 //   * before the wait only weights, norm weights and static scales may be read;
 //   * one exception: the one-CTA grouped GEMM (gemm.cu) reads the routing plan before its wait, to leave early. That is safe
 //     because the kernel in front of it (the activation quantiser, the row gather) triggers only after its own wait, which
 //     the plan kernel's end precedes, or is another grouped GEMM behind such a kernel. One that is put in between must do
 //     the same.
-// At level 1 only GEMMs are launched as dependents, so an early trigger matters where a GEMM follows.
+// At level 1 only GEMMs are launched as dependents, so an early trigger matters where a GEMM follows. Level 2 is the default:
+// the launch latency (0.4 us in a graph) and prologue of every kernel of a step pass behind its predecessor.
 extern "C" int hb_gemm_get_pdl(void);
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

@@ -29,6 +29,8 @@ __global__ void __launch_bounds__(256)
 rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int h, long long ldx,
                long long ldy, float eps, int gemma) {
+  grid_dep_launch();
+  grid_dep_wait();
   __shared__ float red[32];
   const int row = blockIdx.x;
   const int nvec = h >> 3;
@@ -88,6 +90,8 @@ gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
                          long long ldx, long long ldz, float eps, int norm_first, int sigmoid_gate, int gemma,
                          uint8_t* __restrict__ q_out, uint8_t* __restrict__ q_sf, const float* __restrict__ q_gscale,
                          int q_ka) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int groups = h / gs;
   const long long id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / L;
   const bool live = id < static_cast<long long>(rows) * groups;      // (idle lanes still take part in the shuffles)
@@ -182,6 +186,8 @@ __global__ void gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const 
                                      const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows,
                                      int h, int gs, long long ldx, long long ldz, float eps, int norm_first,
                                      int sigmoid_gate, int gemma) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int groups = h / gs;
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -330,6 +336,8 @@ __device__ __forceinline__ float act_one(int mode, float a, float b) {
 }
 __global__ void act_mul_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
                                    __nv_bfloat16* __restrict__ out, long long rows, int inter, long long ldx, int mode) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int per_row = inter >> 3;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= rows * per_row) return;
@@ -365,6 +373,8 @@ __global__ void act_mul_vec_kernel(const __nv_bfloat16* __restrict__ x, const __
 // other. In place on the contiguous y; 8 channels per thread. Five element-wise passes took 230 us at 4096 x 8192, this takes 33.
 __global__ void head_skip_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x, long long ldx,
                                  const float* __restrict__ d, long long rows, int inner, int head_dim) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int per_row = inner >> 3;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= rows * per_row) return;
@@ -384,6 +394,8 @@ __global__ void head_skip_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloa
 
 __global__ void act_mul_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
                                __nv_bfloat16* __restrict__ out, long long rows, int inter, long long ldx, int mode) {
+  grid_dep_wait();
+  grid_dep_launch();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= rows * inter) return;
   const long long r = idx / inter;
@@ -409,6 +421,8 @@ __global__ void act_mul_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 __global__ void gdn_gates_kernel(const __nv_bfloat16* __restrict__ ba, long long ld, const float* __restrict__ a_log,
                                  const float* __restrict__ dt_bias, int rows, int heads, float* __restrict__ beta,
                                  float* __restrict__ g) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * heads) return;
   const int r = i / heads, hd = i - r * heads;
@@ -421,6 +435,8 @@ __global__ void gdn_gates_kernel(const __nv_bfloat16* __restrict__ ba, long long
 
 __global__ void embedding_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                  __nv_bfloat16* __restrict__ out, int h, long long vocab) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int t = blockIdx.x;
   long long id = ids[t];
   if (id < 0 || id >= vocab || !index_ok(id, kBoundVocab, kKerEmbedding)) id = 0;
@@ -431,6 +447,8 @@ __global__ void embedding_kernel(const long long* __restrict__ ids, const __nv_b
 
 __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                            __nv_bfloat16* __restrict__ out, long long n) {
+  grid_dep_wait();
+  grid_dep_launch();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2;
   if (i + 1 < n) {
     const uint32_t x = *reinterpret_cast<const uint32_t*>(a + i), y = *reinterpret_cast<const uint32_t*>(b + i);
@@ -455,11 +473,9 @@ int hb_rmsnorm(const void* x, void* residual, const void* w, void* y, int rows, 
                float eps, int gemma, void* stream) {
   if (h % 8 != 0 || rows <= 0) return 1;
   const int nvec = h / 8;
-  if (nvec <= 256) rmsnorm_kernel<1><<<rows, 256, 0, ST(stream)>>>(BF(x), BFM(residual), BF(w), BFM(y), h, ldx, ldy, eps, gemma);
-  else if (nvec <= 512) rmsnorm_kernel<2><<<rows, 256, 0, ST(stream)>>>(BF(x), BFM(residual), BF(w), BFM(y), h, ldx, ldy, eps, gemma);
-  else if (nvec <= 1024) rmsnorm_kernel<4><<<rows, 256, 0, ST(stream)>>>(BF(x), BFM(residual), BF(w), BFM(y), h, ldx, ldy, eps, gemma);
-  else if (nvec <= 2048) rmsnorm_kernel<8><<<rows, 256, 0, ST(stream)>>>(BF(x), BFM(residual), BF(w), BFM(y), h, ldx, ldy, eps, gemma);
-  else return 1;
+  if (nvec > 2048) return 1;
+  launch_dep(nvec <= 256 ? rmsnorm_kernel<1> : nvec <= 512 ? rmsnorm_kernel<2> : nvec <= 1024 ? rmsnorm_kernel<4> : rmsnorm_kernel<8>,
+             dim3(rows), dim3(256), 0, ST(stream), BF(x), BFM(residual), BF(w), BFM(y), h, ldx, ldy, eps, gemma);
   return OK();
 }
 
@@ -470,7 +486,7 @@ static int gated_rmsnorm_reg(const void* x, const void* z, const void* w, void* 
   const long long threads = static_cast<long long>(rows) * (h / gs) * lanes;
   const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
 #define HB_GN(NC, L)                                                                                                      \
-  gated_rmsnorm_reg_kernel<NC, L><<<blocks, 256, 0, ST(stream)>>>(                                                        \
+  launch_dep(gated_rmsnorm_reg_kernel<NC, L>, dim3(blocks), dim3(256), 0, ST(stream),                                     \
       BF(x), BF(z), BF(w), BFM(y), rows, h, gs, ldx, ldz, eps, norm_first, sigmoid_gate, gemma, static_cast<uint8_t*>(q), \
       static_cast<uint8_t*>(sf), static_cast<const float*>(gscale), ka)
   if (lanes == 8) HB_GN(1, 8);
@@ -491,8 +507,8 @@ int hb_gated_rmsnorm(const void* x, const void* z, const void* w, void* y, int r
                              nullptr, 0, stream);
   const long long warps = static_cast<long long>(rows) * (h / gs);
   const unsigned blocks = static_cast<unsigned>((warps * 32 + 255) / 256);
-  gated_rmsnorm_kernel<<<blocks, 256, 0, ST(stream)>>>(BF(x), BF(z), BF(w), BFM(y), rows, h, gs, ldx, ldz, eps,
-                                                       norm_first, sigmoid_gate, gemma);
+  launch_dep(gated_rmsnorm_kernel, dim3(blocks), dim3(256), 0, ST(stream), BF(x), BF(z), BF(w), BFM(y), rows, h, gs, ldx, ldz, eps,
+             norm_first, sigmoid_gate, gemma);
   return OK();
 }
 
@@ -503,17 +519,17 @@ int hb_head_skip(void* y, const void* x, long long ldx, const void* d, long long
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) != 0)
     return 1;
   const long long n = rows * (inner / 8);
-  head_skip_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, ST(stream)>>>(
-      BFM(y), BF(x), ldx, static_cast<const float*>(d), rows, inner, head_dim);
+  launch_dep(head_skip_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, ST(stream),
+             BFM(y), BF(x), ldx, static_cast<const float*>(d), rows, inner, head_dim);
   return OK();
 }
 
 int hb_gdn_gates(const void* ba, long long ld, const void* a_log, const void* dt_bias, int rows, int heads,
                  void* beta, void* g, void* stream) {
   if (rows <= 0) return 0;
-  gdn_gates_kernel<<<(rows * heads + 255) / 256, 256, 0, ST(stream)>>>(
-      BF(ba), ld, static_cast<const float*>(a_log), static_cast<const float*>(dt_bias), rows, heads,
-      static_cast<float*>(beta), static_cast<float*>(g));
+  launch_dep(gdn_gates_kernel, dim3((rows * heads + 255) / 256), dim3(256), 0, ST(stream),
+             BF(ba), ld, static_cast<const float*>(a_log), static_cast<const float*>(dt_bias), rows, heads,
+             static_cast<float*>(beta), static_cast<float*>(g));
   return OK();
 }
 
@@ -599,6 +615,8 @@ void hb_rope_use_table(const void* table) { g_rope_table = static_cast<const flo
 
 __global__ void rope_table_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq, int tokens,
                                   int half, float2* __restrict__ out) {
+  grid_dep_wait();
+  grid_dep_launch();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<long long>(tokens) * half) return;
   const int t = static_cast<int>(i / half), j = static_cast<int>(i % half);
@@ -611,8 +629,8 @@ __global__ void rope_table_kernel(const int* __restrict__ positions, const float
 int hb_rope_table(const void* positions, const void* inv_freq, int tokens, int half, void* out, void* stream) {
   if (tokens <= 0 || half <= 0) return 0;
   const long long n = static_cast<long long>(tokens) * half;
-  rope_table_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, ST(stream)>>>(
-      static_cast<const int*>(positions), static_cast<const float*>(inv_freq), tokens, half, static_cast<float2*>(out));
+  launch_dep(rope_table_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, ST(stream),
+             static_cast<const int*>(positions), static_cast<const float*>(inv_freq), tokens, half, static_cast<float2*>(out));
   return OK();
 }
 
@@ -647,10 +665,10 @@ int hb_rope_kv_write(const void* qkv, long long ld_qkv, const void* positions, c
   const int heads = hq + 2 * hkv;
   const int ysplit = (heads + 7) / 8;
   launch_dep(rope_kv_write_kernel, dim3(tokens, ysplit), dim3(256), 0, ST(stream),
-      BF(qkv), ld_qkv, static_cast<const int*>(positions), static_cast<const int*>(slots),
-      static_cast<const float*>(inv_freq), BF(q_norm_w), BF(k_norm_w), eps, gemma_norm, BFM(q_out), k_pool, v_pool,
-      pool_stride, head_stride, hq, hkv, d, rot, kv_fp8, kv_inv_scale, q_gate, g_kv_sf.k, g_kv_sf.v,
-      g_kv_sf.pool_stride, g_kv_sf.head_stride, g_rope_table);
+             BF(qkv), ld_qkv, static_cast<const int*>(positions), static_cast<const int*>(slots),
+             static_cast<const float*>(inv_freq), BF(q_norm_w), BF(k_norm_w), eps, gemma_norm, BFM(q_out), k_pool, v_pool,
+             pool_stride, head_stride, hq, hkv, d, rot, kv_fp8, kv_inv_scale, q_gate, g_kv_sf.k, g_kv_sf.v,
+             g_kv_sf.pool_stride, g_kv_sf.head_stride, g_rope_table);
   g_kv_sf = KvSf{};
   g_rope_table = nullptr;
   return OK();
@@ -664,26 +682,27 @@ int hb_act_mul(const void* x, const void* gate, void* out, long long rows, int i
   // A thread of the vector form computes eight exponentials and divisions one after the other, which few elements do not hide:
   // scalar / vector, 1 x 5376 1.7 / 2.1 us, 32 x 5376 2.0 / 2.2, 192 x 1024 2.2 / 2.2, 64 x 5376 2.7 / 2.3. Squared ReLU has neither.
   if (inter % 8 == 0 && ldx % 8 == 0 && (ptrs & 15) == 0 && (mode == 2 || n >= 192 * 1024)) {
-    act_mul_vec_kernel<<<static_cast<unsigned>((n / 8 + 255) / 256), 256, 0, ST(stream)>>>(BF(x), BF(gate), BFM(out), rows,
-                                                                                           inter, ldx, mode);
+    launch_dep(act_mul_vec_kernel, dim3(static_cast<unsigned>((n / 8 + 255) / 256)), dim3(256), 0, ST(stream), BF(x), BF(gate),
+               BFM(out), rows, inter, ldx, mode);
     return OK();
   }
-  act_mul_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, ST(stream)>>>(BF(x), BF(gate), BFM(out), rows,
-                                                                                inter, ldx, mode);
+  launch_dep(act_mul_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, ST(stream), BF(x), BF(gate), BFM(out),
+             rows, inter, ldx, mode);
   return OK();
 }
 
 int hb_embedding(const void* ids, const void* table, void* out, int tokens, int h, long long vocab, void* stream) {
   if (tokens <= 0) return 0;
   if (h % 8 != 0) return 1;
-  embedding_kernel<<<tokens, 128, 0, ST(stream)>>>(static_cast<const long long*>(ids), BF(table), BFM(out), h, vocab);
+  launch_dep(embedding_kernel, dim3(tokens), dim3(128), 0, ST(stream), static_cast<const long long*>(ids), BF(table), BFM(out),
+             h, vocab);
   return OK();
 }
 
 int hb_add(const void* a, const void* b, void* out, long long n, void* stream) {
   if (n <= 0) return 0;
   const long long threads = (n + 1) / 2;
-  add_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, ST(stream)>>>(BF(a), BF(b), BFM(out), n);
+  launch_dep(add_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, ST(stream), BF(a), BF(b), BFM(out), n);
   return OK();
 }
 

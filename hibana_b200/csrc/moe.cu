@@ -35,6 +35,8 @@ __device__ __forceinline__ unsigned route_key(float v) {
 __global__ void __launch_bounds__(1024) moe_route_block_kernel(
     const float* __restrict__ logits, long long ld, const float* __restrict__ sel_bias, int experts, int topk,
     int sigmoid, int renorm, float scale, int* __restrict__ ids, float* __restrict__ weights) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ float s_red[32];
   __shared__ int s_warp_tie[32], s_warp_sel[32];
   __shared__ unsigned s_key[MAX_TOPK];
@@ -111,6 +113,8 @@ template <int PER>
 __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ sel_bias,
                                  int tokens, int experts, int topk, int sigmoid, int renorm, float scale,
                                  int* __restrict__ ids, float* __restrict__ weights) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= tokens) return;
@@ -211,6 +215,8 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
 __global__ void __launch_bounds__(1024)
 moe_share_kernel(int* __restrict__ ids, float* __restrict__ weights, int rows, int k, int experts, int keep, int budget,
                  float scale) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ unsigned score[1024];
   __shared__ unsigned char in_set[1024];
   __shared__ int s_core;
@@ -309,6 +315,8 @@ moe_plan_kernel(const int* __restrict__ ids, int pairs, int topk, int experts, i
                 int* __restrict__ cnt, int* __restrict__ start, int* __restrict__ pos, int* __restrict__ src_row,
                 int rows_cap, int* __restrict__ total_rows, int tile_bn, int* __restrict__ tiles,
                 int* __restrict__ n_tiles, int tile_cap) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ int sm[];   // [experts] own counts, [experts] starts, [experts] running, [warps][experts]
   int* own = sm;
   int* s = sm + experts;
@@ -436,6 +444,8 @@ moe_plan_kernel(const int* __restrict__ ids, int pairs, int topk, int experts, i
 // expert * 4096 + chunk per tile of `tile_bn` rows that has rows. Single CTA.
 __global__ void moe_tiles_kernel(const int* __restrict__ cnt, int experts, int tile_bn, int* __restrict__ tiles,
                                  int* __restrict__ n_tiles, int tile_cap) {
+  grid_dep_wait();
+  grid_dep_launch();
   extern __shared__ int base[];
   __shared__ int wtot[32];
   __shared__ int s_total;
@@ -463,6 +473,8 @@ __global__ void moe_tiles_kernel(const int* __restrict__ cnt, int experts, int t
 
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ src_row,
                                   const int* __restrict__ total_rows, __nv_bfloat16* __restrict__ out, int h) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int r = blockIdx.x;
   if (r >= *total_rows) return;
   const int src = src_row[r];
@@ -480,6 +492,8 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, long lon
                                    const float* __restrict__ weights, const __nv_bfloat16* __restrict__ shared,
                                    long long ld_shared, __nv_bfloat16* __restrict__ out, long long ldo, int topk,
                                    int h) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int t = blockIdx.x;
   __shared__ int ps[MAX_TOPK];
   __shared__ float ws[MAX_TOPK];
@@ -519,13 +533,13 @@ int hb_moe_route(const void* logits, long long ld, const void* sel_bias, int tok
   if (experts > 1024 || topk > MAX_TOPK || topk > experts) return 1;
   if (tokens <= 256 && experts > 128) {      // decode / verify sizes: latency matters, one CTA per token
     const int threads = (experts + 31) / 32 * 32;
-    moe_route_block_kernel<<<tokens, threads, 0, ST(stream)>>>(
-        static_cast<const float*>(logits), ld, static_cast<const float*>(sel_bias), experts, topk, sigmoid, renorm,
-        scale, static_cast<int*>(ids), static_cast<float*>(weights));
+    launch_dep(moe_route_block_kernel, dim3(tokens), dim3(threads), 0, ST(stream),
+               static_cast<const float*>(logits), ld, static_cast<const float*>(sel_bias), experts, topk, sigmoid, renorm,
+               scale, static_cast<int*>(ids), static_cast<float*>(weights));
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
   }
 #define HB_ROUTE(PER)                                                                                        \
-  moe_route_kernel<PER><<<(tokens + 3) / 4, 128, 0, ST(stream)>>>(                                           \
+  launch_dep(moe_route_kernel<PER>, dim3((tokens + 3) / 4), dim3(128), 0, ST(stream),                                            \
       static_cast<const float*>(logits), ld, static_cast<const float*>(sel_bias), tokens, experts, topk, sigmoid, \
       renorm, scale, static_cast<int*>(ids), static_cast<float*>(weights))
   if (experts <= 128) HB_ROUTE(4);
@@ -539,8 +553,8 @@ int hb_moe_share(void* ids, void* weights, int rows, int k, int experts, int kee
                  void* stream) {
   if (rows <= 0) return 0;
   if (experts > 1024 || k > MAX_TOPK || keep < 0 || keep > k || rows * k > 16384) return 1;
-  moe_share_kernel<<<1, 1024, 0, ST(stream)>>>(static_cast<int*>(ids), static_cast<float*>(weights), rows, k, experts,
-                                               keep, budget, scale);
+  launch_dep(moe_share_kernel, dim3(1), dim3(1024), 0, ST(stream), static_cast<int*>(ids), static_cast<float*>(weights), rows, k, experts,
+             keep, budget, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -564,11 +578,13 @@ int hb_moe_plan(const void* ids, int tokens, int topk, int experts, int e_lo, in
   cfg.blockDim = dim3(1024);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ST(stream);
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ranks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = hb_gemm_get_pdl() >= 2 ? 2 : 1;
   (void)cudaLaunchKernelEx(&cfg, moe_plan_kernel,
       static_cast<const int*>(ids), tokens * topk, topk, experts, e_lo, e_n, id_base, static_cast<int*>(cnt),
       static_cast<int*>(start), static_cast<int*>(pos), static_cast<int*>(src_row), rows_cap,
@@ -578,19 +594,19 @@ int hb_moe_plan(const void* ids, int tokens, int topk, int experts, int e_lo, in
 
 int hb_moe_tiles(const void* cnt, int experts, int tile_bn, void* tiles, void* n_tiles, int tile_cap, void* stream) {
   if (experts <= 0 || tile_bn < 16 || tile_cap <= 0) return 1;
-  moe_tiles_kernel<<<1, 1024, experts * sizeof(int), ST(stream)>>>(static_cast<const int*>(cnt), experts, tile_bn,
-                                                                  static_cast<int*>(tiles),
-                                                                  static_cast<int*>(n_tiles), tile_cap);
+  launch_dep(moe_tiles_kernel, dim3(1), dim3(1024), experts * sizeof(int), ST(stream), static_cast<const int*>(cnt), experts, tile_bn,
+             static_cast<int*>(tiles),
+             static_cast<int*>(n_tiles), tile_cap);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
 int hb_moe_gather(const void* x, long long ldx, const void* src_row, const void* total_rows, void* out, int rows_cap,
                   int h, void* stream) {
   if (rows_cap <= 0) return 0;
-  moe_gather_kernel<<<rows_cap, 128, 0, ST(stream)>>>(static_cast<const __nv_bfloat16*>(x), ldx,
-                                                      static_cast<const int*>(src_row),
-                                                      static_cast<const int*>(total_rows),
-                                                      static_cast<__nv_bfloat16*>(out), h);
+  launch_dep(moe_gather_kernel, dim3(rows_cap), dim3(128), 0, ST(stream), static_cast<const __nv_bfloat16*>(x), ldx,
+             static_cast<const int*>(src_row),
+             static_cast<const int*>(total_rows),
+             static_cast<__nv_bfloat16*>(out), h);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -598,10 +614,10 @@ int hb_moe_combine(const void* y, long long ldy, const void* pos, const void* we
                    long long ld_shared, void* out, long long ldo, int tokens, int topk, int h, void* stream) {
   if (tokens <= 0) return 0;
   if (topk > MAX_TOPK || (h & 1)) return 1;
-  moe_combine_kernel<<<tokens, 256, 0, ST(stream)>>>(static_cast<const __nv_bfloat16*>(y), ldy,
-                                                     static_cast<const int*>(pos), static_cast<const float*>(weights),
-                                                     static_cast<const __nv_bfloat16*>(shared), ld_shared,
-                                                     static_cast<__nv_bfloat16*>(out), ldo, topk, h);
+  launch_dep(moe_combine_kernel, dim3(tokens), dim3(256), 0, ST(stream), static_cast<const __nv_bfloat16*>(y), ldy,
+             static_cast<const int*>(pos), static_cast<const float*>(weights),
+             static_cast<const __nv_bfloat16*>(shared), ld_shared,
+             static_cast<__nv_bfloat16*>(out), ldo, topk, h);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

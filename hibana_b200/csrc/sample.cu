@@ -33,6 +33,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 argmax_kernel(const T* __restrict__ logits, long long ld, int vocab, const int* __restrict__ bitmask, int mask_words,
               long long* __restrict__ out, float* __restrict__ out_val) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ float sv[8];
   __shared__ int si[8];
   const int row = blockIdx.x;
@@ -78,6 +80,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 argmax_partial_kernel(const T* __restrict__ logits, long long ld, int vocab, const int* __restrict__ bitmask,
                       int mask_words, int nch, float* __restrict__ pv, int* __restrict__ pi) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ float sv[8];
   __shared__ int si[8];
   const int row = blockIdx.x, ch = blockIdx.y;
@@ -124,6 +128,8 @@ argmax_partial_kernel(const T* __restrict__ logits, long long ld, int vocab, con
 __global__ void argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int nch, int rows,
                                     const float* __restrict__ temperature, long long* __restrict__ out,
                                     float* __restrict__ out_val) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -471,6 +477,8 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
               const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ offsets,
               const int* __restrict__ bitmask, int mask_words, long long* __restrict__ out,
               float* __restrict__ out_prob, int skip_greedy) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ float cv[SAMPLE_K];
   __shared__ int ci[SAMPLE_K];
   __shared__ float wv[LAW_WARPS];
@@ -760,13 +768,13 @@ int hb_argmax(const void* logits, long long ld, int rows, int vocab, int is_f32,
   if (rows <= 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (is_f32)
-    argmax_kernel<float><<<rows, 256, 0, st>>>(static_cast<const float*>(logits), ld, vocab,
-                                               static_cast<const int*>(bitmask), mask_words,
-                                               static_cast<long long*>(out), static_cast<float*>(out_val));
+    launch_dep(argmax_kernel<float>, dim3(rows), dim3(256), 0, st, static_cast<const float*>(logits), ld, vocab,
+               static_cast<const int*>(bitmask), mask_words,
+               static_cast<long long*>(out), static_cast<float*>(out_val));
   else
-    argmax_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), ld, vocab,
-                                                       static_cast<const int*>(bitmask), mask_words,
-                                                       static_cast<long long*>(out), static_cast<float*>(out_val));
+    launch_dep(argmax_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(logits), ld, vocab,
+               static_cast<const int*>(bitmask), mask_words,
+               static_cast<long long*>(out), static_cast<float*>(out_val));
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -780,8 +788,8 @@ int hb_sample(const void* logits, long long ld, int rows, int vocab, int is_f32,
       static_cast<const float*>(top_p), static_cast<const unsigned long long*>(seeds),                     \
       static_cast<const unsigned long long*>(offsets), static_cast<const int*>(bitmask), mask_words,       \
       static_cast<long long*>(out), static_cast<float*>(out_prob), skip_greedy
-  if (is_f32) sample_kernel<float><<<rows, LAW_T, 0, st>>>(static_cast<const float*>(logits), HB_SAMPLE_ARGS);
-  else sample_kernel<__nv_bfloat16><<<rows, LAW_T, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SAMPLE_ARGS);
+  if (is_f32) launch_dep(sample_kernel<float>, dim3(rows), dim3(LAW_T), 0, st, static_cast<const float*>(logits), HB_SAMPLE_ARGS);
+  else launch_dep(sample_kernel<__nv_bfloat16>, dim3(rows), dim3(LAW_T), 0, st, static_cast<const __nv_bfloat16*>(logits), HB_SAMPLE_ARGS);
 #undef HB_SAMPLE_ARGS
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
@@ -854,17 +862,17 @@ int hb_argmax2(const void* logits, long long ld, int rows, int vocab, int is_f32
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const dim3 grid(rows, nch);
   if (is_f32)
-    argmax_partial_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(logits), ld, vocab,
-                                                       static_cast<const int*>(bitmask), mask_words, nch,
-                                                       static_cast<float*>(scratch_v), static_cast<int*>(scratch_i));
+    launch_dep(argmax_partial_kernel<float>, grid, dim3(256), 0, st, static_cast<const float*>(logits), ld, vocab,
+               static_cast<const int*>(bitmask), mask_words, nch,
+               static_cast<float*>(scratch_v), static_cast<int*>(scratch_i));
   else
-    argmax_partial_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(logits), ld, vocab, static_cast<const int*>(bitmask), mask_words, nch,
-        static_cast<float*>(scratch_v), static_cast<int*>(scratch_i));
-  argmax_final_kernel<<<(rows + 3) / 4, 128, 0, st>>>(static_cast<const float*>(scratch_v),
-                                                      static_cast<const int*>(scratch_i), nch, rows,
-                                                      static_cast<const float*>(temperature),
-                                                      static_cast<long long*>(out), static_cast<float*>(out_val));
+    launch_dep(argmax_partial_kernel<__nv_bfloat16>, grid, dim3(256), 0, st,
+               static_cast<const __nv_bfloat16*>(logits), ld, vocab, static_cast<const int*>(bitmask), mask_words, nch,
+               static_cast<float*>(scratch_v), static_cast<int*>(scratch_i));
+  launch_dep(argmax_final_kernel, dim3((rows + 3) / 4), dim3(128), 0, st, static_cast<const float*>(scratch_v),
+             static_cast<const int*>(scratch_i), nch, rows,
+             static_cast<const float*>(temperature),
+             static_cast<long long*>(out), static_cast<float*>(out_val));
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -31,6 +31,8 @@ __global__ void conv1d_kernel(const __nv_bfloat16* __restrict__ x, long long ldx
                               const int* __restrict__ q_indptr, const int* __restrict__ slot_in,
                               const int* __restrict__ slot_out, const int* __restrict__ has_init, int channels,
                               int act_silu) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -76,6 +78,8 @@ __global__ void conv1d_tiled_kernel(const __nv_bfloat16* __restrict__ x, long lo
                                     long long state_stride, const int* __restrict__ q_indptr,
                                     const int* __restrict__ slot_in, const int* __restrict__ slot_out,
                                     const int* __restrict__ has_init, int channels, int act_silu) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int b = blockIdx.z;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -121,6 +125,8 @@ __global__ void conv1d_state_kernel(const __nv_bfloat16* __restrict__ x, long lo
                                     const int* __restrict__ q_indptr, const int* __restrict__ slot_in,
                                     const int* __restrict__ slot_out, const int* __restrict__ has_init,
                                     int channels) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -180,6 +186,8 @@ __device__ __forceinline__ unsigned mix32(unsigned x) {
 
 template <int P, int N, int THREADS, int FMT>
 __global__ void __launch_bounds__(THREADS) mamba2_scan_kernel(const MambaParams p) {
+  grid_dep_wait();
+  grid_dep_launch();
   constexpr int CG = THREADS / P;          // column groups
   constexpr int NC = N / CG;               // state columns per thread
   static_assert(THREADS % P == 0 && N % CG == 0 && CG <= 32 && (CG & (CG - 1)) == 0 && NC % 4 == 0, "bad Mamba tiling");
@@ -324,6 +332,8 @@ struct GdnParams {
 // One CTA per (sequence, value head), V threads: thread v holds state row S[v, 0..K) in registers.
 template <int V, int K>
 __global__ void __launch_bounds__(V) gdn_scan_kernel(const GdnParams p) {
+  grid_dep_wait();
+  grid_dep_launch();
   // The head's [V, K] fp32 state travels through shared memory (rows padded by four floats): global traffic is
   // then whole rows per warp instruction in both directions, and thread v picks up / drops its own row from the
   // padded tile without bank conflicts. Reading rows straight from global, 512 bytes apart per lane, used half of
@@ -434,10 +444,10 @@ using namespace hb;
 
 template <int FMT>
 static int launch_mamba(const MambaParams& p, dim3 grid, int head_dim, int d_state, cudaStream_t st) {
-  if (head_dim == 32 && d_state == 64) mamba2_scan_kernel<32, 64, 128, FMT><<<grid, 128, 0, st>>>(p);
-  else if (head_dim == 64 && d_state == 128) mamba2_scan_kernel<64, 128, 256, FMT><<<grid, 256, 0, st>>>(p);
-  else if (head_dim == 64 && d_state == 64) mamba2_scan_kernel<64, 64, 256, FMT><<<grid, 256, 0, st>>>(p);
-  else if (head_dim == 32 && d_state == 16) mamba2_scan_kernel<32, 16, 128, FMT><<<grid, 128, 0, st>>>(p);
+  if (head_dim == 32 && d_state == 64) launch_dep(mamba2_scan_kernel<32, 64, 128, FMT>, grid, dim3(128), 0, st, p);
+  else if (head_dim == 64 && d_state == 128) launch_dep(mamba2_scan_kernel<64, 128, 256, FMT>, grid, dim3(256), 0, st, p);
+  else if (head_dim == 64 && d_state == 64) launch_dep(mamba2_scan_kernel<64, 64, 256, FMT>, grid, dim3(256), 0, st, p);
+  else if (head_dim == 32 && d_state == 16) launch_dep(mamba2_scan_kernel<32, 16, 128, FMT>, grid, dim3(128), 0, st, p);
   else return 1;
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
@@ -451,18 +461,18 @@ int hb_conv1d(const void* x, long long ldx, const void* w, const void* bias, voi
   if (width != 4) return 1;
   if (max_rows > CONV_TT) {   // prefill: parallel over tiles of tokens, then the new windows
     const dim3 tg((channels + 127) / 128, (max_rows + CONV_TT - 1) / CONV_TT, batch);
-    conv1d_tiled_kernel<4><<<tg, 128, 0, ST(stream)>>>(BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state),
-                                                       state_stride, IP(q_indptr), IP(slot_in), IP(slot_out),
-                                                       IP(has_init), channels, act_silu);
+    launch_dep(conv1d_tiled_kernel<4>, tg, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state),
+               state_stride, IP(q_indptr), IP(slot_in), IP(slot_out),
+               IP(has_init), channels, act_silu);
     if (slot_out != nullptr)
-      conv1d_state_kernel<4><<<dim3((channels + 127) / 128, batch), 128, 0, ST(stream)>>>(
-          BF(x), ldx, BFM(state), state_stride, IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels);
+      launch_dep(conv1d_state_kernel<4>, dim3((channels + 127) / 128, batch), dim3(128), 0, ST(stream),
+                 BF(x), ldx, BFM(state), state_stride, IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
   }
   const dim3 grid((channels + 127) / 128, batch);
-  conv1d_kernel<4><<<grid, 128, 0, ST(stream)>>>(BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state), state_stride,
-                                                 IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels,
-                                                 act_silu);
+  launch_dep(conv1d_kernel<4>, grid, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state), state_stride,
+             IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels,
+             act_silu);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -521,11 +531,11 @@ int hb_gdn_scan(const void* q, const void* k, const void* v, const void* g, cons
         return 3;
       armed = true;
     }
-    gdn_scan_kernel<128, 128><<<grid, 128, SMEM, ST(stream)>>>(p);
+    launch_dep(gdn_scan_kernel<128, 128>, grid, dim3(128), SMEM, ST(stream), p);
   } else if (kdim == 64 && vdim == 64) {
-    gdn_scan_kernel<64, 64><<<grid, 64, 64 * 68 * 4, ST(stream)>>>(p);
+    launch_dep(gdn_scan_kernel<64, 64>, grid, dim3(64), 64 * 68 * 4, ST(stream), p);
   } else if (kdim == 32 && vdim == 32) {
-    gdn_scan_kernel<32, 32><<<grid, 32, 32 * 36 * 4, ST(stream)>>>(p);
+    launch_dep(gdn_scan_kernel<32, 32>, grid, dim3(32), 32 * 36 * 4, ST(stream), p);
   } else {
     return 1;
   }
