@@ -1,5 +1,6 @@
 // Paged GQA prefill attention on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM). Head dim 256 runs the
-// kernel described here; head dims up to 128 run its two-stream form, attn_prefill_pp_kernel below.
+// kernel described here; head dims up to 128 run its two-stream form, attn_prefill_pp_kernel below, and bf16 pools with enough
+// query rows the form with two Q tiles per CTA, attn_prefill_q2_kernel.
 //
 // One CTA owns one (sequence, kv head, block of query tokens). The block's query rows are packed as
 // (token, group member) pairs, 128 rows = floor(128 / g) tokens x g query heads of the kv head, so a K / V tile
@@ -1054,6 +1055,421 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
   if (warp == ISSUER) tmem_dealloc(tmem_base, 512);
 }
 
+// bf16 pools, head dims up to 128: two Q tiles per CTA. The kernel above reads every K / V tile for one tile of 128 packed rows
+// (64 KB from L2 per 128 x 128 scores, near what L2 delivers if the softmax kept up), and the chain scores -> softmax -> P -> O of
+// a stream left the tensor cores idle for four fifths of the time. Here the two streams are two Q tiles on the same K / V tiles:
+// half the traffic, and no merge of accumulators at the end. Tiles are 64 keys, so that a stream has two score buffers in TMEM and the
+// scores of the next tile are there before the softmax of this one ends: the softmax warps never wait for an MMA in the steady
+// state. Q is loaded by the softmax warps while the producers fetch the first tiles, and the heaviest blocks of all heads and
+// sequences start first. Bounds per 64 keys and pair of Q tiles: MMAs 1280 cycles (Q K^T reads 6 KB of shared memory per
+// instruction), exponentials 1024; 1830 to 1930 are spent, 1330 of them in a softmax whose exponentials share their unit with the
+// other stream's. One layer, 40 / 8 heads of 128: 2048 tokens 111 -> 61 us, from scattered slots 200 -> 73, five prompts of 4096
+// 202 -> 103, 4096 tokens 312 -> 173, 2048 new ones over 8192 keys 457 -> 303; 32 / 32 heads of 64, 2048 tokens 75 -> 39; 29 tokens
+// 12.8 -> 8.6.
+constexpr int Q2_KT = 64;
+constexpr int Q2_STAGES = 4;      // tiles of the K and of the V ring
+constexpr int Q2_THREADS = 512;   // warps 0-3 and 4-7 softmax, 8 and 9 fetch K, 10 and 11 V, 12 and 13 issue S = Q K^T, 14 and 15 O += P V
+template <int D>
+struct Q2Cfg {
+  static constexpr int Q_TILE = PF_ROWS * D * 2;
+  static constexpr int KV_TILE = Q2_KT * D * 2;
+  static constexpr int BAR_OFF = 2 * Q_TILE + 2 * Q2_STAGES * KV_TILE;
+  static constexpr int SMEM = BAR_OFF + 256 + 1024;
+  static_assert((4 * Q2_STAGES + 13) * 8 + 8 <= 256, "barriers, TMEM address and abort flag");
+  static_assert(SMEM <= 227 * 1024 && 4 * Q2_KT + 2 * D <= 512, "shared memory, TMEM");
+};
+
+// A CTA's two Q tiles: `tpb` tokens each from tok0 on, of which tile st has rows(st) packed rows and tiles(st) key tiles.
+struct Q2Block {
+  int g, b, kvh, tpb, row0, R, tok0, ctx, kmax, ntiles;
+  int rows0, rows1, tiles0, tiles1;
+  __device__ __forceinline__ int rows(int st) const { return st ? rows1 : rows0; }
+  __device__ __forceinline__ int tiles(int st) const { return st ? tiles1 : tiles0; }
+  __device__ __forceinline__ Q2Block(const PfParams& p) {
+    g = p.hq / p.hkv;
+    tpb = PF_ROWS / g;
+    kvh = blockIdx.x;
+    b = blockIdx.y;
+    row0 = p.q_indptr ? p.q_indptr[b] : b;
+    R = p.q_indptr ? p.q_indptr[b + 1] - row0 : 1;
+    ctx = p.ctx_len[b];
+    tok0 = static_cast<int>(gridDim.z - 1 - blockIdx.z) * 2 * tpb;       // heaviest (latest) blocks first
+    const int n0 = max(0, min(tpb, R - tok0)), n1 = max(0, min(tpb, R - tok0 - tpb));
+    const int vis0 = visible(p, tok0, n0), vis1 = visible(p, tok0 + tpb, n1);
+    rows0 = n0 * g;
+    rows1 = n1 * g;
+    tiles0 = (vis0 + Q2_KT - 1) / Q2_KT;
+    tiles1 = (vis1 + Q2_KT - 1) / Q2_KT;
+    kmax = max(vis0, vis1);
+    ntiles = max(tiles0, tiles1);
+  }
+  // keys that `n` tokens from `tok` on see
+  __device__ __forceinline__ int visible(const PfParams& p, int tok, int n) const {
+    return n > 0 ? max(0, p.causal ? min(ctx, ctx - R + tok + n) : ctx) : 0;
+  }
+};
+
+// P of one row from its scores, written over them in TMEM; returns their sum. `rel` is the last visible column; WHOLE rows
+// see all of them.
+template <bool WHOLE>
+__device__ __forceinline__ float q2_weights(const uint32_t (&v)[2][32], uint32_t s_t, int rel, float scale_log2, float neg_m) {
+  const uint64_t scale2 = pack2(scale_log2, scale_log2), neg2 = pack2(neg_m, neg_m);
+  uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t w[16];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      float p0, p1;
+      unpack2(fma2(pack2(__uint_as_float(v[c][j]), __uint_as_float(v[c][j + 1])), scale2, neg2), p0, p1);
+      p0 = WHOLE || c * 32 + j <= rel ? ex2(p0) : 0.f;
+      p1 = WHOLE || c * 32 + j + 1 <= rel ? ex2(p1) : 0.f;
+      sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], pack2(p0, p1));
+      w[j >> 1] = pack_bf16(p0, p1);
+    }
+    tmem_st_32x16(s_t + c * 32, w);
+  }
+  float a, b;
+  unpack2(add2(sum2[0], sum2[1]), a, b);
+  return a + b;
+}
+
+template <int D>
+__global__ void __launch_bounds__(Q2_THREADS, 1)
+attn_prefill_q2_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, const PfParams p) {
+  grid_dep_launch();
+  grid_dep_wait();
+  using C = Q2Cfg<D>;
+  constexpr int KT = Q2_KT, CPR = D / 8;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = smem + 2 * C::Q_TILE;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::BAR_OFF);
+  uint64_t* empty = full + 2 * Q2_STAGES;      // [K, V][stage], as `full`
+  uint64_t* q_ready = empty + 2 * Q2_STAGES;
+  uint64_t* s_ready = q_ready + 1;             // [stream][score buffer]
+  // Softmax and issuers run up to a tile apart. A wait on a phase parity cannot tell phase n from n + 2, so the even and the odd
+  // tiles of a stream have barriers of their own: the next phase of one (tile t + 2) cannot complete before tile t is through.
+  uint64_t* p_ready = s_ready + 4;
+  uint64_t* pv_done = p_ready + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 4);
+  volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler too
+  const Q2Block x(p);
+  if (x.rows0 <= 0) return;   // uniform: before any barrier or TMEM allocation
+
+  if (tid == 256) {
+    for (int i = 0; i < 2 * Q2_STAGES; ++i) {
+      mbar_init(&full[i], 2);                  // one arrival per producer warp of a tile
+      mbar_init(&empty[i], 2);                 // one per stream
+    }
+    mbar_init(q_ready, 256);
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&s_ready[i], 1);
+      mbar_init(&p_ready[i], PF_ROWS);
+      mbar_init(&pv_done[i], 1);
+    }
+    *abort = 0;
+    fence_mbar_init();
+    if (p.use_tma) {
+      prefetch_tmap(&tmk);
+      prefetch_tmap(&tmv);
+    }
+  }
+  if (warp == 12) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (warp < 8) {      // Q rows, zero padded: row rr of tile st is (token tok0 + st * tpb + rr / g, head kvh * g + rr % g)
+    const uint32_t inv_g = (65536u + x.g - 1) / x.g;      // rr * inv_g >> 16 == rr / g for rr < 128
+#pragma unroll 4
+    for (int i = 0; i < 2 * PF_ROWS * CPR / 256; ++i) {
+      const int c = tid + i * 256, r = c / CPR, part = c % CPR, st = r >> 7, rr = r & 127;
+      const uint32_t dst = smem_u32(smem + st * C::Q_TILE) + sw_off(rr, part, PF_ROWS);
+      if (rr < x.rows(st)) {
+        const int t = static_cast<int>(rr * inv_g >> 16);
+        cp16(dst, p.q + (static_cast<long long>(x.row0 + x.tok0 + st * x.tpb + t) * p.hq + x.kvh * x.g + rr - t * x.g) * D +
+                      part * 8);
+      } else {
+        st_zero16(dst);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  if (warp >= 8 && warp < 12) {
+    // ------------------------------------------------------------------ producers: K or V, half a tile (32 keys) per warp
+    const bool is_v = warp >= 10;
+    const int j = warp & 1;
+    const __nv_bfloat16* pool = is_v ? p.v_pool : p.k_pool;
+    const CUtensorMap* tm = is_v ? &tmv : &tmk;
+    const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? p.seq_rows[x.b] : x.b) * p.ld_idx;
+    auto fetch_slot = [&](int t) {             // -1 beyond the visible keys
+      const int key = t * KT + j * 32 + lane;
+      return t < x.ntiles && key < x.kmax ? __ldg(idx_row + key) : -1;
+    };
+    auto place = [&](int t) { return (is_v ? Q2_STAGES : 0) + t % Q2_STAGES; };
+    int slot = fetch_slot(0), next = fetch_slot(1);
+    uint32_t late = 0;                         // bit i: the rows of tile t - i were gathered and have not been announced
+    int done = 0;
+    auto announce = [&](int t) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[place(t)]);
+    };
+    for (int t = 0; t < x.ntiles; ++t) {
+      const int at = place(t);
+      if (t >= Q2_STAGES && !warp_wait(&empty[at], (t / Q2_STAGES - 1) & 1, abort, p.status, kTimeoutEmpty)) break;
+      uint8_t* tile = ring + at * C::KV_TILE;
+      const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
+      const bool run = p.use_tma && __all_sync(0xffffffffu, slot >= 0 && slot == slot0 + lane);
+      late <<= 1;
+      if (run) {      // 32 consecutive pool rows: bulk tensor copies
+        if (elect_one()) {
+          mbar_expect_tx(&full[at], 32 * D * 2);
+#pragma unroll
+          for (int h = 0; h < D / 64; ++h)
+            tma_load_2d(tile + h * (KT * 128) + j * (32 * 128), tm, &full[at], x.kvh * p.tma_xh + h * 64,
+                        x.kvh * p.tma_yh + slot0);
+        }
+        __syncwarp();
+      } else {        // fragmented pool, tail of the context: 16-byte copies, announced with the next tile
+        constexpr int RPI = 32 / CPR;
+        const int part = lane % CPR;
+#pragma unroll 4
+        for (int ii = 0; ii < 32 / RPI; ++ii) {
+          const int rr = ii * RPI + lane / CPR;
+          const int s1 = __shfl_sync(0xffffffffu, slot, rr);
+          const uint32_t dst = smem_u32(tile) + sw_off(j * 32 + rr, part, KT);
+          if (s1 >= 0)
+            cp16(dst, pool + static_cast<long long>(s1) * p.pool_stride + x.kvh * p.head_stride + part * 8);
+          else
+            st_zero16(dst);
+        }
+        late |= 1;
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (late & 2) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        announce(t - 1);
+      }
+      slot = next;
+      next = fetch_slot(t + 2);
+      ++done;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing may land after the CTA has gone
+    if (done > 0 && (late & 1)) announce(done - 1);
+    if (*abort) {      // nor may the bulk copies (bounded: a tile whose other half was never issued does not complete)
+      volatile int ignore = 0;
+      for (int t = max(done - Q2_STAGES, 0); t < done; ++t)
+        mbar_wait(&full[place(t)], (t / Q2_STAGES) & 1, &ignore, nullptr, kTimeoutDrain);
+    }
+  } else if (warp >= 12) {
+    // ------------------------------------------------------------------ MMA issuers: a stream's Q K^T or its P V
+    // (One warp for both issued 1.6 times as slowly: an issue blocks while the pipe is busy, and a wait, passed or not, costs 100
+    // cycles.) The other stream may see more tiles: those are only passed on.
+    const int st = warp & 1, n = x.ntiles, mine = x.tiles(st);
+    const uint32_t smem_a = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+    const uint32_t ring_a = smem_a + 2 * C::Q_TILE, s_0 = tmem_base + st * 2 * KT, o_t = tmem_base + 4 * KT + st * D;
+    if (warp < 14) {
+      constexpr uint32_t idesc_qk = make_idesc_bf16(PF_ROWS, KT);
+      const uint32_t q_a = smem_a + st * C::Q_TILE;
+      bool ok = warp_wait(q_ready, 0, abort, p.status, kTimeoutFull);
+      for (int t = 0; ok && t < n; ++t) {
+        const int at = t % Q2_STAGES, sb = st * 2 + (t & 1);
+        {
+          PF_T0();
+          ok = warp_wait(&full[at], (t / Q2_STAGES) & 1, abort, p.status, kTimeoutFull);
+          PF_ACC(5, lane == 0 && st == 0);
+        }
+        // score buffer t % 2 holds P(t - 2) until that tile's O += P V is done
+        if (ok && t >= 2 && t < mine) ok = warp_wait(&pv_done[sb], ((t >> 1) - 1) & 1, abort, p.status, kTimeoutAccum);
+        if (!ok) break;
+        if (t < mine) {
+          tc_fence_after();
+          const uint32_t k_a = ring_a + at * C::KV_TILE, s_t = s_0 + (t & 1) * KT;
+          if (elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+              const uint32_t in_row = (ks & 3) * 32;   // 16 elements = 32 bytes inside the 128-byte swizzled row
+              mma_f16(s_t, make_desc_sw128(q_a + (ks >> 2) * (PF_ROWS * 128) + in_row),
+                      make_desc_sw128(k_a + (ks >> 2) * (KT * 128) + in_row), idesc_qk, ks > 0 ? 1u : 0u);
+            }
+            tc_commit(&empty[at]);
+            tc_commit(&s_ready[sb]);
+          }
+        } else if (lane == 0) {
+          mbar_arrive(&empty[at]);
+        }
+        __syncwarp();
+      }
+    } else {
+      constexpr uint32_t idesc_pv = make_idesc_bf16(PF_ROWS, D, 0, 1);
+      for (int t = 0; t < n; ++t) {
+        const int at = Q2_STAGES + t % Q2_STAGES, sb = st * 2 + (t & 1);
+        bool ok;
+        {
+          PF_T0();
+          ok = warp_wait(&full[at], (t / Q2_STAGES) & 1, abort, p.status, kTimeoutFull);
+          PF_ACC(4, lane == 0 && st == 0);
+        }
+        if (ok && t < mine) {
+          PF_T0();
+          ok = warp_wait(&p_ready[sb], (t >> 1) & 1, abort, p.status, kTimeoutAccum);
+          PF_ACC(3, lane == 0 && st == 0);
+        }
+        if (!ok) break;
+        if (t < mine) {
+          tc_fence_after();
+          const uint32_t v_a = ring_a + at * C::KV_TILE, s_t = s_0 + (t & 1) * KT;
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < KT / 16; ++kk)
+              // 16 keys = two 8-row groups 1024 bytes apart; P: 8 columns of packed pairs per 16 keys
+              mma_f16_ts(o_t, s_t + (kk >> 1) * 32 + (kk & 1) * 8, make_desc_sw128_mn(v_a + kk * 2048, KT * 128, 1024),
+                         idesc_pv, (t > 0 || kk > 0) ? 1u : 0u);
+            tc_commit(&empty[at]);
+            tc_commit(&pv_done[sb]);
+          }
+        } else if (lane == 0) {
+          mbar_arrive(&empty[at]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax and output of one stream
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    fence_proxy_async_smem();
+    mbar_arrive(q_ready);
+    const int st = warp >> 2;
+    const int r = tid & (PF_ROWS - 1);                   // packed query row = TMEM lane
+    const uint32_t tlane = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t s_0 = tmem_base + st * 2 * KT + tlane, o_t = tmem_base + 4 * KT + st * D + tlane;
+    const bool row_ok = r < x.rows(st);
+    const int tok = x.tok0 + st * x.tpb + r / x.g;
+    const int mine = x.tiles(st);
+    // last visible key position (inclusive); rows that are not there (zeros of Q) see everything: masking would keep their warp, and
+    // with it the tile, on the slower path (128 x 64 scores of 125 rows: 2400 cycles, 1920 with 128 rows)
+    const int lim = !row_ok ? 0x40000000 : p.causal ? x.ctx - x.R + tok : x.ctx - 1;
+    float m_ref = -INFINITY, l = 0.f;   // O and l are relative to 2^m_ref
+    bool ok = true;
+    const long long t_begin = p.prof ? clock64() : 0;
+    for (int t = 0; t < mine; ++t) {
+      {
+        PF_T0();
+        ok = warp_wait(&s_ready[st * 2 + (t & 1)], (t >> 1) & 1, abort, p.status, kTimeoutAccum);
+        PF_ACC(0, tid == 0);
+      }
+      if (!ok) break;
+      tc_fence_after();
+      const long long t_math = p.prof ? clock64() : 0;
+      const uint32_t s_t = s_0 + (t & 1) * KT;
+      uint32_t v[2][32];
+      tmem_ld_32x32(s_t, v[0]);
+      tmem_ld_32x32(s_t + 32, v[1]);
+      // `rel` = last visible column of this tile for this row; a warp whose rows see the whole tile skips the masking.
+      const int rel = lim - t * KT;
+      const bool whole = __all_sync(0xffffffffu, rel >= KT - 1);
+      tmem_ld_wait();
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (whole) {
+#pragma unroll
+        for (int j = 0; j < KT; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(v[j >> 5][j & 31]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < KT; ++j)
+          mx4[j & 3] = fmaxf(mx4[j & 3], j <= rel ? __uint_as_float(v[j >> 5][j & 31]) : -INFINITY);
+      }
+      const float m_tile = pf_reference<false>(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), p.scale_log2);
+      if (t == 0) {
+        m_ref = m_tile;
+      } else if (__any_sync(0xffffffffu, m_tile > m_ref + PfCfg<D, false>::RESCALE_GAP)) {
+        // Raise the reference (all lanes of the warp: tcgen05.ld / st are warp-wide) and rescale O and l, once O += P V of
+        // the tile before has completed
+        ok = warp_wait(&pv_done[st * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort, p.status, kTimeoutAccum);
+        if (!ok) break;
+        tc_fence_after();
+        const float m_new = fmaxf(m_ref, m_tile);
+        const float alpha = m_new == -INFINITY ? 1.f : ex2(m_ref - m_new);
+        m_ref = m_new;
+        l *= alpha;
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += 16) {
+          uint32_t o[16];
+          tmem_ld_32x16(o_t + c0, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+          tmem_st_32x16(o_t + c0, o);
+        }
+      }
+      const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
+      l += whole ? q2_weights<true>(v, s_t, rel, p.scale_log2, neg_m) : q2_weights<false>(v, s_t, rel, p.scale_log2, neg_m);
+      tmem_st_wait();
+      if (p.prof && tid == 0) atomicAdd(p.prof + 13, (unsigned long long)(clock64() - t_math));
+      tc_fence_before();
+      mbar_arrive(&p_ready[st * 2 + (t & 1)]);
+    }
+    if (p.prof && tid == 0) {
+      atomicAdd(p.prof + 10, (unsigned long long)(clock64() - t_begin));
+      atomicAdd(p.prof + 11, (unsigned long long)mine);
+    }
+    if (ok && mine > 0) ok = warp_wait(&pv_done[st * 2 + ((mine - 1) & 1)], ((mine - 1) >> 1) & 1, abort, p.status, kTimeoutAccum);
+    if (ok) {
+      tc_fence_after();
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      __nv_bfloat16* dst = p.out + (static_cast<long long>(x.row0 + tok) * p.hq + x.kvh * x.g + r % x.g) * D;
+#pragma unroll
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t o[32];
+        if (mine > 0) {
+          tmem_ld_32x32(o_t + c0, o);
+          tmem_ld_wait();
+        } else {                                         // no visible key
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = 0;
+        }
+        if (row_ok) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8)
+            *reinterpret_cast<uint4*>(dst + c0 + j) =
+                make_uint4(pack_bf16(__uint_as_float(o[j]) * inv, __uint_as_float(o[j + 1]) * inv),
+                           pack_bf16(__uint_as_float(o[j + 2]) * inv, __uint_as_float(o[j + 3]) * inv),
+                           pack_bf16(__uint_as_float(o[j + 4]) * inv, __uint_as_float(o[j + 5]) * inv),
+                           pack_bf16(__uint_as_float(o[j + 6]) * inv, __uint_as_float(o[j + 7]) * inv));
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 12) tmem_dealloc(tmem_base, 512);
+}
+
+template <int D>
+int launch_prefill_q2(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int max_rows, int batch,
+                      cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(attn_prefill_q2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q2Cfg<D>::SMEM) !=
+        cudaSuccess)
+      return 3;
+    attr = true;
+  }
+  const int tokens = 2 * (PF_ROWS / (p.hq / p.hkv));
+  launch_dep(attn_prefill_q2_kernel<D>, dim3(p.hkv, batch, (max_rows + tokens - 1) / tokens), dim3(Q2_THREADS),
+             Q2Cfg<D>::SMEM, st, *tk, *tv, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
 template <int D, bool F8>
 int launch_prefill_pp(const PfParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int qblocks, int batch,
                       cudaStream_t st) {
@@ -1111,7 +1527,8 @@ void hb_attn_prefill_place(int t, int* place) {
 // bf16 KV with head dim 64, 128 or 256, or e4m3 KV (`kv_fp8`: x = code * kv_scale) with head dim 128 or 256, slot and head
 // strides multiples of 16 and 16-byte aligned pools; group size hq / hkv <= 128. `max_rows` bounds the new rows of any
 // sequence. With splits > 1 the context is cut into that many ranges of whole tiles, a CTA each, whose normalised
-// partial rows and log2 sums go to part_o / part_lse for hb_attn_merge.
+// partial rows and log2 sums go to part_o / part_lse for hb_attn_merge. splits = 1: one range, and bf16 pools with head dim 64 or
+// 128 run two Q tiles per CTA where a sequence may have two; 0: one range, one Q tile per CTA.
 int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                     long long head_stride,
                     const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,
@@ -1164,8 +1581,12 @@ int hb_attn_prefill(const void* q, const void* k_pool, const void* v_pool, long 
     tk = &t.k;
     tv = &t.v;
   }
-  if (d == 64) return launch_prefill_pp<64, false>(p, tk, tv, qblocks, batch, st);
-  if (d == 128) return launch_prefill_pp<128, false>(p, tk, tv, qblocks, batch, st);
+  // two Q tiles per CTA: the caller knows whether there are enough of them (ops/attention.py, two_q_tiles)
+  const bool q2 = splits == 1 && qblocks > 1 && batch <= 65535 && qblocks <= 2 * 65535;
+  if (d == 64)
+    return q2 ? launch_prefill_q2<64>(p, tk, tv, max_rows, batch, st) : launch_prefill_pp<64, false>(p, tk, tv, qblocks, batch, st);
+  if (d == 128)
+    return q2 ? launch_prefill_q2<128>(p, tk, tv, max_rows, batch, st) : launch_prefill_pp<128, false>(p, tk, tv, qblocks, batch, st);
   if (d == 256) return launch_prefill<256, false>(p, tk, tv, qblocks, batch, st);
   return 1;
 }

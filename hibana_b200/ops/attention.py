@@ -92,6 +92,19 @@ def prefill_splits(batch: int, hq: int, hkv: int, d: int, max_rows: int, max_ctx
     return -(-tiles // per) if tiles - per >= MIN_TILES_SAVED else 1
 
 
+def two_q_tiles(batch: int, hq: int, hkv: int, max_rows: int) -> bool:
+    """Whether an unsplit bf16 prefill (head dims up to 128) runs two 128-row Q tiles per CTA (csrc/attn_prefill.cu,
+    attn_prefill_q2_kernel). Against one tile per CTA, 40 / 8 heads of 128: more tiles than one wave of CTAs 1.2 to 2 times as fast
+    (2048 tokens 111 -> 61 us). Within one wave a CTA has twice the rows to do and SMs stay idle, which costs 10 to 28 % on long
+    contexts (300 rows over 1024 / 4096 keys 22.7 -> 24.8, 59.6 -> 72.6 us) and gains on short ones (29 tokens 12.8 -> 8.6, 128
+    tokens 12.8 -> 10.6, 512 keys 16.8 -> 17.0): taken up to half a wave, where longer contexts are split (`prefill_splits`).
+    One form for all row counts under `stable_numerics`."""
+    if cfgmod.current().stable_numerics:
+        return False
+    ctas = batch * hkv * -(-max_rows // max(1, 128 // (hq // hkv)))
+    return ctas > NUM_SMS or 2 * ctas <= NUM_SMS
+
+
 def forward_splits(k_pool: torch.Tensor, v_pool: torch.Tensor, batch: int, hq: int, hkv: int, d: int, max_rows: int,
                    max_ctx: int) -> int:
     """KV splits of a ragged forward with up to `max_rows` new rows per sequence, for the kernel that will run it."""
@@ -278,8 +291,8 @@ def _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, s
         parts = (workspace.part_o.data_ptr(), workspace.part_lse.data_ptr()) if splits > 1 else (None, None)
         nv.check(nv.lib().hb_attn_prefill(
             q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1), kv_indices.data_ptr(),
-            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts, splits,
-            b, max_rows, hq, hkv, d, scale, int(fp8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
+            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts,
+            splits if splits > 1 else int(two_q_tiles(b, hq, hkv, max_rows)), b, max_rows, hq, hkv, d, scale, int(fp8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
             nv.stream()), "hb_attn_prefill")
         if splits > 1:
             nv.check(nv.lib().hb_attn_merge(*parts, out.data_ptr(), t * hq, splits, d, nv.stream()), "hb_attn_merge")

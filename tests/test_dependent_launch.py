@@ -1,0 +1,46 @@
+"""Programmatic dependent launch changes when kernels start, never what they compute."""
+import pytest
+import torch
+
+from hibana_b200.engine.executor import Executor
+from hibana_b200.engine.request import SamplingParams
+from hibana_b200.models.dense import DenseModel
+from hibana_b200.models.hybrid import HybridModel
+from hibana_b200.target import dense_tiny, tiny_hybrid_moe
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("family", ["dense", "hybrid"])
+@pytest.mark.parametrize("graphs", [False, True])
+def test_launch_levels_give_the_same_bits(family, graphs):
+    """Prefill and decode of short and long prompts: tokens, KV pool and recurrent states of level 2 (every kernel of a step is
+    launched as a dependent and may trigger its successor early) equal those of plain launches, run after run."""
+    from hibana_b200 import _native as nv
+    from hibana_b200.ops import gemm
+    t = dense_tiny() if family == "dense" else tiny_hybrid_moe()
+    model = (DenseModel if family == "dense" else HybridModel)(t, "cuda", seed=0)
+    g = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, t.vocab, (n,), generator=g).tolist() for n in (1, 17, 65, 300)]
+
+    def run(level):
+        gemm.set_pdl(level)
+        ex = Executor(model, max_batch=4, max_ctx=384, kv_slots=1024, radix_cache=False, use_graphs=graphs)
+        if graphs:
+            ex.capture_graphs()
+        out = [r.output_ids for r in ex.generate_batch(prompts, SamplingParams(max_tokens=12, ignore_eos=True))]
+        torch.cuda.synchronize()
+        pools = [ex.kv.storage[:, :, :, 1:].clone()]
+        if ex.state_pool is not None:
+            pools += [ex.state_pool.conv[:, 1:].clone(), ex.state_pool.ssm[:, 1:].clone()]
+        return out, pools
+
+    try:
+        want, pools = run(0)
+        for _ in range(3):
+            got, again = run(2)
+            assert got == want
+            assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(pools, again))
+    finally:
+        from hibana_b200 import config
+        gemm.set_pdl(config.current().pdl)
+    assert nv.read_status() == 0

@@ -1,0 +1,61 @@
+"""Prefill attention with two Q tiles per CTA (csrc/attn_prefill.cu, attn_prefill_q2_kernel) and the rule that chooses it."""
+import math
+
+import pytest
+import torch
+
+from hibana_b200 import config as cfgmod
+from hibana_b200.ops import attention
+
+
+def test_two_q_tiles_rule_cpu():
+    assert attention.two_q_tiles(1, 40, 8, 2048) and attention.two_q_tiles(16, 40, 8, 60)
+    assert attention.two_q_tiles(1, 40, 8, 29) and attention.two_q_tiles(1, 40, 8, 225)
+    assert not attention.two_q_tiles(1, 40, 8, 250) and not attention.two_q_tiles(1, 40, 8, 450)
+    assert attention.two_q_tiles(1, 40, 8, 451) and attention.two_q_tiles(1, 128, 1, 2)
+    with cfgmod.using(stable_numerics=True):
+        assert not attention.two_q_tiles(1, 40, 8, 2048)
+
+
+# rows and contexts: one tile, a second tile of one row, both tiles full, a tile more for the second one, prefixes that end on and
+# off a tile, sequences with one tile or none of the block's rows
+CASES = [([26], [26]), ([50], [50]), ([51], [64]), ([51], [65]), ([100, 1, 27], [128, 1, 192]), ([30, 129, 3], [300, 129, 3]),
+         ([77], [1000])]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hq,hkv,d", [(40, 8, 128), (8, 8, 64), (32, 2, 128), (7, 1, 64), (128, 1, 128)])
+@pytest.mark.parametrize("scattered", [False, True])
+@pytest.mark.parametrize("causal", [True, False])
+def test_two_q_tiles_match_reference(hq, hkv, d, scattered, causal):
+    """bf16 weights and a bf16 result: 2^-9 each relative to the largest value a row's average is made of."""
+    from hibana_b200 import _native as nv
+    g = hq // hkv
+    gen = torch.Generator(device="cuda").manual_seed(hq * d)
+    for rows, ctxs in CASES:
+        rows = [max(1, r * 5 // g) for r in rows]                   # the same tiles at every group size
+        ctxs = [max(r, c) for r, c in zip(rows, ctxs)]
+        slots = sum(ctxs) + 65
+        st = torch.randn(2, hkv, slots, d, generator=gen, device="cuda").bfloat16()
+        k, v = st[0].transpose(0, 1), st[1].transpose(0, 1)
+        perm = torch.randperm(slots - 1, generator=gen, device="cuda") if scattered else torch.arange(slots - 1, device="cuda")
+        idx = torch.zeros(len(ctxs), max(ctxs), dtype=torch.int32, device="cuda")
+        o = 0
+        for i, c in enumerate(ctxs):
+            idx[i, :c] = perm[o:o + c].int() + 1
+            o += c
+        indptr = torch.tensor([0] + torch.tensor(rows).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        q = torch.randn(sum(rows), hq, d, generator=gen, device="cuda").bfloat16() * 2
+        ctx = torch.tensor(ctxs, dtype=torch.int32, device="cuda")
+        kw = dict(q_indptr=indptr, max_rows=max(rows), scale=1 / math.sqrt(d), causal=causal)
+        saved = attention.two_q_tiles
+        try:
+            attention.two_q_tiles = lambda *a: True
+            got = attention.paged_attention(q, k, v, idx, ctx, **kw)
+        finally:
+            attention.two_q_tiles = saved
+        ref = attention.paged_attention_ref(q, k, v, idx, ctx, indptr, 1 / math.sqrt(d), causal=causal).float()
+        vmax = v.float().abs().max().item()
+        assert (got.float() - ref).abs().max().item() <= 3 * 2.0 ** -9 * vmax, (rows, ctxs)
+        assert ((got.float() - ref).norm() / ref.norm()).item() <= 4e-3
+    assert nv.read_status() == 0
