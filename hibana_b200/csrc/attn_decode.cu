@@ -52,6 +52,7 @@ struct DecParams {
   float kv_scale;             // dequantisation scale of an e4m3 pool (1 for bf16)
   int causal;
   int use_tma;
+  int early;                  // tables, and keys before this forward's rows, are complete: see hb_attn_decode_early
   int* status;
   unsigned long long* prof;   // optional cycle counters of warp 0 (null = off)
   // Fused split merge: one int per (sequence, kv head), zero between launches. The CTA that finds splits - 1
@@ -156,7 +157,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   using C = DecCfg<D, F8>;
   constexpr int DEC_WARPS = C::WARPS;
   grid_dep_launch();   // what follows (merge, output projection) waits for this grid before it reads anything
-  grid_dep_wait();     // may run as a programmatic dependent of the RoPE + KV-write kernel
+  // May run as a programmatic dependent of the RoPE + KV-write kernel. With `early` the tables and the tiles of keys that are
+  // older than this forward are fetched before the wait: three round trips to L2 (lengths, slots, tiles) pass behind the
+  // projection and the RoPE.
+  if (!p.early) grid_dep_wait();
   constexpr int KT = C::KT, ROWB = C::QROWB;
   constexpr int NB = KT / 8;     // score n-blocks per tile
   constexpr int KS = D / 16;     // k-steps of Q K^T
@@ -185,6 +189,78 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   const int k0 = split * per;
   const int k1 = min(ctx, k0 + per);
   const int ntiles = k1 > k0 ? (k1 - k0 + KT - 1) / KT : 0;
+
+  const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? ldg_keep(p.seq_rows + b) : b) * p.ld_idx;
+
+  // Issues the copies of this warp's `it`-th tile into its ring stage: one bulk tensor copy per column block of
+  // K and of V when the tile's slots are KT consecutive pool rows, else a row-by-row cp.async gather. `tma_mode`
+  // remembers per stage which way the tile in flight travels, `tma_phase` the parity of the stage's barrier.
+  uint32_t tma_mode = 0, tma_phase = 0;
+  // Slot id of key `lane` of this warp's tile `it` (-1 beyond the split). Fetched one tile ahead of its use so
+  // that the index load's latency is not on the issue path.
+  auto fetch_slot = [&](int it) -> int {
+    const int base = k0 + (warp + it * DEC_WARPS) * KT;
+    int slot = (warp + it * DEC_WARPS < ntiles && lane < KT && base + lane < k1) ? ldg_keep(idx_row + base + lane) : -1;
+    if (slot >= 0 && !index_ok(slot, kBoundKvSlots, kKerAttnDecode)) slot = 0;   // reported; the dummy slot is read
+    return slot;
+  };
+  auto issue = [&](int it, int my_slot) {
+    const int tile = warp + it * DEC_WARPS;
+    if (tile < ntiles) {
+      const int st = it % DEC_STAGES;
+      const int base = k0 + tile * KT;
+      uint8_t* kt = ring + st * C::STAGE_BYTES;
+      const uint32_t kdst = smem_u32(kt);
+      const uint32_t vdst = kdst + C::TILE_BYTES;
+      constexpr int CPR = D * C::ESZ / 16;  // 16-byte chunks per row
+      constexpr int RPI = 32 / CPR > 0 ? 32 / CPR : 1;   // rows per warp instruction
+      const int slot0 = __shfl_sync(0xffffffffu, my_slot, 0);
+      const bool run = p.use_tma && __all_sync(0xffffffffu, lane >= KT || (my_slot >= 0 && my_slot == slot0 + lane));
+      if (run) {
+        tma_mode |= 1u << st;
+        // lane 0 posts the byte count, then 2 * HALVES lanes issue one box each (K / V x column block)
+        if (lane == 0) mbar_expect_tx(&full[st], 2 * C::TILE_BYTES);
+        __syncwarp();
+        if (lane < 2 * C::HALVES) {
+          const int h = lane >> 1, is_v = lane & 1;
+          tma_load_2d(kt + is_v * C::TILE_BYTES + h * C::BLOCK_BYTES, is_v ? &tmv : &tmk, &full[st],
+                      kvh * p.tma_xh + h * C::BLOCK_ELEMS, kvh * p.tma_yh + slot0);
+        }
+      } else {
+        tma_mode &= ~(1u << st);
+        if constexpr (CPR <= 32) {
+          const int part = lane % CPR, sub = lane / CPR;
+#pragma unroll
+          for (int r = 0; r < KT; r += RPI) {
+            const int key = r + sub;
+            const int slot = __shfl_sync(0xffffffffu, my_slot, key);
+            const uint32_t so = dsw<KT>(key, part);
+            if (slot >= 0) {
+              const long long off = (static_cast<long long>(slot) * p.pool_stride +
+                                     static_cast<long long>(kvh) * p.head_stride) * C::ESZ + part * 16;
+              cp16(kdst + so, reinterpret_cast<const uint8_t*>(p.k_pool) + off);
+              cp16(vdst + so, reinterpret_cast<const uint8_t*>(p.v_pool) + off);
+            } else {
+              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kdst + so), "r"(0) : "memory");
+              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vdst + so), "r"(0) : "memory");
+            }
+          }
+        }
+      }
+    }
+    cp_commit();
+  };
+
+  __syncwarp();      // this warp's barriers are initialised
+  int issued = 0;
+  if (p.early) {
+    // tiles that end before this forward's rows (a tile past the range issues nothing)
+    while (issued < 2 && min(k1, k0 + (warp + issued * DEC_WARPS + 1) * KT) <= ctx - R) {
+      issue(issued, fetch_slot(issued));
+      ++issued;
+    }
+    grid_dep_wait();
+  }
 
   // Q rows (zero padded to 16) into shared memory. For an e4m3 pool Q becomes fp16, the type K and V expand to
   // exactly: every row is scaled by a power of two that takes its largest element to [2^14, 2^15), so all that is more
@@ -259,67 +335,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
     }
   }
 
-  const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? ldg_keep(p.seq_rows + b) : b) * p.ld_idx;
-
-  // Issues the copies of this warp's `it`-th tile into its ring stage: one bulk tensor copy per column block of
-  // K and of V when the tile's slots are KT consecutive pool rows, else a row-by-row cp.async gather. `tma_mode`
-  // remembers per stage which way the tile in flight travels, `tma_phase` the parity of the stage's barrier.
-  uint32_t tma_mode = 0, tma_phase = 0;
-  // Slot id of key `lane` of this warp's tile `it` (-1 beyond the split). Fetched one tile ahead of its use so
-  // that the index load's latency is not on the issue path.
-  auto fetch_slot = [&](int it) -> int {
-    const int base = k0 + (warp + it * DEC_WARPS) * KT;
-    int slot = (warp + it * DEC_WARPS < ntiles && lane < KT && base + lane < k1) ? ldg_keep(idx_row + base + lane) : -1;
-    if (slot >= 0 && !index_ok(slot, kBoundKvSlots, kKerAttnDecode)) slot = 0;   // reported; the dummy slot is read
-    return slot;
-  };
-  auto issue = [&](int it, int my_slot) {
-    const int tile = warp + it * DEC_WARPS;
-    if (tile < ntiles) {
-      const int st = it % DEC_STAGES;
-      const int base = k0 + tile * KT;
-      uint8_t* kt = ring + st * C::STAGE_BYTES;
-      const uint32_t kdst = smem_u32(kt);
-      const uint32_t vdst = kdst + C::TILE_BYTES;
-      constexpr int CPR = D * C::ESZ / 16;  // 16-byte chunks per row
-      constexpr int RPI = 32 / CPR > 0 ? 32 / CPR : 1;   // rows per warp instruction
-      const int slot0 = __shfl_sync(0xffffffffu, my_slot, 0);
-      const bool run = p.use_tma && __all_sync(0xffffffffu, lane >= KT || (my_slot >= 0 && my_slot == slot0 + lane));
-      if (run) {
-        tma_mode |= 1u << st;
-        // lane 0 posts the byte count, then 2 * HALVES lanes issue one box each (K / V x column block)
-        if (lane == 0) mbar_expect_tx(&full[st], 2 * C::TILE_BYTES);
-        __syncwarp();
-        if (lane < 2 * C::HALVES) {
-          const int h = lane >> 1, is_v = lane & 1;
-          tma_load_2d(kt + is_v * C::TILE_BYTES + h * C::BLOCK_BYTES, is_v ? &tmv : &tmk, &full[st],
-                      kvh * p.tma_xh + h * C::BLOCK_ELEMS, kvh * p.tma_yh + slot0);
-        }
-      } else {
-        tma_mode &= ~(1u << st);
-        if constexpr (CPR <= 32) {
-          const int part = lane % CPR, sub = lane / CPR;
-#pragma unroll
-          for (int r = 0; r < KT; r += RPI) {
-            const int key = r + sub;
-            const int slot = __shfl_sync(0xffffffffu, my_slot, key);
-            const uint32_t so = dsw<KT>(key, part);
-            if (slot >= 0) {
-              const long long off = (static_cast<long long>(slot) * p.pool_stride +
-                                     static_cast<long long>(kvh) * p.head_stride) * C::ESZ + part * 16;
-              cp16(kdst + so, reinterpret_cast<const uint8_t*>(p.k_pool) + off);
-              cp16(vdst + so, reinterpret_cast<const uint8_t*>(p.v_pool) + off);
-            } else {
-              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kdst + so), "r"(0) : "memory");
-              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(vdst + so), "r"(0) : "memory");
-            }
-          }
-        }
-      }
-    }
-    cp_commit();
-  };
-
   // 16-row form: o[n-block][4], rows g4 / g4 + 8. Transposed form: o[16-wide head-dim block][4] = (d g4 | g4 + 8)
   // x (query rows 2 t4, 2 t4 + 1); "lo" / "hi" then name those two query rows.
   constexpr int OB = T8 ? D / 16 : ONB;
@@ -337,8 +352,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   const bool prof = p.prof != nullptr && tid == 0;
   const long long t_start = prof ? clock64() : 0;
   long long c_issue = 0, c_wait = 0, c_math = 0;
-  issue(0, fetch_slot(0));
-  issue(1, fetch_slot(1));
+  for (; issued < 2; ++issued) issue(issued, fetch_slot(issued));
   int slot_next = fetch_slot(2);
   for (int it = 0; warp + it * DEC_WARPS < ntiles; ++it) {
     // Stage (it + 2) % 3 was read in iteration it - 1: every lane is past it, order it before the async writes.
@@ -807,6 +821,7 @@ struct DecFuse {
   int q_ka = 0;
 };
 static thread_local DecFuse g_dec_fuse;
+static thread_local int g_dec_early = 0;
 
 extern "C" {
 
@@ -824,6 +839,11 @@ void hb_attn_decode_fuse(void* split_counter, void* q_out, void* q_sf, const voi
   g_dec_fuse.q_out = q_out; g_dec_fuse.q_sf = q_sf; g_dec_fuse.q_gscale = q_gscale; g_dec_fuse.q_ka = q_ka;
 }
 
+// Promises, for the NEXT hb_attn_decode call of this thread, that its tables (block table, context lengths, row offsets) and the keys
+// and values in front of every sequence's last rows were complete before the forward began, and that a kernel which triggers
+// its successor only after its own wait (the embedding gather) ran since: the kernel may then read them ahead of its wait.
+void hb_attn_decode_early(void) { g_dec_early = 1; }
+
 // bf16 KV, or e4m3 (`kv_fp8`: x = code * kv_scale; head dim 128 or 256, slot and head strides multiples of 16, 16-byte
 // aligned pools); rows_per_seq * (hq / hkv) must be <= 16. Partials go through hb_attn_merge when splits > 1 unless
 // hb_attn_decode_fuse armed the in-kernel merge.
@@ -833,6 +853,8 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
                    const void* q_indptr, void* out, void* part_o, void* part_lse, int batch, int max_rows, int hq,
                    int hkv, int d, int splits, float scale, int kv_fp8, float kv_scale, int causal, long long pool_slots,
                    void* status, void* stream) {
+  const int early = g_dec_early;
+  g_dec_early = 0;
   if (batch <= 0) return 0;
   if (kv_fp8 && (pool_stride % 16 != 0 || head_stride % 16 != 0 ||
                  ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) != 0))
@@ -864,6 +886,7 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
   p.q_gscale = static_cast<const float*>(g_dec_fuse.q_gscale);
   p.q_ka = g_dec_fuse.q_ka;
   g_dec_fuse = DecFuse{};
+  p.early = early;
   if (p.q_out != nullptr && p.splits > 1 && p.split_counter == nullptr) return 1;
   if (p.splits > 1 && (part_o == nullptr || part_lse == nullptr)) return 1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -56,7 +56,8 @@ struct Cfg {
   static constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES + SFA_BYTES + SFB_BYTES + PACK_BYTES;
   static constexpr int TX_BYTES = KIND == kGemmW3 ? B_TILE_BYTES + PACK_BYTES : STAGE_BYTES;   // bytes copies deliver
   // Token tiles of up to 64 (decode) keep the ring under ~100 KB so that two CTAs share an SM: the second CTA's
-  // prologue and epilogue overlap the first one's streaming, and grids of up to 2 x 148 CTAs are one wave.
+  // prologue and epilogue overlap the first one's streaming, and grids of up to 2 x 148 CTAs are one wave. (A stage more, 110 KB:
+  // 0.4 us slower a projection; the ring is filled while the producer of the activations runs, and slows that down.)
   // 128-token tiles (the grouped MoE GEMMs at prefill) get three stages for the same reason: thousands of short
   // CTAs whose fixed cost would otherwise be paid one after the other on every SM.
   static constexpr int SMEM_BUDGET = BN <= 64 ? 100 * 1024 : BN == 128 ? 110 * 1024 : 200 * 1024;
@@ -868,6 +869,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
           // one partial, this CTA's own: plain shared-memory loads (no cluster addressing), four columns in flight
           const float* part = reinterpret_cast<const float*>(smem);
           constexpr int NC = BN >= 64 ? 8 : 4;      // columns in flight per thread (latency hiding, see epilogue_rows4)
+          if (c_end <= 4) {      // up to four tokens: one per warp, none computed for nothing (1 x 34816 x 5120 18.9 -> 18.4 us)
+            if (cg < c_end) {
+              const float4 v[1] = {*reinterpret_cast<const float4*>(part + cg * BM + lrow0)};
+              const bool live[1] = {true};
+              const int tok[1] = {b_row0 + cg};
+              epilogue_rows4<1>(p, v, live, tok, grow0, row_lim, alpha, q_inv_gs);
+            }
+          } else
           for (int c = c_begin + cg; c < c_end; c += 4 * NC) {
             float4 v[NC];
             bool live[NC];

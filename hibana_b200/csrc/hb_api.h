@@ -152,6 +152,7 @@ int hb_attn_decode_tc(const void* q, const void* k_pool, const void* v_pool, lon
 void hb_attn_decode_tc_profile(void* buf);
 void hb_attn_prefill_profile(void* buf);
 void hb_attn_decode_profile(void* buf);
+void hb_attn_decode_early(void);
 int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                    long long head_stride,
                    const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,

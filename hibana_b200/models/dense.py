@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from .. import config as cfgmod
-from ..engine.context import ForwardContext
+from ..engine.context import DECODE, ForwardContext
 from ..ops import attention, basic, gemm, nvfp4
 from ..target import Target
 from .linear import Linear, interleave_pairs, norm_linear
@@ -224,7 +224,8 @@ class DenseModel:
                                             max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace,
-                                            quant_scale=layer.o.input_scale if fuse else None)
+                                            quant_scale=layer.o.input_scale if fuse else None,
+                                            tables_ready=ctx.mode == DECODE)
             h, slot = self._row_parallel(layer.o, att if isinstance(att, nvfp4.Nvfp4Tensor)
                                          else att.view(att.shape[0], -1), ctx)
             # prefill-sized chunks requantise in the gate/up epilogue too (tokens on the 128-row side of the GEMM):
@@ -267,7 +268,8 @@ class DenseModel:
                                             max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace,
-                                            quant_scale=None if o_gemv else layer.o.input_scale)
+                                            quant_scale=None if o_gemv else layer.o.input_scale,
+                                            tables_ready=ctx.mode == DECODE)
             layer.o(att if isinstance(att, nvfp4.Nvfp4Tensor) else att.view(rows, -1), epilogue=gemm.EPI_RESIDUAL,
                     residual=res, out=res)
             down_gemv = layer.down.takes_gemv(rows)

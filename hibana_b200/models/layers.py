@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from .. import config as cfgmod
-from ..engine.context import ForwardContext
+from ..engine.context import DECODE, ForwardContext
 from ..ops import attention, basic, gemm, moe, recurrent
 from ..target import ATTN, GATED_ATTN, GDN, LATENT_MOE, MAMBA2, MLP, MOE, NONE, Target
 from ..utils import streams
@@ -156,7 +156,7 @@ class AttentionLayer:
             att = attention.paged_attention(q, kv.k[i], kv.v[i], ctx.kv_indices, ctx.ctx_len, q_indptr=ctx.q_indptr,
                                             max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
-                                            workspace=ctx.attn_workspace)
+                                            workspace=ctx.attn_workspace, tables_ready=ctx.mode == DECODE)
         att = att.view(att.shape[0], -1)
         if self.gated:
             d = t.head_dim

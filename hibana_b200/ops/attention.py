@@ -27,6 +27,7 @@ nv.register("hb_attn_merge_quant", [P, P, L, I, I, I, P, P, P, I, P])
 nv.register("hb_attn_decode", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, Fl, I, L, P, P])
 
 nv.register("hb_attn_decode_fuse", [P, P, P, P, I], void=True)
+nv.register("hb_attn_decode_early", [], void=True)
 nv.register("hb_attn_decode_tc", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, L, P, P])
 nv.register("hb_attn_decode_tc_profile", [P], void=True)
 nv.register("hb_attn_prefill_profile", [P], void=True)
@@ -174,7 +175,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                     seq_rows: Optional[torch.Tensor] = None,
                     scale: Optional[float] = None, kv_scale: float = 1.0, causal: bool = True, splits: int = 1,
                     workspace: Optional[AttnWorkspace] = None, out: Optional[torch.Tensor] = None,
-                    quant_scale: Optional[torch.Tensor] = None):
+                    quant_scale: Optional[torch.Tensor] = None, tables_ready: bool = False):
     """q [T, Hq, D] bf16; pools [slots, Hkv, D]; kv_indices [B, max_ctx] int32; ctx_len [B] int32.
 
     Row r of sequence b (rows q_indptr[b]..q_indptr[b+1], or exactly one row when q_indptr is None) sees keys
@@ -183,6 +184,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     `quant_scale` (fp32 scalar tensor): return the rows [T, Hq * D] as an Nvfp4Tensor quantised with that static
     scale (the activation operand of the output projection); on the decode kernel this and the split merge happen
     inside the attention kernel, elsewhere a quantisation pass follows.
+    `tables_ready`: the tables and all keys and values but those of the call's own rows were complete before the forward began
+    with its embedding gather (a decode step): the decode kernel then fetches them while its predecessors still run.
     """
     t, hq, d = q.shape
     hkv = k_pool.shape[1]
@@ -223,6 +226,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                 nv.ptr(out), workspace.part_o.data_ptr() if splits > 1 else None,
                 workspace.part_lse.data_ptr() if splits > 1 else None, b, max_rows, hq, hkv, d, splits, scale)
         tail = (int(causal), k_pool.shape[0], st.status.data_ptr(), nv.stream())
+        if tables_ready and not tc:
+            nv.lib().hb_attn_decode_early()
         code = (nv.lib().hb_attn_decode_tc(*args, *tail) if tc
                 else nv.lib().hb_attn_decode(*args, int(f8), kv_scale, *tail))
         nv.check(code, "hb_attn_decode")
