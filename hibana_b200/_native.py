@@ -119,9 +119,12 @@ def available() -> bool:
 
 def use_native(*tensors: torch.Tensor) -> bool:
     """True when the op should run the CUDA kernel: every tensor is on a CUDA device (and the library loads)."""
-    if not tensors or not all(t.is_cuda for t in tensors if t is not None):
+    if not tensors:
         return False
-    if lib() is None:
+    for t in tensors:
+        if t is not None and not t.is_cuda:
+            return False
+    if _LIB is None and lib() is None:
         raise RuntimeError("CUDA tensors given but the native library is not loaded")
     return True
 

@@ -20,6 +20,14 @@ NVFP4 = "nvfp4"      # pool format: e2m1 values (two per byte) + one ue4m3 scale
 NVFP4_KV_SCALE = 1.0 / 64.0
 
 
+class SlotRun(list):
+    """Consecutive slots as `KvPool.alloc` hands them out. The mark is void once the list has another length."""
+
+    def __init__(self, slots):
+        super().__init__(slots)
+        self.run_start, self.run_length = self[0], len(self)
+
+
 class KvPool:
     """`dtype` torch.bfloat16, torch.float8_e4m3fn or the string "nvfp4" (4.5 bits per element: K / V rows are
     quantised when they are written, csrc/misc.cu, and dequantised inside the attention kernel, csrc/attn.cu;
@@ -88,6 +96,7 @@ class KvPool:
         del self._free[-n:]
         if out == list(range(out[0], out[0] + n)):
             self._owned[out[0]:out[0] + n] = b"\x01" * n
+            out = SlotRun(out)
         else:
             for s in out:
                 self._owned[s] = 1

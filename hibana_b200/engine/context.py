@@ -26,6 +26,7 @@ class ForwardContext:
     max_rows: int = 1                          # host bound on rows per sequence
     batch: int = 1
     state_slots: Optional[torch.Tensor] = None  # int32 [B] recurrent-state slot per sequence
+    state_slots_host: Optional[list] = None     # the same numbers on the host, where they are known there (prefill)
     sample_rows: Optional[torch.Tensor] = None  # int64 [B'] rows whose logits are wanted (None = all rows)
     attn_splits: int = 1
     attn_workspace: Any = None

@@ -221,7 +221,8 @@ class MambaLayer:
                                       heads=t.mamba_heads, groups=t.mamba_groups, head_dim=t.mamba_head_dim,
                                       d_state=t.mamba_state, q_indptr=ctx.q_indptr, has_init=ctx.has_initial_state,
                                       state_scale=states.ssm_scale[li] if getattr(states, "ssm_scale", None) is not None
-                                      else None, sr_seed=ctx.extras.get("sr_seed", 0), host_rows=ctx.seq_starts_host)
+                                      else None, sr_seed=ctx.extras.get("sr_seed", 0), host_rows=ctx.seq_starts_host,
+                                      host_slots=ctx.state_slots_host)
         if self.out_proj.fmt == "nvfp4" and not self.out_proj.calibrating and not self.out_proj.takes_w3(y.shape[0]):
             # the gated norm writes the output projection's NVFP4 input itself
             return self.out_proj(basic.gated_rmsnorm_quant(y, z, self.norm_w, t.norm_eps, inner // t.mamba_groups,
@@ -327,7 +328,8 @@ class GdnLayer:
             o = recurrent.gdn_scan(qkv[:, :self.qk], qkv[:, self.qk:2 * self.qk], qkv[:, 2 * self.qk:], g, beta,
                                    states.ssm[li], ctx.state_slots, so, k_heads=t.gdn_k_heads, v_heads=t.gdn_v_heads,
                                    kdim=kd, vdim=kd, l2norm=True, q_indptr=ctx.q_indptr,
-                                   has_init=ctx.has_initial_state, host_rows=ctx.seq_starts_host)
+                                   has_init=ctx.has_initial_state, host_rows=ctx.seq_starts_host,
+                                   host_slots=ctx.state_slots_host)
         rows = o.shape[0]
         # per-head RMSNorm of the output, then the SiLU gate (norm before gate)
         key = (id(self.norm_w), self.norm_w._version)

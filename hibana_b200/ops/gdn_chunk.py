@@ -120,13 +120,15 @@ def prepare_native(q, k, v, g, beta, *, k_heads: int, v_heads: int, scale: float
 def gdn_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, beta: torch.Tensor,
                 state: torch.Tensor, slot_in: torch.Tensor, slot_out: Optional[torch.Tensor], *, k_heads: int,
                 v_heads: int, kdim: int, vdim: int, scale: float, l2norm: bool,
-                ranges: Sequence[tuple[int, int]], has_init: Optional[Sequence[int]] = None) -> torch.Tensor:
+                ranges: Sequence[tuple[int, int]], has_init: Optional[Sequence[int]] = None,
+                host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
     """Same contract as ops.recurrent.gdn_scan; `ranges` are the (first, last + 1) rows of each sequence."""
     o = torch.empty(q.shape[0], v_heads * vdim, dtype=q.dtype, device=q.device)
     native = (nv.use_native(q) and kdim == 128 and vdim == 128 and state.dtype == torch.float32
               and q.dtype == torch.bfloat16)
-    sin = slot_in.tolist()
-    sout = slot_out.tolist() if slot_out is not None else None
+    # reading the slots back waits for everything queued so far: 50 us of idle GPU a layer
+    sin = list(host_slots) if host_slots is not None else slot_in.tolist()
+    sout = None if slot_out is None else sin if slot_out is slot_in else slot_out.tolist()
     for b, (r0, r1) in enumerate(ranges):
         if r1 <= r0:
             continue

@@ -7,6 +7,7 @@ tactic -> FlashInfer mm_fp4, and FP8 GEMV / cuBLASLt) is hibana/kernels/ops.py:5
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -49,12 +50,18 @@ def set_pdl(on) -> None:
 def _plan(m: int, n: int, k_tiles: int, max_ws_bytes: int) -> tuple[bool, int, int]:
     """(swap, bn, splits) for an [m tokens] x [n features] problem. Negative splits: the launch may lower their number to
     fit the chip, but by the same amount at every tile width."""
+    c = cfgmod.current()
+    return _plan_for(m, n, k_tiles, c.stable_numerics, c.max_splits)
+
+
+@functools.lru_cache(maxsize=4096)
+def _plan_for(m: int, n: int, k_tiles: int, stable: bool, max_splits: int) -> tuple[bool, int, int]:
     if m <= 256:
         bn = next(b for b in (16, 32, 64, 128, 256) if b >= m)
         tiles = (n + 127) // 128
         splits = 1
         slots = NUM_SMS * (2 if bn <= 64 else 1)     # token tiles <= 64 run two CTAs per SM (csrc/gemm.cu Cfg)
-        if cfgmod.current().stable_numerics:
+        if stable:
             # the number of K splits (hence the order every output element is summed in) must not depend on how
             # many rows share the forward: a token then gets the same bits from a decode step, a verify round of
             # any depth and any batch (reference: hibana/kernels/stable.py, HIBANA_STABLE_NUMERICS)
@@ -62,8 +69,8 @@ def _plan(m: int, n: int, k_tiles: int, max_ws_bytes: int) -> tuple[bool, int, i
         if tiles < slots:
             # Fill the resident CTA slots without spilling into a second, mostly empty wave; every split keeps at
             # least two K tiles.
-            splits = max(1, min(slots // tiles, k_tiles // 2, cfgmod.current().max_splits))
-        if cfgmod.current().stable_numerics and splits > 1:
+            splits = max(1, min(slots // tiles, k_tiles // 2, max_splits))
+        if stable and splits > 1:
             splits = -splits
         return True, bn, splits
     return False, (256 if n >= 256 else 128), 1

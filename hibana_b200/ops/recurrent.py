@@ -69,10 +69,12 @@ def mamba2_scan(x: torch.Tensor, bmat: torch.Tensor, cmat: torch.Tensor, dt: tor
                 slot_in: torch.Tensor, slot_out: Optional[torch.Tensor], *, heads: int, groups: int, head_dim: int,
                 d_state: int, q_indptr: Optional[torch.Tensor] = None,
                 has_init: Optional[torch.Tensor] = None, state_scale: Optional[torch.Tensor] = None,
-                sr_seed: int = 0, host_rows: Optional[Sequence[int]] = None) -> torch.Tensor:
+                sr_seed: int = 0, host_rows: Optional[Sequence[int]] = None,
+                host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
     """x [T, heads*P], bmat/cmat [T, groups*N], dt [T, heads] (bf16, column slices allowed);
     state [slots, heads, P, N] in fp32, fp16 (`sr_seed` != 0: stochastic rounding when the state is written back)
-    or int8 with `state_scale` [slots, heads, P] fp32 row scales. Returns y [T, heads*P] bf16."""
+    or int8 with `state_scale` [slots, heads, P] fp32 row scales. Returns y [T, heads*P] bf16. `host_slots`: the numbers in
+    `slot_in`, where the host knows them (the chunked form then need not read them back)."""
     t = x.shape[0]
     batch = slot_in.shape[0]
     fmt = {torch.float32: 0, torch.float16: 1, torch.int8: 2}[state.dtype]
@@ -86,7 +88,8 @@ def mamba2_scan(x: torch.Tensor, bmat: torch.Tensor, cmat: torch.Tensor, dt: tor
             r += n
         return ssd_chunk.mamba2_chunked(x, bmat, cmat, dt, a_log, dt_bias, dskip, state, slot_in, slot_out,
                                         heads=heads, groups=groups, head_dim=head_dim, d_state=d_state,
-                                        ranges=ranges, has_init=None if has_init is None else has_init.tolist())
+                                        ranges=ranges, has_init=None if has_init is None else has_init.tolist(),
+                                        host_slots=host_slots)
     if nv.use_native(x):
         y = torch.empty(t, heads * head_dim, dtype=x.dtype, device=x.device)
         nv.check(nv.lib().hb_mamba2_scan_fmt(
@@ -138,11 +141,12 @@ def gdn_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
              state: torch.Tensor, slot_in: torch.Tensor, slot_out: Optional[torch.Tensor], *, k_heads: int,
              v_heads: int, kdim: int, vdim: int, scale: Optional[float] = None, l2norm: bool = True,
              q_indptr: Optional[torch.Tensor] = None, has_init: Optional[torch.Tensor] = None,
-             host_rows: Optional[Sequence[int]] = None) -> torch.Tensor:
+             host_rows: Optional[Sequence[int]] = None, host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
     """Gated delta rule. q, k [T, k_heads*K] (same row pitch), v [T, v_heads*V] bf16; g (log decay), beta
     [T, v_heads] fp32 contiguous; state [slots, v_heads, V, K] fp32. Returns o [T, v_heads*V] bf16.
     `host_rows` (rows per sequence, known on the host during prefill) lets long sequences take the chunked form
-    (ops/gdn_chunk.py): tensor-core work parallel over chunks instead of one serial step per token."""
+    (ops/gdn_chunk.py): tensor-core work parallel over chunks instead of one serial step per token. `host_slots`: the numbers
+    in `slot_in`, where the host knows them."""
     t = q.shape[0]
     batch = slot_in.shape[0]
     scale = kdim ** -0.5 if scale is None else scale
@@ -154,7 +158,7 @@ def gdn_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
             r += n
         return gdn_chunk.gdn_chunked(q, k, v, g, beta, state, slot_in, slot_out, k_heads=k_heads, v_heads=v_heads,
                                      kdim=kdim, vdim=vdim, scale=scale, l2norm=l2norm, ranges=ranges,
-                                     has_init=None if has_init is None else has_init.tolist())
+                                     has_init=None if has_init is None else has_init.tolist(), host_slots=host_slots)
     if nv.use_native(q):
         assert q.stride(0) == k.stride(0) and g.is_contiguous() and beta.is_contiguous()
         o = torch.empty(t, v_heads * vdim, dtype=q.dtype, device=q.device)

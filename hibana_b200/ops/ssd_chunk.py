@@ -89,13 +89,14 @@ def one_kernel(n: int, heads: int, head_dim: int) -> bool:
 
 def mamba2_chunked(x, bmat, cmat, dt, a_log, dt_bias, dskip, state, slot_in, slot_out, *, heads: int, groups: int,
                    head_dim: int, d_state: int, ranges: Sequence[tuple[int, int]],
-                   has_init: Optional[Sequence[int]] = None) -> torch.Tensor:
+                   has_init: Optional[Sequence[int]] = None, host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
     """Same contract as ops.recurrent.mamba2_scan for an fp32 state [slots, heads, P, N]."""
     y = torch.empty(x.shape[0], heads * head_dim, dtype=x.dtype, device=x.device)
     native = (nv.use_native(x) and d_state == 128 and head_dim % 32 == 0 and state.dtype == torch.float32
               and x.dtype == torch.bfloat16)
-    sin = slot_in.tolist()
-    sout = slot_out.tolist() if slot_out is not None else None
+    # reading the slots back waits for everything queued so far: 50 us of idle GPU a layer
+    sin = list(host_slots) if host_slots is not None else slot_in.tolist()
+    sout = None if slot_out is None else sin if slot_out is slot_in else slot_out.tolist()
     for b, (r0, r1) in enumerate(ranges):
         if r1 <= r0:
             continue
