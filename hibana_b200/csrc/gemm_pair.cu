@@ -22,8 +22,11 @@
 // Grouped (mixture-of-experts) mode: a unit is (chunk of up to 256 rows of an expert's segment, 256 of its weight rows), from
 // the work list that the routing plan left on the device. An expert of a 4096-token chunk has about 176 rows, and its
 // GEMM is 4 to 11 K tiles long: as one CTA per 128 x 128 tile, set-up and epilogue took most of the time (fc1 and
-// fc2 of 512 experts, 1024 x 2688, 544 us each over 4096 and 904 tokens; as units 391 and 235). fc1 requantises its
-// activation for fc2 in the epilogue, for which two warps share each lane quarter (464 us with one).
+// fc2 of 512 experts, 1024 x 2688, 904 / 4096 tokens of 22 experts each: 544 us on average; as units 349 / 359 and 217 / 238). fc1
+// requantises its activation for fc2 in the epilogue, straight from registers: staged in shared memory, which the MMAs keep busy, it
+// took 40 us longer, and with four warps per lane quarter instead of two 90 more. Rows of A that lie past the segment are not
+// fetched and their warps skip the epilogue: 305 / 321 and 205 / 226 us. What is left is the epilogue of fc1 (237 us without) and 1.1 us
+// between the units of a cluster, which share accumulator columns; the weights' bytes take 121.
 #include <algorithm>
 
 #include "gemm.cuh"
@@ -46,7 +49,7 @@ constexpr int B_BYTES = 128 * 128;            // this CTA's half of the 256 colu
 constexpr int SFA_BYTES = 2048;               // one 128-row block x 4 K atoms
 constexpr int SFB_BYTES = 4096;               // two 128-column blocks x 4 K atoms (each CTA holds all columns' scales)
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
-constexpr int ROW_PITCH = 80;                 // staged output row: at most 64 + 8 bytes (conflict-free 16-byte accesses)
+constexpr int ROW_PITCH = 80;                 // staged output row: 64 bytes (conflict-free 16-byte accesses)
 constexpr int STAGING_BYTES = EPI_WARPS * 32 * ROW_PITCH;
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + 256;
 constexpr int ACC1_COL = 208;                 // first column of the second accumulator
@@ -208,9 +211,14 @@ __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.f +
 // One epilogue warp's part of a unit: 32 rows x half of its columns, in steps of 32 columns (one tcgen05.ld), two steps in
 // registers at a time. `acc` is the accumulator's address for the warp's lanes, `release` the leader's acc_free barrier.
 // The columns that the two accumulators share come first: the last ones of the first, the first ones of the second.
-template <int EPI>
+template <int EPI, bool GRP>
 __device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x, int buf, int half, uint32_t acc, int row0,
                                               uint8_t* staging, float alpha, float q_inv_gs, uint32_t release, int lane) {
+  if (GRP && row0 >= x.m_end) {                     // none of these rows is stored (the segment's padding)
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(release);
+    return;
+  }
   const int steps = x.width / 64, groups = (steps + 1) / 2;
   const int col0 = half * (x.width / 2);            // first column of this half, within the unit
   uint8_t* my_row = staging + lane * ROW_PITCH;
@@ -227,34 +235,62 @@ __device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(release);
     }
+    if constexpr (EPI == kEpiSiluMulQuant || EPI == kEpiRelu2Quant) {
+      // The thread's token: two steps are 32 or 64 features, 16 or 32 packed bytes and two or four scale bytes, which go straight
+      // from registers to whole or half sectors. Same arithmetic in the same order as the stand-alone quantiser. Whole steps are
+      // in range or none: ungrouped SiLU-mul calls have a multiple of 64 gate and up columns, grouped calls of 64 features.
+      constexpr int GROUPS = EPI == kEpiSiluMulQuant ? 1 : 2;     // 16-feature groups of a step
+      constexpr int SHIFT = EPI == kEpiSiluMulQuant ? 5 : 4;      // columns per group, log2
+      uint2 pk[2 * GROUPS];
+      uint32_t sfw = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (s0 + h >= steps) break;
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+          float y[16];
+#pragma unroll
+          for (int t = 0; t < 16; ++t) {
+            if constexpr (EPI == kEpiSiluMulQuant) {
+              y[t] = __bfloat162float(__float2bfloat16(silu_fast(__uint_as_float(r[h][2 * t]) * alpha) *
+                                                       (__uint_as_float(r[h][2 * t + 1]) * alpha)));
+            } else {      // squared ReLU, rounded as a bf16 store would
+              const float v = __uint_as_float(r[h][g * 16 + t]) * alpha;
+              y[t] = __bfloat162float(__float2bfloat16(v > 0.f ? v * v : 0.f));
+            }
+          }
+          sfw |= quant16(y, q_inv_gs, &pk[h * GROUPS + g]) << (8 * (h * GROUPS + g));
+        }
+      }
+      const int c = x.n0 + col0 + s0 * 32;          // first column
+      const int ng = c >= p.n ? 0 : s0 + 1 < steps && c + 64 <= p.n ? 2 * GROUPS : GROUPS;      // groups in range
+      if (row < x.m_end && ng > 0) {
+        uint8_t* dst = p.q_out + static_cast<size_t>(row) * p.q_ld + (c >> SHIFT) * 8;
+        uint8_t* sf = p.q_sf + row_sf_off(row, c >> SHIFT, p.q_ka);      // the groups of a K atom are neighbouring bytes
+        if (ng == 2 * GROUPS) {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(pk[0].x, pk[0].y, pk[1].x, pk[1].y);
+          if constexpr (GROUPS == 2) {
+            *reinterpret_cast<uint4*>(dst + 16) = make_uint4(pk[2].x, pk[2].y, pk[3].x, pk[3].y);
+            *reinterpret_cast<uint32_t*>(sf) = sfw;
+          } else {
+            *reinterpret_cast<uint16_t*>(sf) = static_cast<uint16_t>(sfw);
+          }
+        } else {
+          *reinterpret_cast<uint2*>(dst) = pk[0];
+          sf[0] = static_cast<uint8_t>(sfw);
+          if constexpr (GROUPS == 2) {
+            *reinterpret_cast<uint2*>(dst + 8) = pk[1];
+            sf[1] = static_cast<uint8_t>(sfw >> 8);
+          }
+        }
+      }
+    } else
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int s = s0 + h;
       if (s >= steps) break;
       const int c = x.n0 + col0 + s * 32;           // first column of the step
-      if constexpr (EPI == kEpiSiluMulQuant) {
-        // 32 accumulator columns are 16 gate / up pairs: one 16-feature NVFP4 group of the thread's token. Same
-        // arithmetic in the same order as the stand-alone quantiser.
-        float y[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t)
-          y[t] = __bfloat162float(__float2bfloat16(silu_fast(__uint_as_float(r[h][2 * t]) * alpha) *
-                                                   (__uint_as_float(r[h][2 * t + 1]) * alpha)));
-        my_row[64 + s] = static_cast<uint8_t>(quant16(y, q_inv_gs, reinterpret_cast<uint2*>(my_row + s * 8)));
-      } else if constexpr (EPI == kEpiRelu2Quant) {
-        // two groups: squared ReLU, rounded as a bf16 store would, then the same quantiser
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          float y[16];
-#pragma unroll
-          for (int t = 0; t < 16; ++t) {
-            const float v = __uint_as_float(r[h][g * 16 + t]) * alpha;
-            y[t] = __bfloat162float(__float2bfloat16(v > 0.f ? v * v : 0.f));
-          }
-          my_row[64 + 2 * s + g] =
-              static_cast<uint8_t>(quant16(y, q_inv_gs, reinterpret_cast<uint2*>(my_row + s * 16 + g * 8)));
-        }
-      } else {
+      {
         // bf16 rows through shared memory: whole 16-byte chunks, consecutive lanes along a row
         constexpr int CHUNKS = EPI == kEpiSiluMul ? 2 : 4;
 #pragma unroll
@@ -298,42 +334,16 @@ __device__ __forceinline__ void epilogue_unit(const PairParams& p, const Unit& x
     }
   }
   if constexpr (EPI == kEpiSiluMulQuant || EPI == kEpiRelu2Quant) {
-    // Packed bytes of the half: consecutive lanes along a row, 8 bytes per group (SiLU-mul: a step is one group, else two).
-    // Whole steps are in range or none: ungrouped SiLU-mul calls have a multiple of 64 gate and up columns (32 features, so the
-    // last K atom of the next GEMM may hold two groups and two zeroed ones), grouped calls a multiple of 64 features.
-    constexpr int GROUPS = EPI == kEpiSiluMulQuant ? 1 : 2;
-    constexpr int SHIFT = EPI == kEpiSiluMulQuant ? 5 : 4;      // columns per group, log2
-    const int c_half = x.n0 + col0;
-    const int ng = steps * GROUPS;                              // 8, 4, 2 or 1
-    const int g = lane % ng;
-    __syncwarp();
-    for (int r0 = 0; r0 < 32; r0 += 32 / ng) {
-      const int lr = r0 + lane / ng;
-      const int grow = row0 + lr;
-      if (grow < x.m_end && c_half + ((g + 1) << SHIFT) <= p.n)
-        *reinterpret_cast<uint2*>(p.q_out + static_cast<size_t>(grow) * p.q_ld + (c_half >> SHIFT) * 8 + g * 8) =
-            *reinterpret_cast<const uint2*>(staging + lr * ROW_PITCH + g * 8);
-    }
-    if (row < x.m_end) {
-      const int g0 = c_half >> SHIFT;
-      if (ng >= 4 && c_half + (ng << SHIFT) <= p.n) {           // four groups of a K atom are one aligned word
-        for (int w = 0; w < ng; w += 4)
-          *reinterpret_cast<uint32_t*>(p.q_sf + row_sf_off(row, g0 + w, p.q_ka)) =
-              *reinterpret_cast<const uint32_t*>(my_row + 64 + w);
-      } else {
-        for (int w = 0; w < ng; ++w)
-          if (c_half + ((w + 1) << SHIFT) <= p.n) p.q_sf[row_sf_off(row, g0 + w, p.q_ka)] = my_row[64 + w];
-      }
-      if (half == 1 && x.n0 + x.width >= p.n)      // groups that pad the last K tile of the next GEMM read as zero
-        for (int w = p.n >> SHIFT; w < p.q_ka * 4; ++w) p.q_sf[row_sf_off(row, w, p.q_ka)] = 0;
-    }
-    __syncwarp();
+    constexpr int SHIFT = EPI == kEpiSiluMulQuant ? 5 : 4;
+    if (row < x.m_end && half == 1 && x.n0 + x.width >= p.n)      // groups that pad the last K tile of the next GEMM read as zero
+      for (int w = p.n >> SHIFT; w < p.q_ka * 4; ++w) p.q_sf[row_sf_off(row, w, p.q_ka)] = 0;
   }
 }
 
 template <int EPI, bool GRP>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap ta64,
+                 const __grid_constant__ CUtensorMap ta32, const __grid_constant__ CUtensorMap tb,
                  const __grid_constant__ CUtensorMap tb_sub, const __grid_constant__ CUtensorMap tsfa,
                  const __grid_constant__ CUtensorMap tsfb, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -379,9 +389,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
     // The whole warp walks the loop (waits included) and one elected lane issues: see elect_one.
     const uint32_t full0 = __shfl_sync(0xffffffffu, map_to_cta(smem_u32(full), 0), 0);   // the leader's barriers
     int i = 0;             // stage counter over all units
+    // Grouped: rows of A that a CTA fetches, in whole boxes. What lies beyond the segment's rows is not worth its way from L2: the
+    // MMA then reads whatever the stage held, into rows that nobody stores.
+    auto box_rows = [](const Unit& x, int r) {
+      if constexpr (!GRP) return 128;
+      const int n = x.m_end - x.m0 - r * 128;
+      return n > 64 ? 128 : n > 32 ? 64 : n > 0 ? 32 : 0;
+    };
     auto side_a = [&](const Unit& x, int kt, int s) {
       const uint32_t st = smem_base + s * STAGE_BYTES;
-      tma_load_2d_pair(st, &ta, full0 + s * 8, kt * 128, x.m0 + static_cast<int>(rank) * 128);
+      const int box = box_rows(x, static_cast<int>(rank));
+      if (GRP && box == 0) return;
+      tma_load_2d_pair(st, !GRP || box == 128 ? &ta : box == 64 ? &ta64 : &ta32, full0 + s * 8, kt * 128,
+                       x.m0 + static_cast<int>(rank) * 128);
       tma_load_2d_pair(st + A_BYTES + B_BYTES, &tsfa, full0 + s * 8, kt * 256, (x.m0 >> 7) + static_cast<int>(rank));
     };
     auto side_b = [&](const Unit& x, int kt, int s) {
@@ -390,8 +410,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
                        x.b0 + static_cast<int>(rank) * (x.width >> 1));
       tma_load_2d_pair(st + A_BYTES + B_BYTES + SFA_BYTES, &tsfb, full0 + s * 8, kt * 256, x.b0 >> 7);
     };
-    auto tx_bytes = [](const Unit& x) {
-      return 2u * (A_BYTES + SFA_BYTES + SFB_BYTES + static_cast<uint32_t>(x.width) * 64u);
+    auto tx_bytes = [&](const Unit& x) {
+      uint32_t bytes = 2u * (SFB_BYTES + static_cast<uint32_t>(x.width) * 64u);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int box = box_rows(x, r);
+        bytes += static_cast<uint32_t>(box) * 128u + (box > 0 ? SFA_BYTES : 0);
+      }
+      return bytes;
     };
     // The first ring of stages: weights first (they depend on nothing), then the wait for the kernel that produces
     // the activations, then the activations.
@@ -421,6 +447,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
       if constexpr (GRP) {
         x.m0 = __shfl_sync(0xffffffffu, x.m0, 0);
         x.b0 = __shfl_sync(0xffffffffu, x.b0, 0);
+        x.m_end = __shfl_sync(0xffffffffu, x.m_end, 0);
       }
       for (int kt = 0; kt < p.k_tiles; ++kt, ++i) {
         if (i < pre) continue;
@@ -518,7 +545,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
       // one verdict per warp: lanes that give up on a wait must not leave the others alone in a warp-wide TMEM load
       if (!__all_sync(0xffffffffu, mbar_wait(&accum[buf], (it >> 1) & 1, abort, p.status, kTimeoutAccum))) break;
       tc_fence_after();
-      epilogue_unit<EPI>(p, x, buf, half, tlane + (buf ? ACC1_COL : 0), x.m0 + static_cast<int>(rank) * 128 + q * 32, mine,
+      epilogue_unit<EPI, GRP>(p, x, buf, half, tlane + (buf ? ACC1_COL : 0), x.m0 + static_cast<int>(rank) * 128 + q * 32, mine,
                          alpha, q_inv_gs, release, lane);
       ++it;
     }
@@ -531,8 +558,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 }
 
 template <int EPI, bool GRP>
-cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_sub, const CUtensorMap& tsfa,
-                   const CUtensorMap& tsfb, const PairParams& p, int clusters, cudaStream_t stream) {
+cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& ta64, const CUtensorMap& ta32, const CUtensorMap& tb,
+                   const CUtensorMap& tb_sub, const CUtensorMap& tsfa, const CUtensorMap& tsfb, const PairParams& p, int clusters, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
   cfg.blockDim = dim3(THREADS);
@@ -545,13 +572,14 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = hb_gemm_get_pdl() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, GRP>, ta, tb, tb_sub, tsfa, tsfb, p);
+  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, GRP>, ta, ta64, ta32, tb, tb_sub, tsfa, tsfb, p);
 }
 
 // Clusters of two that the device holds at once (0 = the kernels could not be set up).
 template <int EPI, bool GRP>
 int resident_clusters() {
-  if (cudaFuncSetAttribute(gemm_pair_kernel<EPI, GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+  if (cudaFuncSetAttribute(gemm_pair_kernel<EPI, GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
+      cudaSuccess)
     return 0;
   cudaLaunchConfig_t q = {};
   q.gridDim = dim3(2);
@@ -662,11 +690,16 @@ cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
   const uint64_t pa = static_cast<uint64_t>(act_ka) * 512, pb = static_cast<uint64_t>(wgt_ka) * 512;
   const TmapKey ksa{act_sf, static_cast<uint64_t>((rows + 127) / 128), pa / 8, pa, 1, 256, 2};
   const TmapKey ksb{wgt_sf, static_cast<uint64_t>((wgt_rows + 127) / 128), pb / 8, pb, 2, 256, 2};
-  CUtensorMap ta, tb, tb_sub, tsfa, tsfb;
-  if (!get_tmap_2d(ka, &ta) || !get_tmap_2d(kb, &tb) || !get_tmap_2d(kb_sub, &tb_sub) || !get_tmap_2d(ksa, &tsfa) ||
+  CUtensorMap ta, ta64, ta32, tb, tb_sub, tsfa, tsfb;
+  TmapKey k64 = ka, k32 = ka;
+  if (grouped) {
+    k64.box_rows = 64;
+    k32.box_rows = 32;
+  }
+  if (!get_tmap_2d(ka, &ta) || !get_tmap_2d(k64, &ta64) || !get_tmap_2d(k32, &ta32) || !get_tmap_2d(kb, &tb) || !get_tmap_2d(kb_sub, &tb_sub) || !get_tmap_2d(ksa, &tsfa) ||
       !get_tmap_2d(ksb, &tsfb))
     return cudaErrorInvalidValue;
-#define HB_PAIR(EPI, GRP) launch<EPI, GRP>(ta, tb, tb_sub, tsfa, tsfb, p, clusters, stream)
+#define HB_PAIR(EPI, GRP) launch<EPI, GRP>(ta, ta64, ta32, tb, tb_sub, tsfa, tsfb, p, clusters, stream)
   switch (a.epilogue) {
     case kEpiStore: return grouped ? HB_PAIR(kEpiStore, true) : HB_PAIR(kEpiStore, false);
     case kEpiResidual: return HB_PAIR(kEpiResidual, false);
