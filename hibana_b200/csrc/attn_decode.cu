@@ -53,6 +53,13 @@ struct DecParams {
   int causal;
   int use_tma;
   int early;                  // tables, and keys before this forward's rows, are complete: see hb_attn_decode_early
+  // Fused RoPE + KV write (see hb_attn_decode_rope): rows [Hq * D | Hkv * D | Hkv * D] of the projection, null = off
+  const __nv_bfloat16* qkv;
+  long long ld_qkv;
+  const int* positions;
+  const int* slots;
+  const float* inv_freq;
+  float kv_inv_scale;
   int* status;
   unsigned long long* prof;   // optional cycle counters of warp 0 (null = off)
   // Fused split merge: one int per (sequence, kv head), zero between launches. The CTA that finds splits - 1
@@ -140,7 +147,9 @@ struct DecCfg {
   static constexpr int QROWB = D * 2 + 16;              // padded Q row: conflict-free ldmatrix
   static constexpr int Q_BYTES = 16 * QROWB;
   static constexpr int BAR_OFF = WARPS * WARP_BYTES + Q_BYTES;
-  static constexpr int SMEM = BAR_OFF + 256 + 1024;     // +0 barriers and abort flags, +128 row scales, +192 merge flag
+  static constexpr int ROPE_OFF = BAR_OFF + 256;        // +0 barriers and abort flags, +128 row scales, +192 merge flag
+  static constexpr int NEW_OFF = ROPE_OFF + D / 2 * 8;  // fused RoPE: the row's (cos, sin), then its new K and V rows
+  static constexpr int SMEM = NEW_OFF + 2 * D * ESZ + 1024;
   static_assert(16 * D * 4 + 16 * 8 <= WARP_BYTES, "merge scratch must fit a warp's ring");
   static_assert(BLOCK_BYTES % 1024 == 0, "column blocks must keep the swizzle atom alignment");
 };
@@ -149,6 +158,23 @@ struct DecCfg {
 template <int KT>
 __device__ __forceinline__ uint32_t dsw(int row, int c) {
   return static_cast<uint32_t>((c >> 3) * (KT * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
+}
+
+// Chunk c (8 elements) of a row of head dim D at `src`, rotated by the angles cs[D / 2]: the arithmetic of rope_kv_write_kernel.
+template <int D>
+__device__ __forceinline__ void rope_chunk(const __nv_bfloat16* src, int c, const float2* cs, float (&o)[8]) {
+  const bool low = c < D / 16;
+  const int pc = low ? c + D / 16 : c - D / 16;
+  const uint4 a = *reinterpret_cast<const uint4*>(src + c * 8), b = *reinterpret_cast<const uint4*>(src + pc * 8);
+  float v[8], pv[8];
+  unpack8(a, v);
+  unpack8(b, pv);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float2 t = cs[(low ? c : pc) * 8 + e];
+    // (spelled out with the roundings that rope_kv_write_kernel has: left to the compiler they differ between kernels)
+    o[e] = low ? __fmaf_rn(v[e], t.x, -__fmul_rn(pv[e], t.y)) : __fmaf_rn(pv[e], t.y, __fmul_rn(v[e], t.x));
+  }
 }
 
 template <int D, bool T8, bool F8>
@@ -253,13 +279,52 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
 
   __syncwarp();      // this warp's barriers are initialised
   int issued = 0;
+  const bool rope = p.qkv != nullptr;
+  float2* cs = reinterpret_cast<float2*>(smem + C::ROPE_OFF);
+  uint8_t* fresh = smem + C::NEW_OFF;                       // the new token's K row, then its V row, as the pool holds them
+  const bool owns_new = rope && ntiles > 0 && k1 == ctx;    // this range ends with the new token
   if (p.early) {
-    // tiles that end before this forward's rows (a tile past the range issues nothing)
-    while (issued < 2 && min(k1, k0 + (warp + issued * DEC_WARPS + 1) * KT) <= ctx - R) {
+    // Tiles that end before this forward's rows (a tile past the range issues nothing). With fused RoPE the one new row is put
+    // into its tile by this CTA, so that no tile has to wait.
+    while (issued < 2 && (rope || min(k1, k0 + (warp + issued * DEC_WARPS + 1) * KT) <= ctx - R)) {
       issue(issued, fetch_slot(issued));
       ++issued;
     }
+    if (rope) {
+      const float pos = static_cast<float>(ldg_keep(p.positions + b));
+      for (int j = tid; j < D / 2; j += DEC_WARPS * 32) {
+        float sn, co;
+        sincosf(pos * p.inv_freq[j], &sn, &co);
+        cs[j] = make_float2(co, sn);
+      }
+      __syncthreads();
+    }
     grid_dep_wait();
+  }
+  if (owns_new) {      // K and V of the new token: into the pool and, for this CTA's own tile, into shared memory
+    const __nv_bfloat16* krow = p.qkv + b * p.ld_qkv + (p.hq + kvh) * D;
+    int slot = ldg_keep(p.slots + b);
+    if (slot >= 0 && !index_ok(slot, kBoundKvSlots, kKerRopeKvWrite)) slot = -1;   // reported; nothing is written
+    for (int i = tid; i < 2 * (D / 8); i += DEC_WARPS * 32) {
+      const bool is_v = i >= D / 8;
+      const int c = is_v ? i - D / 8 : i;
+      float f[8];
+      if (is_v) unpack8(*reinterpret_cast<const uint4*>(krow + p.hkv * D + c * 8), f);
+      else rope_chunk<D>(krow, c, cs, f);
+      uint8_t* pool = const_cast<uint8_t*>(reinterpret_cast<const uint8_t*>(is_v ? p.v_pool : p.k_pool)) +
+                      (static_cast<long long>(slot) * p.pool_stride + static_cast<long long>(kvh) * p.head_stride) * C::ESZ;
+      if constexpr (F8) {
+        uint32_t w[2] = {0, 0};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e >> 2] |= float_to_e4m3(f[e] * p.kv_inv_scale) << (8 * (e & 3));
+        *reinterpret_cast<uint2*>(fresh + (is_v ? D : 0) + c * 8) = make_uint2(w[0], w[1]);
+        if (slot >= 0) *reinterpret_cast<uint2*>(pool + c * 8) = make_uint2(w[0], w[1]);
+      } else {
+        const uint4 v = pack8(f);
+        *reinterpret_cast<uint4*>(fresh + (is_v ? 2 * D : 0) + c * 16) = v;
+        if (slot >= 0) *reinterpret_cast<uint4*>(pool + c * 16) = v;
+      }
+    }
   }
 
   // Q rows (zero padded to 16) into shared memory. For an e4m3 pool Q becomes fp16, the type K and V expand to
@@ -271,7 +336,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
     uint4 v = make_uint4(0, 0, 0, 0);
     if (qi < nq) {
       const int rr = qi / g, gg = qi % g;
-      v = *reinterpret_cast<const uint4*>(p.q + (static_cast<long long>(row0 + rr) * p.hq + kvh * g + gg) * D + c * 8);
+      if (rope) {
+        float f[8];
+        rope_chunk<D>(p.qkv + b * p.ld_qkv + (kvh * g + gg) * D, c, cs, f);
+        v = pack8(f);
+      } else {
+        v = *reinterpret_cast<const uint4*>(p.q + (static_cast<long long>(row0 + rr) * p.hq + kvh * g + gg) * D + c * 8);
+      }
     }
     if constexpr (F8) {
       uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -377,6 +448,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
     const uint32_t vbase = kbase + C::TILE_BYTES;
     const int tile = warp + it * DEC_WARPS;
     const int kpos0 = k0 + tile * KT;
+    if (owns_new && tile == ntiles - 1) {      // the new token's row over what the copy found in its slot
+      constexpr int CPR = D * C::ESZ / 16;
+      uint8_t* dst = ring + st * C::STAGE_BYTES;
+      for (int i = lane; i < 2 * CPR; i += 32) {
+        const int c = i % CPR, is_v = i / CPR;
+        *reinterpret_cast<uint4*>(dst + is_v * C::TILE_BYTES + dsw<KT>(ctx - 1 - kpos0, c)) =
+            *reinterpret_cast<const uint4*>(fresh + i * 16);
+      }
+      __syncwarp();
+    }
 
     if constexpr (!T8) {
     float s[NB][4];
@@ -822,6 +903,12 @@ struct DecFuse {
 };
 static thread_local DecFuse g_dec_fuse;
 static thread_local int g_dec_early = 0;
+struct DecRope {
+  const void *qkv = nullptr, *positions = nullptr, *slots = nullptr, *inv_freq = nullptr;
+  long long ld = 0;
+  float kv_inv_scale = 1.f;
+};
+static thread_local DecRope g_dec_rope;
 
 extern "C" {
 
@@ -844,6 +931,17 @@ void hb_attn_decode_fuse(void* split_counter, void* q_out, void* q_sf, const voi
 // its successor only after its own wait (the embedding gather) ran since: the kernel may then read them ahead of its wait.
 void hb_attn_decode_early(void) { g_dec_early = 1; }
 
+// RoPE and KV write inside the NEXT hb_attn_decode call of this thread (with hb_attn_decode_early, one row per sequence): row b of
+// `qkv` [Hq * D | Hkv * D | Hkv * D] is rotated over all of D at positions[b], its K and V go to slots[b] (whose place in the
+// block table is the sequence's last) and take part in the attention from shared memory; `q` is not read. 16-byte aligned rows
+// of qkv and of the pools; `kv_inv_scale` as hb_rope_kv_write has it. The separate kernel was 4.4 us of every layer's chain.
+void hb_attn_decode_rope(const void* qkv, long long ld_qkv, const void* positions, const void* slots, const void* inv_freq,
+                         float kv_inv_scale) {
+  g_dec_rope.kv_inv_scale = kv_inv_scale;
+  g_dec_rope.qkv = qkv; g_dec_rope.ld = ld_qkv; g_dec_rope.positions = positions; g_dec_rope.slots = slots;
+  g_dec_rope.inv_freq = inv_freq;
+}
+
 // bf16 KV, or e4m3 (`kv_fp8`: x = code * kv_scale; head dim 128 or 256, slot and head strides multiples of 16, 16-byte
 // aligned pools); rows_per_seq * (hq / hkv) must be <= 16. Partials go through hb_attn_merge when splits > 1 unless
 // hb_attn_decode_fuse armed the in-kernel merge.
@@ -855,6 +953,8 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
                    void* status, void* stream) {
   const int early = g_dec_early;
   g_dec_early = 0;
+  const DecRope rope = g_dec_rope;
+  g_dec_rope = DecRope{};
   if (batch <= 0) return 0;
   if (kv_fp8 && (pool_stride % 16 != 0 || head_stride % 16 != 0 ||
                  ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) != 0))
@@ -887,6 +987,19 @@ int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long l
   p.q_ka = g_dec_fuse.q_ka;
   g_dec_fuse = DecFuse{};
   p.early = early;
+  p.qkv = static_cast<const __nv_bfloat16*>(rope.qkv);
+  p.ld_qkv = rope.ld;
+  p.positions = static_cast<const int*>(rope.positions);
+  p.slots = static_cast<const int*>(rope.slots);
+  p.inv_freq = static_cast<const float*>(rope.inv_freq);
+  p.kv_inv_scale = rope.kv_inv_scale;
+  if (p.qkv != nullptr) {
+    const int align = kv_fp8 ? 16 : 8;      // pool strides are in elements
+    if (!early || q_indptr != nullptr || max_rows != 1 || p.slots == nullptr || p.positions == nullptr || p.inv_freq == nullptr ||
+        rope.ld % 8 != 0 || (reinterpret_cast<uintptr_t>(rope.qkv) & 15) != 0 || pool_stride % align != 0 ||
+        head_stride % align != 0 || ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) != 0)
+      return 1;
+  }
   if (p.q_out != nullptr && p.splits > 1 && p.split_counter == nullptr) return 1;
   if (p.splits > 1 && (part_o == nullptr || part_lse == nullptr)) return 1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

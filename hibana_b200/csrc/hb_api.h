@@ -153,6 +153,8 @@ void hb_attn_decode_tc_profile(void* buf);
 void hb_attn_prefill_profile(void* buf);
 void hb_attn_decode_profile(void* buf);
 void hb_attn_decode_early(void);
+void hb_attn_decode_rope(const void* qkv, long long ld_qkv, const void* positions, const void* slots, const void* inv_freq,
+                         float kv_inv_scale);
 int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,
                    long long head_stride,
                    const void* kv_indices, long long ld_idx, const void* seq_rows, const void* ctx_len,

@@ -213,9 +213,15 @@ class DenseModel:
                 qkv = norm_linear(res, None, layer.input_norm, t.norm_eps, layer.qkv, add_residual=False)
             else:
                 qkv = self._reduce_norm_linear(h, slot, res, layer.input_norm, layer.qkv, ctx)
-            q = basic.rope_kv_write(qkv, ctx.positions, ctx.slots, self.inv_freq, kv.k[i], kv.v[i], t.q_heads,
-                                    t.kv_heads, t.head_dim, rot=t.rot_dim, kv_scale=kv.kv_scale,
-                                    table=basic.rope_table(ctx, self.inv_freq, t.rot_dim))
+            rope = None
+            if ctx.mode == DECODE and ctx.q_indptr is None and attention.rope_in_kernel(
+                    qkv, kv.k[i], kv.v[i], t.q_heads, t.kv_heads, t.head_dim, t.rot_dim):
+                rope = (qkv, ctx.positions, ctx.slots, self.inv_freq)
+                q = qkv[:, :t.q_heads * t.head_dim].unflatten(1, (t.q_heads, t.head_dim))
+            else:
+                q = basic.rope_kv_write(qkv, ctx.positions, ctx.slots, self.inv_freq, kv.k[i], kv.v[i], t.q_heads,
+                                        t.kv_heads, t.head_dim, rot=t.rot_dim, kv_scale=kv.kv_scale,
+                                        table=basic.rope_table(ctx, self.inv_freq, t.rot_dim))
             # decode-shaped steps hand NVFP4 activations from kernel to kernel: the attention kernel merges its KV
             # splits and quantises for o_proj, the gate/up GEMM requantises for down in its epilogue
             fuse = (cfgmod.current().fuse_epilogues and layer.o.fmt == "nvfp4" and not layer.o.calibrating
@@ -225,7 +231,7 @@ class DenseModel:
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace,
                                             quant_scale=layer.o.input_scale if fuse else None,
-                                            tables_ready=ctx.mode == DECODE)
+                                            tables_ready=ctx.mode == DECODE, rope=rope)
             h, slot = self._row_parallel(layer.o, att if isinstance(att, nvfp4.Nvfp4Tensor)
                                          else att.view(att.shape[0], -1), ctx)
             # prefill-sized chunks requantise in the gate/up epilogue too (tokens on the 128-row side of the GEMM):

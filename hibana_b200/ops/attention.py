@@ -28,6 +28,7 @@ nv.register("hb_attn_decode", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I
 
 nv.register("hb_attn_decode_fuse", [P, P, P, P, I], void=True)
 nv.register("hb_attn_decode_early", [], void=True)
+nv.register("hb_attn_decode_rope", [P, L, P, P, P, Fl], void=True)
 nv.register("hb_attn_decode_tc", [P, P, P, L, L, P, L, P, P, P, P, P, P, I, I, I, I, I, I, Fl, I, L, P, P])
 nv.register("hb_attn_decode_tc_profile", [P], void=True)
 nv.register("hb_attn_prefill_profile", [P], void=True)
@@ -175,7 +176,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                     seq_rows: Optional[torch.Tensor] = None,
                     scale: Optional[float] = None, kv_scale: float = 1.0, causal: bool = True, splits: int = 1,
                     workspace: Optional[AttnWorkspace] = None, out: Optional[torch.Tensor] = None,
-                    quant_scale: Optional[torch.Tensor] = None, tables_ready: bool = False):
+                    quant_scale: Optional[torch.Tensor] = None, tables_ready: bool = False, rope: Optional[tuple] = None):
     """q [T, Hq, D] bf16; pools [slots, Hkv, D]; kv_indices [B, max_ctx] int32; ctx_len [B] int32.
 
     Row r of sequence b (rows q_indptr[b]..q_indptr[b+1], or exactly one row when q_indptr is None) sees keys
@@ -186,6 +187,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     inside the attention kernel, elsewhere a quantisation pass follows.
     `tables_ready`: the tables and all keys and values but those of the call's own rows were complete before the forward began
     with its embedding gather (a decode step): the decode kernel then fetches them while its predecessors still run.
+    `rope` = (qkv, positions, slots, inv_freq), where `rope_in_kernel` allows it: q is a view of the projection's rows, and
+    rotation and KV write happen inside the kernel instead of in `basic.rope_kv_write`.
     """
     t, hq, d = q.shape
     hkv = k_pool.shape[1]
@@ -217,7 +220,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
             nv.lib().hb_attn_decode_fuse(workspace.counter.data_ptr() if splits > 1 else None, nv.ptr(qb), nv.ptr(sfb),
                                          nv.ptr(quant_scale), sfb.shape[1] if sfb is not None else 0)
         if xq is None:
-            out = torch.empty_like(q) if out is None else out
+            out = torch.empty(t, hq, d, dtype=q.dtype, device=q.device) if out is None else out
         # decode_attn = "tc" selects the persistent tcgen05 kernel (head dim 128; csrc/attn_decode_tc.cu). It
         # matches the mma.sync kernel in isolation (123 vs 122 us at 64 x 2304 keys) but not yet inside the 27B
         # decode step (18.8 vs 15.8 ms per step), so the mma.sync kernel stays the default.
@@ -228,6 +231,10 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         tail = (int(causal), k_pool.shape[0], st.status.data_ptr(), nv.stream())
         if tables_ready and not tc:
             nv.lib().hb_attn_decode_early()
+        if rope is not None:
+            qkv, positions, slots, inv_freq = rope
+            nv.lib().hb_attn_decode_rope(qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), slots.data_ptr(),
+                                         inv_freq.data_ptr(), 1.0 / kv_scale)
         code = (nv.lib().hb_attn_decode_tc(*args, *tail) if tc
                 else nv.lib().hb_attn_decode(*args, int(f8), kv_scale, *tail))
         nv.check(code, "hb_attn_decode")
@@ -249,6 +256,21 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     res = _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, seq_rows, scale, kv_scale, causal,
                          splits, workspace, out, cfg, fp8, b, t, hq, hkv, d)
     return res if quant_scale is None else nvfp4.quantize(res.view(t, hq * d), quant_scale)
+
+
+def rope_in_kernel(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, hq: int, hkv: int, d: int, rot: int) -> bool:
+    """Whether a decode step (one row per sequence) may hand its projection's rows to `paged_attention(rope=...)`: the
+    tensor-core decode kernel on a bf16 or e4m3 pool, all of the head rotated, no q / k norm or gate in the rows, 16-byte
+    aligned rows everywhere."""
+    cfg = cfgmod.current()
+    if not nv.use_native(qkv, k_pool) or getattr(k_pool, "sf", None) is not None or cfg.decode_attn == "tc":
+        return False
+    if rot != d or hq // hkv > 16 or qkv.stride(0) % 8 or qkv.stride(1) != 1 or qkv.data_ptr() % 16:
+        return False
+    if k_pool.dtype != torch.bfloat16:
+        return _fp8_tensor_cores(k_pool, v_pool, d, cfg)
+    return (d in (64, 128, 256) and k_pool.stride() == v_pool.stride() and k_pool.stride(2) == 1 and k_pool.stride(0) % 8 == 0
+            and k_pool.stride(1) % 8 == 0 and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
 
 
 def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg, q: Optional[torch.Tensor] = None,
