@@ -28,6 +28,7 @@ nv.register("hb_gemm_silu_quant", [nv.I, nv.P, nv.P, nv.P, nv.P, nv.I, nv.I, nv.
                                    nv.I, nv.I, nv.P, nv.I, nv.I, nv.I, nv.P])
 nv.register("hb_gemm_silu_quant_rows", [nv.I, nv.P, nv.P, nv.P, nv.P, nv.I, nv.I, nv.I, nv.L, nv.L, nv.P, nv.P, nv.P,
                                         nv.P, nv.I, nv.P, nv.I, nv.I, nv.I, nv.P])
+nv.register("hb_few_rows_bf16", [nv.P, nv.L, nv.P, nv.L, nv.I, nv.I, nv.I, nv.P, nv.L, nv.I, nv.P])
 
 
 _PDL_INIT = False
@@ -109,6 +110,16 @@ def _ref_epilogue(acc: torch.Tensor, epilogue: int, residual: Optional[torch.Ten
     return acc.to(torch.bfloat16)
 
 
+def few_rows_ok(x: torch.Tensor, w: torch.Tensor, epilogue: int, residual: Optional[torch.Tensor]) -> bool:
+    """Whether a bf16 projection runs in csrc/few_rows.cu: up to 8 rows and 32 MB of weights, up to 16 rows and 16 MB (measured
+    there; 8192 x 5120 takes 17.6 us against 16.7 at one row, 4096 x 4096 11 against 9.8 at 16). Not under `stable_numerics`: its
+    order of sums is its own."""
+    m, n, k = x.shape[0], w.shape[0], w.shape[1]
+    return (1 <= m <= 16 and n * k <= (16 << 20 if m <= 8 else 8 << 20) and residual is None
+            and epilogue in (EPI_STORE, EPI_STORE_F32) and k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and not cfgmod.current().stable_numerics)
+
+
 def linear_bf16(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE, residual: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None, splits: Optional[int] = None) -> torch.Tensor:
     """y = x @ w.T for bf16 x [M, K], w [N, K] (fp32 accumulation)."""
@@ -122,6 +133,12 @@ def linear_bf16(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE, 
         return res
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
     out = _out(m, n, epilogue, x, out)
+    if splits is None and few_rows_ok(x, w, epilogue, residual):
+        if not _PDL_INIT:
+            set_pdl(cfgmod.current().pdl)
+        nv.check(nv.lib().hb_few_rows_bf16(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), m, n, k, out.data_ptr(),
+                                           out.stride(0), int(epilogue == EPI_STORE_F32), nv.stream()), "hb_few_rows_bf16")
+        return out
     swap, bn, auto_splits = _plan(m, n, (k + 63) // 64, nv.WORKSPACE_BYTES)
     splits = auto_splits if splits is None else splits
     if swap:

@@ -28,7 +28,7 @@ CASES = [([26], [26]), ([50], [50]), ([51], [64]), ([51], [65]), ([100, 1, 27], 
 @pytest.mark.parametrize("scattered", [False, True])
 @pytest.mark.parametrize("causal", [True, False])
 def test_two_q_tiles_match_reference(hq, hkv, d, scattered, causal):
-    """bf16 weights and a bf16 result: 2^-9 each relative to the largest value a row's average is made of."""
+    """bf16 weights and a bf16 result: half an ulp each (2^-8) of the largest value that a row averages is an upper bound."""
     from hibana_b200 import _native as nv
     g = hq // hkv
     gen = torch.Generator(device="cuda").manual_seed(hq * d)
@@ -56,6 +56,6 @@ def test_two_q_tiles_match_reference(hq, hkv, d, scattered, causal):
             attention.two_q_tiles = saved
         ref = attention.paged_attention_ref(q, k, v, idx, ctx, indptr, 1 / math.sqrt(d), causal=causal).float()
         vmax = v.float().abs().max().item()
-        assert (got.float() - ref).abs().max().item() <= 3 * 2.0 ** -9 * vmax, (rows, ctxs)
+        assert (got.float() - ref).abs().max().item() <= 2 * 2.0 ** -8 * vmax, (rows, ctxs)
         assert ((got.float() - ref).norm() / ref.norm()).item() <= 4e-3
     assert nv.read_status() == 0
