@@ -352,7 +352,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
                                   uint8_t* __restrict__ q_out, uint8_t* __restrict__ q_sf,
                                   const float* __restrict__ q_gscale, int q_ka) {
   grid_dep_launch();   // the output projection may become resident and fetch its weights
-  grid_dep_wait();     // may run as a programmatic dependent of the split kernel
+  grid_dep_wait(part_o, part_lse);     // may run as a programmatic dependent of the split kernel
   __shared__ __align__(32) __nv_bfloat16 fin[256];
   extern __shared__ float weight[];     // [splits]
   const long long rh = blockIdx.x;

@@ -226,14 +226,14 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const int key = kbeg + t * KT + r0 + i * RSTEP;
-        sl[i] = t < ntiles && key < kmax ? __ldg(idx_row + key) : -1;
+        sl[i] = t < ntiles && key < kmax ? ld_step(idx_row + key) : -1;
       }
     };
     auto load = [&](const void* pool, const int (&sl)[PER], uint4 (&reg)[PER]) {
 #pragma unroll
       for (int i = 0; i < PER; ++i)
         reg[i] = sl[i] < 0 ? make_uint4(0, 0, 0, 0)
-                           : __ldg(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(pool) +
+                           : ld_step(reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(pool) +
                                                                   static_cast<long long>(sl[i]) * p.pool_stride +
                                                                   kvh * p.head_stride + part * 16));
     };
@@ -285,7 +285,7 @@ __device__ __forceinline__ void pf_produce(const PfParams& p, const PfBlock& x, 
     for (int i = 0; i < SB; ++i) {
       const int j = pw + 3 * i;
       const int key = kbeg + t * KT + j * 32 + lane;
-      sl[i] = (j < KT / 32 && t < ntiles && key < kmax) ? __ldg(idx_row + key) : -1;
+      sl[i] = (j < KT / 32 && t < ntiles && key < kmax) ? ld_step(idx_row + key) : -1;
     }
   };
   auto copy_tile = [&](int t, const int (&sl)[SB], const __nv_bfloat16* pool, const CUtensorMap* tm, uint8_t* ring,
@@ -1212,7 +1212,7 @@ attn_prefill_q2_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
     const int* idx_row = p.kv_indices + static_cast<long long>(p.seq_rows ? p.seq_rows[x.b] : x.b) * p.ld_idx;
     auto fetch_slot = [&](int t) {             // -1 beyond the visible keys
       const int key = t * KT + j * 32 + lane;
-      return t < x.ntiles && key < x.kmax ? __ldg(idx_row + key) : -1;
+      return t < x.ntiles && key < x.kmax ? ld_step(idx_row + key) : -1;
     };
     auto place = [&](int t) { return (is_v ? Q2_STAGES : 0) + t % Q2_STAGES; };
     int slot = fetch_slot(0), next = fetch_slot(1);

@@ -43,14 +43,9 @@ few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __re
     const int f = f0 + g4 + 8 * half, kk = kl + i * STRIDE;
     return f < n && kk < k ? __ldg(reinterpret_cast<const uint4*>(w + f * ldw + kk)) : zero;
   };
-  // x is another kernel's output: a load that stays behind the wait (one through a const __restrict__ pointer may move ahead of it)
   auto rows = [&](int i, int blk) -> uint4 {
     const int t = blk * 8 + g4, kk = kl + i * STRIDE;
-    uint4 v = zero;
-    if (t < m && kk < k)
-      asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(x + t * ldx + kk) : "memory");
-    return v;
+    return t < m && kk < k ? ld_step(reinterpret_cast<const uint4*>(x + t * ldx + kk)) : zero;
   };
   uint4 a[DEPTH][2], b[DEPTH][NB];
   grid_dep_launch();

@@ -6,6 +6,7 @@
 // returns; nothing traps and nothing spins forever.
 #pragma once
 #include <cstdint>
+#include <cstring>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -202,7 +203,48 @@ __device__ __forceinline__ float4 ld_dsmem_v4(uint32_t cluster_addr) {   // 16-b
 // The grid this one depends on (programmatic stream serialisation) has completed and its writes are visible.
 // A no-op when the kernel was launched without the attribute.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The same for a kernel with const __restrict__ parameters that earlier kernels of the step wrote: the compiler may move a load through
+// such a pointer ahead of the wait (a promise about the whole kernel overrides the asm's clobber), so they are named here and come out
+// as values that do not exist before it. Loads through them are plain ones then, not read-only ones.
+template <typename P>
+__device__ __forceinline__ void behind_wait(P& p) {          // (stays a global address: no generic loads)
+  size_t a = __cvta_generic_to_global(p);
+  asm volatile("" : "+l"(a)::"memory");
+  p = static_cast<P>(__cvta_global_to_generic(a));
+}
+template <typename P, typename... Q>
+__device__ __forceinline__ void grid_dep_wait(P& p, Q&... q) {
+  grid_dep_wait();
+  behind_wait(p);
+  (behind_wait(q), ...);
+}
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Load of what an earlier kernel of the step wrote where a const __restrict__ view or __ldg would be wanted for speed (loads that need
+// not keep their order with this kernel's stores): stays behind the wait, and is a plain load, not a read-only one.
+template <typename T>
+__device__ __forceinline__ T ld_step(const T* p) {
+  static_assert(sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "2, 4, 8 or 16 bytes");
+  T r;
+  if constexpr (sizeof(T) == 2) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    memcpy(&r, &v, 2);
+  } else if constexpr (sizeof(T) == 4) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    memcpy(&r, &v, 4);
+  } else if constexpr (sizeof(T) == 8) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    memcpy(&r, &v, 8);
+  } else {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    memcpy(&r, &v, 16);
+  }
+  return r;
+}
 
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -30,7 +30,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int h, long long ldx,
                long long ldy, float eps, int gemma) {
   grid_dep_launch();
-  grid_dep_wait();
+  grid_dep_wait(x, residual);
   __shared__ float red[32];
   const int row = blockIdx.x;
   const int nvec = h >> 3;
@@ -83,15 +83,16 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
 // 66 us with a warp per group and four predicated chunks, 19 us so; 4096 rows of 8 groups of 1024, 115 -> 99.
 // Lanes beyond the end of a group that does not fill them (16, 96 or 640 channels) divide ones, not zeros: a zero dividend sends
 // its warp through the division's slow path (one row of 6 groups of 640: 8.9 us with zeros and four chunks, 4.1 so).
+// (two blocks to an SM asked for: with plain loads the compiler takes 138 registers at four chunks, one block, 5000 x 10240 70 -> 117 us)
 template <int NC, int L>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows, int h, int gs,
                          long long ldx, long long ldz, float eps, int norm_first, int sigmoid_gate, int gemma,
                          uint8_t* __restrict__ q_out, uint8_t* __restrict__ q_sf, const float* __restrict__ q_gscale,
                          int q_ka) {
   grid_dep_launch();
-  grid_dep_wait();
+  grid_dep_wait(x, z);
   const int groups = h / gs;
   const long long id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / L;
   const bool live = id < static_cast<long long>(rows) * groups;      // (idle lanes still take part in the shuffles)
@@ -186,7 +187,7 @@ __global__ void gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const 
                                      const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows,
                                      int h, int gs, long long ldx, long long ldz, float eps, int norm_first,
                                      int sigmoid_gate, int gemma) {
-  grid_dep_wait();
+  grid_dep_wait(x, z);
   grid_dep_launch();
   const int groups = h / gs;
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -233,7 +234,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, long
                                      uint8_t* __restrict__ v_sf, long long sf_pool_stride, long long sf_head_stride,
                                      const float2* __restrict__ table) {
   grid_dep_launch();   // at level 2 the attention kernel is a dependent and its launch overlaps the rest of the projection
-  grid_dep_wait();     // may run as a programmatic dependent of the QKV projection
+  grid_dep_wait(qkv, positions, slots, table);     // may run as a programmatic dependent of the QKV projection
   const int t = blockIdx.x;
   const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int nw = gridDim.y * (blockDim.x >> 5);
@@ -336,7 +337,7 @@ __device__ __forceinline__ float act_one(int mode, float a, float b) {
 }
 __global__ void act_mul_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
                                    __nv_bfloat16* __restrict__ out, long long rows, int inter, long long ldx, int mode) {
-  grid_dep_wait();
+  grid_dep_wait(x, gate);
   grid_dep_launch();
   const int per_row = inter >> 3;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -373,7 +374,7 @@ __global__ void act_mul_vec_kernel(const __nv_bfloat16* __restrict__ x, const __
 // other. In place on the contiguous y; 8 channels per thread. Five element-wise passes took 230 us at 4096 x 8192, this takes 33.
 __global__ void head_skip_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x, long long ldx,
                                  const float* __restrict__ d, long long rows, int inner, int head_dim) {
-  grid_dep_wait();
+  grid_dep_wait(x, y);
   grid_dep_launch();
   const int per_row = inner >> 3;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -394,7 +395,7 @@ __global__ void head_skip_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloa
 
 __global__ void act_mul_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
                                __nv_bfloat16* __restrict__ out, long long rows, int inter, long long ldx, int mode) {
-  grid_dep_wait();
+  grid_dep_wait(x, gate);
   grid_dep_launch();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= rows * inter) return;
@@ -421,7 +422,7 @@ __global__ void act_mul_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 __global__ void gdn_gates_kernel(const __nv_bfloat16* __restrict__ ba, long long ld, const float* __restrict__ a_log,
                                  const float* __restrict__ dt_bias, int rows, int heads, float* __restrict__ beta,
                                  float* __restrict__ g) {
-  grid_dep_wait();
+  grid_dep_wait(ba);
   grid_dep_launch();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * heads) return;
@@ -435,7 +436,7 @@ __global__ void gdn_gates_kernel(const __nv_bfloat16* __restrict__ ba, long long
 
 __global__ void embedding_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                  __nv_bfloat16* __restrict__ out, int h, long long vocab) {
-  grid_dep_wait();
+  grid_dep_wait(ids);
   grid_dep_launch();
   const int t = blockIdx.x;
   long long id = ids[t];
@@ -447,7 +448,7 @@ __global__ void embedding_kernel(const long long* __restrict__ ids, const __nv_b
 
 __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                            __nv_bfloat16* __restrict__ out, long long n) {
-  grid_dep_wait();
+  grid_dep_wait(a, b);
   grid_dep_launch();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2;
   if (i + 1 < n) {
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(
     long long pool_stride, long long head_stride, int tokens, int hq, int hkv, int d, int q_gate,
     const float2* __restrict__ table) {
   grid_dep_launch();
-  grid_dep_wait();
+  grid_dep_wait(qkv, slots, table);
   const int lanes_per_head = d >> 3;                       // 8, 16 or 32
   const int heads_per_warp = 32 / lanes_per_head;
   const int lane = threadIdx.x & 31;
@@ -615,7 +616,7 @@ void hb_rope_use_table(const void* table) { g_rope_table = static_cast<const flo
 
 __global__ void rope_table_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq, int tokens,
                                   int half, float2* __restrict__ out) {
-  grid_dep_wait();
+  grid_dep_wait(positions);
   grid_dep_launch();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<long long>(tokens) * half) return;

@@ -35,7 +35,7 @@ __device__ __forceinline__ unsigned route_key(float v) {
 __global__ void __launch_bounds__(1024) moe_route_block_kernel(
     const float* __restrict__ logits, long long ld, const float* __restrict__ sel_bias, int experts, int topk,
     int sigmoid, int renorm, float scale, int* __restrict__ ids, float* __restrict__ weights) {
-  grid_dep_wait();
+  grid_dep_wait(logits);
   grid_dep_launch();
   __shared__ float s_red[32];
   __shared__ int s_warp_tie[32], s_warp_sel[32];
@@ -113,7 +113,7 @@ template <int PER>
 __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ sel_bias,
                                  int tokens, int experts, int topk, int sigmoid, int renorm, float scale,
                                  int* __restrict__ ids, float* __restrict__ weights) {
-  grid_dep_wait();
+  grid_dep_wait(logits);
   grid_dep_launch();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -215,7 +215,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
 __global__ void __launch_bounds__(1024)
 moe_share_kernel(int* __restrict__ ids, float* __restrict__ weights, int rows, int k, int experts, int keep, int budget,
                  float scale) {
-  grid_dep_wait();
+  grid_dep_wait(ids, weights);
   grid_dep_launch();
   __shared__ unsigned score[1024];
   __shared__ unsigned char in_set[1024];
@@ -315,7 +315,7 @@ moe_plan_kernel(const int* __restrict__ ids, int pairs, int topk, int experts, i
                 int* __restrict__ cnt, int* __restrict__ start, int* __restrict__ pos, int* __restrict__ src_row,
                 int rows_cap, int* __restrict__ total_rows, int tile_bn, int* __restrict__ tiles,
                 int* __restrict__ n_tiles, int tile_cap) {
-  grid_dep_wait();
+  grid_dep_wait(ids);
   grid_dep_launch();
   extern __shared__ int sm[];   // [experts] own counts, [experts] starts, [experts] running, [warps][experts]
   int* own = sm;
@@ -444,7 +444,7 @@ moe_plan_kernel(const int* __restrict__ ids, int pairs, int topk, int experts, i
 // expert * 4096 + chunk per tile of `tile_bn` rows that has rows. Single CTA.
 __global__ void moe_tiles_kernel(const int* __restrict__ cnt, int experts, int tile_bn, int* __restrict__ tiles,
                                  int* __restrict__ n_tiles, int tile_cap) {
-  grid_dep_wait();
+  grid_dep_wait(cnt);
   grid_dep_launch();
   extern __shared__ int base[];
   __shared__ int wtot[32];
@@ -473,7 +473,7 @@ __global__ void moe_tiles_kernel(const int* __restrict__ cnt, int experts, int t
 
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ src_row,
                                   const int* __restrict__ total_rows, __nv_bfloat16* __restrict__ out, int h) {
-  grid_dep_wait();
+  grid_dep_wait(x, src_row, total_rows);
   grid_dep_launch();
   const int r = blockIdx.x;
   if (r >= *total_rows) return;
@@ -493,7 +493,7 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, long lon
                                    long long ld_shared, __nv_bfloat16* __restrict__ out, long long ldo, int topk,
                                    int h) {
   grid_dep_launch();
-  grid_dep_wait();
+  grid_dep_wait(y, pos, weights, shared);
   const int t = blockIdx.x;
   __shared__ int ps[MAX_TOPK];
   __shared__ float ws[MAX_TOPK];

@@ -22,7 +22,7 @@ __global__ void quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long lon
                                    const float* __restrict__ gscale, uint8_t* __restrict__ q,
                                    uint8_t* __restrict__ sf, int mode, const int* __restrict__ src_rows,
                                    const int* __restrict__ total_rows) {
-  grid_dep_wait();     // launched as a programmatic dependent: the producer of x must have completed
+  grid_dep_wait(x, src_rows, total_rows);     // launched as a programmatic dependent: the producer of x must have completed
   grid_dep_launch();   // a GEMM may start prefetching its weights; behind the wait, as a grouped one reads the plan (launch_dep)
   const int groups_pad = ka * 4;
   const int rows_pad = ((m + 127) >> 7) << 7;
@@ -76,7 +76,7 @@ __global__ void quant_nvfp4_pairs_kernel(const __nv_bfloat16* __restrict__ x, lo
                                          const int* __restrict__ pos, int pairs, int topk, int k, int ka,
                                          const float* __restrict__ gscale, uint8_t* __restrict__ q,
                                          uint8_t* __restrict__ sf) {
-  grid_dep_wait();
+  grid_dep_wait(x, pos);
   grid_dep_launch();   // behind the wait: the grouped GEMM that follows reads the routing plan at once (see launch_dep)
   const int groups_pad = ka * 4;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -121,7 +121,7 @@ norm_quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
       if (tid + i * T < nchunk) wa[i] = __ldg(reinterpret_cast<const uint4*>(w) + tid + i * T);
     if (q != nullptr) gs_early = __ldg(gscale);
   }
-  grid_dep_wait();
+  grid_dep_wait(x, residual);
   if (row >= m) {   // padding rows of the last 128-row scale block: zero scales, nothing else
     for (int g = tid; g < ka * 4; g += T) sf[row_sf_off(row, g, ka)] = 0;
     return;

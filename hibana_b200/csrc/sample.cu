@@ -33,7 +33,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 argmax_kernel(const T* __restrict__ logits, long long ld, int vocab, const int* __restrict__ bitmask, int mask_words,
               long long* __restrict__ out, float* __restrict__ out_val) {
-  grid_dep_wait();
+  grid_dep_wait(logits, bitmask);
   grid_dep_launch();
   __shared__ float sv[8];
   __shared__ int si[8];
@@ -80,7 +80,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 argmax_partial_kernel(const T* __restrict__ logits, long long ld, int vocab, const int* __restrict__ bitmask,
                       int mask_words, int nch, float* __restrict__ pv, int* __restrict__ pi) {
-  grid_dep_wait();
+  grid_dep_wait(logits, bitmask);
   grid_dep_launch();
   __shared__ float sv[8];
   __shared__ int si[8];
@@ -128,7 +128,7 @@ argmax_partial_kernel(const T* __restrict__ logits, long long ld, int vocab, con
 __global__ void argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int nch, int rows,
                                     const float* __restrict__ temperature, long long* __restrict__ out,
                                     float* __restrict__ out_val) {
-  grid_dep_wait();
+  grid_dep_wait(pv, pi, temperature);
   grid_dep_launch();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -477,7 +477,7 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
               const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ offsets,
               const int* __restrict__ bitmask, int mask_words, long long* __restrict__ out,
               float* __restrict__ out_prob, int skip_greedy) {
-  grid_dep_wait();
+  grid_dep_wait(logits, temperature, top_k, top_p, seeds, offsets, bitmask);
   grid_dep_launch();
   __shared__ float cv[SAMPLE_K];
   __shared__ int ci[SAMPLE_K];

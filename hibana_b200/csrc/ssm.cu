@@ -31,7 +31,7 @@ __global__ void conv1d_kernel(const __nv_bfloat16* __restrict__ x, long long ldx
                               const int* __restrict__ q_indptr, const int* __restrict__ slot_in,
                               const int* __restrict__ slot_out, const int* __restrict__ has_init, int channels,
                               int act_silu) {
-  grid_dep_wait();
+  grid_dep_wait(x, state, q_indptr, slot_in, slot_out, has_init);
   grid_dep_launch();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -78,7 +78,7 @@ __global__ void conv1d_tiled_kernel(const __nv_bfloat16* __restrict__ x, long lo
                                     long long state_stride, const int* __restrict__ q_indptr,
                                     const int* __restrict__ slot_in, const int* __restrict__ slot_out,
                                     const int* __restrict__ has_init, int channels, int act_silu) {
-  grid_dep_wait();
+  grid_dep_wait(x, state, q_indptr, slot_in, slot_out, has_init);
   grid_dep_launch();
   const int b = blockIdx.z;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -125,7 +125,7 @@ __global__ void conv1d_state_kernel(const __nv_bfloat16* __restrict__ x, long lo
                                     const int* __restrict__ q_indptr, const int* __restrict__ slot_in,
                                     const int* __restrict__ slot_out, const int* __restrict__ has_init,
                                     int channels) {
-  grid_dep_wait();
+  grid_dep_wait(x, state, q_indptr, slot_in, slot_out, has_init);
   grid_dep_launch();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
