@@ -200,100 +200,329 @@ __device__ __forceinline__ int block_sum_i(int v, int* red) {
   return __reduce_add_sync(0xffffffffu, red[threadIdx.x & 31]);
 }
 
-// Largest key x of [lo, hi] with f(x) >= want, where f(x) is the sum of weight(v) over the allowed tokens of key >= x (f(lo) >=
-// want, f falls with x, no token is above hi). Every pass over the row sums the tokens above WAYS - 1 thresholds at once, so
-// 32 bits take 8 passes instead of 32, and what lies above the range is carried along, so later passes only look at
-// the few tokens inside it. Deterministic. Whole CTA; `sums` is shared scratch.
-constexpr int WAYS = 16;
-template <typename V, typename T, typename W>
-__device__ unsigned search_key(const T* __restrict__ lr, int vocab, const int* __restrict__ mask, unsigned lo, unsigned hi,
-                               V want, W weight, V (*sums)[LAW_WARPS]) {
+// A row as order keys, 0 for what is out of the law (masked, NaN, -inf: finite and +inf values have keys above 0x007fffff). Rows that
+// fit are brought into shared memory once (STAGED), others are read and converted at each pass. ONE_ZERO: -0.0 has the key of 0.0.
+template <typename T, bool STAGED, bool ONE_ZERO = false>
+struct RowKeys {
+  const T* lr;
+  const int* mask;
+  const unsigned* staged;
+  // keys of i, i + step, ... (0 from `end` on), all loads in flight before the first is used
+  template <bool RAW, int U>
+  __device__ __forceinline__ void load(unsigned (&k)[U], int i, int step, int end) const {
+    if (STAGED && !RAW) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) k[u] = i + u * step < end ? staged[i + u * step] : 0u;
+    } else {
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = ldf<T>(lr, min(i + u * step, end - 1));
+      if (mask != nullptr) {
+        int m[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) m[u] = mask[min(i + u * step, end - 1) >> 5];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (!((m[u] >> ((i + u * step) & 31)) & 1)) v[u] = -INFINITY;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) k[u] = i + u * step < end && v[u] > -INFINITY ? order_key(v[u]) : 0u;
+    }
+    if (ONE_ZERO)
+#pragma unroll
+      for (int u = 0; u < U; ++u) k[u] = k[u] == 0x7fffffffu ? 0x80000000u : k[u];
+  }
+  __device__ __forceinline__ unsigned operator()(int i) const {
+    unsigned k[1];
+    load<false>(k, i, 1, i + 1);
+    return k[0];
+  }
+};
+
+// f(key, index) over begin, begin + step, ... < end in order, U loads at once (0 past the end).
+template <int U = 8, typename R, typename F>
+__device__ __forceinline__ void scan(const R& row, int begin, int end, int step, F f) {
+  for (int i = begin; i < end; i += U * step) {
+    unsigned k[U];
+    row.template load<false>(k, i, step, end);
+#pragma unroll
+    for (int u = 0; u < U; ++u) f(k[u], i + u * step);
+  }
+}
+
+// The largest key of a row (at least that of -inf); a staged row is in shared memory afterwards. Whole CTA.
+template <typename R>
+__device__ unsigned stage_row(const R& row, bool keep, unsigned* keys, int vocab, unsigned* red) {
+  unsigned mk = order_key(-INFINITY);
+  for (int i = threadIdx.x; i < vocab; i += 16 * LAW_T) {
+    unsigned k[16];
+    row.template load<true>(k, i, LAW_T, vocab);
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      if (keep && i + u * LAW_T < vocab) keys[i + u * LAW_T] = k[u];
+      mk = max(mk, k[u]);
+    }
+  }
+  mk = __reduce_max_sync(0xffffffffu, mk);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mk;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, red[threadIdx.x & 31]);
+}
+
+// Largest key x of [lo, hi] with f(x) >= want, where f(x) is the sum of weight(v) over the tokens of key >= x (f(lo) >= want, f falls
+// with x, no token is above hi = the key of `top`, weights are at most 1).
+// One pass adds the weights up in BUCKETS of 1/16 `width` below `top` (a nucleus ends within some temperatures of the maximum), as
+// whole numbers of 2^-41, so the order of the atomics does not matter; the bucket where the sum reaches `want` holds the answer. Its tokens
+// are listed and each finds its own f; the largest key that holds is it. More than RANKED of them (ties, long rows, the
+// last bucket) are narrowed first, each pass summing above 15 thresholds. At 18992 tokens that is one pass and the list where
+// narrowing 32 bits by 16 took eight passes. Deterministic. Whole CTA.
+constexpr int WAYS = 16, BUCKETS = 256, RANKED = 1024;
+constexpr int FIX = 41, FIX_PART = 14;    // a sum is kept in three parts: 2^14 * 2^18 tokens fill 32 bits
+template <typename V>
+struct SearchScratch {
+  union {
+    unsigned bucket[3][BUCKETS];
+    uint2 list[RANKED];      // key, weight
+  };
+  V sums[WAYS][LAW_WARPS];
+  V totals[WAYS];
+  V before;
+  int count[LAW_WARPS];
+  unsigned best, low;
+  int at;
+  uint4 thr[WAYS / 4];       // thresholds (in registers they would spill: 64 a thread)
+};
+__device__ __forceinline__ float as_weight(unsigned b, float) { return __uint_as_float(b); }
+__device__ __forceinline__ int as_weight(unsigned b, int) { return static_cast<int>(b); }
+__device__ __forceinline__ unsigned weight_bits(float w) { return __float_as_uint(w); }
+__device__ __forceinline__ unsigned weight_bits(int w) { return static_cast<unsigned>(w); }
+__device__ __forceinline__ unsigned long long fixed(float w) { return __float2ull_rn(w * static_cast<float>(1ull << FIX)); }
+__device__ __forceinline__ unsigned long long fixed(int w) { return w; }
+__device__ __forceinline__ float from_fixed(unsigned long long s, float) {
+  return static_cast<float>(static_cast<double>(s) * (1.0 / static_cast<double>(1ull << FIX)));
+}
+__device__ __forceinline__ int from_fixed(unsigned long long s, int) { return static_cast<int>(s); }
+
+// Sixteen sums over a warp at once: at each step a lane keeps half of its sums and hands the other half to its partner (the
+// additions of a tree over each). Sum j ends in acc[0] of lanes 2 j and 2 j + 1.
+template <typename V>
+__device__ __forceinline__ void warp_sums(V (&acc)[WAYS], int lane) {
+#pragma unroll
+  for (int o = 16, c = WAYS / 2; o > 1; o >>= 1, c >>= 1)
+#pragma unroll
+    for (int j = 0; j < WAYS / 2; ++j)
+      if (j < c) {
+        const V keep = (lane & o) ? acc[j + c] : acc[j], give = (lane & o) ? acc[j] : acc[j + c];
+        acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+  acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+}
+
+template <typename V, typename R, typename W>
+__device__ unsigned search_key(const R& row, int vocab, unsigned lo, unsigned hi, V want, float top, float width, W weight,
+                               SearchScratch<V>& sc) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (!(lo < hi)) return lo;
+  if (V(0) >= want) return hi;
   V beyond = V(0);           // f(hi + 1)
+  // Lists the tokens that are `in`; if they are few the answer is found (true).
+  auto ranked = [&](auto in, unsigned& answer) {
+    int mine = 0;
+    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) { mine += in(k); });
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    if (lane == 31) sc.count[warp] = upto;
+    if (tid == 0) sc.best = 0u;
+    __syncthreads();
+    const int c = sc.count[lane];
+    const int total = __reduce_add_sync(0xffffffffu, c);
+    if (total > RANKED) return false;
+    int at = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0) + upto - mine;
+    if (mine != 0)
+      scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
+        if (in(k)) sc.list[at++] = make_uint2(k, weight_bits(weight(key_value(k))));
+      });
+    __syncthreads();
+    if (tid < total) {
+      const unsigned k = sc.list[tid].x;
+      V f = V(0);
+#pragma unroll 8
+      for (int i = 0; i < total; ++i) {
+        const uint2 e = sc.list[i];
+        f += e.x >= k ? as_weight(e.y, V(0)) : V(0);
+      }
+      if (f + beyond >= want) atomicMax(&sc.best, k);
+    }
+    __syncthreads();
+    answer = max(sc.best, lo);
+    return true;
+  };
+  unsigned answer;
+  if (vocab <= (1 << 18)) {
+    const float per = 16.f / width;
+    auto bucket = [&](unsigned k) {         // rises as the key falls, by roundings that keep the order
+      return static_cast<int>(fminf((top - key_value(k)) * per, static_cast<float>(BUCKETS - 1)));
+    };
+    __syncthreads();
+    for (int i = tid; i < 3 * BUCKETS; i += LAW_T) sc.bucket[0][i] = 0u;
+    if (tid == 0) sc.at = BUCKETS;
+    __syncthreads();
+    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
+      if (k > lo) {
+        const int b = bucket(k);
+        const unsigned long long w = fixed(weight(key_value(k)));
+        constexpr unsigned PART = (1u << FIX_PART) - 1u;
+        atomicAdd(&sc.bucket[0][b], static_cast<unsigned>(w) & PART);
+        if (sizeof(V) == 4 && static_cast<V>(0.5f) != V(0)) {      // (counts need one part)
+          atomicAdd(&sc.bucket[1][b], static_cast<unsigned>(w >> FIX_PART) & PART);
+          atomicAdd(&sc.bucket[2][b], static_cast<unsigned>(w >> (2 * FIX_PART)));
+        }
+      }
+    });
+    __syncthreads();
+    if (tid < 32) {          // the first bucket whose end reaches `want`: each lane owns BUCKETS / 32 in a row
+      constexpr int OWN = BUCKETS / 32;
+      unsigned long long own[OWN], upto = 0;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) {
+        const int b = tid * OWN + j;
+        upto += sc.bucket[0][b] + (static_cast<unsigned long long>(sc.bucket[1][b]) << FIX_PART) +
+                (static_cast<unsigned long long>(sc.bucket[2][b]) << (2 * FIX_PART));
+        own[j] = upto;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const unsigned long long before = upto - own[OWN - 1];
+      const unsigned reached = __ballot_sync(0xffffffffu, from_fixed(upto, V(0)) >= want);
+      if (reached && lane == __ffs(reached) - 1)
+#pragma unroll
+        for (int j = OWN - 1; j >= 0; --j)
+          if (from_fixed(before + own[j], V(0)) >= want) {
+            sc.at = tid * OWN + j;
+            sc.before = from_fixed(before + (j == 0 ? 0ull : own[j - 1]), V(0));
+          }
+    }
+    __syncthreads();
+    const int at = sc.at;
+    if (at == BUCKETS) return lo;
+    beyond = sc.before;
+    auto in = [&](unsigned k) { return k > lo && bucket(k) == at; };
+    if (ranked(in, answer)) return answer;
+    unsigned kmin = 0xffffffffu, kmax = 0u;
+    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
+      if (in(k)) {
+        kmin = min(kmin, k);
+        kmax = max(kmax, k);
+      }
+    });
+    if (tid == 0) sc.low = 0xffffffffu;
+    __syncthreads();
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) {
+      atomicMin(&sc.low, kmin);
+      atomicMax(&sc.best, kmax);
+    }
+    __syncthreads();
+    lo = sc.low - 1;         // f(the lowest key of the bucket) >= want
+    hi = sc.best;
+    __syncthreads();
+  }
   while (lo < hi) {
+    if (ranked([&](unsigned k) { return k > lo && k <= hi; }, answer)) return answer;
     const unsigned span = hi - lo, step = span / WAYS + 1;
-    V acc[WAYS - 1];
-#pragma unroll
-    for (int j = 0; j < WAYS - 1; ++j) acc[j] = V(0);
-#pragma unroll 4
-    for (int i = threadIdx.x; i < vocab; i += LAW_T) {
-      const float v = ldf<T>(lr, i);
-      const unsigned k = order_key(v);
-      if (k > lo && k <= hi && v > -INFINITY && mask_ok(mask, i)) {
-        const unsigned above = (k - lo) / step;          // thresholds lo + step, lo + 2 step, ... at or below k
-        const V w = weight(v);
-#pragma unroll
-        for (int j = 0; j < WAYS - 1; ++j) acc[j] += above > static_cast<unsigned>(j) ? w : V(0);
-      }
-    }
+    const int n = static_cast<int>(span / step);
+    if (tid < WAYS) reinterpret_cast<unsigned*>(sc.thr)[tid] = lo + (tid + 1) * step;      // lo + step, ... up to hi
     __syncthreads();
+    V acc[WAYS];
 #pragma unroll
-    for (int j = 0; j < WAYS - 1; ++j) {
-      V t = acc[j];
+    for (int j = 0; j < WAYS; ++j) acc[j] = V(0);
+    bool some = false;
+    scan<4>(row, tid, vocab, LAW_T, [&](unsigned k, int) {
+      if (k > lo && k <= hi) {
+        const V w = weight(key_value(k));
+        some = true;
+#pragma unroll
+        for (int j = 0; j < WAYS / 4; ++j) {
+          const uint4 t = sc.thr[j];
+          acc[4 * j] += k >= t.x ? w : V(0);
+          acc[4 * j + 1] += k >= t.y ? w : V(0);
+          acc[4 * j + 2] += k >= t.z ? w : V(0);
+          if (j < WAYS / 4 - 1) acc[4 * j + 3] += k >= t.w ? w : V(0);
+        }
+      }
+    });
+    if (__any_sync(0xffffffffu, some)) warp_sums(acc, lane);
+    if ((lane & 1) == 0) sc.sums[lane >> 1][warp] = acc[0];
+    __syncthreads();
+    if (warp < n) {
+      V t = sc.sums[warp][lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if ((threadIdx.x & 31) == 0) sums[j][threadIdx.x >> 5] = t;
+      if (lane == 0) sc.totals[warp] = t + beyond;
     }
     __syncthreads();
-    unsigned best = 0;       // thresholds that hold
-#pragma unroll 1
-    for (; best < span / step; ++best) {
-      V t = sums[best][threadIdx.x & 31];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      t += beyond;
-      if (!(t >= want)) {
-        hi = lo + (best + 1) * step - 1;
-        beyond = t;
-        break;
-      }
+    const unsigned failed = __ballot_sync(0xffffffffu, lane < n && !(sc.totals[lane < WAYS ? lane : 0] >= want));
+    const int best = failed ? __ffs(failed) - 1 : n;       // thresholds that hold
+    if (best < n) {
+      hi = lo + (best + 1) * step - 1;
+      beyond = sc.totals[best];
     }
     lo += best * step;
   }
   return lo;
 }
 
+// The 32 values of a warp added to `acc` one after the other; `after` = the running sum behind this lane's own. Every lane gets the end.
+__device__ __forceinline__ float sum_lanes(float acc, float w, int lane, float& after) {
+#pragma unroll
+  for (int src = 0; src < 32; ++src) {
+    acc += __shfl_sync(0xffffffffu, w, src);
+    if (lane == src) after = acc;
+  }
+  return acc;
+}
+
 // The sampling law of one row as engine/rejection.py `distribution` defines it: softmax(logits / temp) over the
 // allowed tokens, cut to the first `k_lim` tokens in (value desc, index asc) order (0 = no cut), then to the
 // smallest prefix of that order whose mass reaches p_lim. Draws one token by inverse CDF in index order from the
 // law with token `exclude` removed (-1: nothing removed; the residual of a point-mass draft in speculative
-// sampling) and reports the probability of token `probe` under the law. LAW_T threads, whole CTA. With a nucleus
-// cut, 256 threads and one threshold per pass took 165 us at 18992 tokens and 2040 us at 151936; this takes 87 and 480 us (0 of
-// 36000 draws differed).
-template <typename T>
-__device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restrict__ mask, float temp, int k_lim,
-                        float p_lim, float u01, int exclude, int probe, long long* out, float* out_prob,
-                        float* out_probe) {
+// sampling) and reports the probability of token `probe` under the law. LAW_T threads, whole CTA. Bound by the chain of its passes
+// over the row, so the row is staged where it fits. With a nucleus cut, us at 11 rows, a pass over the row for every 4
+// bits of the cut / now: 18992 tokens 85 / 32, 31040 113 / 42, 52224 167 / 65, 151936 (not staged) 479 / 318; cut off 26 / 18, 36 / 22, 53 / 33,
+// 163 / 117 (0 of 13824 draws and probabilities differed).
+template <typename T, bool STAGED>
+__device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int k_lim, float p_lim, float u01, int exclude,
+                        int probe, long long* out, float* out_prob, float* out_probe, SearchScratch<float>& sc) {
   constexpr int CHUNKS = 256;              // contiguous pieces of the row for the draw
+  extern __shared__ unsigned row_keys[];   // STAGED: vocab of them
+  __shared__ unsigned redu[LAW_WARPS];
   __shared__ float red[LAW_WARPS];
   __shared__ int redi[LAW_WARPS];
-  __shared__ float csum[CHUNKS];
-  __shared__ int ceq[CHUNKS];
-  __shared__ int s_pick, s_eq_base;
-  __shared__ float s_base;
-  __shared__ float sums_f[WAYS - 1][LAW_WARPS];
-  __shared__ int sums_i[WAYS - 1][LAW_WARPS];
+  __shared__ float cweight[CHUNKS];
+  __shared__ int ceq[CHUNKS];              // threshold tokens in front of a chunk
+  __shared__ int ceq_warp[CHUNKS / 32];
   const int tid = threadIdx.x;
   const float inv_t = 1.f / temp;
-  float mx = -INFINITY;
-  for (int i = tid; i < vocab; i += LAW_T)
-    if (mask_ok(mask, i)) mx = fmaxf(mx, ldf<T>(lr, i));
-  mx = warp_max(mx);
-  __syncthreads();
-  if ((tid & 31) == 0) red[tid >> 5] = mx;
-  __syncthreads();
-  mx = warp_max(red[tid & 31]);
+  const RowKeys<T, STAGED> row{lr, mask, row_keys};
+  const unsigned mk = stage_row(row, STAGED, row_keys, vocab, redu);
+  const float mx = key_value(mk);
   // ---- top-k cut: tk_key = value of the k-th token, need_k = how many of the tokens equal to it are inside
-  unsigned tk_key = 0;     // finite values have keys above 0x007fffff: 0 keeps everything
+  unsigned tk_key = 0;
   int need_k = 0x7fffffff;
   const bool cut_k = k_lim > 0 && k_lim < vocab;
   if (cut_k) {
-    tk_key = search_key<int>(lr, vocab, mask, 0u, order_key(mx), k_lim, [](float) { return 1; }, sums_i);
+    tk_key = search_key<int>(row, vocab, 0u, mk, k_lim, mx, temp, [](float) { return 1; },
+                             reinterpret_cast<SearchScratch<int>&>(sc));
     int above = 0;
-    for (int i = tid; i < vocab; i += LAW_T)
-      if (mask_ok(mask, i)) {
-        const float v = ldf<T>(lr, i);
-        above += v > -INFINITY && order_key(v) > tk_key;
-      }
+    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) { above += k > tk_key; });
     need_k = k_lim - block_sum_i(above, redi);
   }
   // mass above a key and number of tokens equal to it
@@ -302,16 +531,12 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   auto mass_above = [&](unsigned key) {
     m_above = 0.f;
     n_eq = 0;
-    if (tid < SUM_T) {
-#pragma unroll 8
-      for (int i = tid; i < vocab; i += SUM_T) {
-        const float v = ldf<T>(lr, i);
-        const bool live = v > -INFINITY && mask_ok(mask, i);
-        const unsigned k = order_key(v);
-        m_above += live && k > key ? __expf((v - mx) * inv_t) : 0.f;
-        n_eq += live && k == key;
-      }
-    }
+    if (tid < SUM_T)
+      scan(row, tid, vocab, SUM_T, [&](unsigned k, int) {
+        const float w = __expf((key_value(max(k, 0x00800000u)) - mx) * inv_t);    // (no branch around it)
+        m_above += k > key ? w : 0.f;
+        n_eq += k == key && k != 0u;
+      });
     m_above = sum_in_order(m_above, red);
     n_eq = block_sum_i(n_eq, redi);
   };
@@ -324,8 +549,8 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   if (p_lim < 1.f) {
     const float want = p_lim * kept;
     // mass(key >= tk_key) = kept >= want, and every token above tk_key is inside the cut
-    const unsigned lo = search_key<float>(lr, vocab, mask, tk_key, order_key(mx), want,
-                                          [&](float v) { return __expf((v - mx) * inv_t); }, sums_f);
+    const unsigned lo = search_key<float>(row, vocab, tk_key, mk, want, mx, temp,
+                                          [&](float v) { return __expf((v - mx) * inv_t); }, sc);
     if (lo != tk_key || !cut_k) {
       t_key = lo;
       mass_above(t_key);
@@ -340,26 +565,19 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   float w_probe = 0.f, w_ex = 0.f;
   for (int pass = 0; pass < 2; ++pass) {
     const int tok = pass == 0 ? probe : exclude;
-    if (tok < 0 || tok >= vocab || !mask_ok(mask, tok)) continue;
+    if (tok < 0 || tok >= vocab) continue;
     if (pass == 1 && exclude == probe) {
       w_ex = w_probe;
       continue;
     }
-    const float v = ldf<T>(lr, tok);
+    const unsigned k = row(tok);
     float w = 0.f;
-    if (v > -INFINITY) {
-      const unsigned k = order_key(v);
-      if (k > t_key) w = __expf((v - mx) * inv_t);
-      else if (k == t_key) {
-        int before = 0;
-        for (int i = tid; i < tok; i += LAW_T)
-          if (mask_ok(mask, i)) {
-            const float o = ldf<T>(lr, i);
-            before += o > -INFINITY && order_key(o) == t_key;
-          }
-        before = block_sum_i(before, redi);
-        if (before < need_eq) w = w_t;
-      }
+    if (k > t_key) w = __expf((key_value(k) - mx) * inv_t);
+    else if (k == t_key && k != 0u) {
+      int before = 0;
+      scan(row, tid, tok, LAW_T, [&](unsigned k2, int) { before += k2 == t_key; });
+      before = block_sum_i(before, redi);
+      if (before < need_eq) w = w_t;
     }
     if (pass == 0) w_probe = w;
     else w_ex = w;
@@ -373,79 +591,73 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   // ---- draw: mass and number of threshold tokens per chunk, the chunk the draw falls into, then the token in it; all sums in
   // index order
   const int per = (vocab + CHUNKS - 1) / CHUNKS;
+  const int ex_chunk = exclude >= 0 ? exclude / per : -1;
+  float mine = 0.f;
+  int my_eq = 0, eq_before = 0;
   if (tid < CHUNKS) {
-    float mine = 0.f;
-    int my_eq = 0;
-    const int hi_i = min(vocab, (tid + 1) * per);
-#pragma unroll 8
-    for (int i = tid * per; i < hi_i; ++i) {
-      const float v = ldf<T>(lr, i);
-      const bool live = v > -INFINITY && mask_ok(mask, i);
-      const unsigned k = order_key(v);
-      mine += live && k > t_key ? __expf((v - mx) * inv_t) : 0.f;
-      my_eq += live && k == t_key;
+    scan(row, tid * per, min(vocab, (tid + 1) * per), 1, [&](unsigned k, int) {
+      const float w = __expf((key_value(max(k, 0x00800000u)) - mx) * inv_t);
+      mine += k > t_key ? w : 0.f;
+      my_eq += k == t_key && k != 0u;
+    });
+    eq_before = my_eq;                      // running count over the chunks: whole numbers, any order
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, eq_before, o);
+      if ((tid & 31) >= o) eq_before += v;
     }
-    csum[tid] = mine;
-    ceq[tid] = my_eq;
+    if ((tid & 31) == 31) ceq_warp[tid >> 5] = eq_before;
+    eq_before -= my_eq;
+  }
+  __syncthreads();
+  if (tid < CHUNKS) {
+    for (int w = 0; w < (tid >> 5); ++w) eq_before += ceq_warp[w];
+    const int take = max(0, min(my_eq, need_eq - eq_before));
+    float w = mine + take * w_t;
+    if (tid == ex_chunk) w = fmaxf(w - w_ex, 0.f);
+    cweight[tid] = w;
+    ceq[tid] = eq_before;
   }
   __syncthreads();
   const float u = u01 * kept_draw;
-  const int ex_chunk = exclude >= 0 ? exclude / per : -1;
-  if (tid == 0) {
-    float acc = 0.f;
-    int eq_seen = 0, pick = -1, last = 0;
-    float base = 0.f;
-    int eq_base = 0;
-    for (int t = 0; t < CHUNKS; ++t) {
-      const int take = max(0, min(ceq[t], need_eq - eq_seen));
-      float w = csum[t] + take * w_t;
-      if (t == ex_chunk) w = fmaxf(w - w_ex, 0.f);
-      if (w > 0.f) last = t;
-      if (pick < 0 && u < acc + w) {
-        pick = t;
-        base = acc;
-        eq_base = eq_seen;
+  if (tid < 32) {        // one warp adds 32 chunks, then 32 tokens of the chunk, at a time and in order
+    float acc = 0.f, base = -1.f, after = 0.f;
+    int pick = -1, last = 0;
+    for (int t = 0; t < CHUNKS && pick < 0; t += 32) {
+      const float w = cweight[t + tid], before = acc;
+      acc = sum_lanes(acc, w, tid, after);
+      const unsigned kept_mask = __ballot_sync(0xffffffffu, w > 0.f), hit = __ballot_sync(0xffffffffu, u < after);
+      if (kept_mask) last = t + 31 - __clz(kept_mask);
+      if (hit) {
+        const int at = __ffs(hit) - 1;
+        pick = t + at;
+        base = at == 0 ? before : __shfl_sync(0xffffffffu, after, at - 1);
       }
-      acc += w;
-      eq_seen += ceq[t];
     }
-    if (pick < 0) {   // rounding: u landed past the last kept token
-      pick = last;
-      base = -1.f;
-    }
-    s_pick = pick;
-    s_base = base;
-    s_eq_base = eq_base;
-  }
-  __syncthreads();
-  if (tid < 32) {        // one warp loads 32 tokens at a time and adds them up in order
-    float acc = s_base;
-    int eq_seen = s_eq_base, chosen = -1, last_kept = -1;
+    if (pick < 0) pick = last;             // rounding: u landed past the last kept token (base stays -1)
+    acc = base;
+    int eq_seen = ceq[pick], chosen = -1, last_kept = -1;
     float w_chosen = 0.f, w_last = 0.f;
-    const int hi_i = min(vocab, (s_pick + 1) * per);
-    for (int i0 = s_pick * per; i0 < hi_i && chosen < 0; i0 += 32) {
+    const int hi_i = min(vocab, (pick + 1) * per);
+    for (int i0 = pick * per; i0 < hi_i && chosen < 0; i0 += 32) {
       const int i = i0 + tid;
-      float v = -INFINITY;
-      if (i < hi_i && mask_ok(mask, i)) v = ldf<T>(lr, i);
-      const bool live = v > -INFINITY;
-      const unsigned k = order_key(v);
-      const unsigned equal = __ballot_sync(0xffffffffu, live && k == t_key);
+      const unsigned k = i < hi_i ? row(i) : 0u;
+      const unsigned equal = __ballot_sync(0xffffffffu, k == t_key && k != 0u);
       float w = 0.f;
-      if (live && k > t_key) w = __expf((v - mx) * inv_t);
-      else if (live && k == t_key && eq_seen + __popc(equal & ((1u << tid) - 1u)) < need_eq) w = w_t;
-      if (i == exclude) w = 0.f;
+      if (k > t_key) w = __expf((key_value(k) - mx) * inv_t);
+      else if (k == t_key && k != 0u && eq_seen + __popc(equal & ((1u << tid) - 1u)) < need_eq) w = w_t;
+      if (i == exclude || !(w > 0.f)) w = 0.f;
       eq_seen += __popc(equal);
-      for (unsigned left = __ballot_sync(0xffffffffu, w > 0.f); left != 0u; left &= left - 1u) {
-        const int src = __ffs(left) - 1;
-        const float ws = __shfl_sync(0xffffffffu, w, src);
-        last_kept = i0 + src;
-        w_last = ws;
-        if (s_base >= 0.f && u < acc + ws) {
-          chosen = last_kept;
-          w_chosen = ws;
-          break;
-        }
-        acc += ws;
+      acc = sum_lanes(acc, w, tid, after);                 // (a dropped token's zero changes nothing)
+      const unsigned kept_mask = __ballot_sync(0xffffffffu, w > 0.f);
+      const unsigned hit = __ballot_sync(0xffffffffu, w > 0.f && base >= 0.f && u < after);
+      if (kept_mask == 0u) continue;
+      const int at = hit ? __ffs(hit) - 1 : 31 - __clz(kept_mask);
+      last_kept = i0 + at;
+      w_last = __shfl_sync(0xffffffffu, w, at);
+      if (hit) {
+        chosen = last_kept;
+        w_chosen = w_last;
       }
     }
     if (chosen < 0) {
@@ -460,17 +672,71 @@ __device__ void law_row(const T* __restrict__ lr, int vocab, const int* __restri
   __syncthreads();
 }
 
-template <typename T>
-__device__ void sample_full_row(const T* __restrict__ lr, int vocab, const int* __restrict__ mask, float temp,
-                                int k_lim, float p_lim, float u01, long long* out, float* out_prob) {
-  law_row<T>(lr, vocab, mask, temp, k_lim, p_lim, u01, -1, -1, out, out_prob, nullptr);
-}
-
 constexpr int SAMPLE_K = 64;  // candidates kept per row for 1 <= top-k <= 64 (top-p is applied inside them)
 
-// One CTA per row. Keeps the SAMPLE_K largest logits by repeated threshold passes (vocab is read a few times from
-// L2), then softmax / top-p / inverse-CDF draw on the candidates. temperature <= 0 means greedy.
-template <typename T>
+// The k first tokens of a row in (value desc, index asc) order, 0.0 and -0.0 equal: value and index to cv, ci. False, and nothing
+// written, when the row has fewer. Whole CTA.
+template <typename T, bool STAGED>
+__device__ bool list_candidates(const T* lr, int vocab, const int* mask, int k, float temp, float* cv, int* ci,
+                                SearchScratch<float>& sc) {
+  extern __shared__ unsigned row_keys[];
+  __shared__ unsigned redu[LAW_WARPS], gk[SAMPLE_K];
+  __shared__ int gi[SAMPLE_K], ei[SAMPLE_K], n_above, n_equal;
+  const int tid = threadIdx.x;
+  const RowKeys<T, STAGED, true> row{lr, mask, row_keys};
+  const unsigned mk = stage_row(row, STAGED, row_keys, vocab, redu);
+  const unsigned tk = search_key<int>(row, vocab, 0u, mk, k, key_value(mk), temp, [](float) { return 1; },
+                                      reinterpret_cast<SearchScratch<int>&>(sc));
+  if (tk <= 0x007fffffu) return false;
+  if (tid == 0) n_above = n_equal = 0;
+  __syncthreads();
+  scan(row, tid, vocab, LAW_T, [&](unsigned x, int i) {
+    if (x > tk) {
+      const int at = atomicAdd(&n_above, 1);               // fewer than k of them
+      gk[at] = x;
+      gi[at] = i;
+    } else if (x == tk) {
+      const int at = atomicAdd(&n_equal, 1);
+      if (at < SAMPLE_K) ei[at] = i;
+    }
+  });
+  __syncthreads();
+  const int above = n_above, equal = n_equal;
+  if (tid < above) {
+    int rank = 0;
+    for (int j = 0; j < above; ++j) rank += gk[j] > gk[tid] || (gk[j] == gk[tid] && gi[j] < gi[tid]);
+    cv[rank] = key_value(gk[tid]);
+    ci[rank] = gi[tid];
+  }
+  if (equal <= SAMPLE_K) {
+    if (tid < equal) {
+      int rank = above;
+      for (int j = 0; j < equal; ++j) rank += ei[j] < ei[tid];
+      if (rank < k) {
+        cv[rank] = key_value(tk);
+        ci[rank] = ei[tid];
+      }
+    }
+  } else {                                                 // many: in index order, a warp at a time
+    if (tid < 32)
+      for (int i0 = 0, got = above; i0 < vocab && got < k; i0 += 32) {
+        const bool is = i0 + tid < vocab && row(i0 + tid) == tk;
+        const unsigned m = __ballot_sync(0xffffffffu, is);
+        const int rank = got + __popc(m & ((1u << tid) - 1u));
+        if (is && rank < k) {
+          cv[rank] = key_value(tk);
+          ci[rank] = i0 + tid;
+        }
+        got += __popc(m);
+      }
+  }
+  __syncthreads();
+  return true;
+}
+
+// One CTA per row. Lists the k <= SAMPLE_K largest logits, then softmax / top-p / inverse-CDF draw on the candidates; k off or
+// above: the law of the whole row. temperature <= 0 means greedy.
+template <typename T, bool STAGED>
 __global__ void __launch_bounds__(LAW_T)
 sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
@@ -485,6 +751,7 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
   __shared__ int wi[LAW_WARPS];
   __shared__ float s_prev_v;
   __shared__ int s_prev_i;
+  __shared__ SearchScratch<float> sc;
   const int row = blockIdx.x;
   const T* lr = logits + row * ld;
   const int* mask = bitmask ? bitmask + static_cast<long long>(row) * mask_words : nullptr;
@@ -494,19 +761,22 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
   if (temp > 0.f && (k <= 0 || k > SAMPLE_K)) {
     // top-k off (the API default) or wider than the candidate list: the law is the softmax over the whole
     // vocabulary (then top-p), not over the SAMPLE_K largest logits
-    sample_full_row<T>(lr, vocab, mask, temp, k > SAMPLE_K ? k : 0, top_p ? top_p[row] : 1.f,
-                       uniform01(seeds ? seeds[row] : 0ull, offsets ? offsets[row] : 0ull), out + row,
-                       out_prob ? out_prob + row : nullptr);
+    law_row<T, STAGED>(lr, vocab, mask, temp, k > SAMPLE_K ? k : 0, top_p ? top_p[row] : 1.f,
+                       uniform01(seeds ? seeds[row] : 0ull, offsets ? offsets[row] : 0ull), -1, -1, out + row,
+                       out_prob ? out_prob + row : nullptr, nullptr, sc);
     return;
   }
   if (temp <= 0.f) k = 1;
+  // From four candidates on by the key of the k-th one (a search and a list against k passes over the row; 50 of
+  // 18992 169 -> 29 us, of 151936 1772 -> 126). Fewer live tokens than candidates: the passes.
+  const bool listed = k > 3 && list_candidates<T, STAGED>(lr, vocab, mask, k, temp, cv, ci, sc);
   if (threadIdx.x == 0) {
     s_prev_v = INFINITY;
     s_prev_i = -1;
   }
   __syncthreads();
   // Selection by successive maxima in (value desc, index asc) order: exact and deterministic.
-  for (int c = 0; c < k; ++c) {
+  for (int c = listed ? k : 0; c < k; ++c) {
     const float pv = s_prev_v;
     const int pi = s_prev_i;
     float best = -INFINITY;
@@ -645,7 +915,7 @@ __global__ void lattice_walk_kernel(const long long* __restrict__ cand, const fl
 // then yields the emitted tokens, so sampled and greedy rounds share one accept path (greedy requests, temp <= 0,
 // fall out of the same rule: their law is the one-hot argmax). Uniforms are counter draws at (seed, 2 * (draws + j)
 // + 1) for the test and + 2 for the draw.
-template <typename T>
+template <typename T, bool STAGED>
 __global__ void __launch_bounds__(LAW_T)
 spec_targets_kernel(const T* __restrict__ logits, long long ld, int vocab, int k, const long long* __restrict__ drafts,
                     const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -655,6 +925,7 @@ spec_targets_kernel(const T* __restrict__ logits, long long ld, int vocab, int k
                     long long* __restrict__ target, float* __restrict__ p_draft) {
   __shared__ long long s_tok;
   __shared__ float s_probe;
+  __shared__ SearchScratch<float> sc;
   const int row = blockIdx.x, b = row / (k + 1), j = row - b * (k + 1);
   const T* lr = logits + row * ld;
   const int* mask = bitmask ? bitmask + static_cast<long long>(row) * mask_words : nullptr;
@@ -675,8 +946,8 @@ spec_targets_kernel(const T* __restrict__ logits, long long ld, int vocab, int k
   }
   const unsigned long long seed = seeds ? seeds[b] : 0ull, base = draws ? draws[b] : 0ull;
   const int d = j < k ? static_cast<int>(drafts[static_cast<long long>(b) * k + j]) : -1;
-  law_row<T>(lr, vocab, mask, temp, k_lim, p_lim, uniform01(seed, 2 * (base + j) + 2), d, d, &s_tok, nullptr,
-             &s_probe);
+  law_row<T, STAGED>(lr, vocab, mask, temp, k_lim, p_lim, uniform01(seed, 2 * (base + j) + 2), d, d, &s_tok, nullptr,
+                     &s_probe, sc);
   if (threadIdx.x == 0) {
     long long tok = s_tok;
     if (j < k) {
@@ -756,6 +1027,14 @@ rank_gap_kernel(const T* __restrict__ logits, long long ld, int vocab, const lon
   }
 }
 
+// Rows of up to 52224 tokens (204 KB of keys beside 15 KB of scratch) are staged.
+inline size_t staged_bytes(int vocab) { return vocab <= 52224 ? static_cast<size_t>(vocab) * sizeof(unsigned) : 0; }
+template <typename K>
+bool row_kernel(K kern, size_t smem) {
+  return smem <= 32 * 1024 ||
+         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess;
+}
+
 }  // namespace
 }  // namespace hb
 
@@ -788,10 +1067,17 @@ int hb_sample(const void* logits, long long ld, int rows, int vocab, int is_f32,
       static_cast<const float*>(top_p), static_cast<const unsigned long long*>(seeds),                     \
       static_cast<const unsigned long long*>(offsets), static_cast<const int*>(bitmask), mask_words,       \
       static_cast<long long*>(out), static_cast<float*>(out_prob), skip_greedy
-  if (is_f32) launch_dep(sample_kernel<float>, dim3(rows), dim3(LAW_T), 0, st, static_cast<const float*>(logits), HB_SAMPLE_ARGS);
-  else launch_dep(sample_kernel<__nv_bfloat16>, dim3(rows), dim3(LAW_T), 0, st, static_cast<const __nv_bfloat16*>(logits), HB_SAMPLE_ARGS);
+  const size_t smem = staged_bytes(vocab);
+  auto go = [&](auto kern, auto* p) {
+    return row_kernel(kern, smem) &&
+           launch_dep(kern, dim3(rows), dim3(LAW_T), smem, st, p, HB_SAMPLE_ARGS) == cudaSuccess;
+  };
+  const float* lf = static_cast<const float*>(logits);
+  const __nv_bfloat16* lb = static_cast<const __nv_bfloat16*>(logits);
+  const bool ok = smem ? (is_f32 ? go(sample_kernel<float, true>, lf) : go(sample_kernel<__nv_bfloat16, true>, lb))
+                       : (is_f32 ? go(sample_kernel<float, false>, lf) : go(sample_kernel<__nv_bfloat16, false>, lb));
 #undef HB_SAMPLE_ARGS
-  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  return cudaGetLastError() == cudaSuccess && ok ? 0 : 2;
 }
 
 int hb_lattice_walk(const void* cand, const void* scores, const void* temperature, const void* uniforms, int batch,
@@ -819,11 +1105,18 @@ int hb_spec_targets(const void* logits, long long ld, int batch, int k, int voca
       static_cast<const unsigned long long*>(seeds), static_cast<const unsigned long long*>(draws),           \
       static_cast<const float*>(soft), static_cast<const int*>(bitmask), mask_words,                          \
       static_cast<const long long*>(greedy_pick), static_cast<long long*>(target), static_cast<float*>(p_draft)
-  if (is_f32) spec_targets_kernel<float><<<rows, LAW_T, 0, st>>>(static_cast<const float*>(logits), HB_SPEC_ARGS);
-  else
-    spec_targets_kernel<__nv_bfloat16><<<rows, LAW_T, 0, st>>>(static_cast<const __nv_bfloat16*>(logits), HB_SPEC_ARGS);
+  const size_t smem = staged_bytes(vocab);
+  auto go = [&](auto kern, auto* p) {
+    if (!row_kernel(kern, smem)) return false;
+    kern<<<rows, LAW_T, smem, st>>>(p, HB_SPEC_ARGS);
+    return true;
+  };
+  const float* lf = static_cast<const float*>(logits);
+  const __nv_bfloat16* lb = static_cast<const __nv_bfloat16*>(logits);
+  const bool ok = smem ? (is_f32 ? go(spec_targets_kernel<float, true>, lf) : go(spec_targets_kernel<__nv_bfloat16, true>, lb))
+                       : (is_f32 ? go(spec_targets_kernel<float, false>, lf) : go(spec_targets_kernel<__nv_bfloat16, false>, lb));
 #undef HB_SPEC_ARGS
-  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  return cudaGetLastError() == cudaSuccess && ok ? 0 : 2;
 }
 
 int hb_accept_greedy(const void* target, const void* drafts, const void* stop_ids, int n_stop, const void* budget,

@@ -1,0 +1,91 @@
+"""Full-vocabulary and listed-candidate sampling at the edges of the row kernel: one warp of tokens, the longest row staged in
+shared memory and the first that is not, more equal tokens than the ranking list holds, candidate counts around the listed form."""
+import pytest
+import torch
+
+from hibana_b200.engine.rejection import distribution
+from hibana_b200.ops import sampling
+
+ROWS = 12
+
+
+def _rows(kind: str, vocab: int) -> torch.Tensor:
+    g = torch.Generator().manual_seed(vocab)
+    x = torch.randn(ROWS, vocab, generator=g)
+    if kind == "plain":
+        return x * 2
+    if kind == "ties":                     # a few distinct values, zeros of both signs: thousands of equal tokens at every cut
+        return (x * 2).round() / 2
+    x = x * 3
+    x[:, ::3] = float("-inf")
+    x[:, 1::7] = float("nan")
+    return x
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [33, 4096, 52224, 52225])
+@pytest.mark.parametrize("kind", ["plain", "ties", "holes"])
+@pytest.mark.parametrize("top_k,top_p", [(0, 0.95), (0, 0.3), (65, 0.9), (3, 1.0), (4, 0.9), (64, 0.95)])
+def test_row_kernel_draws_from_the_law(vocab, kind, top_k, top_p):
+    x = _rows(kind, vocab)
+    masked = kind == "holes"
+    mask = None
+    if masked:
+        g = torch.Generator().manual_seed(1)
+        mask = torch.randint(-2 ** 31, 2 ** 31 - 1, (ROWS, (vocab + 31) // 32), generator=g).to(torch.int32)
+    temp = torch.tensor([0.8, 1.0, 0.3, 2.0] * 3)
+    full = lambda v, dt: torch.full((ROWS,), v, dtype=dt)
+    seeds, offs = torch.arange(ROWS) * 7919 + 5, torch.arange(ROWS) + 3
+    dev = [t.cuda() for t in (x, temp, full(top_k, torch.int32), full(top_p, torch.float32), seeds, offs)]
+    got = sampling.sample(*dev, mask.cuda() if masked else None).cpu()
+    for r in range(ROWS):
+        lg = x[r].double()
+        allowed = ~lg.isnan()
+        if masked:
+            allowed &= ((mask[r][torch.arange(vocab) // 32] >> (torch.arange(vocab) % 32)) & 1).bool()
+        lg[~allowed] = float("-inf")
+        if 1 <= top_k <= 64:               # candidates in (value desc, index asc) order
+            order = torch.sort(lg, descending=True, stable=True).indices[:top_k]
+            w = torch.exp((lg[order] - lg[order[0]]) / float(temp[r]))
+        else:
+            order = torch.arange(vocab)
+            w = distribution(lg[None].float(), float(temp[r]), top_k, 1.0)[0].double()
+        w = w / w.sum()
+        if top_p < 1:                      # smallest prefix in value order that reaches top_p
+            by = torch.sort(lg[order], descending=True, stable=True).indices
+            cum = torch.cumsum(w[by], 0)
+            cut = int((cum >= top_p).nonzero()[0]) + 1
+            drop = by[cut:]
+            edge = float(w[by[cut - 1]])
+            w[drop] = 0
+        else:
+            edge = 0.0
+        kept = float(w.sum())
+        u = sampling.uniform01(int(seeds[r]), int(offs[r])) * kept
+        at = int((order == got[r]).nonzero()[0])
+        after = float(w[:at + 1].sum())
+        before = after - float(w[at])
+        # fp32 sums of at most ceil(52225 / 256) + 256 + 13 terms, one after the other: 473 * 2^-24 < 3e-5 of the mass, and as much
+        # again for the cut; a cut moved by that rounding moves the mass by the token at the edge where sums tie
+        tol = 6e-5 + (edge if edge < 6e-5 else 0.0)
+        assert before - tol <= u <= after + tol, (r, u, before, after)
+
+
+@pytest.mark.gpu
+def test_speculative_targets_on_staged_and_long_rows_agree():
+    """The same law over a staged row and over one padded with forbidden tokens past the staging limit."""
+    vocab, longer, b, k = 5000, 52300, 4, 2
+    g = torch.Generator().manual_seed(2)
+    x = torch.randn(b * (k + 1), vocab, generator=g).cuda() * 2
+    pad = torch.full((b * (k + 1), longer), float("-inf"), device="cuda")
+    pad[:, :vocab] = x
+    drafts = x.argmax(1).view(b, k + 1)[:, :k].contiguous()
+    drafts[0] = 17
+    t = lambda v, dt: torch.full((b,), v, dtype=dt, device="cuda")
+    args = (t(0.8, torch.float32), t(0, torch.int32), t(0.9, torch.float32), torch.arange(b, device="cuda") + 9,
+            torch.arange(b, device="cuda"))
+    a, pa = sampling.spec_targets(x, drafts, *args)
+    c, pc = sampling.spec_targets(pad, drafts, *args)
+    # other strides of the sums (the draw's chunks are 1/256 of the row): 473 * 2^-24 of the mass
+    assert torch.allclose(pa, pc, atol=6e-5, rtol=0)
+    assert (a == c).float().mean() > 0.8 and bool((a < vocab).all() and (c < vocab).all())
