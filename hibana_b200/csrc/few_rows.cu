@@ -27,17 +27,19 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NB = blocks of 8 rows of x.
-template <int NB, int WARPS, int DEPTH>
+// NB = blocks of 8 rows of x. SPLIT CTAs (a cluster) share a block of features, each with its turns of K; the first adds their sums up.
+template <int NB, int WARPS, int DEPTH, int SPLIT = 1>
 __global__ void __launch_bounds__(WARPS * 32)
 few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __restrict__ w, long long ldw, int m, int n, int k,
                 void* out, long long ldo, int f32) {
   __shared__ float red[WARPS][8 * NB][FEATS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g4 = lane >> 2, t4 = lane & 3;
-  const int f0 = blockIdx.x * FEATS;
-  const int kl = (warp * 4 + t4) * 8;                       // this lane's first element of its warp's first step
-  constexpr int STRIDE = WARPS * 32;                        // elements between two steps of a warp
-  const int steps = k > warp * 32 ? (k - warp * 32 + STRIDE - 1) / STRIDE : 0;
+  __shared__ float parts[SPLIT][SPLIT > 1 ? 8 * NB * FEATS : 1];     // of the first CTA: the sums of each
+  const int part = SPLIT > 1 ? blockIdx.x % SPLIT : 0, turn = part * WARPS + warp;
+  const int f0 = blockIdx.x / SPLIT * FEATS;
+  const int kl = (turn * 4 + t4) * 8;                       // this lane's first element of its warp's first step
+  constexpr int STRIDE = SPLIT * WARPS * 32;                // elements between two steps of a warp
+  const int steps = k > turn * 32 ? (k - turn * 32 + STRIDE - 1) / STRIDE : 0;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   auto weights = [&](int i, int half) -> uint4 {
     const int f = f0 + g4 + 8 * half, kk = kl + i * STRIDE;
@@ -49,6 +51,7 @@ few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __re
   };
   uint4 a[DEPTH][2], b[DEPTH][NB];
   grid_dep_launch();
+  if (SPLIT > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // (its shared memory may be written)
 #pragma unroll
   for (int i = 0; i < DEPTH; ++i) {
     a[i][0] = weights(i, 0);
@@ -84,14 +87,34 @@ few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __re
 #pragma unroll
     for (int e = 0; e < 4; ++e) red[warp][q * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = acc[q][e];
   __syncthreads();
-  for (int i = threadIdx.x; i < m * FEATS; i += WARPS * 32) {
-    const int t = i / FEATS, f = i % FEATS;
-    if (f0 + f >= n) continue;
+  auto sum = [&](int i) {
     float s = 0.f;
 #pragma unroll
-    for (int j = 0; j < WARPS; ++j) s += red[j][t][f];
-    if (f32) static_cast<float*>(out)[t * ldo + f0 + f] = s;
-    else static_cast<__nv_bfloat16*>(out)[t * ldo + f0 + f] = __float2bfloat16(s);
+    for (int j = 0; j < WARPS; ++j) s += red[j][i / FEATS][i % FEATS];
+    return s;
+  };
+  auto store = [&](int i, float s) {
+    const int t = i / FEATS, f = f0 + i % FEATS;
+    if (f >= n) return;
+    if (f32) static_cast<float*>(out)[t * ldo + f] = s;
+    else static_cast<__nv_bfloat16*>(out)[t * ldo + f] = __float2bfloat16(s);
+  };
+  if constexpr (SPLIT == 1) {
+    for (int i = threadIdx.x; i < m * FEATS; i += WARPS * 32) store(i, sum(i));
+  } else {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < m * FEATS; i += WARPS * 32) {
+      const float s = sum(i);
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(smem_u32(&parts[part][i]), 0)), "f"(s) : "memory");
+    }
+    cluster_sync_all();
+    if (part == 0)
+      for (int i = threadIdx.x; i < m * FEATS; i += WARPS * 32) {
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < SPLIT; ++j) s += parts[j][i];
+        store(i, s);
+      }
   }
 }
 
@@ -112,13 +135,18 @@ int hb_few_rows_bf16(const void* x, long long ldx, const void* w, long long ldw,
   // eight warps, several CTAs to an SM. A matrix of a megabyte runs beside a larger projection on a parallel branch: four warps
   // (13K registers) fit next to its two CTAs of 192 threads, sixteen would wait until that projection has left the SM, which put
   // 11 us a layer on the critical path of the delta rule's gates.
+  // From 2048 elements of K on eight CTAs share a block of features, all of K in flight at once: beside the projection, which
+  // keeps the memory busy, each round of loads takes 3 us, and the gates of 4 rows (96 x 5120) left 5 us after the convolution.
   const int ctas = (n + FEATS - 1) / FEATS;
-  auto kern = static_cast<long long>(n) * k <= (1 << 19) ? (m <= 8 ? few_rows_kernel<1, 4, 8> : few_rows_kernel<2, 4, 4>)
+  const bool small = static_cast<long long>(n) * k <= (1 << 19);
+  const int split = small && k >= 2048 ? 8 : 1;
+  auto kern = split > 1 ? (m <= 8 ? few_rows_kernel<1, 4, 8, 8> : few_rows_kernel<2, 4, 4, 8>)
+              : small ? (m <= 8 ? few_rows_kernel<1, 4, 8> : few_rows_kernel<2, 4, 4>)
               : m <= 8 ? (ctas <= 148 && k > 1024 ? few_rows_kernel<1, 16, 8> : few_rows_kernel<1, 8, 8>)
                        : (k > 1024 ? few_rows_kernel<2, 8, 8> : few_rows_kernel<2, 8, 4>);
-  const int warps = static_cast<long long>(n) * k <= (1 << 19) ? 4 : m <= 8 && ctas <= 148 && k > 1024 ? 16 : 8;
-  launch_dep(kern, dim3(ctas), dim3(warps * 32), 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), ldx,
-             static_cast<const __nv_bfloat16*>(w), ldw, m, n, k, out, ldo, f32);
+  const int warps = small ? 4 : m <= 8 && ctas <= 148 && k > 1024 ? 16 : 8;
+  launch_dep_cluster(kern, dim3(ctas * split), dim3(warps * 32), split, 0, static_cast<cudaStream_t>(stream),
+                     static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w), ldw, m, n, k, out, ldo, f32);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -155,6 +155,7 @@ void hb_attn_decode_profile(void* buf);
 int hb_few_rows_bf16(const void* x, long long ldx, const void* w, long long ldw, int m, int n, int k, void* out, long long ldo,
                      int f32, void* stream);
 void hb_attn_decode_early(void);
+void hb_state_early(void);
 void hb_attn_decode_rope(const void* qkv, long long ld_qkv, const void* positions, const void* slots, const void* inv_freq,
                          float kv_inv_scale);
 int hb_attn_decode(const void* q, const void* k_pool, const void* v_pool, long long pool_stride,

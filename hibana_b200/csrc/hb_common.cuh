@@ -302,19 +302,30 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
 // the launch latency (0.4 us in a graph) and prologue of every kernel of a step pass behind its predecessor.
 extern "C" int hb_gemm_get_pdl(void);
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args&&... args) {
+inline cudaError_t launch_dep_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st,
+                                      Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
   cfg.attrs = at;
-  cfg.numAttrs = hb_gemm_get_pdl() >= 2 ? 1 : 0;     // level 1: GEMMs only; level 2: these kernels as well
+  if (hb_gemm_get_pdl() >= 2) {     // level 1: GEMMs only; level 2: these kernels as well
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = cluster;
+    at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  return launch_dep_cluster(kern, grid, block, 1, smem, st, static_cast<Args&&>(args)...);
 }
 
 // ---------------------------------------------------------------- tcgen05 / TMEM

@@ -422,8 +422,8 @@ __global__ void act_mul_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 __global__ void gdn_gates_kernel(const __nv_bfloat16* __restrict__ ba, long long ld, const float* __restrict__ a_log,
                                  const float* __restrict__ dt_bias, int rows, int heads, float* __restrict__ beta,
                                  float* __restrict__ g) {
-  grid_dep_wait(ba);
   grid_dep_launch();
+  grid_dep_wait(ba);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * heads) return;
   const int r = i / heads, hd = i - r * heads;

@@ -211,7 +211,7 @@ class MambaLayer:
             ctx.extras["ring"].append((self, (xbc, dt)))
         xbc = recurrent.conv1d(xbc, self.conv_w, self.conv_b, states.conv[li], ctx.state_slots, so,
                                q_indptr=ctx.q_indptr, has_init=ctx.has_initial_state, silu=True,
-                               max_rows=ctx.max_rows if ctx.q_indptr is not None else 0)
+                               max_rows=ctx.max_rows if ctx.q_indptr is not None else 0, state_ready=ctx.mode == DECODE)
         if getattr(states, "window", 0):
             y = self._scan_window(xbc, dt, states, ctx.state_slots, ctx.q_indptr, ctx.has_initial_state,
                                   ctx.seq_starts_host, commit="state_out" not in ctx.extras)
@@ -222,7 +222,7 @@ class MambaLayer:
                                       d_state=t.mamba_state, q_indptr=ctx.q_indptr, has_init=ctx.has_initial_state,
                                       state_scale=states.ssm_scale[li] if getattr(states, "ssm_scale", None) is not None
                                       else None, sr_seed=ctx.extras.get("sr_seed", 0), host_rows=ctx.seq_starts_host,
-                                      host_slots=ctx.state_slots_host)
+                                      host_slots=ctx.state_slots_host, state_ready=ctx.mode == DECODE)
         if self.out_proj.fmt == "nvfp4" and not self.out_proj.calibrating and not self.out_proj.takes_w3(y.shape[0]):
             # the gated norm writes the output projection's NVFP4 input itself
             return self.out_proj(basic.gated_rmsnorm_quant(y, z, self.norm_w, t.norm_eps, inner // t.mamba_groups,
@@ -318,7 +318,7 @@ class GdnLayer:
             ctx.extras["ring"].append((self, (qkvz[:, :2 * self.qk + self.vd], g, beta)))
         qkv = recurrent.conv1d(qkvz[:, :2 * self.qk + self.vd], self.conv_w, None, states.conv[li], ctx.state_slots,
                                so, q_indptr=ctx.q_indptr, has_init=ctx.has_initial_state, silu=True,
-                               max_rows=ctx.max_rows if ctx.q_indptr is not None else 0)
+                               max_rows=ctx.max_rows if ctx.q_indptr is not None else 0, state_ready=ctx.mode == DECODE)
         z = qkvz[:, 2 * self.qk + self.vd:]
         br.join(beta, g)
         if getattr(states, "window", 0):
@@ -329,7 +329,7 @@ class GdnLayer:
                                    states.ssm[li], ctx.state_slots, so, k_heads=t.gdn_k_heads, v_heads=t.gdn_v_heads,
                                    kdim=kd, vdim=kd, l2norm=True, q_indptr=ctx.q_indptr,
                                    has_init=ctx.has_initial_state, host_rows=ctx.seq_starts_host,
-                                   host_slots=ctx.state_slots_host)
+                                   host_slots=ctx.state_slots_host, state_ready=ctx.mode == DECODE)
         rows = o.shape[0]
         # per-head RMSNorm of the output, then the SiLU gate (norm before gate)
         key = (id(self.norm_w), self.norm_w._version)

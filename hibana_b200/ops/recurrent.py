@@ -17,6 +17,7 @@ import torch.nn.functional as F
 from .. import _native as nv
 
 P, I, L, Fl = nv.P, nv.I, nv.L, nv.F
+nv.register("hb_state_early", [], void=True)
 nv.register("hb_conv1d", [P, L, P, P, P, L, P, L, P, P, P, P, I, I, I, I, I, P])
 nv.register("hb_mamba2_scan", [P, P, P, P, L, L, L, P, P, P, P, L, P, L, P, P, P, P, I, I, I, I, I, P])
 nv.register("hb_mamba2_scan_fmt", [P, P, P, P, L, L, L, P, P, P, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, ctypes.c_uint, P])
@@ -35,14 +36,19 @@ def _ranges(q_indptr, batch):
 
 def conv1d(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], state: torch.Tensor,
            slot_in: torch.Tensor, slot_out: Optional[torch.Tensor], *, q_indptr: Optional[torch.Tensor] = None,
-           has_init: Optional[torch.Tensor] = None, silu: bool = True, max_rows: int = 0) -> torch.Tensor:
+           has_init: Optional[torch.Tensor] = None, silu: bool = True, max_rows: int = 0,
+           state_ready: bool = False) -> torch.Tensor:
     """x [T, C] bf16 (may be a column slice), weight [C, W], state [slots, C, W-1] bf16 (raw inputs). `max_rows`
-    (host bound on rows per sequence; 0 = unknown) lets prefill chunks run parallel over tiles of tokens."""
+    (host bound on rows per sequence; 0 = unknown) lets prefill chunks run parallel over tiles of tokens. `state_ready` (here and
+    in the scans): tables and states were complete before the forward began with its embedding gather (a decode step), so the
+    kernel fetches them while its predecessors still run."""
     t, c = x.shape
     w = weight.shape[1]
     batch = slot_in.shape[0]
     if nv.use_native(x):
         y = torch.empty(t, c, dtype=x.dtype, device=x.device)
+        if state_ready:
+            nv.lib().hb_state_early()
         nv.check(nv.lib().hb_conv1d(x.data_ptr(), x.stride(0), weight.data_ptr(), nv.ptr(bias), y.data_ptr(),
                                     y.stride(0), state.data_ptr(), state.stride(0), nv.ptr(q_indptr),
                                     slot_in.data_ptr(), nv.ptr(slot_out), nv.ptr(has_init), batch, c, w, int(silu),
@@ -70,7 +76,7 @@ def mamba2_scan(x: torch.Tensor, bmat: torch.Tensor, cmat: torch.Tensor, dt: tor
                 d_state: int, q_indptr: Optional[torch.Tensor] = None,
                 has_init: Optional[torch.Tensor] = None, state_scale: Optional[torch.Tensor] = None,
                 sr_seed: int = 0, host_rows: Optional[Sequence[int]] = None,
-                host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
+                host_slots: Optional[Sequence[int]] = None, state_ready: bool = False) -> torch.Tensor:
     """x [T, heads*P], bmat/cmat [T, groups*N], dt [T, heads] (bf16, column slices allowed);
     state [slots, heads, P, N] in fp32, fp16 (`sr_seed` != 0: stochastic rounding when the state is written back)
     or int8 with `state_scale` [slots, heads, P] fp32 row scales. Returns y [T, heads*P] bf16. `host_slots`: the numbers in
@@ -92,6 +98,8 @@ def mamba2_scan(x: torch.Tensor, bmat: torch.Tensor, cmat: torch.Tensor, dt: tor
                                         host_slots=host_slots)
     if nv.use_native(x):
         y = torch.empty(t, heads * head_dim, dtype=x.dtype, device=x.device)
+        if state_ready:
+            nv.lib().hb_state_early()
         nv.check(nv.lib().hb_mamba2_scan_fmt(
             x.data_ptr(), bmat.data_ptr(), cmat.data_ptr(), dt.data_ptr(), x.stride(0), bmat.stride(0), dt.stride(0),
             a_log.data_ptr(), nv.ptr(dt_bias), nv.ptr(dskip), y.data_ptr(), y.stride(0), state.data_ptr(),
@@ -141,7 +149,8 @@ def gdn_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
              state: torch.Tensor, slot_in: torch.Tensor, slot_out: Optional[torch.Tensor], *, k_heads: int,
              v_heads: int, kdim: int, vdim: int, scale: Optional[float] = None, l2norm: bool = True,
              q_indptr: Optional[torch.Tensor] = None, has_init: Optional[torch.Tensor] = None,
-             host_rows: Optional[Sequence[int]] = None, host_slots: Optional[Sequence[int]] = None) -> torch.Tensor:
+             host_rows: Optional[Sequence[int]] = None, host_slots: Optional[Sequence[int]] = None,
+             state_ready: bool = False) -> torch.Tensor:
     """Gated delta rule. q, k [T, k_heads*K] (same row pitch), v [T, v_heads*V] bf16; g (log decay), beta
     [T, v_heads] fp32 contiguous; state [slots, v_heads, V, K] fp32. Returns o [T, v_heads*V] bf16.
     `host_rows` (rows per sequence, known on the host during prefill) lets long sequences take the chunked form
@@ -162,6 +171,8 @@ def gdn_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor,
     if nv.use_native(q):
         assert q.stride(0) == k.stride(0) and g.is_contiguous() and beta.is_contiguous()
         o = torch.empty(t, v_heads * vdim, dtype=q.dtype, device=q.device)
+        if state_ready:
+            nv.lib().hb_state_early()
         nv.check(nv.lib().hb_gdn_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
                                       q.stride(0), v.stride(0), o.data_ptr(), o.stride(0), state.data_ptr(),
                                       state.stride(0), nv.ptr(q_indptr), slot_in.data_ptr(), nv.ptr(slot_out),

@@ -19,9 +19,9 @@ def test_few_rows_rule_cpu():
         assert not ok(1, 512, 4096)
 
 
-# n and k around the tiles (16 features, 32-element steps, turns of 4, 8 and 16 warps) and each of the kernel's forms
+# n and k around the tiles (16 features, 32-element steps, turns of 4, 8 and 16 warps, clusters of 8) and each of the kernel's forms
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,k", [(1, 8), (17, 72), (96, 5120), (50, 1000), (512, 4096), (520, 2056), (4096, 1024), (4100, 264),
+@pytest.mark.parametrize("n,k", [(1, 8), (17, 72), (16, 2048), (31, 2056), (96, 5120), (50, 1000), (512, 4096), (520, 2056), (4096, 1024), (4100, 264),
                                  (2368, 1032), (2384, 3304)])
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("f32", [True, False])
