@@ -133,7 +133,15 @@ gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     }
   }
 #pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  for (int o = (L < 32 ? L : 32) / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if constexpr (L > 32) {                  // (the CTA is one group)
+    __shared__ float part[L / 32];
+    if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = ss;
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < L / 32; ++i) ss += part[i];
+  }
   const float rstd = rsqrtf(ss / gs + eps);
   uint4* yr = reinterpret_cast<uint4*>(y + static_cast<long long>(row) * h + g * gs);
 #pragma unroll
@@ -483,15 +491,20 @@ int hb_rmsnorm(const void* x, void* residual, const void* w, void* y, int rows, 
 static int gated_rmsnorm_reg(const void* x, const void* z, const void* w, void* y, int rows, int h, int gs, long long ldx,
                              long long ldz, float eps, int norm_first, int sigmoid_gate, int gemma, void* q, void* sf,
                              const void* gscale, int ka, void* stream) {
-  const int nchunk = gs / 8, lanes = nchunk <= 8 ? 8 : nchunk <= 16 ? 16 : 32;
+  // Few groups: four warps on each, one chunk a lane, so that the chip is not one SM working through exponentials and divisions
+  // (behind one row's scan, 8 groups of 1024: 7.7 -> 3.5 us).
+  const int nchunk = gs / 8;
+  const bool few = nchunk > 32 && static_cast<long long>(rows) * (h / gs) <= 2 * 148;
+  const int lanes = nchunk <= 8 ? 8 : nchunk <= 16 ? 16 : few ? 128 : 32, block = few ? 128 : 256;
   const long long threads = static_cast<long long>(rows) * (h / gs) * lanes;
-  const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
+  const unsigned blocks = static_cast<unsigned>((threads + block - 1) / block);
 #define HB_GN(NC, L)                                                                                                      \
-  launch_dep(gated_rmsnorm_reg_kernel<NC, L>, dim3(blocks), dim3(256), 0, ST(stream),                                     \
+  launch_dep(gated_rmsnorm_reg_kernel<NC, L>, dim3(blocks), dim3(block), 0, ST(stream),                                   \
       BF(x), BF(z), BF(w), BFM(y), rows, h, gs, ldx, ldz, eps, norm_first, sigmoid_gate, gemma, static_cast<uint8_t*>(q), \
       static_cast<uint8_t*>(sf), static_cast<const float*>(gscale), ka)
   if (lanes == 8) HB_GN(1, 8);
   else if (lanes == 16) HB_GN(1, 16);
+  else if (few) HB_GN(1, 128);
   else if (nchunk <= 32) HB_GN(1, 32);
   else if (nchunk <= 64) HB_GN(2, 32);
   else if (nchunk <= 96) HB_GN(3, 32);
