@@ -491,7 +491,7 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, long long
 
 // out[t, :] = sum_k w[t, k] * y[pos[t, k], :] (+ shared[t, :]). VEC outputs a thread (8, 16-byte rows; else 2), one CTA per token and
 // 128 * VEC columns, eight experts' rows in flight. Bytes bound it at many tokens; at one it is a chain of loads: with 256 threads
-// walking all columns and one load at a time it took 6.1 us at 2048 columns and 22 experts, 4.2 so.
+// walking all columns and one load at a time it took 6.1 us at 1024 columns and 22 experts, 4.2 so.
 template <int VEC>
 __global__ void __launch_bounds__(128)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ y, long long ldy, const int* __restrict__ pos,

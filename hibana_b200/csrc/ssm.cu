@@ -124,6 +124,72 @@ __global__ void conv1d_tiled_kernel(const __nv_bfloat16* __restrict__ x, long lo
   }
 }
 
+// The same for two channels a thread (even channel count and pitches, 4-byte rows), eight rows in flight: issue bounds it (an exponential
+// and an IEEE division per element), so loads, stores and addresses are shared. 5000 rows of 10240
+// channels 130 -> 72 us, 1500 38 -> 30 (with the window kernel behind it).
+template <int W>
+__global__ void __launch_bounds__(128)
+conv1d_tiled2_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
+                     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y, long long ldy,
+                     __nv_bfloat16* __restrict__ state, long long state_stride, const int* __restrict__ q_indptr,
+                     const int* __restrict__ slot_in, const int* __restrict__ slot_out, const int* __restrict__ has_init,
+                     int channels, int act_silu) {
+  grid_dep_wait(x, state, q_indptr, slot_in, slot_out, has_init);
+  grid_dep_launch();
+  const int b = blockIdx.z;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
+  if (c >= channels) return;
+  if (!index_ok(slot_in[b], kBoundStateSlots, kKerConvState) ||
+      (slot_out != nullptr && !index_ok(slot_out[b], kBoundStateSlots, kKerConvState)))
+    return;   // reported; the sequence is skipped
+  const int r0 = q_indptr ? q_indptr[b] : b;
+  const int r1 = q_indptr ? q_indptr[b + 1] : b + 1;
+  const int t0 = r0 + blockIdx.y * CONV_TT;
+  if (t0 >= r1) return;
+  const int t1 = min(t0 + CONV_TT, r1);
+  const bool init = has_init == nullptr || has_init[b] != 0;
+  const __nv_bfloat16* sin = state + static_cast<long long>(slot_in[b]) * state_stride + static_cast<long long>(c) * (W - 1);
+  float win[2][W - 1], wt[2][W], bs[2];
+#pragma unroll
+  for (int j = 0; j < W - 1; ++j) {
+    const int t = t0 - (W - 1) + j;        // as above: rows before r0 live in the state
+    const uint32_t v = t >= r0 ? *reinterpret_cast<const uint32_t*>(x + t * ldx + c) : 0u;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      win[e][j] = t >= r0 ? (e ? bf16_hi(v) : bf16_lo(v)) : init ? __bfloat162float(sin[e * (W - 1) + j + (t0 - r0)]) : 0.f;
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) wt[e][j] = __bfloat162float(w[static_cast<long long>(c + e) * W + j]);
+    bs[e] = bias ? __bfloat162float(bias[c + e]) : 0.f;
+  }
+  const __nv_bfloat16* xr = x + t0 * ldx + c;
+  __nv_bfloat16* yr = y + t0 * ldy + c;
+  constexpr int U = 8;
+  for (int n = t1 - t0; n > 0; n -= U, xr += U * ldx, yr += U * ldy) {
+    uint32_t v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = u < n ? *reinterpret_cast<const uint32_t*>(xr + u * ldx) : 0u;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float o[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float xv = e ? bf16_hi(v[u]) : bf16_lo(v[u]);
+        float acc = bs[e] + wt[e][W - 1] * xv;
+#pragma unroll
+        for (int j = 0; j < W - 1; ++j) acc += wt[e][j] * win[e][j];
+#pragma unroll
+        for (int j = 0; j < W - 2; ++j) win[e][j] = win[e][j + 1];
+        win[e][W - 2] = xv;
+        o[e] = act_silu ? silu_f(acc) : acc;
+      }
+      if (u < n) *reinterpret_cast<uint32_t*>(yr + u * ldy) = pack_bf16(o[0], o[1]);
+    }
+  }
+}
+
 // New window of every sequence after a tiled pass: the last W - 1 raw inputs (rows before the sequence start come
 // from the old state). One thread per (sequence, channel) reads everything it needs before it writes, so the input
 // and output slots may be the same.
@@ -489,8 +555,10 @@ int hb_conv1d(const void* x, long long ldx, const void* w, const void* bias, voi
   if (batch <= 0) return 0;
   if (width != 4) return 1;
   if (max_rows > CONV_TT) {   // prefill: parallel over tiles of tokens, then the new windows
-    const dim3 tg((channels + 127) / 128, (max_rows + CONV_TT - 1) / CONV_TT, batch);
-    launch_dep(conv1d_tiled_kernel<4>, tg, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state),
+    const bool two = ((channels | ldx | ldy) & 1) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 3) == 0;
+    const int per = two ? 256 : 128;
+    const dim3 tg((channels + per - 1) / per, (max_rows + CONV_TT - 1) / CONV_TT, batch);
+    launch_dep(two ? conv1d_tiled2_kernel<4> : conv1d_tiled_kernel<4>, tg, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state),
                state_stride, IP(q_indptr), IP(slot_in), IP(slot_out),
                IP(has_init), channels, act_silu);
     if (slot_out != nullptr)

@@ -52,3 +52,25 @@ def test_gated_norm_of_few_and_many_groups(rows, gs, norm_first):
     n = (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5)).view(rows, -1) * w.double() * (gate if norm_first else 1.0)
     # the fast exponential is good to some 2^-21 for arguments of a few units
     assert ((got.double() - n).abs() <= (2.0 ** -8 + 2.0 ** -18) * n.abs() + 1e-6).all()
+
+
+# one and two channels a thread (odd counts and pitches take one), tiles of 32 rows in batches of 8, sequences with and without a state
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,pitch", [(6, 6), (258, 320), (131, 131), (64, 67)])
+@pytest.mark.parametrize("rows", [(33, 1, 40), (64, 65, 7), (3, 96, 2)])
+def test_tiled_convolution(channels, pitch, rows):
+    from hibana_b200.ops import recurrent
+    g = torch.Generator().manual_seed(channels)
+    x = torch.randn(sum(rows), pitch, generator=g).bfloat16()
+    w, bias = torch.randn(channels, 4, generator=g).bfloat16(), torch.randn(channels, generator=g).bfloat16()
+    state = torch.randn(5, channels, 3, generator=g).bfloat16()
+    ip = torch.tensor([0, rows[0], rows[0] + rows[1], sum(rows)], dtype=torch.int32)
+    slots, init = torch.tensor([3, 1, 4], dtype=torch.int32), torch.tensor([1, 0, 1], dtype=torch.int32)
+    kw = dict(silu=True, max_rows=max(rows))
+    want_state, got_state = state.clone(), state.cuda()
+    want = recurrent.conv1d(x[:, :channels], w, bias, want_state, slots, slots, q_indptr=ip, has_init=init, **kw)
+    got = recurrent.conv1d(x.cuda()[:, :channels], w.cuda(), bias.cuda(), got_state, slots.cuda(), slots.cuda(), q_indptr=ip.cuda(),
+                           has_init=init.cuda(), **kw)
+    # five fp32 terms of at most 16 and the fast exponential, then bf16
+    assert ((got.cpu().double() - want.double()).abs() <= 2.0 ** -7 * want.double().abs() + 5 * 16 * 2.0 ** -23).all()
+    assert torch.equal(got_state.cpu(), want_state)
