@@ -77,15 +77,14 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
 }
 
 // Gated grouped RMSNorm (Mamba-2 / GDN output): y = rmsnorm_g(x * silu(z)) * w with groups of `gs` channels, or norm-before-gate
-// when norm_first != 0: y = rmsnorm_g(x) * w * silu(z). Groups of up to 1024 channels sit in registers: L lanes per group, NC
-// 16-byte chunks per lane; one read of x and z, 16-byte stores. The kernel is bound by issue (an exponential and an IEEE
+// when norm_first != 0: y = rmsnorm_g(x) * w * silu(z). Groups of up to 1024 channels sit in registers: L lanes per group, a
+// 16-byte chunk per lane; one read of x and z, 16-byte stores. The kernel is bound by issue (an exponential and an IEEE
 // division per element), so no lane idles and no chunk is computed that is not there: 1237 rows of 48 groups of 128 took
-// 66 us with a warp per group and four predicated chunks, 19 us so; 4096 rows of 8 groups of 1024, 115 -> 99.
+// 66 us with a warp per group and four predicated chunks, 19 us so.
 // Lanes beyond the end of a group that does not fill them (16, 96 or 640 channels) divide ones, not zeros: a zero dividend sends
 // its warp through the division's slow path (one row of 6 groups of 640: 8.9 us with zeros and four chunks, 4.1 so).
-// (two blocks to an SM asked for: with plain loads the compiler takes 138 registers at four chunks, one block, 5000 x 10240 70 -> 117 us)
-template <int NC, int L>
-__global__ void __launch_bounds__(256, 2)
+template <int L>
+__global__ void __launch_bounds__(256)
 gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows, int h, int gs,
                          long long ldx, long long ldz, float eps, int norm_first, int sigmoid_gate, int gemma,
@@ -102,35 +101,27 @@ gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   const uint4* zr = z ? reinterpret_cast<const uint4*>(z + row * ldz + g * gs) : nullptr;
   const uint4* wr = reinterpret_cast<const uint4*>(w + g * gs);
   const int nchunk = live ? gs >> 3 : 0;
-  uint4 xa[NC], za[NC], wa[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int ci = lane + c * L;
-    xa[c] = wa[c] = make_uint4(0, 0, 0, 0);
-    za[c] = make_uint4(0x3f803f80, 0x3f803f80, 0x3f803f80, 0x3f803f80);
-    if (ci < nchunk) {
-      xa[c] = xr[ci];
-      if (zr) za[c] = zr[ci];
-      wa[c] = wr[ci];
-    }
+  const int ci = lane;                     // this lane's chunk of eight channels
+  uint4 xa = make_uint4(0, 0, 0, 0), wa = xa, za = make_uint4(0x3f803f80, 0x3f803f80, 0x3f803f80, 0x3f803f80);
+  if (ci < nchunk) {
+    xa = xr[ci];
+    if (zr) za = zr[ci];
+    wa = wr[ci];
   }
-  float v[NC][8], gt[NC][8];
+  float v[8], gt[8];
   float ss = 0.f;
+  const uint32_t xw[4] = {xa.x, xa.y, xa.z, xa.w}, zw[4] = {za.x, za.y, za.z, za.w};
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const uint32_t xw[4] = {xa[c].x, xa[c].y, xa[c].z, xa[c].w}, zw[4] = {za[c].x, za[c].y, za[c].z, za[c].w};
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float xv = (e & 1) ? bf16_hi(xw[e >> 1]) : bf16_lo(xw[e >> 1]);
-      float gate = 1.f;
-      if (zr) {
-        const float zz = (e & 1) ? bf16_hi(zw[e >> 1]) : bf16_lo(zw[e >> 1]);
-        gate = sigmoid_gate ? 1.f / (1.f + __expf(-zz)) : zz / (1.f + __expf(-zz));
-      }
-      gt[c][e] = gate;
-      v[c][e] = norm_first ? xv : xv * gate;
-      if (lane + c * L < nchunk) ss += v[c][e] * v[c][e];
+  for (int e = 0; e < 8; ++e) {
+    const float xv = (e & 1) ? bf16_hi(xw[e >> 1]) : bf16_lo(xw[e >> 1]);
+    float gate = 1.f;
+    if (zr) {
+      const float zz = (e & 1) ? bf16_hi(zw[e >> 1]) : bf16_lo(zw[e >> 1]);
+      gate = sigmoid_gate ? 1.f / (1.f + __expf(-zz)) : zz / (1.f + __expf(-zz));
     }
+    gt[e] = gate;
+    v[e] = norm_first ? xv : xv * gate;
+    if (ci < nchunk) ss += v[e] * v[e];
   }
 #pragma unroll
   for (int o = (L < 32 ? L : 32) / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -144,50 +135,46 @@ gated_rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   }
   const float rstd = rsqrtf(ss / gs + eps);
   uint4* yr = reinterpret_cast<uint4*>(y + static_cast<long long>(row) * h + g * gs);
+  const uint32_t ww4[4] = {wa.x, wa.y, wa.z, wa.w};
+  uint32_t o4[4];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int ci = lane + c * L;
-    const uint32_t ww4[4] = {wa[c].x, wa[c].y, wa[c].z, wa[c].w};
-    uint32_t o4[4];
+  for (int e = 0; e < 8; e += 2) {
+    float o2[2];
 #pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      float o2[2];
-#pragma unroll
-      for (int d = 0; d < 2; ++d) {
-        const float ww = d ? bf16_hi(ww4[e >> 1]) : bf16_lo(ww4[e >> 1]);
-        const float wv = gemma ? 1.f + ww : ww;
-        o2[d] = norm_first ? v[c][e + d] * rstd * wv * gt[c][e + d] : v[c][e + d] * rstd * wv;
-      }
-      o4[e >> 1] = pack_bf16(o2[0], o2[1]);
+    for (int d = 0; d < 2; ++d) {
+      const float ww = d ? bf16_hi(ww4[e >> 1]) : bf16_lo(ww4[e >> 1]);
+      const float wv = gemma ? 1.f + ww : ww;
+      o2[d] = norm_first ? v[e + d] * rstd * wv * gt[e + d] : v[e + d] * rstd * wv;
     }
-    if (q_out == nullptr) {
-      if (ci < nchunk) yr[ci] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-      continue;
-    }
-    // NVFP4 output for the projection that follows: chunks ci and ci ^ 1 (neighbouring lanes) are one 16-element scale
-    // group; values are the bf16-rounded outputs, as a separate quantiser would see them
-    float f[8];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      f[2 * e] = bf16_lo(o4[e]);
-      f[2 * e + 1] = bf16_hi(o4[e]);
-    }
-    float amax = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    if (ci >= nchunk) continue;
-    const float inv_gs = 1.f / *q_gscale;
-    const uint32_t sfb = float_to_e4m3(amax * (1.f / 6.f) * inv_gs);
-    const float sfv = e4m3_to_float(sfb);
-    const float inv = sfv > 0.f ? 1.f / (sfv * (1.f / inv_gs)) : 0.f;
-    uint32_t wq = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) wq |= e2m1x2(f[2 * e] * inv, f[2 * e + 1] * inv) << (8 * e);
-    const int col8 = (g * gs >> 3) + ci;                  // 8-element chunk index inside the row
-    reinterpret_cast<uint32_t*>(q_out + static_cast<size_t>(row) * (h >> 1))[col8] = wq;
-    if ((ci & 1) == 0) q_sf[row_sf_off(row, col8 >> 1, q_ka)] = static_cast<uint8_t>(sfb);
+    o4[e >> 1] = pack_bf16(o2[0], o2[1]);
   }
+  if (q_out == nullptr) {
+    if (ci < nchunk) yr[ci] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+    return;
+  }
+  // NVFP4 output for the projection that follows: chunks ci and ci ^ 1 (neighbouring lanes) are one 16-element scale
+  // group; values are the bf16-rounded outputs, as a separate quantiser would see them
+  float f[8];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    f[2 * e] = bf16_lo(o4[e]);
+    f[2 * e + 1] = bf16_hi(o4[e]);
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  if (ci >= nchunk) return;
+  const float inv_gs = 1.f / *q_gscale;
+  const uint32_t sfb = float_to_e4m3(amax * (1.f / 6.f) * inv_gs);
+  const float sfv = e4m3_to_float(sfb);
+  const float inv = sfv > 0.f ? 1.f / (sfv * (1.f / inv_gs)) : 0.f;
+  uint32_t wq = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) wq |= e2m1x2(f[2 * e] * inv, f[2 * e + 1] * inv) << (8 * e);
+  const int col8 = (g * gs >> 3) + ci;                  // 8-element chunk index inside the row
+  reinterpret_cast<uint32_t*>(q_out + static_cast<size_t>(row) * (h >> 1))[col8] = wq;
+  if ((ci & 1) == 0) q_sf[row_sf_off(row, col8 >> 1, q_ka)] = static_cast<uint8_t>(sfb);
 }
 
 // Any other group size, width or pitch: one warp per (row, group), two passes.
@@ -491,24 +478,24 @@ int hb_rmsnorm(const void* x, void* residual, const void* w, void* y, int rows, 
 static int gated_rmsnorm_reg(const void* x, const void* z, const void* w, void* y, int rows, int h, int gs, long long ldx,
                              long long ldz, float eps, int norm_first, int sigmoid_gate, int gemma, void* q, void* sf,
                              const void* gscale, int ka, void* stream) {
-  // Few groups: four warps on each, one chunk a lane, so that the chip is not one SM working through exponentials and divisions
-  // (behind one row's scan, 8 groups of 1024: 7.7 -> 3.5 us).
+  // One chunk a lane: a group of more than 256 channels is a CTA of two to four warps. A warp with up to four chunks a lane held 97 to
+  // 138 registers, half the threads per SM: 5000 rows of 8 groups of 1024 (NVFP4 out) 125 -> 99 us, of 512 54 -> 48, 6 of
+  // 640 72 -> 58; and one row was a single CTA
+  // working through exponentials and divisions (behind its scan 7.7 -> 3.5 us).
   const int nchunk = gs / 8;
-  const bool few = nchunk > 32 && static_cast<long long>(rows) * (h / gs) <= 2 * 148;
-  const int lanes = nchunk <= 8 ? 8 : nchunk <= 16 ? 16 : few ? 128 : 32, block = few ? 128 : 256;
+  const int lanes = nchunk <= 8 ? 8 : nchunk <= 16 ? 16 : (nchunk + 31) / 32 * 32, block = lanes > 32 ? lanes : 256;
   const long long threads = static_cast<long long>(rows) * (h / gs) * lanes;
   const unsigned blocks = static_cast<unsigned>((threads + block - 1) / block);
-#define HB_GN(NC, L)                                                                                                      \
-  launch_dep(gated_rmsnorm_reg_kernel<NC, L>, dim3(blocks), dim3(block), 0, ST(stream),                                   \
+#define HB_GN(L)                                                                                                          \
+  launch_dep(gated_rmsnorm_reg_kernel<L>, dim3(blocks), dim3(block), 0, ST(stream),                                       \
       BF(x), BF(z), BF(w), BFM(y), rows, h, gs, ldx, ldz, eps, norm_first, sigmoid_gate, gemma, static_cast<uint8_t*>(q), \
       static_cast<uint8_t*>(sf), static_cast<const float*>(gscale), ka)
-  if (lanes == 8) HB_GN(1, 8);
-  else if (lanes == 16) HB_GN(1, 16);
-  else if (few) HB_GN(1, 128);
-  else if (nchunk <= 32) HB_GN(1, 32);
-  else if (nchunk <= 64) HB_GN(2, 32);
-  else if (nchunk <= 96) HB_GN(3, 32);
-  else HB_GN(4, 32);
+  if (lanes == 8) HB_GN(8);
+  else if (lanes == 16) HB_GN(16);
+  else if (lanes == 32) HB_GN(32);
+  else if (lanes == 64) HB_GN(64);
+  else if (lanes == 96) HB_GN(96);
+  else HB_GN(128);
 #undef HB_GN
   return OK();
 }
