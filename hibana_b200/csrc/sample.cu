@@ -179,8 +179,8 @@ __device__ __forceinline__ float key_value(unsigned k) {
 }
 // A row's kernels run 1024 threads: a pass over the vocabulary is a chain of L2 loads per thread, so its length is what counts.
 // The mass above a key and the sums of the draw keep one fixed order of additions whatever the thread count: SUM_T strided
-// accumulators, a tree over each warp, then the warps one after the other. The threshold masses of the nucleus search do not
-// (search_key): the cut may move by one key where a mass ties p_lim * kept within fp32 rounding.
+// accumulators, a tree over each warp, then the warps one after the other. The masses that the nucleus search compares with p_lim * kept
+// are whole numbers, which have no order (search_key).
 constexpr int LAW_T = 1024, LAW_WARPS = LAW_T / 32, SUM_T = 256;
 __device__ __forceinline__ float sum_in_order(float v, float* red) {   // v counts on the first SUM_T threads; whole CTA
   v = warp_sum(v);
@@ -269,62 +269,94 @@ __device__ unsigned stage_row(const R& row, bool keep, unsigned* keys, int vocab
   return __reduce_max_sync(0xffffffffu, red[threadIdx.x & 31]);
 }
 
-// Largest key x of [lo, hi] with f(x) >= want, where f(x) is the sum of weight(v) over the tokens of key >= x (f(lo) >= want, f falls
-// with x, no token is above hi = the key of `top`, weights are at most 1).
-// One pass adds the weights up in BUCKETS of 1/16 `width` below `top` (a nucleus ends within some temperatures of the maximum), as
-// whole numbers of 2^-41, so the order of the atomics does not matter; the bucket where the sum reaches `want` holds the answer. Its tokens
-// are listed and each finds its own f; the largest key that holds is it. More than RANKED of them (ties, long rows, the
-// last bucket) are narrowed first, each pass summing above 15 thresholds. At 18992 tokens that is one pass and the list where
-// narrowing 32 bits by 16 took eight passes. Deterministic. Whole CTA.
-constexpr int WAYS = 16, BUCKETS = 256, RANKED = 1024;
-constexpr int FIX = 41, FIX_PART = 14;    // a sum is kept in three parts: 2^14 * 2^18 tokens fill 32 bits
-template <typename V>
+// Largest key x above `lo` that a token has and for which holds(f(x)), where f(x) is the sum of whole(k) over the tokens of keys
+// k >= x above `lo`; `lo` if there is none. holds() stays true as its argument grows, no token is above hi = the key of `top`.
+// Weights are whole numbers (at most 2^FIX each, 1 with ONES), so f has one value however it is added up, and every step asks
+// holds() about that value: a bucket that reaches the goal has a token that does. (With fp32 sums in the second step one draw in
+// about a million found none.)
+// One pass adds the weights up in BUCKETS of 1/16 `width` below `top` (a nucleus ends within some temperatures of the maximum); the
+// first bucket whose end holds has the answer. Its tokens are listed and each finds its own f; the largest key that holds is it. More than
+// RANKED of them (ties, long rows, the last bucket) are narrowed first: buckets again, of keys, 256 to a pass. At 18992 tokens that is one
+// pass and the list where narrowing 32 bits by 16 took eight passes. Whole CTA.
+constexpr int BUCKETS = 256, RANKED = 1024;
+constexpr int FIX = 41, FIX_PART = 14, SLAB = 1 << 18;    // a sum is kept in three parts: 2^14 * 2^18 tokens fill 32 bits
+constexpr int LIST_PART = 21;                             // a listed weight in two: 2^21 * 2^10 tokens
 struct SearchScratch {
   union {
-    unsigned bucket[3][BUCKETS];
-    uint2 list[RANKED];      // key, weight
+    struct {
+      unsigned bucket[3][BUCKETS];
+      unsigned long long sum[BUCKETS];
+    };
+    uint4 list[RANKED];      // key, weight in two parts
   };
-  V sums[WAYS][LAW_WARPS];
-  V totals[WAYS];
-  V before;
+  unsigned long long before;
   int count[LAW_WARPS];
   unsigned best, low;
   int at;
-  uint4 thr[WAYS / 4];       // thresholds (in registers they would spill: 64 a thread)
 };
-__device__ __forceinline__ float as_weight(unsigned b, float) { return __uint_as_float(b); }
-__device__ __forceinline__ int as_weight(unsigned b, int) { return static_cast<int>(b); }
-__device__ __forceinline__ unsigned weight_bits(float w) { return __float_as_uint(w); }
-__device__ __forceinline__ unsigned weight_bits(int w) { return static_cast<unsigned>(w); }
 __device__ __forceinline__ unsigned long long fixed(float w) { return __float2ull_rn(w * static_cast<float>(1ull << FIX)); }
-__device__ __forceinline__ unsigned long long fixed(int w) { return w; }
-__device__ __forceinline__ float from_fixed(unsigned long long s, float) {
+__device__ __forceinline__ float from_fixed(unsigned long long s) {
   return static_cast<float>(static_cast<double>(s) * (1.0 / static_cast<double>(1ull << FIX)));
 }
-__device__ __forceinline__ int from_fixed(unsigned long long s, int) { return static_cast<int>(s); }
 
-// Sixteen sums over a warp at once: at each step a lane keeps half of its sums and hands the other half to its partner (the
-// additions of a tree over each). Sum j ends in acc[0] of lanes 2 j and 2 j + 1.
-template <typename V>
-__device__ __forceinline__ void warp_sums(V (&acc)[WAYS], int lane) {
-#pragma unroll
-  for (int o = 16, c = WAYS / 2; o > 1; o >>= 1, c >>= 1)
-#pragma unroll
-    for (int j = 0; j < WAYS / 2; ++j)
-      if (j < c) {
-        const V keep = (lane & o) ? acc[j + c] : acc[j], give = (lane & o) ? acc[j] : acc[j + c];
-        acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-      }
-  acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-}
-
-template <typename V, typename R, typename W>
-__device__ unsigned search_key(const R& row, int vocab, unsigned lo, unsigned hi, V want, float top, float width, W weight,
-                               SearchScratch<V>& sc) {
+template <bool ONES, typename R, typename W, typename H>
+__device__ unsigned search_key(const R& row, int vocab, unsigned lo, unsigned hi, float top, float width, W whole, H holds,
+                               SearchScratch& sc) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!(lo < hi)) return lo;
-  if (V(0) >= want) return hi;
-  V beyond = V(0);           // f(hi + 1)
+  if (holds(0ull)) return hi;
+  unsigned long long beyond = 0;           // f of the keys above the range that is left
+  // The first bucket of the keys that are `in` whose end holds (BUCKETS: none); `beyond` is then the sum in front of it. bucket(k) rises
+  // as the key falls.
+  auto reached = [&](auto in, auto bucket) {
+    __syncthreads();
+    if (tid < BUCKETS) sc.sum[tid] = 0ull;
+    if (tid == 0) sc.at = BUCKETS;
+    for (int from = 0; from < vocab; from += SLAB) {
+      if (tid < 3 * BUCKETS) sc.bucket[0][tid] = 0u;
+      __syncthreads();
+      scan(row, from + tid, min(vocab - from, SLAB) + from, LAW_T, [&](unsigned k, int) {
+        if (in(k)) {
+          const int b = bucket(k);
+          const unsigned long long w = whole(k);
+          constexpr unsigned PART = (1u << FIX_PART) - 1u;
+          atomicAdd(&sc.bucket[0][b], static_cast<unsigned>(w) & PART);
+          if (!ONES) {
+            atomicAdd(&sc.bucket[1][b], static_cast<unsigned>(w >> FIX_PART) & PART);
+            atomicAdd(&sc.bucket[2][b], static_cast<unsigned>(w >> (2 * FIX_PART)));
+          }
+        }
+      });
+      __syncthreads();
+      if (tid < BUCKETS)
+        sc.sum[tid] += sc.bucket[0][tid] + (static_cast<unsigned long long>(sc.bucket[1][tid]) << FIX_PART) +
+                       (static_cast<unsigned long long>(sc.bucket[2][tid]) << (2 * FIX_PART));
+      __syncthreads();
+    }
+    if (tid < 32) {          // each lane owns BUCKETS / 32 in a row
+      constexpr int OWN = BUCKETS / 32;
+      unsigned long long own[OWN], upto = 0;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) own[j] = upto += sc.sum[tid * OWN + j];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const unsigned long long front = beyond + upto - own[OWN - 1];
+      const unsigned there = __ballot_sync(0xffffffffu, holds(beyond + upto));
+      if (there && lane == __ffs(there) - 1)
+#pragma unroll
+        for (int j = OWN - 1; j >= 0; --j)
+          if (holds(front + own[j])) {
+            sc.at = tid * OWN + j;
+            sc.before = front + (j == 0 ? 0ull : own[j - 1]);
+          }
+    }
+    __syncthreads();
+    if (sc.at < BUCKETS) beyond = sc.before;
+    return sc.at;
+  };
   // Lists the tokens that are `in`; if they are few the answer is found (true).
   auto ranked = [&](auto in, unsigned& answer) {
     int mine = 0;
@@ -344,140 +376,62 @@ __device__ unsigned search_key(const R& row, int vocab, unsigned lo, unsigned hi
     int at = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0) + upto - mine;
     if (mine != 0)
       scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
-        if (in(k)) sc.list[at++] = make_uint2(k, weight_bits(weight(key_value(k))));
+        if (in(k)) {
+          const unsigned long long w = whole(k);
+          sc.list[at++] = make_uint4(k, static_cast<unsigned>(w) & ((1u << LIST_PART) - 1u), static_cast<unsigned>(w >> LIST_PART), 0u);
+        }
       });
     __syncthreads();
     if (tid < total) {
       const unsigned k = sc.list[tid].x;
-      V f = V(0);
+      unsigned f0 = 0u, f1 = 0u;
 #pragma unroll 8
       for (int i = 0; i < total; ++i) {
-        const uint2 e = sc.list[i];
-        f += e.x >= k ? as_weight(e.y, V(0)) : V(0);
+        const uint4 e = sc.list[i];
+        f0 += e.x >= k ? e.y : 0u;
+        f1 += e.x >= k ? e.z : 0u;
       }
-      if (f + beyond >= want) atomicMax(&sc.best, k);
+      if (holds(beyond + f0 + (static_cast<unsigned long long>(f1) << LIST_PART))) atomicMax(&sc.best, k);
     }
     __syncthreads();
-    answer = max(sc.best, lo);
+    answer = sc.best;
     return true;
   };
+  const float per = 16.f / width;
+  auto bucket = [&](unsigned k) {           // by roundings that keep the order
+    return static_cast<int>(fminf((top - key_value(k)) * per, static_cast<float>(BUCKETS - 1)));
+  };
+  const int at = reached([&](unsigned k) { return k > lo; }, bucket);
+  if (at == BUCKETS) return lo;
+  auto in = [&](unsigned k) { return k > lo && bucket(k) == at; };
   unsigned answer;
-  if (vocab <= (1 << 18)) {
-    const float per = 16.f / width;
-    auto bucket = [&](unsigned k) {         // rises as the key falls, by roundings that keep the order
-      return static_cast<int>(fminf((top - key_value(k)) * per, static_cast<float>(BUCKETS - 1)));
-    };
-    __syncthreads();
-    for (int i = tid; i < 3 * BUCKETS; i += LAW_T) sc.bucket[0][i] = 0u;
-    if (tid == 0) sc.at = BUCKETS;
-    __syncthreads();
-    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
-      if (k > lo) {
-        const int b = bucket(k);
-        const unsigned long long w = fixed(weight(key_value(k)));
-        constexpr unsigned PART = (1u << FIX_PART) - 1u;
-        atomicAdd(&sc.bucket[0][b], static_cast<unsigned>(w) & PART);
-        if (sizeof(V) == 4 && static_cast<V>(0.5f) != V(0)) {      // (counts need one part)
-          atomicAdd(&sc.bucket[1][b], static_cast<unsigned>(w >> FIX_PART) & PART);
-          atomicAdd(&sc.bucket[2][b], static_cast<unsigned>(w >> (2 * FIX_PART)));
-        }
-      }
-    });
-    __syncthreads();
-    if (tid < 32) {          // the first bucket whose end reaches `want`: each lane owns BUCKETS / 32 in a row
-      constexpr int OWN = BUCKETS / 32;
-      unsigned long long own[OWN], upto = 0;
-#pragma unroll
-      for (int j = 0; j < OWN; ++j) {
-        const int b = tid * OWN + j;
-        upto += sc.bucket[0][b] + (static_cast<unsigned long long>(sc.bucket[1][b]) << FIX_PART) +
-                (static_cast<unsigned long long>(sc.bucket[2][b]) << (2 * FIX_PART));
-        own[j] = upto;
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const unsigned long long before = upto - own[OWN - 1];
-      const unsigned reached = __ballot_sync(0xffffffffu, from_fixed(upto, V(0)) >= want);
-      if (reached && lane == __ffs(reached) - 1)
-#pragma unroll
-        for (int j = OWN - 1; j >= 0; --j)
-          if (from_fixed(before + own[j], V(0)) >= want) {
-            sc.at = tid * OWN + j;
-            sc.before = from_fixed(before + (j == 0 ? 0ull : own[j - 1]), V(0));
-          }
+  if (ranked(in, answer)) return answer;
+  unsigned kmin = 0xffffffffu, kmax = 0u;
+  scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
+    if (in(k)) {
+      kmin = min(kmin, k);
+      kmax = max(kmax, k);
     }
-    __syncthreads();
-    const int at = sc.at;
-    if (at == BUCKETS) return lo;
-    beyond = sc.before;
-    auto in = [&](unsigned k) { return k > lo && bucket(k) == at; };
-    if (ranked(in, answer)) return answer;
-    unsigned kmin = 0xffffffffu, kmax = 0u;
-    scan(row, tid, vocab, LAW_T, [&](unsigned k, int) {
-      if (in(k)) {
-        kmin = min(kmin, k);
-        kmax = max(kmax, k);
-      }
-    });
-    if (tid == 0) sc.low = 0xffffffffu;
-    __syncthreads();
-    kmin = __reduce_min_sync(0xffffffffu, kmin);
-    kmax = __reduce_max_sync(0xffffffffu, kmax);
-    if (lane == 0) {
-      atomicMin(&sc.low, kmin);
-      atomicMax(&sc.best, kmax);
-    }
-    __syncthreads();
-    lo = sc.low - 1;         // f(the lowest key of the bucket) >= want
-    hi = sc.best;
-    __syncthreads();
+  });
+  if (tid == 0) sc.low = 0xffffffffu;
+  __syncthreads();
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  if (lane == 0) {
+    atomicMin(&sc.low, kmin);
+    atomicMax(&sc.best, kmax);
   }
-  while (lo < hi) {
-    if (ranked([&](unsigned k) { return k > lo && k <= hi; }, answer)) return answer;
-    const unsigned span = hi - lo, step = span / WAYS + 1;
-    const int n = static_cast<int>(span / step);
-    if (tid < WAYS) reinterpret_cast<unsigned*>(sc.thr)[tid] = lo + (tid + 1) * step;      // lo + step, ... up to hi
-    __syncthreads();
-    V acc[WAYS];
-#pragma unroll
-    for (int j = 0; j < WAYS; ++j) acc[j] = V(0);
-    bool some = false;
-    scan<4>(row, tid, vocab, LAW_T, [&](unsigned k, int) {
-      if (k > lo && k <= hi) {
-        const V w = weight(key_value(k));
-        some = true;
-#pragma unroll
-        for (int j = 0; j < WAYS / 4; ++j) {
-          const uint4 t = sc.thr[j];
-          acc[4 * j] += k >= t.x ? w : V(0);
-          acc[4 * j + 1] += k >= t.y ? w : V(0);
-          acc[4 * j + 2] += k >= t.z ? w : V(0);
-          if (j < WAYS / 4 - 1) acc[4 * j + 3] += k >= t.w ? w : V(0);
-        }
-      }
-    });
-    if (__any_sync(0xffffffffu, some)) warp_sums(acc, lane);
-    if ((lane & 1) == 0) sc.sums[lane >> 1][warp] = acc[0];
-    __syncthreads();
-    if (warp < n) {
-      V t = sc.sums[warp][lane];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) sc.totals[warp] = t + beyond;
-    }
-    __syncthreads();
-    const unsigned failed = __ballot_sync(0xffffffffu, lane < n && !(sc.totals[lane < WAYS ? lane : 0] >= want));
-    const int best = failed ? __ffs(failed) - 1 : n;       // thresholds that hold
-    if (best < n) {
-      hi = lo + (best + 1) * step - 1;
-      beyond = sc.totals[best];
-    }
-    lo += best * step;
+  __syncthreads();
+  kmin = sc.low;
+  kmax = sc.best;
+  while (kmin < kmax) {
+    const int shift = max(0, 24 - __clz(kmax - kmin));
+    auto left = [&](unsigned k) { return k >= kmin && k <= kmax; };
+    kmax -= static_cast<unsigned>(reached(left, [&](unsigned k) { return static_cast<int>((kmax - k) >> shift); })) << shift;
+    kmin = kmax - min(kmax - kmin, (1u << shift) - 1u);
+    if (ranked(left, answer)) return answer;
   }
-  return lo;
+  return kmax;
 }
 
 // The 32 values of a warp added to `acc` one after the other; `after` = the running sum behind this lane's own. Every lane gets the end.
@@ -496,11 +450,11 @@ __device__ __forceinline__ float sum_lanes(float acc, float w, int lane, float& 
 // law with token `exclude` removed (-1: nothing removed; the residual of a point-mass draft in speculative
 // sampling) and reports the probability of token `probe` under the law. LAW_T threads, whole CTA. Bound by the chain of its passes
 // over the row, so the row is staged where it fits. With a nucleus cut, us at 11 rows, a pass over the row for every 4
-// bits of the cut / now: 18992 tokens 85 / 32, 31040 113 / 42, 52224 167 / 65, 151936 (not staged) 479 / 318; cut off 26 / 18, 36 / 22, 53 / 33,
-// 163 / 117 (0 of 13824 draws and probabilities differed).
+// bits of the cut / now: 18992 tokens 85 / 31, 31040 113 / 43, 52224 167 / 68, 151936 (not staged) 479 / 287; cut off 26 / 17, 36 / 22, 53 / 31,
+// 163 / 116 (0 of 23040 draws differed).
 template <typename T, bool STAGED>
 __device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int k_lim, float p_lim, float u01, int exclude,
-                        int probe, long long* out, float* out_prob, float* out_probe, SearchScratch<float>& sc) {
+                        int probe, long long* out, float* out_prob, float* out_probe, SearchScratch& sc) {
   constexpr int CHUNKS = 256;              // contiguous pieces of the row for the draw
   extern __shared__ unsigned row_keys[];   // STAGED: vocab of them
   __shared__ unsigned redu[LAW_WARPS];
@@ -519,8 +473,8 @@ __device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int
   int need_k = 0x7fffffff;
   const bool cut_k = k_lim > 0 && k_lim < vocab;
   if (cut_k) {
-    tk_key = search_key<int>(row, vocab, 0u, mk, k_lim, mx, temp, [](float) { return 1; },
-                             reinterpret_cast<SearchScratch<int>&>(sc));
+    tk_key = search_key<true>(row, vocab, 0u, mk, mx, temp, [](unsigned) { return 1ull; },
+                              [&](unsigned long long n) { return n >= k_lim; }, sc);
     int above = 0;
     scan(row, tid, vocab, LAW_T, [&](unsigned k, int) { above += k > tk_key; });
     need_k = k_lim - block_sum_i(above, redi);
@@ -549,8 +503,17 @@ __device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int
   if (p_lim < 1.f) {
     const float want = p_lim * kept;
     // mass(key >= tk_key) = kept >= want, and every token above tk_key is inside the cut
-    const unsigned lo = search_key<float>(row, vocab, tk_key, mk, want, mx, temp,
-                                          [&](float v) { return __expf((v - mx) * inv_t); }, sc);
+    unsigned lo = search_key<false>(row, vocab, tk_key, mk, mx, temp,
+                                    [&](unsigned k) { return fixed(__expf((key_value(k) - mx) * inv_t)); },
+                                    [&](unsigned long long m) { return from_fixed(m) >= want; }, sc);
+    if (lo == 0u) {        // the whole numbers' mass is a rounding short of p_lim * kept (p_lim next to 1): all tokens are inside
+      lo = 0xffffffffu;
+      scan(row, tid, vocab, LAW_T, [&](unsigned k, int) { lo = min(lo, k - 1u); });      // (0, no token's, becomes the largest)
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      if (tid % 32 == 0) redu[tid / 32] = lo;
+      __syncthreads();
+      lo = __reduce_min_sync(0xffffffffu, redu[tid % 32]) + 1u;
+    }
     if (lo != tk_key || !cut_k) {
       t_key = lo;
       mass_above(t_key);
@@ -678,15 +641,15 @@ constexpr int SAMPLE_K = 64;  // candidates kept per row for 1 <= top-k <= 64 (t
 // written, when the row has fewer. Whole CTA.
 template <typename T, bool STAGED>
 __device__ bool list_candidates(const T* lr, int vocab, const int* mask, int k, float temp, float* cv, int* ci,
-                                SearchScratch<float>& sc) {
+                                SearchScratch& sc) {
   extern __shared__ unsigned row_keys[];
   __shared__ unsigned redu[LAW_WARPS], gk[SAMPLE_K];
   __shared__ int gi[SAMPLE_K], ei[SAMPLE_K], n_above, n_equal;
   const int tid = threadIdx.x;
   const RowKeys<T, STAGED, true> row{lr, mask, row_keys};
   const unsigned mk = stage_row(row, STAGED, row_keys, vocab, redu);
-  const unsigned tk = search_key<int>(row, vocab, 0u, mk, k, key_value(mk), temp, [](float) { return 1; },
-                                      reinterpret_cast<SearchScratch<int>&>(sc));
+  const unsigned tk = search_key<true>(row, vocab, 0u, mk, key_value(mk), temp, [](unsigned) { return 1ull; },
+                                       [&](unsigned long long n) { return n >= k; }, sc);
   if (tk <= 0x007fffffu) return false;
   if (tid == 0) n_above = n_equal = 0;
   __syncthreads();
@@ -751,7 +714,7 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
   __shared__ int wi[LAW_WARPS];
   __shared__ float s_prev_v;
   __shared__ int s_prev_i;
-  __shared__ SearchScratch<float> sc;
+  __shared__ SearchScratch sc;
   const int row = blockIdx.x;
   const T* lr = logits + row * ld;
   const int* mask = bitmask ? bitmask + static_cast<long long>(row) * mask_words : nullptr;
@@ -768,7 +731,7 @@ sample_kernel(const T* __restrict__ logits, long long ld, int vocab, const float
   }
   if (temp <= 0.f) k = 1;
   // From four candidates on by the key of the k-th one (a search and a list against k passes over the row; 50 of
-  // 18992 169 -> 29 us, of 151936 1772 -> 126). Fewer live tokens than candidates: the passes.
+  // 18992 169 -> 30 us, of 151936 1772 -> 133). Fewer live tokens than candidates: the passes.
   const bool listed = k > 3 && list_candidates<T, STAGED>(lr, vocab, mask, k, temp, cv, ci, sc);
   if (threadIdx.x == 0) {
     s_prev_v = INFINITY;
@@ -925,7 +888,7 @@ spec_targets_kernel(const T* __restrict__ logits, long long ld, int vocab, int k
                     long long* __restrict__ target, float* __restrict__ p_draft) {
   __shared__ long long s_tok;
   __shared__ float s_probe;
-  __shared__ SearchScratch<float> sc;
+  __shared__ SearchScratch sc;
   const int row = blockIdx.x, b = row / (k + 1), j = row - b * (k + 1);
   const T* lr = logits + row * ld;
   const int* mask = bitmask ? bitmask + static_cast<long long>(row) * mask_words : nullptr;
@@ -1027,7 +990,7 @@ rank_gap_kernel(const T* __restrict__ logits, long long ld, int vocab, const lon
   }
 }
 
-// Rows of up to 52224 tokens (204 KB of keys beside 15 KB of scratch) are staged.
+// Rows of up to 52224 tokens (204 KB of keys beside 20 KB of scratch) are staged.
 inline size_t staged_bytes(int vocab) { return vocab <= 52224 ? static_cast<size_t>(vocab) * sizeof(unsigned) : 0; }
 template <typename K>
 bool row_kernel(K kern, size_t smem) {

@@ -89,3 +89,39 @@ def test_speculative_targets_on_staged_and_long_rows_agree():
     # other strides of the sums (the draw's chunks are 1/256 of the row): 473 * 2^-24 of the mass
     assert torch.allclose(pa, pc, atol=6e-5, rtol=0)
     assert (a == c).float().mean() > 0.8 and bool((a < vocab).all() and (c < vocab).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [18992, 52300])
+@pytest.mark.parametrize("top_k", [0, 3000])
+def test_nucleus_that_ends_with_a_bucket(vocab, top_k):
+    """top-p at the mass where a bucket of the nucleus search ends, give or take some floats, and just below 1: always a finite
+    probability and a token of the nucleus (a search whose two tests disagree by a rounding finds no key there)."""
+    temp, ulps = 0.8, 8
+    x = torch.randn(vocab, generator=torch.Generator().manual_seed(1)) * 2
+    order = torch.sort(x, descending=True, stable=True).indices[:top_k or vocab]
+    v = x[order]
+    w = torch.exp((v.double() - float(v[0])) / temp)
+    cum = torch.cumsum(w, 0) / w.sum()
+    bucket = ((v[0] - v) * (16 / temp)).floor()
+    ends = (bucket[1:] != bucket[:-1]).nonzero().flatten()
+    at = cum[ends][(cum[ends] > 0.05) & (cum[ends] < 0.9995)].float()
+    ps = torch.cat([(at.view(torch.int32)[:, None] + torch.arange(-ulps, ulps + 1)).flatten().int().view(torch.float32),
+                    torch.tensor([1 - 2.0 ** -24, 1 - 2.0 ** -23, 0.999999])])
+    b = len(ps)
+    full = lambda val, dt: torch.full((b,), val, dtype=dt, device="cuda")
+    args = (full(temp, torch.float32), full(top_k, torch.int32), ps.cuda(), torch.arange(b, device="cuda") + 3,
+            torch.arange(b, device="cuda"))
+    rank = torch.full((vocab,), vocab, dtype=torch.long)
+    rank[order] = torch.arange(len(order))
+    before = torch.cat([cum - w / w.sum(), torch.tensor([2.0])])      # mass in front of a token; past the top-k cut: none of the law
+    tol = 6e-5      # as above: fp32 sums
+    tok = sampling.sample(x.cuda().expand(b, vocab), *args).cpu()
+    assert (before[rank[tok].clamp_max(len(order))] <= ps.double() + tol).all()
+    drafts = full(int(order[0]), torch.int64)[:, None]
+    target, p_draft = (t.cpu() for t in sampling.spec_targets(x.cuda().expand(2 * b, vocab), drafts, *args))
+    assert (before[rank[target[:, 1]].clamp_max(len(order))] <= ps.double() + tol).all()
+    # the first token's share of the nucleus, whose mass is at least p and less than p and one more token
+    kept = 1 / (w.sum() * p_draft[:, 0].double())
+    edge = (w / w.sum())[torch.searchsorted(cum, ps.double()).clamp_max(len(order) - 1)]
+    assert (kept >= ps.double() - tol).all() and (kept <= ps.double() + edge + tol).all()
