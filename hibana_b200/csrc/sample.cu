@@ -471,10 +471,13 @@ __device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int
   // ---- top-k cut: tk_key = value of the k-th token, need_k = how many of the tokens equal to it are inside
   unsigned tk_key = 0;
   int need_k = 0x7fffffff;
-  const bool cut_k = k_lim > 0 && k_lim < vocab;
+  bool cut_k = k_lim > 0 && k_lim < vocab;
   if (cut_k) {
     tk_key = search_key<true>(row, vocab, 0u, mk, mx, temp, [](unsigned) { return 1ull; },
                               [&](unsigned long long n) { return n >= k_lim; }, sc);
+    cut_k = tk_key != 0u;                  // fewer live tokens than that: all of them are inside
+  }
+  if (cut_k) {
     int above = 0;
     scan(row, tid, vocab, LAW_T, [&](unsigned k, int) { above += k > tk_key; });
     need_k = k_lim - block_sum_i(above, redi);

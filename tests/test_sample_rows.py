@@ -125,3 +125,28 @@ def test_nucleus_that_ends_with_a_bucket(vocab, top_k):
     kept = 1 / (w.sum() * p_draft[:, 0].double())
     edge = (w / w.sum())[torch.searchsorted(cum, ps.double()).clamp_max(len(order) - 1)]
     assert (kept >= ps.double() - tol).all() and (kept <= ps.double() + edge + tol).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [4096, 52225])
+@pytest.mark.parametrize("top_p", [1.0, 0.8])
+def test_fewer_live_tokens_than_top_k(vocab, top_p):
+    """A grammar that leaves 10 tokens and a top-k of 100: the law of those 10."""
+    b = 32
+    g = torch.Generator().manual_seed(4)
+    x = torch.randn(2 * b, vocab, generator=g)
+    live = torch.randperm(vocab, generator=g)[:10]
+    words = torch.zeros((vocab + 31) // 32, dtype=torch.int64)
+    for t in live.tolist():
+        words[t // 32] |= 1 << (t % 32)
+    mask = ((words + 2 ** 31) % 2 ** 32 - 2 ** 31).to(torch.int32).expand(2 * b, -1).contiguous()
+    full = lambda val, dt: torch.full((2 * b,), val, dtype=dt)
+    args = (full(0.8, torch.float32), full(100, torch.int32), full(top_p, torch.float32), torch.arange(2 * b) * 31 + 7,
+            torch.arange(2 * b))
+    got = sampling.sample(x.cuda(), *[a.cuda() for a in args], mask.cuda()).cpu()
+    assert torch.equal(got, sampling.sample_ref(x, *args, mask))
+    drafts = live[torch.arange(b) % 10][:, None]
+    half = [a[:b] for a in args]
+    got, p = sampling.spec_targets(x.cuda(), drafts.cuda(), *[a.cuda() for a in half], None, mask.cuda())
+    want, pw = sampling.spec_targets_ref(x, drafts, *half, None, mask)
+    assert torch.equal(got.cpu(), want) and torch.allclose(p.cpu(), pw, atol=1e-5, rtol=1e-5)
