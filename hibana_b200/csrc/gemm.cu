@@ -417,11 +417,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
   const float* alpha_ptr = p.alpha_ptr;
   if (p.grp_cnt != nullptr) {
     int e = blockIdx.z, chunk = blockIdx.y;
+    // CTAs without rows leave at once: waiting for the kernel in front they would keep others off their SM. The first one waits all the
+    // same: a grid none of whose CTAs did (no expert of this call has rows) could end before its predecessors (see launch_dep).
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
     if (p.grp_tiles != nullptr) {
       if (static_cast<int>(blockIdx.y) >= *p.grp_ntiles) {   // uniform, before any barrier or TMEM allocation
-        // an empty list (no rows routed to this rank) still owes every rank its "returned" flag: one CTA says so
-        if (p.epilogue == kEpiReturn && *p.grp_ntiles == 0 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-          ep_publish_returned(p);
+        if (first) {      // an empty list (no rows routed to this rank) still owes every rank its "returned" flag
+          grid_dep_wait();
+          if (p.epilogue == kEpiReturn && threadIdx.x == 0) ep_publish_returned(p);
+        }
         return;
       }
       const int code = p.grp_tiles[blockIdx.y];
@@ -430,6 +434,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
     }
     const int cnt = p.grp_cnt[e];
     if (chunk * BN >= cnt) {   // uniform: before any barrier or TMEM allocation
+      if (first) grid_dep_wait();
       if (p.epilogue == kEpiReturn && threadIdx.x == 0) ep_cta_done(p, false);
       return;
     }

@@ -44,3 +44,40 @@ def test_launch_levels_give_the_same_bits(family, graphs):
         from hibana_b200 import config
         gemm.set_pdl(config.current().pdl)
     assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["bf16", "nvfp4", "w3"])
+@pytest.mark.parametrize("t", [3, 100])
+def test_expert_range_without_rows(fmt, t):
+    """An expert range that no token is routed to, in a chain of dependents: its grouped GEMMs have nothing to do, but end behind
+    what runs in front of them. Bits of the chain equal those of plain launches."""
+    from hibana_b200 import _native as nv
+    from hibana_b200 import config
+    from hibana_b200.ops import gemm, moe
+    g = torch.Generator().manual_seed(t)
+    e, h, inter = 8, 512, 256
+    ew = moe.ExpertWeights.create((torch.randn(e, 2 * inter, h, generator=g) * 0.05).cuda(),
+                                  (torch.randn(e, h, inter, generator=g) * 0.05).cuda(), "swiglu", fmt, in_amax=5.0, mid_amax=2.0)
+    x = torch.randn(t, 8192, generator=g).bfloat16().cuda()
+    wide, back = ((torch.randn(n, k, generator=g) * 0.02).bfloat16().cuda() for n, k in ((h, 8192), (8192, h)))
+    ids = torch.randint(0, 4, (t, 2), generator=g).int().cuda()
+    w = torch.rand(t, 2, generator=g).cuda()
+
+    def chain():
+        y = x
+        for _ in range(4):
+            shared = gemm.linear_bf16(y, wide)
+            y = gemm.linear_bf16(moe.experts_forward(shared, ids, w, ew, shared=shared, e_lo=4, e_n=4), back)
+        return y, shared
+
+    try:
+        gemm.set_pdl(0)
+        want, shared = chain()
+        assert torch.equal(moe.experts_forward(shared, ids, w, ew, shared=shared, e_lo=4, e_n=4), shared)
+        gemm.set_pdl(2)
+        for _ in range(5):
+            assert torch.equal(chain()[0], want)
+    finally:
+        gemm.set_pdl(config.current().pdl)
+    assert nv.read_status() == 0
