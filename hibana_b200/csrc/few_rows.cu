@@ -8,8 +8,9 @@
 // not by bytes; so as much of K as possible is in flight at once.
 //
 // In a chain of launches, tcgen05 / this, us: 512 x 4096 5.8 / 3.1 (1 row), 1024 x 4096 6.0 / 3.3, 2048 x 2048 5.3 / 2.9, 4096 x 1024
-// 5.5 / 3.4, 4096 x 4096 9.5 / 7.8; 16 rows 6.0 / 5.3, 6.2 / 5.5, 5.7 / 3.5, 5.6 / 3.5, 9.8 / 11. Error against 64 bits 2.4e-7 / 4.7e-7 at
-// 4096, fp32 accumulation in both.
+// 5.5 / 3.4, 4096 x 4096 9.5 / 7.8; 16 rows 6.0 / 5.3, 6.2 / 5.5, 5.7 / 3.5, 5.6 / 3.5, 9.8 / 11. Relative error against 64 bits (fp32
+// accumulation in both): 512 x 4096 4.9e-7 / 1.4e-7 at 1 row, 4.8e-7 / 2.4e-7 at 16; 4096 x 1024 1.7e-7 / 0.9e-7; 256 x 1000, whose K the
+// tcgen05 form cuts finer than these warps do, 1.3e-7 / 1.3e-7 (2.3e-7 with one accumulator).
 #include "hb_api.h"
 #include "hb_common.cuh"
 
@@ -62,17 +63,17 @@ few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __re
   for (int i = 0; i < DEPTH; ++i)
 #pragma unroll
     for (int q = 0; q < NB; ++q) b[i][q] = rows(i, q);
-  float acc[NB][4];
+  float acc[2][NB][4];       // of the even and the odd instructions: the longer a chain, the more its fp32 additions lose
 #pragma unroll
-  for (int q = 0; q < NB; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
+  for (int q = 0; q < 2 * NB; ++q) acc[q & 1][q >> 1][0] = acc[q & 1][q >> 1][1] = acc[q & 1][q >> 1][2] = acc[q & 1][q >> 1][3] = 0.f;
   for (int i0 = 0; i0 < steps; i0 += DEPTH) {
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) {
       // (steps past the end multiply zeros)
 #pragma unroll
       for (int q = 0; q < NB; ++q) {
-        mma_bf16(acc[q], a[i][0].x, a[i][1].x, a[i][0].y, a[i][1].y, b[i][q].x, b[i][q].y);
-        mma_bf16(acc[q], a[i][0].z, a[i][1].z, a[i][0].w, a[i][1].w, b[i][q].z, b[i][q].w);
+        mma_bf16(acc[0][q], a[i][0].x, a[i][1].x, a[i][0].y, a[i][1].y, b[i][q].x, b[i][q].y);
+        mma_bf16(acc[1][q], a[i][0].z, a[i][1].z, a[i][0].w, a[i][1].w, b[i][q].z, b[i][q].w);
       }
       if (i0 + DEPTH < steps) {
         a[i][0] = weights(i0 + DEPTH + i, 0);
@@ -85,7 +86,7 @@ few_rows_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __re
 #pragma unroll
   for (int q = 0; q < NB; ++q)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) red[warp][q * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = acc[q][e];
+    for (int e = 0; e < 4; ++e) red[warp][q * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = acc[0][q][e] + acc[1][q][e];
   __syncthreads();
   auto sum = [&](int i) {
     float s = 0.f;
@@ -133,7 +134,7 @@ int hb_few_rows_bf16(const void* x, long long ldx, const void* w, long long ldw,
     return 1;
   // One wave of CTAs: sixteen warps take 4096 elements of K at once. More CTAs (or 9 to 16 rows, whose fragments of x take registers):
   // eight warps, several CTAs to an SM. A matrix of a megabyte runs beside a larger projection on a parallel branch: four warps
-  // (13K registers) fit next to its two CTAs of 192 threads, sixteen would wait until that projection has left the SM, which put
+  // (12K to 16K registers) find room next to its CTAs of 192 threads, sixteen would wait until that projection has left the SM, which put
   // 11 us a layer on the critical path of the delta rule's gates.
   // From 2048 elements of K on eight CTAs share a block of features, all of K in flight at once: beside the projection, which
   // keeps the memory busy, each round of loads takes 3 us, and the gates of 4 rows (96 x 5120) left 5 us after the convolution.
