@@ -1063,9 +1063,17 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
 // state. Q is loaded by the softmax warps while the producers fetch the first tiles, and the heaviest blocks of all heads and
 // sequences start first. Bounds per 64 keys and pair of Q tiles: MMAs 1280 cycles (Q K^T reads 6 KB of shared memory per
 // instruction), exponentials 1024; 1830 to 1930 are spent, 1330 of them in a softmax whose exponentials share their unit with the
-// other stream's. One layer, 40 / 8 heads of 128: 2048 tokens 111 -> 61 us, from scattered slots 200 -> 73, five prompts of 4096
-// 202 -> 103, 4096 tokens 312 -> 173, 2048 new ones over 8192 keys 457 -> 303; 32 / 32 heads of 64, 2048 tokens 75 -> 39; 29 tokens
-// 12.8 -> 8.6.
+// other stream's. One layer, 40 / 8 heads of 128: 2048 tokens 111 -> 62 us, from scattered slots 200 -> 75, five prompts of 4096
+// 202 -> 104, 4096 tokens 313 -> 175, 2048 new ones over 8192 keys 465 -> 303; 32 / 32 heads of 64, 2048 tokens 75 -> 41; 29 tokens
+// 13.1 -> 8.8.
+// The reference of a row's weights: a weight that is the reference itself is 1 and has no rounding error, and it is the largest weights
+// whose rounding to bf16 shows. So the reference follows the maximum exactly for the first 256 keys (what the two streams of the kernel
+// above see first), afterwards in steps of 2^4. With the maximum of the first 64 keys and steps of 2^8 the error against 64 bits
+// was up to 10 % above that kernel's, now it is the same or less. 40 / 8 heads of 128, queries times 1 / 1.5 / 3, 1e-3: 512 tokens, above 1.977 /
+// 1.913 / 1.826, before 2.013 / 2.015 / 2.024, now 1.974 / 1.913 / 1.796; 2048 tokens 2.047 / 2.017 / 2.029, 2.084 / 2.107 / 2.145, 2.046 /
+// 2.010 / 1.911 (rounding the result alone: 1.66). It costs 2048 tokens 61.8 -> 62.5 us, 512 17.4 -> 18.4, five prompts of 4096 102 -> 104.
+constexpr int Q2_SETTLE = 4;      // tiles
+constexpr float Q2_GAP = 4.f;     // log2
 constexpr int Q2_KT = 64;
 constexpr int Q2_STAGES = 4;      // tiles of the K and of the V ring
 constexpr int Q2_THREADS = 512;   // warps 0-3 and 4-7 softmax, 8 and 9 fetch K, 10 and 11 V, 12 and 13 issue S = Q K^T, 14 and 15 O += P V
@@ -1390,9 +1398,9 @@ attn_prefill_q2_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
       const float m_tile = pf_reference<false>(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), p.scale_log2);
       if (t == 0) {
         m_ref = m_tile;
-      } else if (__any_sync(0xffffffffu, m_tile > m_ref + PfCfg<D, false>::RESCALE_GAP)) {
+      } else if (__any_sync(0xffffffffu, m_tile > m_ref + (t < Q2_SETTLE ? 0.f : Q2_GAP))) {
         // Raise the reference (all lanes of the warp: tcgen05.ld / st are warp-wide) and rescale O and l, once O += P V of
-        // the tile before has completed
+        // the tile before has completed. The scores make room for 64 columns of O at a time and are read again.
         ok = warp_wait(&pv_done[st * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort, p.status, kTimeoutAccum);
         if (!ok) break;
         tc_fence_after();
@@ -1401,14 +1409,18 @@ attn_prefill_q2_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
         m_ref = m_new;
         l *= alpha;
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 16) {
-          uint32_t o[16];
-          tmem_ld_32x16(o_t + c0, o);
+        for (int c0 = 0; c0 < D; c0 += 64) {
+          tmem_ld_32x32(o_t + c0, v[0]);
+          tmem_ld_32x32(o_t + c0 + 32, v[1]);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-          tmem_st_32x16(o_t + c0, o);
+          for (int j = 0; j < 64; ++j) v[j >> 5][j & 31] = __float_as_uint(__uint_as_float(v[j >> 5][j & 31]) * alpha);
+          tmem_st_32x32(o_t + c0, v[0]);
+          tmem_st_32x32(o_t + c0 + 32, v[1]);
         }
+        tmem_ld_32x32(s_t, v[0]);
+        tmem_ld_32x32(s_t + 32, v[1]);
+        tmem_ld_wait();
       }
       const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
       l += whole ? q2_weights<true>(v, s_t, rel, p.scale_log2, neg_m) : q2_weights<false>(v, s_t, rel, p.scale_log2, neg_m);

@@ -50,11 +50,12 @@ def test_few_rows_match_fp64(n, k, m, f32):
 @pytest.mark.parametrize("n,k", [(256, 1000), (300, 1536), (512, 4096), (4096, 1024)])
 @pytest.mark.parametrize("m", [1, 8, 16])
 def test_few_rows_are_as_close_as_the_tiles(n, k, m):
-    """2-norm of the error against fp64 over n * m sums: both are averages over hundreds of roundings, 10 % apart at most by chance."""
+    """2-norm of the error against fp64 over N = n * m sums. A norm of N independent errors varies by 1 / sqrt(2 N) of itself, the
+    quotient of two by 1 / sqrt(N): four times that is allowed, 25 % at N = 256 (chains twice as long are off by 75 % there)."""
     g = torch.Generator(device="cuda").manual_seed(n + k + m)
     x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
     w = torch.randn(n, k, generator=g, device="cuda").bfloat16()
     want = x.double() @ w.double().t()
     splits = gemm._plan(m, n, (k + 63) // 64, 0)[2]
     few, tiles = ((gemm.linear_bf16(x, w, epilogue=gemm.EPI_STORE_F32, splits=s).double() - want).norm().item() for s in (None, splits))
-    assert few <= 1.1 * tiles, (few, tiles)
+    assert few <= (1 + 4 / (n * m) ** 0.5) * tiles, (few, tiles)
