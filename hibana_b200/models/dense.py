@@ -176,7 +176,7 @@ class DenseModel:
                                     t.kv_heads, t.head_dim, rot=t.rot_dim, kv_scale=kv.kv_scale,
                                     table=basic.rope_table(ctx, self.inv_freq, t.rot_dim))
             att = attention.paged_attention(q, kv.k[i], kv.v[i], ctx.kv_indices, ctx.ctx_len, q_indptr=ctx.q_indptr,
-                                            max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
+                                            max_rows=ctx.max_rows, max_ctx=ctx.max_ctx_host, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace)
             comm.sp_gemm_scatter(layer.o, att.view(rows, -1))
@@ -227,7 +227,7 @@ class DenseModel:
             fuse = (cfgmod.current().fuse_epilogues and layer.o.fmt == "nvfp4" and not layer.o.calibrating
                     and q.shape[0] <= 128 and q.is_cuda and not layer.o.takes_w3(q.shape[0]))
             att = attention.paged_attention(q, kv.k[i], kv.v[i], ctx.kv_indices, ctx.ctx_len, q_indptr=ctx.q_indptr,
-                                            max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
+                                            max_rows=ctx.max_rows, max_ctx=ctx.max_ctx_host, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace,
                                             quant_scale=layer.o.input_scale if fuse else None,
@@ -271,7 +271,7 @@ class DenseModel:
                                     table=basic.rope_table(ctx, self.inv_freq, t.rot_dim))
             o_gemv = layer.o.takes_gemv(rows)
             att = attention.paged_attention(q, kv.k[i], kv.v[i], ctx.kv_indices, ctx.ctx_len, q_indptr=ctx.q_indptr,
-                                            max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
+                                            max_rows=ctx.max_rows, max_ctx=ctx.max_ctx_host, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace,
                                             quant_scale=None if o_gemv else layer.o.input_scale,

@@ -154,7 +154,7 @@ class AttentionLayer:
             att = self._sparse(x, q, ctx, kv)
         else:
             att = attention.paged_attention(q, kv.k[i], kv.v[i], ctx.kv_indices, ctx.ctx_len, q_indptr=ctx.q_indptr,
-                                            max_rows=ctx.max_rows, seq_rows=ctx.seq_rows, scale=self.scale,
+                                            max_rows=ctx.max_rows, max_ctx=ctx.max_ctx_host, seq_rows=ctx.seq_rows, scale=self.scale,
                                             kv_scale=kv.kv_scale, splits=ctx.attn_splits,
                                             workspace=ctx.attn_workspace, tables_ready=ctx.mode == DECODE)
         att = att.view(att.shape[0], -1)

@@ -94,17 +94,22 @@ def prefill_splits(batch: int, hq: int, hkv: int, d: int, max_rows: int, max_ctx
     return -(-tiles // per) if tiles - per >= MIN_TILES_SAVED else 1
 
 
-def two_q_tiles(batch: int, hq: int, hkv: int, max_rows: int) -> bool:
-    """Whether an unsplit bf16 prefill (head dims up to 128) runs two 128-row Q tiles per CTA (csrc/attn_prefill.cu,
-    attn_prefill_q2_kernel). Against one tile per CTA, 40 / 8 heads of 128: more tiles than one wave of CTAs 1.2 to 2 times as fast
-    (2048 tokens 111 -> 61 us). Within one wave a CTA has twice the rows to do and SMs stay idle, which costs 10 to 28 % on long
-    contexts (300 rows over 1024 / 4096 keys 22.7 -> 24.8, 59.6 -> 72.6 us) and gains on short ones (29 tokens 12.8 -> 8.6, 128
-    tokens 12.8 -> 10.6, 512 keys 16.8 -> 17.0): taken up to half a wave, where longer contexts are split (`prefill_splits`).
+# Keys that a row sees on average up to which two Q tiles per CTA pay within half a wave of CTAs (`two_q_tiles`).
+TWO_TILES_KEYS = 192
+
+
+def two_q_tiles(batch: int, hq: int, hkv: int, max_rows: int, max_ctx: int = 0) -> bool:
+    """Whether an unsplit bf16 prefill (head dims up to 128) over contexts of up to `max_ctx` keys runs two 128-row Q tiles per CTA
+    (csrc/attn_prefill.cu, attn_prefill_q2_kernel). Against one tile per CTA, 40 / 8 heads of 128: more tiles than one wave of CTAs 1.4
+    to 1.9 times as fast (460 tokens 24.9 -> 17.5 us, over 16000 keys 382 -> 253, 2048 tokens 111 -> 62). Within one wave a CTA has twice the
+    rows to do while SMs stay idle, which every key tile pays for: prompts of 29 / 128 / 225 tokens 13.1 / 13.1 / 14.0 -> 8.8 / 11.1 /
+    12.3, but four times 50 rows over 256 / 512 / 1024 keys 13.2 / 15.9 / 22.0 -> 13.9 / 17.9 / 26.0 (longer contexts are split,
+    `prefill_splits`). So up to half a wave a row may see 192 keys on average: 150 rows over 256 keys gain 5 %, 100 lose 3 %.
     One form for all row counts under `stable_numerics`."""
     if cfgmod.current().stable_numerics:
         return False
     ctas = batch * hkv * -(-max_rows // max(1, 128 // (hq // hkv)))
-    return ctas > NUM_SMS or 2 * ctas <= NUM_SMS
+    return ctas > NUM_SMS or 2 * ctas <= NUM_SMS and max_ctx - max_rows // 2 <= TWO_TILES_KEYS
 
 
 def forward_splits(k_pool: torch.Tensor, v_pool: torch.Tensor, batch: int, hq: int, hkv: int, d: int, max_rows: int,
@@ -176,7 +181,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                     seq_rows: Optional[torch.Tensor] = None,
                     scale: Optional[float] = None, kv_scale: float = 1.0, causal: bool = True, splits: int = 1,
                     workspace: Optional[AttnWorkspace] = None, out: Optional[torch.Tensor] = None,
-                    quant_scale: Optional[torch.Tensor] = None, tables_ready: bool = False, rope: Optional[tuple] = None):
+                    quant_scale: Optional[torch.Tensor] = None, tables_ready: bool = False, rope: Optional[tuple] = None,
+                    max_ctx: int = 0):
     """q [T, Hq, D] bf16; pools [slots, Hkv, D]; kv_indices [B, max_ctx] int32; ctx_len [B] int32.
 
     Row r of sequence b (rows q_indptr[b]..q_indptr[b+1], or exactly one row when q_indptr is None) sees keys
@@ -189,6 +195,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     with its embedding gather (a decode step): the decode kernel then fetches them while its predecessors still run.
     `rope` = (qkv, positions, slots, inv_freq), where `rope_in_kernel` allows it: q is a view of the projection's rows, and
     rotation and KV write happen inside the kernel instead of in `basic.rope_kv_write`.
+    `max_ctx` (host value) bounds the context lengths; 0: the width of kv_indices does.
     """
     t, hq, d = q.shape
     hkv = k_pool.shape[1]
@@ -254,7 +261,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         return out if quant_scale is None else nvfp4.quantize(out.view(t, hq * d), quant_scale)
     out = torch.empty_like(q) if out is None else out
     res = _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, seq_rows, scale, kv_scale, causal,
-                         splits, workspace, out, cfg, fp8, b, t, hq, hkv, d)
+                         splits, workspace, out, cfg, fp8, b, t, hq, hkv, d, max_ctx or kv_indices.shape[1])
     return res if quant_scale is None else nvfp4.quantize(res.view(t, hq * d), quant_scale)
 
 
@@ -309,17 +316,19 @@ def _quant_bufs(rows: int, k: int, device):
 
 
 def _paged_general(q, k_pool, v_pool, kv_indices, ctx_len, q_indptr, max_rows, seq_rows, scale, kv_scale, causal,
-                   splits, workspace, out, cfg, fp8, b, t, hq, hkv, d):
+                   splits, workspace, out, cfg, fp8, b, t, hq, hkv, d, max_ctx):
     if getattr(k_pool, "sf", None) is not None:
         fp8 = 2       # NVFP4 pool: the split-KV kernel dequantises rows as it loads them
         nv.lib().hb_attn_fp4_scales(k_pool.sf.data_ptr(), v_pool.sf.data_ptr(), k_pool.sf.stride(0), k_pool.sf.stride(1))
     if q_indptr is not None and _prefill_tensor_cores(k_pool, v_pool, d, cfg, q, out):
         st = nv.device_state(q.device)
         parts = (workspace.part_o.data_ptr(), workspace.part_lse.data_ptr()) if splits > 1 else (None, None)
+        if splits <= 1:      # 1: two Q tiles per CTA, 0: one
+            splits = int(two_q_tiles(b, hq, hkv, max_rows, max_ctx))
         nv.check(nv.lib().hb_attn_prefill(
             q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0), k_pool.stride(1), kv_indices.data_ptr(),
-            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts,
-            splits if splits > 1 else int(two_q_tiles(b, hq, hkv, max_rows)), b, max_rows, hq, hkv, d, scale, int(fp8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
+            kv_indices.stride(0), nv.ptr(seq_rows), ctx_len.data_ptr(), q_indptr.data_ptr(), out.data_ptr(), *parts, splits,
+            b, max_rows, hq, hkv, d, scale, int(fp8), kv_scale, int(causal), k_pool.shape[0], st.status.data_ptr(),
             nv.stream()), "hb_attn_prefill")
         if splits > 1:
             nv.check(nv.lib().hb_attn_merge(*parts, out.data_ptr(), t * hq, splits, d, nv.stream()), "hb_attn_merge")

@@ -17,6 +17,37 @@ def test_two_q_tiles_rule_cpu():
         assert not attention.two_q_tiles(1, 40, 8, 2048)
 
 
+def test_two_q_tiles_rule_looks_at_the_context_cpu():
+    """Within half a wave: 192 keys per row on average, whatever the prefix is; beyond one wave any context."""
+    assert attention.two_q_tiles(1, 40, 8, 225, 225) and attention.two_q_tiles(1, 40, 8, 150, 256)
+    assert not attention.two_q_tiles(1, 40, 8, 100, 256) and not attention.two_q_tiles(4, 40, 8, 50, 1024)
+    assert not attention.two_q_tiles(1, 40, 8, 250, 250) and attention.two_q_tiles(1, 40, 8, 451, 16000)
+
+
+def test_context_bound_reaches_the_rule_cpu(monkeypatch):
+    """`max_ctx` of the call, or the width of the block table where the caller gives none."""
+    from hibana_b200 import _native as nv
+    seen = []
+
+    class Lib:
+        def hb_attn_prefill(self, *args):
+            seen.append(args[13])
+            return 0
+
+    monkeypatch.setattr(nv, "use_native", lambda *t: True)
+    monkeypatch.setattr(nv, "lib", Lib)
+    monkeypatch.setattr(nv, "stream", lambda: 0)
+    monkeypatch.setattr(nv, "device_state", lambda dev: type("S", (), {"status": torch.zeros(1)}))
+    monkeypatch.setattr(attention, "_prefill_tensor_cores", lambda *a: True)
+    pool = torch.empty(1100, 8, 128, dtype=torch.bfloat16)
+    ip = torch.tensor([0, 100], dtype=torch.int32)
+    call = lambda width, **kw: attention.paged_attention(  # noqa: E731
+        torch.empty(100, 40, 128, dtype=torch.bfloat16), pool, pool, torch.zeros(1, width, dtype=torch.int32),
+        torch.tensor([100], dtype=torch.int32), q_indptr=ip, max_rows=100, **kw)
+    call(1000), call(200), call(1000, max_ctx=100), call(1000, max_ctx=1000)
+    assert seen == [0, 1, 1, 0]
+
+
 # rows and contexts: one tile, a second tile of one row, both tiles full, a tile more for the second one, prefixes that end on and
 # off a tile, sequences with one tile or none of the block's rows
 CASES = [([26], [26]), ([50], [50]), ([51], [64]), ([51], [65]), ([100, 1, 27], [128, 1, 192]), ([30, 129, 3], [300, 129, 3]),
