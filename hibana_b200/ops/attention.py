@@ -201,6 +201,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     hkv = k_pool.shape[1]
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     if not nv.use_native(q, k_pool):
+        if rope is not None:
+            raise ValueError("rope in the attention kernel: no such kernel on the CPU (see rope_in_kernel)")
         idx = kv_indices if seq_rows is None else kv_indices[seq_rows.long()]
         res = paged_attention_ref(q, k_pool, v_pool, idx, ctx_len, q_indptr, scale, kv_scale, causal)
         if out is not None:
@@ -210,13 +212,14 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     b = ctx_len.shape[0]
     if splits > 1 and (workspace is None or workspace.rows < t or workspace.part_o.shape[1:] != (hq, splits, d)):
         workspace = AttnWorkspace(t, hq, d, splits, q.device)
-    fp4 = getattr(k_pool, "sf", None) is not None
     fp8 = k_pool.dtype != torch.bfloat16
     cfg = cfgmod.current()
-    f8 = fp8 and not fp4 and _fp8_tensor_cores(k_pool, v_pool, d, cfg, q, out)
-    if (not fp8 and d in (64, 128, 256) or f8) and max_rows * (hq // hkv) <= 16:
+    kernel = _decode_kernel(k_pool, v_pool, d, max_rows * (hq // hkv), cfg, q, out)
+    if rope is not None and not (kernel == "mma" and tables_ready and q_indptr is None):
+        raise ValueError("rope in the attention kernel: a decode step that rope_in_kernel() allows, with tables_ready")
+    if kernel is not None:
         st = nv.device_state(q.device)
-        tc = d == 128 and cfg.decode_attn == "tc" and not f8
+        f8, tc = fp8, kernel == "tc"
         fuse = cfg.fuse_epilogues and not tc and (cfg.fuse_attn_tail or splits == 1)
         xq = None
         if fuse:
@@ -270,14 +273,22 @@ def rope_in_kernel(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor
     tensor-core decode kernel on a bf16 or e4m3 pool, all of the head rotated, no q / k norm or gate in the rows, 16-byte
     aligned rows everywhere."""
     cfg = cfgmod.current()
-    if not nv.use_native(qkv, k_pool) or getattr(k_pool, "sf", None) is not None or cfg.decode_attn == "tc":
+    if not nv.use_native(qkv, k_pool) or cfg.decode_attn == "tc" or _decode_kernel(k_pool, v_pool, d, hq // hkv, cfg, qkv) != "mma":
         return False
-    if rot != d or hq // hkv > 16 or qkv.stride(0) % 8 or qkv.stride(1) != 1 or qkv.data_ptr() % 16:
-        return False
-    if k_pool.dtype != torch.bfloat16:
-        return _fp8_tensor_cores(k_pool, v_pool, d, cfg)
-    return (d in (64, 128, 256) and k_pool.stride() == v_pool.stride() and k_pool.stride(2) == 1 and k_pool.stride(0) % 8 == 0
+    return (rot == d and qkv.stride(0) % 8 == 0 and qkv.stride(1) == 1 and qkv.data_ptr() % 16 == 0
+            and k_pool.stride() == v_pool.stride() and k_pool.stride(2) == 1 and k_pool.stride(0) % 8 == 0
             and k_pool.stride(1) % 8 == 0 and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
+
+
+def _decode_kernel(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, rows: int, cfg, q: Optional[torch.Tensor] = None,
+                   out: Optional[torch.Tensor] = None) -> Optional[str]:
+    """Kernel for `rows` query rows per kv head: "mma" (csrc/attn_decode.cu), "tc" (csrc/attn_decode_tc.cu, `decode_attn` setting) or
+    None, the prefill and general kernels."""
+    if rows > 16 or getattr(k_pool, "sf", None) is not None:
+        return None
+    if k_pool.dtype != torch.bfloat16:
+        return "mma" if _fp8_tensor_cores(k_pool, v_pool, d, cfg, q, out) else None
+    return None if d not in (64, 128, 256) else "tc" if d == 128 and cfg.decode_attn == "tc" else "mma"
 
 
 def _fp8_tensor_cores(k_pool: torch.Tensor, v_pool: torch.Tensor, d: int, cfg, q: Optional[torch.Tensor] = None,

@@ -12,6 +12,42 @@ def test_rope_in_kernel_needs_the_native_path_cpu():
     assert not attention.rope_in_kernel(torch.empty(1, 7 * 128, dtype=torch.bfloat16), pool, pool, 4, 2, 128, 128)
 
 
+def test_rope_that_would_not_reach_its_kernel_is_refused_cpu(monkeypatch):
+    """Calls whose dispatch leads elsewhere would attend with unrotated queries and write no K and V (or leave the kernel's rope armed
+    for the next call): a ValueError, before anything is armed or launched."""
+    from hibana_b200 import _native as nv
+    from hibana_b200 import config as cfgmod
+    called = []
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: called.append(name) or 0
+
+    def call(dtype=torch.bfloat16, d=128, q_indptr=None, ready=True):
+        pool = torch.zeros(40, 2, d, dtype=dtype)
+        qkv = torch.zeros(1, 8 * d, dtype=torch.bfloat16)
+        one = torch.ones(1, dtype=torch.int32)
+        return attention.paged_attention(qkv[:, :4 * d].unflatten(1, (4, d)), pool, pool, torch.ones(1, 32, dtype=torch.int32), one,
+                                         q_indptr=q_indptr, tables_ready=ready, rope=(qkv, one, one, torch.ones(d // 2)))
+
+    with pytest.raises(ValueError, match="rope"):
+        call()                                      # the CPU path
+    monkeypatch.setattr(nv, "use_native", lambda *t: True)
+    monkeypatch.setattr(nv, "lib", Lib)
+    monkeypatch.setattr(nv, "stream", lambda: 0)
+    monkeypatch.setattr(nv, "device_state", lambda dev: type("S", (), {"status": torch.zeros(1)}))
+    for kw in (dict(d=96), dict(dtype=torch.float8_e4m3fn, d=64), dict(q_indptr=torch.tensor([0, 1], dtype=torch.int32)), dict(ready=False)):
+        with pytest.raises(ValueError, match="rope"):
+            call(**kw)
+    with cfgmod.using(decode_attn="tc"), pytest.raises(ValueError, match="rope"):
+        call()
+    with cfgmod.using(stable_numerics=True), pytest.raises(ValueError, match="rope"):
+        call(dtype=torch.float8_e4m3fn)
+    assert called == []
+    call()
+    assert called[-3:] == ["hb_attn_decode_early", "hb_attn_decode_rope", "hb_attn_decode"]
+
+
 # contexts that end in the first and the last row of a key tile, in the tile after, in one key, and across splits
 CTX = [1, 2, 16, 17, 31, 32, 33, 64, 65, 500, 513, 1300]
 
