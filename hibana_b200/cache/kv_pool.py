@@ -11,7 +11,8 @@ list, pad pages, `write`).
 """
 from __future__ import annotations
 
-from typing import Iterable
+import functools
+from typing import Iterable, Optional
 
 import torch
 
@@ -21,11 +22,26 @@ NVFP4_KV_SCALE = 1.0 / 64.0
 
 
 class SlotRun(list):
-    """Consecutive slots as `KvPool.alloc` hands them out. The mark is void once the list has another length."""
+    """Consecutive slots from `run_start` on, as `KvPool.alloc` hands them out. Any change of the list takes the mark off (None)."""
+
+    run_start: Optional[int] = None
 
     def __init__(self, slots):
         super().__init__(slots)
-        self.run_start, self.run_length = self[0], len(self)
+        self.run_start = self[0]
+
+
+def _unmarked(change):
+    @functools.wraps(change)
+    def method(self, *args, **kw):
+        self.run_start = None
+        return change(self, *args, **kw)
+    return method
+
+
+for _name in ("__setitem__", "__delitem__", "__iadd__", "__imul__", "append", "extend", "insert", "pop", "remove", "clear", "sort",
+              "reverse"):
+    setattr(SlotRun, _name, _unmarked(getattr(list, _name)))
 
 
 class KvPool:

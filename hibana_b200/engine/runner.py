@@ -335,7 +335,7 @@ class ModelRunner:
             h["ids"][r:r + c] = toks
             h["pos"][r:r + c] = np.arange(start, start + c, dtype=np.int32)
             run = getattr(sl, "run_start", None)           # slots handed out as a run need no look at each of them
-            h["slots"][r:r + c] = sl if run is None or len(sl) != sl.run_length else np.arange(run, run + c, dtype=np.int32)
+            h["slots"][r:r + c] = sl if run is None else np.arange(run, run + c, dtype=np.int32)
             h["tok_rows"][r:r + c] = rows[i]
             h["indptr"][i] = r
             h["ctx"][i] = start + c

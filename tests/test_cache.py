@@ -193,3 +193,23 @@ def test_kv_pool_runs_of_slots_cpu(n):
     pool.free(b)
     pool.check()
     assert pool.free_count == 300
+
+
+def test_slot_run_loses_its_mark_with_any_change():
+    from hibana_b200.cache.kv_pool import KvPool
+    pool = KvPool(1, 300, 1, 8)
+    changes = [lambda r: r.__setitem__(1, 99), lambda r: r.append(7), lambda r: r.extend([7]), lambda r: r.insert(0, 7), lambda r: r.pop(),
+               lambda r: r.remove(r[2]), lambda r: r.reverse(), lambda r: r.sort(), lambda r: r.__delitem__(0), lambda r: r.__iadd__([7]),
+               lambda r: r.__imul__(2), lambda r: r.clear()]
+    for change in changes:
+        run = pool.alloc(20)
+        assert run.run_start == run[0] and run == list(range(run[0], run[0] + 20))
+        change(run)
+        assert run.run_start is None
+    run = pool.alloc(20)
+    run += [5]
+    assert run.run_start is None and run[-1] == 5 and len(run) == 21
+    # what is made from a run carries no mark
+    run = pool.alloc(20)
+    assert all(getattr(x, "run_start", None) is None for x in (run[:5], run + [1], list(run), run.copy(), sorted(run)))
+    assert run.run_start == run[0]
