@@ -308,10 +308,16 @@ class ModelRunner:
         every row (verify), 'none' skips the head. Returns a host list (or None).
         """
         dev = self.device
-        self._enter_forward()
         counts = [len(t) for t in token_lists]
         total = sum(counts)
         b = len(rows)
+        # (one value in the place of many would be spread over them, and a run continued past its end)
+        if not len(counts) == len(starts) == len(slot_lists) == b or [len(s) for s in slot_lists] != counts:
+            raise ValueError("forward_rows: one row, start and token list per sequence, and a slot for every token")
+        for name, given in (("state_slots", state_slots), ("has_initial_state", has_initial_state)):
+            if given is not None and len(given) < b:
+                raise ValueError(f"forward_rows: {name} for {len(given)} of {b} sequences")
+        self._enter_forward()
         max_len = max(s + c for s, c in zip(starts, counts))
         # Everything the forward needs travels in one copy: eight of their own cost 18 us each before the first kernel. The
         # 64-bit fields come first, every field starts on 16 bytes.
@@ -346,9 +352,9 @@ class ModelRunner:
         if want_last:
             h["last"][:] = h["indptr"][1:] - 1
         if state_slots is not None:
-            h["state"][:] = state_slots
+            h["state"][:] = state_slots[:b]
         if has_initial_state is not None:
-            h["init"][:] = has_initial_state
+            h["init"][:] = has_initial_state[:b]
         packed = host.to(dev, non_blocking=True) if pin else host
         self.h2d_bytes += words * 4
         d = {k: packed[o:o + n] for k, (o, n) in place.items()}
@@ -376,7 +382,7 @@ class ModelRunner:
                              q_indptr=d["indptr"], seq_rows=d["rows"], max_rows=max_rows, batch=b, sample_rows=last,
                              attn_splits=splits, attn_workspace=workspace, comm=self.comm, seq_starts_host=list(counts),
                              state_slots=d["state"] if state_slots is not None else d["rows"],
-                             state_slots_host=list(state_slots if state_slots is not None else rows),
+                             state_slots_host=list(state_slots[:b] if state_slots is not None else rows),
                              has_initial_state=d["init"] if has_initial_state is not None else None,
                              checkpoints=checkpoints, max_ctx_host=max_len,
                              extras=extras if extras is not None else {})
