@@ -934,7 +934,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUt
     }
     prof_mark(p, 5, t_entry);
     __syncwarp();
-    if (p.splits > 1) cluster_sync_exit();   // nobody leaves while a peer may still read its partial
+    // Nobody leaves while a peer may still read its partial. With `swap` every warp that has read one has also issued a store of the sum
+    // (a tile has at least one row, and each warp spans all of its rows), so its loads have returned; otherwise a warp whose rows all lie
+    // past the end may have loads in flight that nothing waited for.
+    if (p.splits > 1) {
+      if (p.swap) cluster_sync_exit();
+      else cluster_sync_all();
+    }
     prof_mark(p, 6, t_entry);
   }
   prof_mark(p, 7, t_entry);

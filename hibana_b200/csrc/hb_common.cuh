@@ -177,8 +177,9 @@ __device__ __forceinline__ void cluster_sync_all() {   // every thread of every 
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The same meeting without ordering of memory: for CTAs that only must not leave while a peer still reads their shared memory
-// (whose values the peer has used by then). The release above first waits for the thread's global stores to be acknowledged,
-// which nobody in the cluster reads: 1.3 us at the end of a split-K projection.
+// (whose values the peer has used by then: in every warp an instruction that needs them, such as a store of them, has been issued;
+// a load whose value nothing needs may still be under way). The release above first waits for the thread's global stores to be
+// acknowledged, which nobody in the cluster reads: 1.3 us at the end of a split-K projection.
 __device__ __forceinline__ void cluster_sync_exit() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }

@@ -331,3 +331,19 @@ def test_requant_epilogue_on_sm_pairs_ragged(m, n, k):
     groups = 4 * one.sf.shape[1]
     assert torch.equal(nvfp4.unswizzle_sf(one.sf, m, groups), nvfp4.unswizzle_sf(two.sf, m, groups))
     assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [300, 257, 400])
+def test_split_k_with_the_tokens_on_the_128_row_side(m):
+    """A cluster per tile, the last of which has warps without rows: they read the peers' partials too and must not outlive them."""
+    from hibana_b200 import _native as nv
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, 2048, generator=g, device="cuda").bfloat16()
+    w = torch.randn(320, 2048, generator=g, device="cuda").bfloat16()
+    want = x.double() @ w.double().t()
+    for _ in range(20):
+        y = gemm.linear_bf16(x, w, epilogue=gemm.EPI_STORE_F32, splits=4)
+        # fp32 sums of k exact products: k * 2^-24 of the sum of their magnitudes
+        assert ((y.double() - want).abs() <= 2048 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())).all()
+    assert nv.read_status() == 0
