@@ -981,6 +981,7 @@ std::unordered_map<TmapKey, std::unique_ptr<CUtensorMap>, KeyHash> g_tmaps;
 unsigned long long* g_gemm_prof = nullptr;
 int g_local_reduce = 1;
 int g_pdl = 0;   // launch with programmatic stream serialisation (set through hb_gemm_set_pdl)
+thread_local int g_plain = 0;
 
 template <int KIND, int BN>
 cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorMap* ta, const CUtensorMap* tb,
@@ -1043,7 +1044,7 @@ cudaError_t launch_t(const GemmArgs& a, DevParams& p, dim3 grid, const CUtensorM
       ++na;
     }
   }
-  if (g_pdl) {
+  if (g_pdl && !hb_take_plain()) {
     attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
@@ -1455,5 +1456,15 @@ void hb_clear_tmap_cache(void) { hb::clear_tmap_cache(); }
 
 void hb_gemm_set_pdl(int on) { hb::g_pdl = on < 0 ? 0 : on > 2 ? 2 : on; }
 int hb_gemm_get_pdl(void) { return hb::g_pdl; }
+
+// The NEXT projection of this thread (hb_gemm*, hb_few_rows_bf16, hb_nvfp4_gemv) is launched behind all that was launched before it, not
+// as a dependent: for weights that a kernel of this library may have written just now. A dependent fetches its weights before its
+// wait, and kernels in front of it (embedding gather, norms, GEMMs, quantisers) let it start before they have written anything.
+void hb_gemm_plain(void) { hb::g_plain = 1; }
+int hb_take_plain(void) {
+  const int plain = hb::g_plain;
+  hb::g_plain = 0;
+  return plain;
+}
 
 }  // extern "C"

@@ -571,7 +571,7 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& ta64, const CUtenso
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = hb_gemm_get_pdl() ? 2 : 1;
+  cfg.numAttrs = hb_gemm_get_pdl() && !hb_take_plain() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, GRP>, ta, ta64, ta32, tb, tb_sub, tsfa, tsfb, p);
 }
 

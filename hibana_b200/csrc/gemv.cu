@@ -336,7 +336,7 @@ cudaError_t launch_gemv(const GemvParams& p, int ctas, size_t smem, cudaStream_t
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = hb_gemm_get_pdl() >= 1 ? 1 : 0;
+  cfg.numAttrs = hb_gemm_get_pdl() >= 1 && !hb_take_plain() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, nvfp4_gemv_kernel<KSPLIT, DEQ>, p);
 }
 

@@ -90,6 +90,8 @@ void hb_clear_tmap_cache(void);
 // GEMM launches use programmatic dependent launch (weight prefetch overlaps the preceding kernel) when on.
 void hb_gemm_set_pdl(int on);
 int hb_gemm_get_pdl(void);
+void hb_gemm_plain(void);
+int hb_take_plain(void);
 
 // ---- quantisers (quant.cu) -----------------------------------------------------------------------------
 int hb_quant_nvfp4(const void* x, long long ldx, int m, int k, int ka, const void* gscale, void* q, void* sf,

@@ -302,6 +302,7 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
 // At level 1 only GEMMs are launched as dependents, so an early trigger matters where a GEMM follows. Level 2 is the default:
 // the launch latency (0.4 us in a graph) and prologue of every kernel of a step pass behind its predecessor.
 extern "C" int hb_gemm_get_pdl(void);
+extern "C" int hb_take_plain(void);     // see hb_gemm_plain
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st,
                                       Args&&... args) {
@@ -312,7 +313,7 @@ inline cudaError_t launch_dep_cluster(void (*kern)(KArgs...), dim3 grid, dim3 bl
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   cfg.attrs = at;
-  if (hb_gemm_get_pdl() >= 2) {     // level 1: GEMMs only; level 2: these kernels as well
+  if (hb_gemm_get_pdl() >= 2 && !hb_take_plain()) {     // level 1: GEMMs only; level 2: these kernels as well
     at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }

@@ -117,7 +117,7 @@ class BoltMoeLayer:
             inp = self.fc1_latent(x) if t.latent else x
             lat_ready = br.mark()
             shared = self.shared.forward(x) if self.shared is not None and self.shared_owner else None
-        logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32)
+        logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         ids, w = moe.route(logits, t.top_k, sigmoid=True, sel_bias=self.sel_bias, renorm=True, scale=t.router_scale)
         br.wait(lat_ready, inp if t.latent else None)
         y = self.experts.forward(inp, ids, w, id_base=self.e_lo)

@@ -293,7 +293,7 @@ class DenseModel:
         each rank takes the maximum of its shard and the ranks exchange one (value, id) pair per row
         (`Communicator.pick_exchange`). Reference pattern: hibana/proposers/draft_head.py:229-285."""
         from ..ops import sampling
-        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32)
+        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         if not (self.vocab_shard and comm is not None):
             return sampling.argmax(lg)
         idx, val = sampling.argmax_with_value(lg)
@@ -302,7 +302,7 @@ class DenseModel:
         return sampling.argmax(comm.all_gather_last(lg))
 
     def logits(self, normed: torch.Tensor, comm=None) -> torch.Tensor:
-        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32)
+        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         if self.vocab_shard and comm is not None:
             lg = comm.all_gather_last(lg)
         return lg

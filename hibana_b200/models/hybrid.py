@@ -265,7 +265,7 @@ class HybridModel:
         return basic.rmsnorm(h, self.final_norm, t.norm_eps, residual=res, gemma=t.gemma_norm)
 
     def logits(self, normed: torch.Tensor, comm=None) -> torch.Tensor:
-        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32)
+        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         if self.vocab_shard and comm is not None:
             lg = comm.all_gather_last(lg)
         return lg
@@ -273,7 +273,7 @@ class HybridModel:
     def greedy_tokens(self, normed: torch.Tensor, comm=None) -> torch.Tensor:
         """Greedy token per row; with a vocab-parallel head the ranks exchange one (value, id) pair per row."""
         from ..ops import sampling
-        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32)
+        lg = gemm.linear_bf16(normed, self.lm_head, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         if not (self.vocab_shard and comm is not None):
             return sampling.argmax(lg)
         idx, val = sampling.argmax_with_value(lg)

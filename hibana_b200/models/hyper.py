@@ -64,13 +64,13 @@ class HyperConnection:
         n = self.normed(hyper)
         both = None
         if nv.use_native(hyper) and self.down_inject is not None:
-            both = gemm.linear_bf16(n, self.down_inject, epilogue=gemm.EPI_STORE_F32)      # [T, rank + 16] fp32
+            both = gemm.linear_bf16(n, self.down_inject, epilogue=gemm.EPI_STORE_F32, static_weight=True)      # [T, rank + 16] fp32
             low = torch.empty(t, self.rank, dtype=torch.bfloat16, device=hyper.device)
             nv.check(nv.lib().hb_hc_low(both.data_ptr(), both.stride(0), low.data_ptr(), t, self.rank, nv.stream()),
                      "hb_hc_low")
         else:
-            low = F.silu(gemm.linear_bf16(n, self.down))    # one elementwise launch (fp32 math inside, bf16 out)
-        gate = gemm.linear_bf16(low, self.up)
+            low = F.silu(gemm.linear_bf16(n, self.down, static_weight=True))    # one elementwise launch (fp32 math inside, bf16 out)
+        gate = gemm.linear_bf16(low, self.up, static_weight=True)
         if nv.use_native(hyper):
             mixed = torch.empty(t, self.hidden, dtype=torch.bfloat16, device=hyper.device)
             nv.check(nv.lib().hb_hc_gate_mean(gate.data_ptr(), n.data_ptr(), mixed.data_ptr(), t, self.hc, self.hidden,
@@ -86,7 +86,7 @@ class HyperConnection:
         if both is not None:          # the inject logits came with the gate's first projection (mix)
             logits = both[:, self.rank:]
         else:
-            logits = gemm.linear_bf16(n, self.inject, epilogue=gemm.EPI_STORE_F32)[:, :self.hc]
+            logits = gemm.linear_bf16(n, self.inject, epilogue=gemm.EPI_STORE_F32, static_weight=True)[:, :self.hc]
         if nv.use_native(hyper):
             out = torch.empty_like(hyper)
             nv.check(nv.lib().hb_hc_inject(hyper.data_ptr(), block_output.data_ptr(), logits.data_ptr(),

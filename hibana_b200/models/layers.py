@@ -510,7 +510,7 @@ class MoeLayer:
                 lat = self.fc1_latent(x) if t.latent else None
                 lat_ready = br.mark()
                 shared = self.shared.forward(x) if self.shared is not None else None
-            logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32)
+            logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
             ids, w = self._route(logits)
             if t.latent:
                 br.wait(lat_ready, lat)
@@ -520,7 +520,7 @@ class MoeLayer:
                 return basic.add(out, shared) if shared is not None else out
             br.join(shared)
             return moe.experts_forward(x, ids, w, self._ew(x), shared=shared, id_base=self.e_lo)
-        logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32)
+        logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         ids, w = self._route(logits)
         shared = self.shared.forward(x) if self.shared is not None else None
         if shared is not None and self.shared_split and ctx is not None and ctx.comm is not None:
@@ -544,7 +544,7 @@ def _moe_forward_ep(self, x, comm) -> torch.Tensor:
         inp = self.fc1_latent(x) if t.latent else x
         lat_ready = br.mark()
         shared = self.shared.forward(x) if self.shared is not None else None
-    logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32)
+    logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
     ids, w = self._route(logits)
     br.wait(lat_ready, inp if t.latent else None)
     part = moe.experts_forward(inp, ids, w, self._ew(inp), id_base=self.e_lo)
@@ -580,7 +580,7 @@ def _moe_forward_a2a(self, x, ep) -> torch.Tensor:
         lat = self.fc1_latent(x) if t.latent else None
         lat_ready = br.mark()
         shared = self.shared.forward(x) if self.shared is not None and x.shape[0] else None
-    logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32)
+    logits = gemm.linear_bf16(x, self.router.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
     ids, w = self._route(logits)
     if t.latent:
         br.wait(lat_ready, lat)

@@ -145,16 +145,16 @@ class Linear:
             y = self.w3(x, epilogue=epilogue, residual=residual, out=out)
             return y if requant is None else nvfp4.quantize(y, requant)
         if self.fmt == "bf16":
-            y = gemm.linear_bf16(x, self.weight, epilogue=epilogue, residual=residual, out=out)
+            y = gemm.linear_bf16(x, self.weight, epilogue=epilogue, residual=residual, out=out, static_weight=True)
             return y if requant is None else nvfp4.quantize(y, requant)
         if (not isinstance(x, Nvfp4Tensor) and epilogue in (gemm.EPI_STORE, gemm.EPI_RESIDUAL, gemm.EPI_SILU_MUL)
                 and self.takes_gemv(x.shape[0])):
-            y = gemv.nvfp4_gemv(x, self.wq, epilogue=epilogue, residual=residual, out=out)
+            y = gemv.nvfp4_gemv(x, self.wq, epilogue=epilogue, residual=residual, out=out, static_weight=True)
             return y if requant is None else nvfp4.quantize(y, requant)
         xq = x if isinstance(x, Nvfp4Tensor) else self.quantize_input(x)
         if requant is not None and epilogue == gemm.EPI_SILU_MUL:
-            return gemm.linear_nvfp4_silu_quant(xq, self.wq, self.alpha, requant)
-        y = gemm.linear_nvfp4(xq, self.wq, self.alpha, epilogue=epilogue, residual=residual, out=out)
+            return gemm.linear_nvfp4_silu_quant(xq, self.wq, self.alpha, requant, static_weight=True)
+        y = gemm.linear_nvfp4(xq, self.wq, self.alpha, epilogue=epilogue, residual=residual, out=out, static_weight=True)
         return y if requant is None else nvfp4.quantize(y, requant)
 
 
@@ -169,7 +169,7 @@ def norm_linear(x: torch.Tensor, residual: Optional[torch.Tensor], norm_weight: 
         if res is not None:            # the sum has to land in the residual before any CTA normalises it
             y = lin(basic.rmsnorm(x, norm_weight, eps, residual=res, gemma=gemma), epilogue=epilogue)
         else:                          # the norm runs in the GEMV's prologue
-            y = gemv.nvfp4_gemv(x, lin.wq, norm_weight=norm_weight, eps=eps, gemma=gemma, epilogue=epilogue)
+            y = gemv.nvfp4_gemv(x, lin.wq, norm_weight=norm_weight, eps=eps, gemma=gemma, epilogue=epilogue, static_weight=True)
         return y if requant is None else nvfp4.quantize(y, requant)
     if lin.fmt == "nvfp4":
         if lin.calibrating:

@@ -94,16 +94,16 @@ class VisionEncoder:
         cfg = self.cfg
         b = pixels.shape[0]
         n = cfg.grid * cfg.grid
-        x = gemm.linear_bf16(self.patchify(pixels.to(self.device)), self.patch_w)
+        x = gemm.linear_bf16(self.patchify(pixels.to(self.device)), self.patch_w, static_weight=True)
         x = (x.view(b, n, cfg.width) + self.pos).view(b * n, cfg.width)
         for blk in self.blocks:
             h = F.layer_norm(x.float(), (cfg.width,), *blk["ln1"], cfg.eps).to(torch.bfloat16)
-            att = self._attention(gemm.linear_bf16(h, blk["qkv"]), b, n)
-            x = gemm.linear_bf16(att, blk["proj"], epilogue=gemm.EPI_RESIDUAL, residual=x)
+            att = self._attention(gemm.linear_bf16(h, blk["qkv"], static_weight=True), b, n)
+            x = gemm.linear_bf16(att, blk["proj"], epilogue=gemm.EPI_RESIDUAL, residual=x, static_weight=True)
             h = F.layer_norm(x.float(), (cfg.width,), *blk["ln2"], cfg.eps).to(torch.bfloat16)
-            m = F.gelu(gemm.linear_bf16(h, blk["fc1"]).float()).to(torch.bfloat16)
-            x = gemm.linear_bf16(m, blk["fc2"], epilogue=gemm.EPI_RESIDUAL, residual=x)
+            m = F.gelu(gemm.linear_bf16(h, blk["fc1"], static_weight=True).float()).to(torch.bfloat16)
+            x = gemm.linear_bf16(m, blk["fc2"], epilogue=gemm.EPI_RESIDUAL, residual=x, static_weight=True)
         x = F.layer_norm(x.float(), (cfg.width,), *self.ln_out, cfg.eps).to(torch.bfloat16)
         x = self.pixel_shuffle(x, b)
-        x = F.gelu(gemm.linear_bf16(x, self.proj1).float()).to(torch.bfloat16)
-        return gemm.linear_bf16(x, self.proj2)
+        x = F.gelu(gemm.linear_bf16(x, self.proj1, static_weight=True).float()).to(torch.bfloat16)
+        return gemm.linear_bf16(x, self.proj2, static_weight=True)

@@ -23,6 +23,7 @@ EPI_RELU2 = 6       # grouped (weights on the 128-row side) GEMMs only: out = re
 from ..hardware.b200 import NUM_SMS  # noqa: E402
 
 nv.register("hb_gemm_set_pdl", [nv.I], void=True)
+nv.register("hb_gemm_plain", [], void=True)
 nv.register("hb_gemm_set_local_reduce", [nv.I], void=True)
 nv.register("hb_gemm_silu_quant", [nv.I, nv.P, nv.P, nv.P, nv.P, nv.I, nv.I, nv.I, nv.L, nv.L, nv.P, nv.P, nv.P, nv.P,
                                    nv.I, nv.I, nv.P, nv.I, nv.I, nv.I, nv.P])
@@ -121,8 +122,10 @@ def few_rows_ok(x: torch.Tensor, w: torch.Tensor, epilogue: int, residual: Optio
 
 
 def linear_bf16(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE, residual: Optional[torch.Tensor] = None,
-                out: Optional[torch.Tensor] = None, splits: Optional[int] = None) -> torch.Tensor:
-    """y = x @ w.T for bf16 x [M, K], w [N, K] (fp32 accumulation)."""
+                out: Optional[torch.Tensor] = None, splits: Optional[int] = None, static_weight: bool = False) -> torch.Tensor:
+    """y = x @ w.T for bf16 x [M, K], w [N, K] (fp32 accumulation). `static_weight` (here and in the NVFP4 forms) promises that no
+    kernel of this library that was launched just before writes `w` (a model's weights: laid out long ago): they are then fetched
+    while the kernels in front still run. Without it the projection starts when all of those have ended."""
     m, k = x.shape
     n = w.shape[0]
     if not nv.use_native(x, w):
@@ -133,6 +136,8 @@ def linear_bf16(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE, 
         return res
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
     out = _out(m, n, epilogue, x, out)
+    if not static_weight:
+        nv.lib().hb_gemm_plain()
     if splits is None and few_rows_ok(x, w, epilogue, residual):
         if not _PDL_INIT:
             set_pdl(cfgmod.current().pdl)
@@ -152,7 +157,7 @@ def linear_bf16(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_STORE, 
 
 def linear_nvfp4(x: Nvfp4Tensor, w: Nvfp4Tensor, alpha: torch.Tensor, *, epilogue: int = EPI_STORE,
                  residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                 splits: Optional[int] = None) -> torch.Tensor:
+                 splits: Optional[int] = None, static_weight: bool = False) -> torch.Tensor:
     """y = dequant(x) @ dequant(w).T with block-scaled FP4 MMAs; `alpha` = x.gscale * w.gscale (device scalar)."""
     m, k, n = x.rows, x.k, w.rows
     assert w.k == k
@@ -164,6 +169,8 @@ def linear_nvfp4(x: Nvfp4Tensor, w: Nvfp4Tensor, alpha: torch.Tensor, *, epilogu
             return out
         return res
     out = _out(m, n, epilogue, x.q, out)
+    if not static_weight:
+        nv.lib().hb_gemm_plain()
     swap, bn, auto_splits = _plan(m, n, (k + 255) // 256, nv.WORKSPACE_BYTES)
     splits = auto_splits if splits is None else splits
     if swap:
@@ -186,7 +193,7 @@ def requant_ok(m: int, n: int) -> bool:
 
 
 def linear_nvfp4_silu_quant(x: Nvfp4Tensor, w: Nvfp4Tensor, alpha: torch.Tensor, out_scale: torch.Tensor, *,
-                            splits: Optional[int] = None) -> Nvfp4Tensor:
+                            splits: Optional[int] = None, static_weight: bool = False) -> Nvfp4Tensor:
     """silu(gate) * up of y = x @ w.T (gate / up rows of `w` interleaved pairwise), requantised to NVFP4 with the
     static scale `out_scale` inside the GEMM epilogue: the result feeds the next NVFP4 projection directly.
     Bit-identical to `linear_nvfp4(..., epilogue=EPI_SILU_MUL)` followed by `nvfp4.quantize`.
@@ -194,8 +201,10 @@ def linear_nvfp4_silu_quant(x: Nvfp4Tensor, w: Nvfp4Tensor, alpha: torch.Tensor,
     from . import nvfp4
     m, k, n = x.rows, x.k, w.rows
     if not nv.use_native(x.q, w.q) or not requant_ok(m, n):
-        return nvfp4.quantize(linear_nvfp4(x, w, alpha, epilogue=EPI_SILU_MUL), out_scale)
+        return nvfp4.quantize(linear_nvfp4(x, w, alpha, epilogue=EPI_SILU_MUL, static_weight=static_weight), out_scale)
     ko = n // 2
+    if not static_weight:
+        nv.lib().hb_gemm_plain()
     if m > 128:
         # prefill-sized: fresh buffers (chunk lengths vary and nothing here is captured); scale bytes the kernel
         # does not write (padding rows of the last 128-row block, padding groups of the last K atom) must read zero

@@ -39,7 +39,8 @@ def max_rows(n: int, k: int) -> int:
 
 def nvfp4_gemv(x: torch.Tensor, w: Nvfp4Tensor, *, norm_weight: Optional[torch.Tensor] = None, eps: float = 1e-6,
                gemma: bool = False, epilogue: int = EPI_STORE, residual: Optional[torch.Tensor] = None,
-               out: Optional[torch.Tensor] = None) -> torch.Tensor:
+               out: Optional[torch.Tensor] = None, static_weight: bool = False) -> torch.Tensor:
+    """`static_weight`: see `gemm.linear_bf16`."""
     m, k = x.shape
     n = w.rows
     assert k == w.k and x.dtype == torch.bfloat16 and x.stride(1) == 1
@@ -53,6 +54,8 @@ def nvfp4_gemv(x: torch.Tensor, w: Nvfp4Tensor, *, norm_weight: Optional[torch.T
     if nv.use_native(x, w.q):
         if not 1 <= m <= max_rows(n, k):
             raise ValueError(f"nvfp4_gemv takes 1..{max_rows(n, k)} rows of K = {k}, got {m}")
+        if not static_weight:
+            nv.lib().hb_gemm_plain()
         nv.check(nv.lib().hb_nvfp4_gemv(
             w.q.data_ptr(), w.sf.data_ptr(), w.gscale.data_ptr(), n, k, w.ka, x.data_ptr(), x.stride(0), m,
             nv.ptr(norm_weight), float(eps), int(gemma), nv.ptr(residual),

@@ -53,7 +53,7 @@ def main() -> None:
             out = torch.empty(m, n // 2 if args.epi == "silu" else n, dtype=torch.bfloat16, device=dev)
 
             def run(w_):
-                return gemv.nvfp4_gemv(x, w_, norm_weight=nw, out=out,
+                return gemv.nvfp4_gemv(x, w_, norm_weight=nw, out=out, static_weight=True,
                                        epilogue=gemm.EPI_SILU_MUL if args.epi == "silu" else gemm.EPI_STORE)
             fn = lambda: run(wq)  # noqa: E731
             bytes_moved = n * k * 0.5625 + m * k * 2 + m * n * 2
@@ -67,14 +67,14 @@ def main() -> None:
 
             def run(w_):
                 if args.epi == "silu_quant":
-                    return gemm.linear_nvfp4_silu_quant(xq, w_, alpha, oscale)
-                return gemm.linear_nvfp4(xq, w_, alpha, out=out,
+                    return gemm.linear_nvfp4_silu_quant(xq, w_, alpha, oscale, static_weight=True)
+                return gemm.linear_nvfp4(xq, w_, alpha, out=out, static_weight=True,
                                          epilogue=gemm.EPI_SILU_MUL if args.epi == "silu" else gemm.EPI_STORE)
             fn = lambda: run(wq)  # noqa: E731
             bytes_moved = n * k * 0.5625 + m * k * 0.5625 + m * n * 2
         else:
             out = torch.empty(m, n, dtype=torch.bfloat16, device=dev)
-            fn = lambda: gemm.linear_bf16(x, w, out=out)  # noqa: E731
+            fn = lambda: gemm.linear_bf16(x, w, out=out, static_weight=True)  # noqa: E731
             bytes_moved = (n * k + m * k + m * n) * 2
         if args.once:
             fn()
@@ -88,7 +88,7 @@ def main() -> None:
                 calls = [lambda w_=w_: run(w_) for w_ in ws]
             else:
                 ws = [w.clone() for _ in range(reps)]
-                calls = [lambda w_=w_: gemm.linear_bf16(x, w_, out=out) for w_ in ws]
+                calls = [lambda w_=w_: gemm.linear_bf16(x, w_, out=out, static_weight=True) for w_ in ws]
             for c in calls:
                 c()
             torch.cuda.synchronize()

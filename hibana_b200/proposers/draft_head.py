@@ -99,7 +99,7 @@ class ShortlistHead:
         if self.w3 is not None:
             lg = self.w3(flat.contiguous()).float()
         else:
-            lg = gemm.linear_bf16(flat.contiguous(), self.rows, epilogue=gemm.EPI_STORE_F32)
+            lg = gemm.linear_bf16(flat.contiguous(), self.rows, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         return lg[:, :self.real_rows] if lg.shape[1] != self.real_rows and self.ids is None else lg
 
     def _global(self, local: torch.Tensor) -> torch.Tensor:
@@ -167,7 +167,7 @@ class VocabParallelHead:
     def _logits(self, flat: torch.Tensor) -> torch.Tensor:
         if self.w3 is not None:
             return self.w3(flat.contiguous()).float()[:, :self.local]
-        return gemm.linear_bf16(flat.contiguous(), self.shard, epilogue=gemm.EPI_STORE_F32)
+        return gemm.linear_bf16(flat.contiguous(), self.shard, epilogue=gemm.EPI_STORE_F32, static_weight=True)
 
     def candidates(self, x: torch.Tensor, r: int):
         flat = x.reshape(-1, x.shape[-1])

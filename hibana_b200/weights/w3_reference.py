@@ -208,7 +208,7 @@ class CodebookLinear:
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         from ..ops import gemm
-        y = gemm.linear_bf16(x, self.weight, epilogue=gemm.EPI_STORE_F32)
+        y = gemm.linear_bf16(x, self.weight, epilogue=gemm.EPI_STORE_F32, static_weight=True)
         return (y * self.row_scale).to(torch.bfloat16)
 
     def nbytes(self) -> int:

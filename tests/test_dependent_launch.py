@@ -81,3 +81,73 @@ def test_expert_range_without_rows(fmt, t):
     finally:
         gemm.set_pdl(config.current().pdl)
     assert nv.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["bf16", "nvfp4"])
+@pytest.mark.parametrize("m", [4, 64, 300])
+def test_weights_written_by_the_kernel_in_front(fmt, m):
+    """A projection whose weights this library's kernels have just been launched to write (gathered, projected or quantised) waits for
+    them, also where a norm that releases its successor at once runs in between."""
+    from hibana_b200 import _native as nv
+    from hibana_b200.ops import basic, gemm, nvfp4
+    g = torch.Generator(device="cuda").manual_seed(m)
+    n, k = 8192, 2048
+    table = torch.randn(2 * n, k, generator=g, device="cuda").bfloat16() * 0.05
+    x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    probe = torch.randn(32, n, generator=g, device="cuda").bfloat16()
+    nw, gs = torch.ones(k, device="cuda").bfloat16(), torch.tensor(0.01, device="cuda")
+    alpha = (gs * gs).reshape(1)
+    step = torch.cuda.synchronize
+
+    def run(between):
+        out = []
+        for i in range(4):
+            ids = torch.randperm(2 * n, generator=torch.Generator().manual_seed(i))[:n].cuda()
+            step()
+            w = basic.embedding(ids, table)
+            if fmt == "bf16":
+                between()
+                a = basic.rmsnorm(x, nw, 1e-6)
+                between()
+                y = gemm.linear_bf16(a, w)
+                between()
+                out += [y, gemm.linear_bf16(probe, y)]
+            else:
+                wq = nvfp4.quantize(w, gs)
+                between()
+                xq, _ = nvfp4.rmsnorm_quantize(x, nw, 1e-6, gs)
+                between()
+                out.append(gemm.linear_nvfp4(xq, wq, alpha))
+                between()
+                out.append(gemm.linear_nvfp4_silu_quant(xq, nvfp4.quantize(w, gs), alpha, gs).q.clone())
+            step()
+        return out
+
+    got, want = run(lambda: None), run(step)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert nv.read_status() == 0
+
+
+def test_only_promised_weights_are_fetched_early_cpu(monkeypatch):
+    from hibana_b200 import _native as nv
+    from hibana_b200.models.linear import Linear
+    from hibana_b200.ops import gemm
+    called = []
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: called.append(name) or 0
+
+    lin = Linear(torch.randn(128, 64), "bf16")
+    for name, fake in (("use_native", lambda *t: True), ("lib", Lib), ("stream", lambda: 0),
+                       ("device_state", lambda dev: type("S", (), {"status": torch.zeros(1)}))):
+        monkeypatch.setattr(nv, name, fake)
+    monkeypatch.setattr(gemm, "_PDL_INIT", True)
+    for rows, kernel in ((4, "hb_few_rows_bf16"), (40, "hb_gemm")):
+        x = torch.randn(rows, 64).bfloat16()
+        called.clear()
+        lin(x)
+        assert called == [kernel]
+        gemm.linear_bf16(x, lin.weight)
+        assert called == [kernel, "hb_gemm_plain", kernel]
