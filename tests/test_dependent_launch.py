@@ -6,7 +6,7 @@ from hibana_b200.engine.executor import Executor
 from hibana_b200.engine.request import SamplingParams
 from hibana_b200.models.dense import DenseModel
 from hibana_b200.models.hybrid import HybridModel
-from hibana_b200.target import dense_tiny, tiny_hybrid_moe
+from hibana_b200.target import dense_tiny, get_target, scaled, tiny_hybrid_moe
 
 
 @pytest.mark.gpu
@@ -42,6 +42,52 @@ def test_launch_levels_give_the_same_bits(family, graphs):
             assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(pools, again))
     finally:
         from hibana_b200 import config
+        gemm.set_pdl(config.current().pdl)
+    assert nv.read_status() == 0
+
+
+# RoPE and KV write inside the attention of an e4m3 pool; the delta rule with its gates in clusters on a side stream and the scan that reads
+# its states early; latent experts beside a shared one
+SERVED = {
+    "dense": lambda: dense_tiny(),
+    "delta": lambda: scaled(get_target("qwen38"), layers=4, hidden=2048, ffn=1024, vocab=2048, mtp_layers=0, mtp_depth=0),
+    "latent": lambda: scaled(get_target("nemotron"), layers=9, hidden=1024, vocab=2048, experts=32, top_k=4, expert_ffn=256,
+                             shared_ffn=512, latent=256, mtp_layers=0, mtp_depth=0),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("family", sorted(SERVED))
+@pytest.mark.parametrize("sampled", [False, True])
+def test_launch_levels_with_fp8_caches_and_sampled_rows(family, sampled):
+    """As above: captured decode steps after prompts of odd lengths, fp8 caches, greedy and sampled with a nucleus cut."""
+    from hibana_b200 import _native as nv
+    from hibana_b200 import config
+    from hibana_b200.ops import gemm
+    t = SERVED[family]()
+    model = (DenseModel if t.family == "dense" else HybridModel)(t, "cuda", seed=0)
+    g = torch.Generator().manual_seed(6)
+    prompts = [torch.randint(0, t.vocab, (n,), generator=g).tolist() for n in (1, 17, 130)]
+    params = SamplingParams(max_tokens=16, ignore_eos=True, **(dict(temperature=0.8, top_p=0.9, seed=11) if sampled else {}))
+
+    def run(level):
+        gemm.set_pdl(level)
+        ex = Executor(model, max_batch=4, max_ctx=256, kv_slots=1024, radix_cache=False, kv_dtype=torch.float8_e4m3fn)
+        ex.capture_graphs()
+        out = [r.output_ids for r in ex.generate_batch(prompts, params)]
+        torch.cuda.synchronize()
+        pools = [ex.kv.storage[:, :, :, 1:].clone()]
+        if ex.state_pool is not None:
+            pools += [ex.state_pool.conv[:, 1:].clone(), ex.state_pool.ssm[:, 1:].clone()]
+        return out, pools
+
+    try:
+        want, pools = run(0)
+        for _ in range(3):
+            got, again = run(2)
+            assert got == want
+            assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(pools, again))
+    finally:
         gemm.set_pdl(config.current().pdl)
     assert nv.read_status() == 0
 
