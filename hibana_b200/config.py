@@ -92,7 +92,7 @@ class EngineConfig:
     attn_ctas_per_sm: int = 1              # CTA slots per SM assumed when choosing KV splits (the kernel runs two per
                                            # SM, but modelling both measured slower: more splits, more partials to merge)
     max_splits: int = 8                    # split-K cluster size cap (8 = portable)
-    pdl: int = 2                           # programmatic dependent launch level (0 off, 1 GEMMs, 2 small kernels too)
+    pdl: int = 2                           # programmatic dependent launch level (0 off, 1 GEMMs, 2 most kernels)
     overlap_rows: int = 64                 # up to this many rows a MoE layer's independent chains (shared expert,
                                            # latent projection) run on a side stream beside the routed experts; 0 = off
     expert_budget: int = 0                 # > 0: decode-sized MoE calls read at most this many distinct experts

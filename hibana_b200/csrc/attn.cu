@@ -502,7 +502,8 @@ int hb_attn_paged(const void* q, const void* k_pool, const void* v_pool, long lo
   }
   if (rc != 0) return rc;
   if (p.splits > 1) {
-    launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(static_cast<long long>(total_rows) * hq)), dim3(128), p.splits * sizeof(float), st,
+    launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(static_cast<long long>(total_rows) * hq)), dim3(128),
+               p.splits * sizeof(float), st,
                p.part_o, p.part_lse, p.out, p.splits, d, hq, nullptr, nullptr, nullptr, 0);
     if (cudaGetLastError() != cudaSuccess) return 2;
   }
@@ -512,7 +513,8 @@ int hb_attn_paged(const void* q, const void* k_pool, const void* v_pool, long lo
 int hb_attn_merge(const void* part_o, const void* part_lse, void* out, long long rows_heads, int splits, int d,
                   void* stream) {
   if (rows_heads <= 0) return 0;
-  launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows_heads)), dim3(128), splits * sizeof(float), static_cast<cudaStream_t>(stream),
+  launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows_heads)), dim3(128), splits * sizeof(float),
+             static_cast<cudaStream_t>(stream),
              static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(out), splits,
              d, 1, static_cast<uint8_t*>(nullptr), static_cast<uint8_t*>(nullptr), static_cast<const float*>(nullptr), 0);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
@@ -524,7 +526,8 @@ int hb_attn_merge_quant(const void* part_o, const void* part_lse, long long rows
                         void* q_out, void* q_sf, const void* q_gscale, int q_ka, void* stream) {
   if (rows <= 0) return 0;
   if (d > 256 || d % 16 != 0 || q_out == nullptr || q_sf == nullptr || q_gscale == nullptr) return 1;
-  launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows * hq)), dim3(128), splits * sizeof(float), static_cast<cudaStream_t>(stream),
+  launch_dep(attn_merge_kernel, dim3(static_cast<unsigned>(rows * hq)), dim3(128), splits * sizeof(float),
+             static_cast<cudaStream_t>(stream),
              static_cast<const float*>(part_o), static_cast<const float*>(part_lse), static_cast<__nv_bfloat16*>(nullptr),
              splits, d, hq, static_cast<uint8_t*>(q_out), static_cast<uint8_t*>(q_sf), static_cast<const float*>(q_gscale),
              q_ka);

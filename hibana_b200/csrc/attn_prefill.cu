@@ -1069,9 +1069,10 @@ attn_prefill_pp_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
 // The reference of a row's weights: a weight that is the reference itself is 1 and has no rounding error, and it is the largest weights
 // whose rounding to bf16 shows. So the reference follows the maximum exactly for the first 256 keys (what the two streams of the kernel
 // above see first), afterwards in steps of 2^4. With the maximum of the first 64 keys and steps of 2^8 the error against 64 bits
-// was up to 10 % above that kernel's, now it is the same or less. 40 / 8 heads of 128, queries times 1 / 1.5 / 3, 1e-3: 512 tokens, above 1.977 /
-// 1.913 / 1.826, before 2.013 / 2.015 / 2.024, now 1.974 / 1.913 / 1.796; 2048 tokens 2.047 / 2.017 / 2.029, 2.084 / 2.107 / 2.145, 2.046 /
-// 2.010 / 1.911 (rounding the result alone: 1.66). It costs 2048 tokens 61.8 -> 62.5 us, 512 17.4 -> 18.4, five prompts of 4096 102 -> 104.
+// was up to 11 % above that kernel's, now it is the same or less. 40 / 8 heads of 128, queries times 1 / 1.5 / 3, 1e-3: 512 tokens,
+// above 1.977 / 1.913 / 1.826, before 2.013 / 2.015 / 2.024, now 1.974 / 1.913 / 1.796; 2048 tokens 2.047 / 2.017 / 2.029,
+// 2.084 / 2.107 / 2.145, 2.046 / 2.010 / 1.911 (rounding the result alone: 1.66). It costs 2048 tokens 61.8 -> 62.5 us, 512
+// 17.4 -> 18.4, five prompts of 4096 102 -> 104.
 constexpr int Q2_SETTLE = 4;      // tiles
 constexpr float Q2_GAP = 4.f;     // log2
 constexpr int Q2_KT = 64;

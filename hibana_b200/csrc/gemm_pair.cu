@@ -559,7 +559,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__
 
 template <int EPI, bool GRP>
 cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& ta64, const CUtensorMap& ta32, const CUtensorMap& tb,
-                   const CUtensorMap& tb_sub, const CUtensorMap& tsfa, const CUtensorMap& tsfb, const PairParams& p, int clusters, cudaStream_t stream) {
+                   const CUtensorMap& tb_sub, const CUtensorMap& tsfa, const CUtensorMap& tsfb, const PairParams& p, int clusters,
+                   cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
   cfg.blockDim = dim3(THREADS);
@@ -696,8 +697,8 @@ cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
     k64.box_rows = 64;
     k32.box_rows = 32;
   }
-  if (!get_tmap_2d(ka, &ta) || !get_tmap_2d(k64, &ta64) || !get_tmap_2d(k32, &ta32) || !get_tmap_2d(kb, &tb) || !get_tmap_2d(kb_sub, &tb_sub) || !get_tmap_2d(ksa, &tsfa) ||
-      !get_tmap_2d(ksb, &tsfb))
+  if (!get_tmap_2d(ka, &ta) || !get_tmap_2d(k64, &ta64) || !get_tmap_2d(k32, &ta32) || !get_tmap_2d(kb, &tb) ||
+      !get_tmap_2d(kb_sub, &tb_sub) || !get_tmap_2d(ksa, &tsfa) || !get_tmap_2d(ksb, &tsfb))
     return cudaErrorInvalidValue;
 #define HB_PAIR(EPI, GRP) launch<EPI, GRP>(ta, ta64, ta32, tb, tb_sub, tsfa, tsfb, p, clusters, stream)
   switch (a.epilogue) {

@@ -290,17 +290,24 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
 
 // Launch as a programmatic dependent of the kernel before it in the stream (when the library-wide switch is on,
 // see hb_gemm_set_pdl): the grid may be scheduled while its predecessor drains, which hides launch latency. The rules:
-//   * every kernel calls grid_dep_wait() in every CTA, before it reads anything that ANY kernel of the step wrote, and before it
-//     writes anything (a grid none of whose CTAs waits could end before its predecessor, and its dependent's wait with it).
-//     Kernels may call grid_dep_launch() ahead of their own wait (norms, RoPE + KV write, attention, merges, plain GEMMs do), so
+//   * a CTA calls grid_dep_wait() before it reads anything that ANY kernel of the step wrote, and before it writes anything. CTAs that do
+//     neither (grouped GEMM tiles without rows) may leave without it, but one CTA of every grid waits: a grid none of whose CTAs
+//     does could end before its predecessor, and its dependents' waits with it.
+//     Kernels may call grid_dep_launch() ahead of their own wait (norms, RoPE + KV write, attention, merges, scans, GEMMs do), so
 //     when a dependent starts, kernels further back than its predecessor may still run;
-//   * before the wait only weights, norm weights and static scales may be read;
+//   * before the wait only what was complete long ago may be read: norm weights, static scales, a model's weights (projections fetch
+//     theirs early only where the caller promises that, see hb_gemm_plain), and, where the caller promises it for a decode
+//     step, its tables, older keys and recurrent states (hb_attn_decode_early, hb_state_early: attention, convolution, scans). The
+//     promise holds because the step's embedding gather triggers only after its own wait: nothing behind the gather starts before
+//     everything in front of it has ended. A kernel of the step that writes such data runs ahead of the gather;
 //   * one exception: the one-CTA grouped GEMM (gemm.cu) reads the routing plan before its wait, to leave early. That is safe
 //     because the kernel in front of it (the activation quantiser, the row gather) triggers only after its own wait, which
 //     the plan kernel's end precedes, or is another grouped GEMM behind such a kernel. One that is put in between must do
 //     the same.
 // At level 1 only GEMMs are launched as dependents, so an early trigger matters where a GEMM follows. Level 2 is the default:
-// the launch latency (0.4 us in a graph) and prologue of every kernel of a step pass behind its predecessor.
+// the launch latency (0.4 us in a graph) and prologue of most kernels of a step pass behind their predecessors. Kernels that are
+// launched with <<<>>> (qsa.cu, hyper.cu, ggml.cu, ssm_window.cu, ep.cu, comm.cu, attn_decode_tc.cu, the fp8 quantisers, the speculative
+// ones of sample.cu) start when all in front of them have ended and let their successor start when they end.
 extern "C" int hb_gemm_get_pdl(void);
 extern "C" int hb_take_plain(void);     // see hb_gemm_plain
 template <typename... KArgs, typename... Args>

@@ -450,8 +450,8 @@ __device__ __forceinline__ float sum_lanes(float acc, float w, int lane, float& 
 // law with token `exclude` removed (-1: nothing removed; the residual of a point-mass draft in speculative
 // sampling) and reports the probability of token `probe` under the law. LAW_T threads, whole CTA. Bound by the chain of its passes
 // over the row, so the row is staged where it fits. With a nucleus cut, us at 11 rows, a pass over the row for every 4
-// bits of the cut / now: 18992 tokens 85 / 31, 31040 113 / 43, 52224 167 / 68, 151936 (not staged) 479 / 287; cut off 26 / 17, 36 / 22, 53 / 31,
-// 163 / 116 (0 of 23040 draws differed).
+// bits of the cut / now: 18992 tokens 85 / 31, 31040 113 / 43, 52224 167 / 68, 151936 (not staged) 479 / 287; cut off
+// 26 / 17, 36 / 22, 53 / 31, 163 / 116 (0 of 23040 draws differed).
 template <typename T, bool STAGED>
 __device__ void law_row(const T* lr, int vocab, const int* mask, float temp, int k_lim, float p_lim, float u01, int exclude,
                         int probe, long long* out, float* out_prob, float* out_probe, SearchScratch& sc) {

@@ -558,9 +558,8 @@ int hb_conv1d(const void* x, long long ldx, const void* w, const void* bias, voi
     const bool two = ((channels | ldx | ldy) & 1) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 3) == 0;
     const int per = two ? 256 : 128;
     const dim3 tg((channels + per - 1) / per, (max_rows + CONV_TT - 1) / CONV_TT, batch);
-    launch_dep(two ? conv1d_tiled2_kernel<4> : conv1d_tiled_kernel<4>, tg, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias), BFM(y), ldy, BFM(state),
-               state_stride, IP(q_indptr), IP(slot_in), IP(slot_out),
-               IP(has_init), channels, act_silu);
+    launch_dep(two ? conv1d_tiled2_kernel<4> : conv1d_tiled_kernel<4>, tg, dim3(128), 0, ST(stream), BF(x), ldx, BF(w), BF(bias),
+               BFM(y), ldy, BFM(state), state_stride, IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels, act_silu);
     if (slot_out != nullptr)
       launch_dep(conv1d_state_kernel<4>, dim3((channels + 127) / 128, batch), dim3(128), 0, ST(stream),
                  BF(x), ldx, BFM(state), state_stride, IP(q_indptr), IP(slot_in), IP(slot_out), IP(has_init), channels);

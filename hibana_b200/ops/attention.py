@@ -2,8 +2,9 @@
 
 `paged_attention` is the single entry: query rows of a ragged batch attend to their sequence's context through
 the block table. Kernels: csrc/attn_prefill.cu (tcgen05 prefill, two Q tiles per CTA where `two_q_tiles` says so),
-csrc/attn_decode.cu (tensor-core flash-decoding, up to 16 query rows per kv head, RoPE and KV write of a decode step inside), csrc/attn.cu (general split-KV + LSE merge: NVFP4 KV, and fp8 KV under
-`stable_numerics`, with head dim 64 or off 16-byte boundaries). The plain-PyTorch reference below is the CPU path
+csrc/attn_decode.cu (tensor-core flash-decoding, up to 16 query rows per kv head, RoPE and KV write of a decode step inside),
+csrc/attn.cu (general split-KV + LSE merge: NVFP4 KV, and fp8 KV under `stable_numerics`, with head dim 64 or off 16-byte
+boundaries). The plain-PyTorch reference below is the CPU path
 and the GPU tests' oracle. Reference counterparts: hibana/kernels/ops.py:131-161 (ragged prefill),
 hibana/model/attention.py:69-126, hibana/kernels/csrc/verify_attn.cu.
 """

@@ -37,8 +37,8 @@ _PDL_INIT = False
 
 def set_pdl(on) -> None:
     """Programmatic dependent launch. Level 1 (True): GEMMs launch as dependents, their weight prefetch overlaps the
-    kernel before them. Level 2 (the default): every kernel of a forward does so too, and those that may release their
-    successor at their start. 0 / False: off."""
+    kernel before them. Level 2 (the default): so do the other kernels of a forward (which ones do not: csrc/hb_common.cuh,
+    launch_dep), and those that may release their successor at their start. 0 / False: off."""
     global _PDL_INIT
     _PDL_INIT = True
     if nv.available():

@@ -287,9 +287,8 @@ def tile_hint(pairs: int, experts: int, max_rows: int, fmt: str) -> int:
 def pair_rows(ew: "ExpertWeights", max_rows: int) -> bool:
     """Whether the grouped GEMMs run on SM pairs over 256-row chunks (csrc/gemm_pair.cu): NVFP4 experts as soon as a chunk
     would otherwise be a 128-token tile, in geometries whose activation can be requantised in fc1's epilogue. One-CTA tiles /
-    pairs, whole call: 512 experts, top 22, 1024-2688-1024, 129 tokens 659 / 561 us, 256 693 / 583, 904 995 / 616, 4096
-    2361 / 758; 64 experts, top 8, 2048-768-2048 (SwiGLU), 129 tokens 119 / 86, 904 188 / 126. (Measured before fc1 fetched only a
-    segment's rows and stored its packed output from registers: at 5000 tokens fc1 349 -> 305, fc2 217 -> 205.)"""
+    pairs, whole call: 512 experts, top 22, 1024-2688-1024, 129 tokens 603 / 511 us, 256 639 / 531, 904 867 / 560, 4096
+    1910 / 697; 64 experts, top 8, 2048-768-2048 (SwiGLU), 129 tokens 108 / 79, 256 124 / 89, 904 178 / 120, 4096 551 / 236."""
     return (ew.fmt == "nvfp4" and max_rows > 128 and ew.act in ("swiglu", "relu2") and ew.inter % 64 == 0
             and ew.n1 % 128 == 0 and ew.fc2_rows % 128 == 0)
 
