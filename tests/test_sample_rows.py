@@ -150,3 +150,34 @@ def test_fewer_live_tokens_than_top_k(vocab, top_p):
     got, p = sampling.spec_targets(x.cuda(), drafts.cuda(), *[a.cuda() for a in half], None, mask.cuda())
     want, pw = sampling.spec_targets_ref(x, drafts, *half, None, mask)
     assert torch.equal(got.cpu(), want) and torch.allclose(p.cpu(), pw, atol=1e-5, rtol=1e-5)
+
+
+# more tokens than are listed within one bucket: rows whose logits lie close together, the last bucket, rows in several slabs of 2^18
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [4097, 52224, 262145, 300000])
+@pytest.mark.parametrize("spread", [0.001, 0.05, 40.0])
+@pytest.mark.parametrize("top_k", [0, 2000])
+def test_searches_that_have_to_be_narrowed(vocab, spread, top_k):
+    """The nucleus' mass and its tokens, as at the bucket ends; with a top-k the candidates' search is narrowed first."""
+    temp, tol = 0.8, 6e-5
+    x = torch.randn(vocab, generator=torch.Generator().manual_seed(vocab)) * spread
+    order = torch.sort(x, descending=True, stable=True).indices[:top_k or vocab]
+    w = torch.exp((x[order].double() - float(x[order[0]])) / temp)
+    cum = torch.cumsum(w, 0) / w.sum()
+    ps = torch.tensor([0.01, 0.3, 0.77, 0.999, 1.0])
+    b = len(ps)
+    full = lambda val, dt: torch.full((b,), val, dtype=dt, device="cuda")
+    args = (full(temp, torch.float32), full(top_k, torch.int32), ps.cuda(), torch.arange(b, device="cuda") + 3,
+            torch.arange(b, device="cuda"))
+    rank = torch.full((vocab,), vocab, dtype=torch.long)
+    rank[order] = torch.arange(len(order))
+    before = torch.cat([cum - w / w.sum(), torch.tensor([2.0])])
+    tok = sampling.sample(x.cuda().expand(b, vocab), *args).cpu()
+    assert (before[rank[tok].clamp_max(len(order))] <= ps.double() + tol).all()
+    target, p_draft = (t.cpu() for t in sampling.spec_targets(x.cuda().expand(2 * b, vocab), full(int(order[0]), torch.int64)[:, None], *args))
+    assert (before[rank[target[:, 1]].clamp_max(len(order))] <= ps.double() + tol).all()
+    kept = 1 / (w.sum() * p_draft[:, 0].double())
+    edge = (w / w.sum())[torch.searchsorted(cum, ps.double()).clamp_max(len(order) - 1)]
+    # (sums of ceil(300000 / 256) terms one after the other and a tree: 1185 * 2^-24 of the mass)
+    tol = max(tol, 1200 * 2.0 ** -24)
+    assert (kept >= ps.double() - tol).all() and (kept <= ps.double() + edge + tol).all()
